@@ -5,9 +5,10 @@
 // about one thread per tile so that registers stay low and several CTAs share an SM.
 // Same arithmetic as the small-block kernels:
 //   k_big_step      (c, step)   H_i, U_i = exp(-i 2pi tau H_i) by Taylor + squaring
-//   k_big_dyson     (c)         A_{i+1} = U_i A_i for i < n (A stays in shared memory)
+//   k_big_dyson     (c, segment) A_{i+1} = U_i A_i within a segment (A stays in shared memory)
 //   k_big_floquet   (c)         A_n = V diag(lam) V^H: Cayley transform, parallel Jacobi
-//   k_big_eigframe  (c)         W_i = A_{i+1} V_F for i < n
+//   k_big_seg_frame (c, segment) V_s = E_s V_F
+//   k_big_eigframe  (c, segment) W_i = A_{i+1} V_F
 //   k_big_qr        (c, step) per pair  Q = W_a^H M_ab W_b for block pairs with a big block
 // and, for the mixed form, the same step and Dyson in double-float on the FP32 pipe:
 //   k_big_step_df   (c, step)   U_i in double-float (the Taylor series term by term)
@@ -301,22 +302,24 @@ __global__ void __launch_bounds__(1024) k_big_step(DevSys s, int k) {
   }
 }
 
-// One CTA per crystallite: A_{i+1} = U_i A_i for all steps; A lives in shared memory.
+// One CTA per (crystallite, segment): the segment's products P_i = U_i P_{i-1}, P in shared
+// memory; or (prefix) one per crystallite, the chain over the segments' last products.
 template <int NT>
-__global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_dyson(DevSys s, int k) {
+__global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_dyson(DevSys s, int k, bool prefix) {
   extern __shared__ double2 bsc[];
-  const int c = blockIdx.x;
+  const int c = blockIdx.x % s.C;
   const int b = s.bs[k], bp = s.bpoff[k], bb = b * b;
   double2 *Us = bsc, *As = Us + bb;
   for (int e = threadIdx.x; e < bb; e += blockDim.x) As[e] = cmk(e / b == e % b ? 1.0 : 0.0, 0.0);
   double2 acc[NT][4];
-  for (int i = 0; i < s.n; ++i) {
-    const double2 *Ub = s.U + size_t(i) * s.S2 * s.Cpad;
+  const Chain ch = seg_chain(s, b, blockIdx.x / s.C, prefix);
+  for (int i = 0; i < ch.count; ++i) {
+    const double2 *Ub = ch.from(s, i);
     for (int e = threadIdx.x; e < bb; e += blockDim.x) Us[e] = Ub[at(bp + e, c, s.Cpad)];
     __syncthreads();
     cta_mm_cplx_regs<NT, false, double2>(Us, b, As, b, b, b, b, acc);
     __syncthreads();
-    double2 *Ab = s.A + size_t(i) * s.S2 * s.Cpad;
+    double2 *Ab = ch.to(s, i);
     cta_tiles_store<NT>(b, b, acc, [&](int r, int q, double2 v) {
       As[r * b + q] = v;
       Ab[at(bp + r * b + q, c, s.Cpad)] = v;
@@ -325,31 +328,66 @@ __global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_dyson(DevSys s, in
   }
 }
 
-// One CTA per crystallite: W_i = A_{i+1} V_F (in place over A in FP64; into the
-// single-precision W array in the mixed form).
+// One CTA per (crystallite, segment t): V_t = E_t V_F (k_seg_frame's for the large blocks): FP64
+// over E_t, t >= 1; mixed form in double-float, rounded to float2, t = 0 (V_F itself) included.
+template <bool MIX>
+__global__ void __launch_bounds__(1024) k_big_seg_frame(DevSys s, int k) {
+  extern __shared__ __align__(16) unsigned char bsr[];
+  const int c = blockIdx.x % s.C, t = blockIdx.x / s.C + (MIX ? 0 : 1);
+  const int b = s.bs[k], bp = s.bpoff[k], bb = b * b;
+  if constexpr (MIX) {
+    float2 *Vo = seg_Vf(s, t);
+    float4 *Vs = reinterpret_cast<float4 *>(bsr), *Es = Vs + bb;
+    if (t == 0) {
+      for (int e = threadIdx.x; e < bb; e += blockDim.x)
+        Vo[big_at(s, b, bp, e, c)] = cvt<float2>(s.VF[at(bp + e, c, s.Cpad)]);
+      return;
+    }
+    const float4 *E = reinterpret_cast<const float4 *>(seg_E(s, t - 1));
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+      Vs[e] = df_store(s.VF[at(bp + e, c, s.Cpad)]);
+      Es[e] = E[big_at(s, b, bp, e, c)];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+      const int r = e / b, q = e % b;
+      CdfAcc a = {{0.f, 0.f}, {0.f, 0.f}};
+      for (int l = 0; l < b; ++l) cdf_mac(a, Es[r * b + l], Vs[l * b + q]);
+      const float4 w = cdf_fin(a);
+      Vo[big_at(s, b, bp, e, c)] = make_float2(w.x, w.y);
+    }
+  } else {
+    double2 *Vs = reinterpret_cast<double2 *>(bsr), *Es = Vs + bb, *E = seg_E(s, t - 1);
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+      Vs[e] = s.VF[at(bp + e, c, s.Cpad)];
+      Es[e] = E[at(bp + e, c, s.Cpad)];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+      const int r = e / b, q = e % b;
+      double2 acc = cmk(0, 0);
+      for (int l = 0; l < b; ++l) acc = cfma(Es[r * b + l], Vs[l * b + q], acc);
+      E[at(bp + e, c, s.Cpad)] = acc;
+    }
+  }
+}
+
+// One CTA per (crystallite, kSegLen steps): W_i = A_{i+1} V_F = P_i V_s (FP64, in place over A).
 template <int NT, class C>
 __global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_eigframe(DevSys s, int k) {
   extern __shared__ __align__(16) unsigned char bsr[];
-  const int c = blockIdx.x;
+  const int c = blockIdx.x % s.C, i0 = int(blockIdx.x / s.C) * kSegLen, i1 = min(s.n, i0 + kSegLen);
   const int b = s.bs[k], bp = s.bpoff[k], bb = b * b;
   C *Vs = reinterpret_cast<C *>(bsr), *As = Vs + bb;
-  for (int e = threadIdx.x; e < bb; e += blockDim.x) Vs[e] = cvt<C>(s.VF[at(bp + e, c, s.Cpad)]);
+  for (int e = threadIdx.x; e < bb; e += blockDim.x) Vs[e] = frame_elem<C>(s, segmented(s, b), i0, at(bp + e, c, s.Cpad));
   C acc[NT][4];
-  for (int i = 0; i < s.n; ++i) {
+  for (int i = i0; i < i1; ++i) {
     const double2 *Ab = s.A + size_t(i) * s.S2 * s.Cpad;
     C *Wb = Bufs<C>::W(s) + size_t(i) * s.S2 * s.Cpad;
-    const float4 *Ab4 = reinterpret_cast<const float4 *>(Ab);  // mixed form: double-float A, high parts
-    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
-      if (s.mixed) {
-        const float4 v = Ab4[big_at(s, b, bp, e, c)];
-        As[e] = mkc<C>(v.x, v.y);
-      } else {
-        As[e] = cvt<C>(Ab[at(bp + e, c, s.Cpad)]);
-      }
-    }
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) As[e] = cvt<C>(Ab[at(bp + e, c, s.Cpad)]);
     __syncthreads();
     cta_mm_cplx_regs<NT, false, C>(As, b, Vs, b, b, b, b, acc);
-    cta_tiles_store<NT>(b, b, acc, [&](int r, int q, C v) { Wb[big_at(s, b, bp, r * b + q, c)] = v; });
+    cta_tiles_store<NT>(b, b, acc, [&](int r, int q, C v) { Wb[at(bp + r * b + q, c, s.Cpad)] = v; });
     __syncthreads();
   }
 }
@@ -558,7 +596,7 @@ __device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk, int swee
   const int b = s.bs[k], bp = s.bpoff[k], bo = s.boff[k], bb = b * b;
   double2 *Mm = wk.Mm, *Xk = wk.Xk, *fv = wk.fv, *lam = wk.lam;
   double *red = wk.red;
-  const double2 *U = s.A + size_t(s.n - 1) * s.S2 * s.Cpad;  // U(r,q) = U[at(bp + r*b + q, c)]
+  const double2 *U = period_prop(s, b);  // U(r,q) = U[at(bp + r*b + q, c)]
   const float4 *U4 = reinterpret_cast<const float4 *>(U);      // dfA: double-float A (mixed form)
   auto Ug = [&](int r, int q) {
     return dfA ? df_load(U4[big_at(s, b, bp, r * b + q, c)]) : U[big_at(s, b, bp, r * b + q, c)];
@@ -869,32 +907,21 @@ __global__ void __launch_bounds__(1024) k_big_step_df(DevSys s, int k) {
   }
 }
 
-// Complex double-float 2x2-tiled product into registers (compensated sums per re / im).
-struct CdfAcc {
-  DfAcc re, im;
-};
-__device__ __forceinline__ void cdf_mac(CdfAcc &a, float4 x, float4 y) {  // a += x y
-  df_dot(a.re, x.x, x.z, y.x, y.z);
-  df_dot(a.re, -x.y, -x.w, y.y, y.w);
-  df_dot(a.im, x.x, x.z, y.y, y.w);
-  df_dot(a.im, x.y, x.w, y.x, y.z);
-}
-__device__ __forceinline__ float4 cdf_fin(const CdfAcc &a) {
-  const float2 r = df_fin(a.re), m = df_fin(a.im);
-  return make_float4(r.x, m.x, r.y, m.y);
-}
-
+// The segment's (or prefix) products in double-float, 2 x 2 tiles per thread.
 template <int NT>
-__global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_dyson_df(DevSys s, int k) {
+__global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_dyson_df(DevSys s, int k, bool prefix) {
   extern __shared__ __align__(16) unsigned char bsy[];
-  const int c = blockIdx.x;
+  const int c = blockIdx.x % s.C;
   const int b = s.bs[k], bp = s.bpoff[k], bb = b * b;
   float4 *Us = reinterpret_cast<float4 *>(bsy), *As = Us + bb;
   for (int e = threadIdx.x; e < bb; e += blockDim.x) As[e] = make_float4(e / b == e % b ? 1.f : 0.f, 0.f, 0.f, 0.f);
   const int tm = (b + 1) / 2;
-  for (int i = 0; i < s.n; ++i) {
-    const float4 *Ub = reinterpret_cast<const float4 *>(s.U + size_t(i) * s.S2 * s.Cpad);
-    for (int e = threadIdx.x; e < bb; e += blockDim.x) Us[e] = Ub[at(bp + e, c, s.Cpad)];
+  const Chain ch = seg_chain(s, b, blockIdx.x / s.C, prefix);
+  for (int i = 0; i < ch.count; ++i) {
+    const float4 *Ub = reinterpret_cast<const float4 *>(ch.from(s, i));
+    // U lies [item][c]; the segments' products crystallite-major (big_at)
+    for (int e = threadIdx.x; e < bb; e += blockDim.x)
+      Us[e] = Ub[prefix ? big_at(s, b, bp, e, c) : at(bp + e, c, s.Cpad)];
     __syncthreads();
     float4 out[NT][4];
 #pragma unroll
@@ -911,7 +938,7 @@ __global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_dyson_df(DevSys s,
       out[q][0] = cdf_fin(c00), out[q][1] = cdf_fin(c01), out[q][2] = cdf_fin(c10), out[q][3] = cdf_fin(c11);
     }
     __syncthreads();
-    float4 *Ab = reinterpret_cast<float4 *>(s.A + size_t(i) * s.S2 * s.Cpad);
+    float4 *Ab = reinterpret_cast<float4 *>(ch.to(s, i));
 #pragma unroll
     for (int q = 0; q < NT; ++q) {
       const int t = threadIdx.x + q * blockDim.x;
@@ -1109,7 +1136,7 @@ __device__ void floquet_cta_df(const DevSys &s, int k, int c, FloqWork wk, bool 
   double2 *lam = wk.lam;
   double *red = wk.red;
   float2 *Kf = wk.Kf;
-  const double2 *An = s.A + size_t(s.n - 1) * s.S2 * s.Cpad;
+  const double2 *An = period_prop(s, b);
   const float4 *U4 = reinterpret_cast<const float4 *>(An);
   auto Ug = [&](int r, int q) {
     return a64 ? df_store(An[at(bp + r * b + q, c, s.Cpad)]) : U4[big_at(s, b, bp, r * b + q, c)];
@@ -1296,16 +1323,18 @@ __device__ __forceinline__ void cta_tiles4_store(int m, int n, const float2 (&ac
       if (i0 + a < m && j0 + b < n) f(i0 + a, j0 + b, acc[a][b]);
 }
 
-// One CTA per crystallite: W_i = A_{i+1} V_F for i < n (mixed form: high parts of the
-// double-float A, single-precision V and W), 4 x 4 tiles.
+// One CTA per (crystallite, kSegLen steps): W_i = A_{i+1} V_F = P_i V_s (mixed form: high parts
+// of the double-float A, single-precision V and W), 4 x 4 tiles.
 __global__ void __launch_bounds__(384) k_big_eigframe4(DevSys s, int k) {
   extern __shared__ __align__(16) unsigned char bsr4[];
-  const int c = blockIdx.x;
+  const int c = blockIdx.x % s.C, i0 = int(blockIdx.x / s.C) * kSegLen, i1 = min(s.n, i0 + kSegLen);
   const int b = s.bs[k], bp = s.bpoff[k], bb = b * b;
   float2 *Vs = reinterpret_cast<float2 *>(bsr4), *As = Vs + bb;
-  for (int e = threadIdx.x; e < bb; e += blockDim.x) Vs[e] = cvt<float2>(s.VF[at(bp + e, c, s.Cpad)]);
+  const bool seg = segmented(s, b);
+  for (int e = threadIdx.x; e < bb; e += blockDim.x)
+    Vs[e] = frame_elem<float2>(s, seg, i0, seg ? big_at(s, b, bp, e, c) : at(bp + e, c, s.Cpad));
   float2 acc[4][4];
-  for (int i = 0; i < s.n; ++i) {
+  for (int i = i0; i < i1; ++i) {
     const float4 *Ab4 = reinterpret_cast<const float4 *>(s.A + size_t(i) * s.S2 * s.Cpad);
     float2 *Wb = s.Wf + size_t(i) * s.S2 * s.Cpad;
     for (int e = threadIdx.x; e < bb; e += blockDim.x) {

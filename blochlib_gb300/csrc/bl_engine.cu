@@ -163,6 +163,21 @@ __device__ __forceinline__ float2 dfv_mul(float2 a, float2 b) {
   return make_float2(h, __fsub_rn(e, __fsub_rn(h, p)));
 }
 
+// complex double-float elements as float4 (re.hi, im.hi, re.lo, im.lo): compensated sums
+struct CdfAcc {
+  DfAcc re, im;
+};
+__device__ __forceinline__ void cdf_mac(CdfAcc &a, float4 x, float4 y) {  // a += x y
+  df_dot(a.re, x.x, x.z, y.x, y.z);
+  df_dot(a.re, -x.y, -x.w, y.y, y.w);
+  df_dot(a.im, x.x, x.z, y.y, y.w);
+  df_dot(a.im, x.y, x.w, y.x, y.z);
+}
+__device__ __forceinline__ float4 cdf_fin(const CdfAcc &a) {
+  const float2 r = df_fin(a.re), m = df_fin(a.im);
+  return make_float4(r.x, m.x, r.y, m.y);
+}
+
 // ------------------------------------------------------------------ job description
 struct DevSys {
   int C, Cpad, n, npts, N, nb, S2, nint, nq, nr, ne, J, rosym, step_method;
@@ -221,6 +236,9 @@ struct DevSys {
   // stored crystallite-major inside each (step, block) region (big_at), so that the
   // one-CTA-per-crystallite kernels move contiguous rows; the other blocks keep [item][c]
   int clay;
+  // Segments of the Dyson products: nseg = ceil(n / kSegLen); blocks up to seg_max are segmented
+  // (none when nseg == 1).  See seg_E.
+  int nseg, seg_max;
 };
 
 // Precision-dependent arrays: W (eigenframe; in place over A in FP64), Q, R, G, Z, twiddles.
@@ -495,6 +513,54 @@ __device__ int unitary_eig(const double2 (&U)[B][B], double2 (&lam)[B], double2 
 
 // ------------------------------------------------------------------ kernels
 __device__ __forceinline__ size_t at(int item, int c, int Cpad) { return size_t(item) * Cpad + c; }
+
+// Segmented Dyson products.  The chain A_{i+1} = U_i A_i of n dependent products is cut into
+// segments of kSegLen steps that run side by side, each from the identity: A[i] then holds
+// P_i = U_i .. U_{first step of its segment}.  A short chain over the segments' last products
+// gives E_{s+1} = P_last(s) E_s (E_0 = I, E_nseg = A_n, which the Floquet step decomposes), and
+// the eigenframe takes W_i = A_{i+1} V = P_i V_s with V_s = E_s V formed once per segment: the
+// full A_i are never needed.  What bounded the chain was the serial steps, not FP64 issue: a
+// warp holds 32 crystallites of one (block, column), so 320 crystallites of a 10-block gave
+// 320 one-warp CTAs on 608 sub-partitions, each stepping 157 times (1.28 ms per block, FP64
+// pipe 32 % busy).  The extra products are 1/kSegLen of the Dyson and eigenframe work; 16 keeps
+// that near 6 % of a stage that gets up to nseg times the threads.  The split depends on n
+// alone, so a crystallite's result does not depend on how many others run.  Measured (Dyson,
+// eigenframe; before -> after): 5 like spins, 320 crystallites, n = 157, FP64 1.73 -> 1.07 and
+// 4.76 -> 1.00 ms; 7 spins, 144, n = 120, FP64 23.5 -> 14.6 and 23.3 -> 14.2 ms; 4 spins, 3722,
+// n = 128, FP64 1.83 -> 1.33 and 1.14 -> 1.23 ms (the latter FP64-issue bound before too); one
+// 3-spin crystallite, n = 64, Dyson 0.151 -> 0.061 ms.
+// E_s and V_s live in the U buffer, which is dead once a block's segments are done: E_{s+1} in
+// the slots of step s (the same block's items), V_s as float2 (mixed form) from step nseg + s;
+// the FP64 form writes V_s over E_s.
+constexpr int kSegLen = 16;
+__device__ __forceinline__ bool segmented(const DevSys &s, int b) { return b <= s.seg_max; }
+__device__ __forceinline__ double2 *seg_E(const DevSys &s, int t) { return s.U + size_t(t) * s.S2 * s.Cpad; }
+__device__ __forceinline__ float2 *seg_Vf(const DevSys &s, int t) {
+  return reinterpret_cast<float2 *>(s.U + size_t(s.nseg + t) * s.S2 * s.Cpad);
+}
+// the period propagator A_n of a block of size b
+__device__ __forceinline__ const double2 *period_prop(const DevSys &s, int b) {
+  return segmented(s, b) ? seg_E(s, s.nseg - 1) : s.A + size_t(s.n - 1) * s.S2 * s.Cpad;
+}
+// A chain of products x <- M_t x from the identity: the steps of one segment (M = U, results to
+// A), or the segments' last products (M = A at each segment's last step, results to E).
+struct Chain {
+  const double2 *src;
+  double2 *dst;
+  int first, stride, last, count, dst0;  // M_t = src step min(first + t stride, last); result t to dst step dst0 + t
+  __device__ __forceinline__ const double2 *from(const DevSys &s, int t) const {
+    return src + size_t(min(first + t * stride, last)) * s.S2 * s.Cpad;
+  }
+  __device__ __forceinline__ double2 *to(const DevSys &s, int t) const {
+    return dst + size_t(dst0 + t) * s.S2 * s.Cpad;
+  }
+};
+__device__ __forceinline__ Chain seg_chain(const DevSys &s, int b, int seg, bool prefix) {
+  if (prefix) return Chain{s.A, s.U, kSegLen - 1, kSegLen, s.n - 1, s.nseg, 0};
+  if (!segmented(s, b)) return Chain{s.U, s.A, 0, 1, s.n - 1, s.n, 0};
+  const int i0 = seg * kSegLen;
+  return Chain{s.U, s.A, i0, 1, s.n - 1, min(kSegLen, s.n - i0), i0};
+}
 
 // Rows of M = R_rotor(phi, beta) R_powder for crystallite c, phi the rotor phase (sin sp,
 // cos cp): row 2 always, rows 0 and 1 only when second-order quadrupolar terms need them.
@@ -1077,22 +1143,26 @@ __global__ void __launch_bounds__(kThreads) k_step_taylor(DevSys s, const int *_
     }
 }
 
-// One thread per (crystallite, block, column j): column j of A_{i+1} = U_i A_i.
+// One thread per (crystallite, block, segment, column j): column j of the segment's products
+// P_i = U_i P_{i-1}, or (prefix) of the chain over the segments' last products (seg_chain).
 template <int B>
-__global__ void __launch_bounds__(kThreads) k_dyson(DevSys s, const int *__restrict__ blist, int nblist) {
+__global__ void __launch_bounds__(kThreads) k_dyson(DevSys s, const int *__restrict__ blist, int nblist, int nseg,
+                                                    bool prefix) {
   long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
   int c = int(tid % s.Cpad);
   long rest = tid / s.Cpad;
-  if (rest >= long(nblist) * B) return;
+  if (rest >= long(nblist) * B * nseg) return;
   int j = int(rest % B);
-  int k = blist[rest / B];
+  const int seg = int(rest / B % nseg);
+  int k = blist[rest / B / nseg];
   if (c >= s.C) return;
   const int bp = s.bpoff[k];
+  const Chain ch = seg_chain(s, B, seg, prefix);
   double2 x[B];
 #pragma unroll
   for (int r = 0; r < B; ++r) x[r] = cmk(r == j ? 1.0 : 0.0, 0.0);
-  for (int i = 0; i < s.n; ++i) {
-    const double2 *Ub = s.U + size_t(i) * s.S2 * s.Cpad;
+  for (int i = 0; i < ch.count; ++i) {
+    const double2 *Ub = ch.from(s, i);
     double2 y[B];
 #pragma unroll
     for (int r = 0; r < B; ++r) {
@@ -1101,7 +1171,7 @@ __global__ void __launch_bounds__(kThreads) k_dyson(DevSys s, const int *__restr
       for (int l = 0; l < B; ++l) acc = cfma(Ub[at(bp + r * B + l, c, s.Cpad)], x[l], acc);
       y[r] = acc;
     }
-    double2 *Ab = s.A + size_t(i) * s.S2 * s.Cpad;
+    double2 *Ab = ch.to(s, i);
 #pragma unroll
     for (int r = 0; r < B; ++r) {
       x[r] = y[r];
@@ -1110,11 +1180,12 @@ __global__ void __launch_bounds__(kThreads) k_dyson(DevSys s, const int *__restr
   }
 }
 
-// The mixed form's Dyson product in double-float: one lane per (crystallite, block, column,
-// row), U_i and A_{i+1} as float4 double-float elements; each element of U_i x is four
+// The mixed form's Dyson product in double-float: one lane per (crystallite, block, segment,
+// column, row), U_i and A_{i+1} as float4 double-float elements; each element of U_i x is four
 // compensated dot products (re and im, each of a U-hi/lo x-hi/lo expansion).
 template <int B>
-__global__ void __launch_bounds__(kThreads) k_dyson_df(DevSys s, const int *__restrict__ blist, int nblist) {
+__global__ void __launch_bounds__(kThreads) k_dyson_df(DevSys s, const int *__restrict__ blist, int nblist, int nseg,
+                                                       bool prefix) {
   // G lanes per (crystallite, column j): lane r < B owns row r of the column; a warp holds
   // 32/G consecutive crystallites of one (block, column), so the U rows it loads are whole
   // 16-byte runs of consecutive crystallites.  y_r = sum_l U_rl x_l, l ascending, each x_l
@@ -1128,21 +1199,22 @@ __global__ void __launch_bounds__(kThreads) k_dyson_df(DevSys s, const int *__re
   const long rest = tid / G;
   const int c = int(rest % s.Cpad);
   const long rest2 = rest / s.Cpad;
-  if (rest2 >= long(nblist) * B) return;  // warp-uniform (G Cpad is a multiple of 32)
-  const int j = int(rest2 % B), k = blist[rest2 / B];
+  if (rest2 >= long(nblist) * B * nseg) return;  // warp-uniform (G Cpad is a multiple of 32)
+  const int j = int(rest2 % B), seg = int(rest2 / B % nseg), k = blist[rest2 / B / nseg];
   const int bp = s.bpoff[k];
+  const Chain ch = seg_chain(s, B, seg, prefix);
   const bool own = r < B;
   const int lane0 = int(threadIdx.x & 31) & ~(G - 1);
   float4 u[B], un[B];
   auto load_row = [&](int i, float4(&d)[B]) {
-    const float4 *Ub = reinterpret_cast<const float4 *>(s.U + size_t(i) * s.S2 * s.Cpad);
+    const float4 *Ub = reinterpret_cast<const float4 *>(ch.from(s, i));
 #pragma unroll
     for (int l = 0; l < B; ++l) d[l] = own ? Ub[at(bp + r * B + l, c, s.Cpad)] : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   load_row(0, u);
   float4 x = make_float4(r == j ? 1.f : 0.f, 0.f, 0.f, 0.f);
-  for (int i = 0; i < s.n; ++i) {
-    if (i + 1 < s.n) load_row(i + 1, un);
+  for (int i = 0; i < ch.count; ++i) {
+    if (i + 1 < ch.count) load_row(i + 1, un);
     DfAcc re = {0.f, 0.f}, im = {0.f, 0.f};
 #pragma unroll
     for (int l = 0; l < B; ++l) {
@@ -1160,7 +1232,7 @@ __global__ void __launch_bounds__(kThreads) k_dyson_df(DevSys s, const int *__re
     const float2 a = df_fin(re), b = df_fin(im);
     x = make_float4(a.x, b.x, a.y, b.y);
     if (own && c < s.C) {
-      float4 *Ab = reinterpret_cast<float4 *>(s.A + size_t(i) * s.S2 * s.Cpad);
+      float4 *Ab = reinterpret_cast<float4 *>(ch.to(s, i));
       Ab[at(bp + r * B + j, c, s.Cpad)] = x;
     }
 #pragma unroll
@@ -1178,7 +1250,7 @@ __global__ void __launch_bounds__(kThreads) k_floquet(DevSys s, const int *__res
   int k = blist[rest];
   if (c >= s.C) return;
   const int bp = s.bpoff[k], bo = s.boff[k];
-  const double2 *An = s.A + size_t(s.n - 1) * s.S2 * s.Cpad;
+  const double2 *An = period_prop(s, B);
   const float4 *An4 = reinterpret_cast<const float4 *>(An);  // mixed form: double-float A
   double2 U[B][B], lam[B], V[B][B];
 #pragma unroll
@@ -1248,7 +1320,7 @@ __global__ void __launch_bounds__(kThreads) k_floquet_lanes(DevSys s, const int 
   if (c >= s.C) return;  // the whole group leaves together
   const LaneGroup<B> g{((1u << B) - 1u) << (gi * B), gi * B};
   const int bp = s.bpoff[k], bo = s.boff[k];
-  const double2 *An = s.A + size_t(s.n - 1) * s.S2 * s.Cpad;
+  const double2 *An = period_prop(s, B);
   const float4 *An4 = reinterpret_cast<const float4 *>(An);  // mixed form: double-float A
   double2 U[B], lam[B], V[B];  // V accumulates in FP64 in both forms
   CT K[B];
@@ -1487,8 +1559,73 @@ __global__ void __launch_bounds__(kThreads) k_floquet_lanes(DevSys s, const int 
   s.L[at(bo + r, c, s.Cpad)] = cmk(log(hypot(lr.x, lr.y)), atan2(lr.y, lr.x));
 }
 
-// One thread per (crystallite, block, step): W_i = A_{i+1} V_F (in place over A in FP64;
-// into the single-precision W array in the mixed form).
+// One thread per (crystallite, block, segment s): V_s = E_s V_F, s = 1 .. nseg - 1, in FP64 over
+// E_s; in the mixed form (s = 0 included, where it is V_F) in double-float, rounded to float2.
+template <int B, bool MIX>
+__global__ void __launch_bounds__(kThreads) k_seg_frame(DevSys s, const int *__restrict__ blist, int nblist) {
+  const long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int c = int(tid % s.Cpad), ns = MIX ? s.nseg : s.nseg - 1;
+  const long rest = tid / s.Cpad;
+  if (rest >= long(nblist) * ns) return;
+  const int t = int(rest % ns) + (MIX ? 0 : 1), k = blist[rest / ns];
+  if (c >= s.C) return;
+  const int bp = s.bpoff[k];
+  if constexpr (MIX) {
+    float2 *Vo = seg_Vf(s, t);
+    if (t == 0) {
+#pragma unroll
+      for (int e = 0; e < B * B; ++e) Vo[at(bp + e, c, s.Cpad)] = cvt<float2>(s.VF[at(bp + e, c, s.Cpad)]);
+      return;
+    }
+    const float4 *E = reinterpret_cast<const float4 *>(seg_E(s, t - 1));
+#pragma unroll 1
+    for (int q = 0; q < B; ++q) {  // a column of V at a time
+      float4 v[B];
+#pragma unroll
+      for (int l = 0; l < B; ++l) v[l] = df_store(s.VF[at(bp + l * B + q, c, s.Cpad)]);
+#pragma unroll
+      for (int r = 0; r < B; ++r) {
+        CdfAcc a = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+        for (int l = 0; l < B; ++l) cdf_mac(a, E[at(bp + r * B + l, c, s.Cpad)], v[l]);
+        const float4 w = cdf_fin(a);
+        Vo[at(bp + r * B + q, c, s.Cpad)] = make_float2(w.x, w.y);
+      }
+    }
+  } else {
+    double2 *E = seg_E(s, t - 1);
+    double2 V[B][B];
+#pragma unroll
+    for (int r = 0; r < B; ++r)
+#pragma unroll
+      for (int q = 0; q < B; ++q) V[r][q] = s.VF[at(bp + r * B + q, c, s.Cpad)];
+#pragma unroll
+    for (int r = 0; r < B; ++r) {
+      double2 e[B];
+#pragma unroll
+      for (int l = 0; l < B; ++l) e[l] = E[at(bp + r * B + l, c, s.Cpad)];
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        double2 acc = cmk(0, 0);
+#pragma unroll
+        for (int l = 0; l < B; ++l) acc = cfma(e[l], V[l][q], acc);
+        E[at(bp + r * B + q, c, s.Cpad)] = acc;
+      }
+    }
+  }
+}
+
+// V of step i in the precision of C: V_F, or the V_s of the step's segment.
+template <class C>
+__device__ __forceinline__ C frame_elem(const DevSys &s, bool seg, int i, size_t x) {
+  if constexpr (std::is_same<C, float2>::value)
+    return seg ? seg_Vf(s, i / kSegLen)[x] : cvt<C>(s.VF[x]);
+  else
+    return seg && i >= kSegLen ? seg_E(s, i / kSegLen - 1)[x] : s.VF[x];
+}
+
+// One thread per (crystallite, block, step): W_i = A_{i+1} V_F = P_i V_s (in place over A in
+// FP64; into the single-precision W array in the mixed form).
 template <int B, class C>
 __global__ void __launch_bounds__(kThreads) k_eigframe(DevSys s, const int *__restrict__ blist, int nblist) {
   long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -1503,7 +1640,7 @@ __global__ void __launch_bounds__(kThreads) k_eigframe(DevSys s, const int *__re
 #pragma unroll
   for (int r = 0; r < B; ++r)
 #pragma unroll
-    for (int q = 0; q < B; ++q) V[r][q] = cvt<C>(s.VF[at(bp + r * B + q, c, s.Cpad)]);
+    for (int q = 0; q < B; ++q) V[r][q] = frame_elem<C>(s, segmented(s, B), i, at(bp + r * B + q, c, s.Cpad));
   const double2 *Ab = s.A + size_t(i) * s.S2 * s.Cpad;
   const float4 *Ab4 = reinterpret_cast<const float4 *>(Ab);  // mixed form: double-float A
   C *Wb = Bufs<C>::W(s) + size_t(i) * s.S2 * s.Cpad;
@@ -2848,8 +2985,8 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
       }
       attr((const void *)k_big_eigframe<1, double2>, smem_mat);
       attr((const void *)k_big_eigframe<2, double2>, smem_mat);
-      attr((const void *)k_big_eigframe<1, float2>, smem_mat);
-      attr((const void *)k_big_eigframe<2, float2>, smem_mat);
+      attr((const void *)k_big_seg_frame<false>, smem_mat);
+      attr((const void *)k_big_seg_frame<true>, smem_mat);
       attr((const void *)k_big_eigframe4, smem_mat);
       attr((const void *)k_big_floquet, smem_mat + (J.mixed ? smem_mat / 4 : 0));  // + b^2 float2 (K)
       size_t smem_hf = 0;
@@ -3127,6 +3264,9 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   s.tc_flops = J.tcf.p;
   s.clay = (J.mixed && J.huge_blocks.empty()) ? 1 : 0;
   s.Cpad = J.Cb;
+  // the tensor-core blocks (mixed form) keep one chain per crystallite
+  s.nseg = J.is_static ? 1 : (J.n + kSegLen - 1) / kSegLen;
+  s.seg_max = s.nseg > 1 ? (J.tc ? tc::kMinB - 1 : kMaxBigBlock) : 0;
 }
 
 Job::~Job() {}
@@ -3154,9 +3294,13 @@ static void launch_block_kernels(JobImpl &J, DevSys &s, int stage) {
     case 1:
       if (s.mixed) {
         constexpr int G = B <= 1 ? 1 : B <= 2 ? 2 : B <= 4 ? 4 : 8;
-        k_dyson_df<B><<<grid_for(Cp * nl * B * G), kThreads, 0, st>>>(s, bl, nl);
+        k_dyson_df<B><<<grid_for(Cp * nl * s.nseg * B * G), kThreads, 0, st>>>(s, bl, nl, s.nseg, false);
+        if (s.nseg > 1) k_dyson_df<B><<<grid_for(Cp * nl * B * G), kThreads, 0, st>>>(s, bl, nl, 1, true);
+      } else {
+        k_dyson<B><<<grid_for(Cp * nl * s.nseg * B), kThreads, 0, st>>>(s, bl, nl, s.nseg, false);
+        if (s.nseg > 1) k_dyson<B><<<grid_for(Cp * nl * B), kThreads, 0, st>>>(s, bl, nl, 1, true);
       }
-      else k_dyson<B><<<grid_for(Cp * nl * B), kThreads, 0, st>>>(s, bl, nl);
+      if (s.nseg > 1) ++J.launches;
       break;
     case 2:
       if (B == 1) {
@@ -3168,6 +3312,11 @@ static void launch_block_kernels(JobImpl &J, DevSys &s, int stage) {
       }
       break;
     case 3:
+      if (s.nseg > 1) {
+        if (s.mixed) k_seg_frame<B, true><<<grid_for(Cp * nl * s.nseg), kThreads, 0, st>>>(s, bl, nl);
+        else k_seg_frame<B, false><<<grid_for(Cp * nl * (s.nseg - 1)), kThreads, 0, st>>>(s, bl, nl);
+        ++J.launches;
+      }
       if (s.mixed) k_eigframe<B, float2><<<grid_for(Cp * nl * s.n), kThreads, 0, st>>>(s, bl, nl);
       else k_eigframe<B, double2><<<grid_for(Cp * nl * s.n), kThreads, 0, st>>>(s, bl, nl);
       break;
@@ -3395,23 +3544,34 @@ static void launch_stage(JobImpl &J, DevSys &s, int stage) {
             k_tc_dyson_stk<<<unsigned(s.C), tc::kTcThreads, tc_dyson_stk_smem(b), st>>>(s, k, J.usl.p + J.usl_off[k]);
           else
             k_tc_dyson<<<unsigned(s.C), tc::kTcThreads, tc_dyson_smem(b), st>>>(s, k, J.usl.p + J.usl_off[k]);
-        } else if (s.mixed) {
-          if (nt1) k_big_dyson_df<1><<<unsigned(s.C), th, smat, st>>>(s, k);
-          else k_big_dyson_df<2><<<unsigned(s.C), th, smat, st>>>(s, k);
         } else {
-          if (nt1) k_big_dyson<1><<<unsigned(s.C), th, smat, st>>>(s, k);
-          else k_big_dyson<2><<<unsigned(s.C), th, smat, st>>>(s, k);
+          for (int prefix = 0; prefix < (s.nseg > 1 ? 2 : 1); ++prefix) {
+            const unsigned grid = unsigned(s.C) * unsigned(prefix ? 1 : s.nseg);
+            if (s.mixed) {
+              if (nt1) k_big_dyson_df<1><<<grid, th, smat, st>>>(s, k, prefix != 0);
+              else k_big_dyson_df<2><<<grid, th, smat, st>>>(s, k, prefix != 0);
+            } else {
+              if (nt1) k_big_dyson<1><<<grid, th, smat, st>>>(s, k, prefix != 0);
+              else k_big_dyson<2><<<grid, th, smat, st>>>(s, k, prefix != 0);
+            }
+            J.launches += prefix;
+          }
         }
         break;
       case 2:  // the mixed form's single-precision K follows the two b x b double2 arrays
         k_big_floquet<<<unsigned(s.C), kBigThreads, smat + (s.floq32 ? sizeof(float2) * size_t(b) * b : 0), st>>>(s, k);
         break;
       case 3:
+        if (b <= s.seg_max) {
+          if (s.mixed) k_big_seg_frame<true><<<unsigned(s.C) * unsigned(s.nseg), th, smat, st>>>(s, k);
+          else k_big_seg_frame<false><<<unsigned(s.C) * unsigned(s.nseg - 1), th, smat, st>>>(s, k);
+          ++J.launches;
+        }
         if (s.mixed) {
-          k_big_eigframe4<<<unsigned(s.C), unsigned(big4_threads(b, b)), sw, st>>>(s, k);
+          k_big_eigframe4<<<unsigned(s.C) * unsigned(s.nseg), unsigned(big4_threads(b, b)), sw, st>>>(s, k);
         } else {
-          if (nt1) k_big_eigframe<1, double2><<<unsigned(s.C), th, sw, st>>>(s, k);
-          else k_big_eigframe<2, double2><<<unsigned(s.C), th, sw, st>>>(s, k);
+          if (nt1) k_big_eigframe<1, double2><<<unsigned(s.C) * unsigned(s.nseg), th, sw, st>>>(s, k);
+          else k_big_eigframe<2, double2><<<unsigned(s.C) * unsigned(s.nseg), th, sw, st>>>(s, k);
         }
         break;
     }
