@@ -23,7 +23,7 @@
 //   k_qr         (c, step, pair)    Q_i = W^H D W (and R_i = W^H rho W when needed)
 //   k_fave       (c, element, p)    G_p = sum_i q_{(i+p)%n} r_i (with the period twist)
 //   k_p2p_elems  (c, element)       point-to-point FID terms from Q/R and the Floquet phases
-//   k_fid        (c, j, p)          fid[jn+p] = sum_e z_e^j G_p(e); weighted warp sum
+//   k_fid_pair   (c, j pairs, p)    fid[jn+p] = sum_e z_e^j G_p(e); weighted warp sum
 //   k_reduce     (k)                compensated sum of warp partials (fixed order)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -562,6 +562,11 @@ __device__ __forceinline__ Chain seg_chain(const DevSys &s, int b, int seg, bool
   return Chain{s.U, s.A, i0, 1, s.n - 1, min(kSegLen, s.n - i0), i0};
 }
 
+// Powers of z = e^{i theta} that k_fid_pair takes (FP64 form): Z row m < pair_rows(J) holds
+// z^(m + h), h = 1/2 for an even J and 0 for an odd one; the last row is z^((J-1)/2).
+__host__ __device__ __forceinline__ int pair_rows(int J) { return (J + 1) / 2; }
+__device__ __forceinline__ double pair_power(int J, int m) { return double(m) + (J % 2 == 0 ? 0.5 : 0.0); }
+
 // Rows of M = R_rotor(phi, beta) R_powder for crystallite c, phi the rotor phase (sin sp,
 // cos cp): row 2 always, rows 0 and 1 only when second-order quadrupolar terms need them.
 __device__ __forceinline__ void orient_rows(const DevSys &s, int c, double sp, double cp, double (&m)[3][3]) {
@@ -725,76 +730,64 @@ __global__ void __launch_bounds__(kThreads) k_static_eig(DevSys s, const int *__
   }
 }
 
-// Static powder FID, step 2 (oneFID.h:312-334): one thread per (crystallite, block pair
-// (a,b) of D with rho_ba != 0).  Do = V_a^T D_ab V_b, sig0 = V_b^T rho_ba V_a,
-// A_ij = Do(i,j) sig0(j,i) (dropped when |A|^2 <= 1e-10, as the reference does),
-// B_ij = conj(e_i) e_j with e = exp(-2 pi i dt lambda).  fid[k] = sum A B^k is written for
-// the reconstruction kernel as G_p = A B^p (p < ns) and Z_j = (B^ns)^j.
+// Static powder FID, step 2 (oneFID.h:312-334): one thread per (crystallite, element (i, j) of
+// D's block pairs (a,b) with rho_ba != 0, chunk of kStaticRun values of p).  Do = V_a^T D_ab V_b,
+// sig0 = V_b^T rho_ba V_a, A_ij = Do(i,j) sig0(j,i) (dropped when |A|^2 <= 1e-10, as the
+// reference does), B_ij = e^{i th}, th = 2 pi dt (lambda_i - lambda_j).  fid[k] = sum A B^k is
+// written for the reconstruction kernel as G_p = A B^p (p < n, by products within a chunk) and,
+// by one further thread per element, the powers of B^n that k_fid_pair takes.  A thread per
+// element and chunk instead of one per block pair: 113 -> 26 us for three spins, 1154
+// crystallites (65 of 152 SMs had a CTA).
+constexpr int kStaticRun = 32;
 __global__ void __launch_bounds__(kThreads) k_static_elems(DevSys s) {
-  long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  int c = int(tid % s.Cpad);
-  long rest = tid / s.Cpad;
-  if (rest >= s.npq) return;
-  const int pq = int(rest);
-  if (c >= s.C || s.srp[pq] < 0) return;
-  const int a = s.qa[pq], b = s.qb[pq], rp = s.srp[pq], e0 = s.seo[pq];
+  const long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int c = int(tid % s.Cpad), nch = (s.n + kStaticRun - 1) / kStaticRun;
+  const long rest = tid / s.Cpad;
+  if (rest >= long(s.ne) * (nch + 1) || c >= s.C) return;
+  const int e = int(rest % s.ne), ch = int(rest / s.ne);
+  const double th = s.dt * kPi2 * (s.L[at(s.erg[e], c, s.Cpad)].x - s.L[at(s.esg[e], c, s.Cpad)].x);
+  if (ch == nch) {  // the powers of B^n: by products, each restarted from sincos every 16
+    double2 z1, zm = cmk(1, 0);
+    sincos(double(s.n) * th, &z1.y, &z1.x);
+    for (int m = 0; m < pair_rows(s.J); ++m) {
+      if (m % 16 == 0) sincos(pair_power(s.J, m) * double(s.n) * th, &zm.y, &zm.x);
+      s.Z[at(m * s.ne + e, c, s.Cpad)] = zm;
+      zm = cmul(zm, z1);
+    }
+    return;
+  }
+  int pq = 0;  // the element's block pair: the last one that starts at or before e
+  for (int t = 0; t < s.npq; ++t)
+    if (s.seo[t] >= 0 && s.seo[t] <= e) pq = t;
+  const int a = s.qa[pq], b = s.qb[pq];
   const int ba = s.bs[a], bb = s.bs[b], pa = s.bpoff[a], pb = s.bpoff[b];
-  const double2 *D = s.Dblk + s.doff[pq], *Rh = s.Rhoblk + s.rhooff[rp];  // D_ab (ba x bb), rho_ba (bb x ba)
-  double2 X[kMaxBlock * kMaxBlock], Do[kMaxBlock * kMaxBlock];
-  // Do = V_a^T (D_ab V_b)
-  for (int l = 0; l < ba; ++l)
-    for (int q = 0; q < bb; ++q) {
-      double2 acc = cmk(0, 0);
-      for (int m = 0; m < bb; ++m) {
-        double2 d = D[l * bb + m];
-        if (d.x == 0.0 && d.y == 0.0) continue;
-        acc = cfma(d, cmk(s.VF[at(pb + m * bb + q, c, s.Cpad)].x, 0.0), acc);
-      }
-      X[l * bb + q] = acc;
+  const int i = (e - s.seo[pq]) / bb, j = (e - s.seo[pq]) % bb;
+  const double2 *D = s.Dblk + s.doff[pq], *Rh = s.Rhoblk + s.rhooff[s.srp[pq]];  // D_ab (ba x bb), rho_ba (bb x ba)
+  double2 dij = cmk(0, 0), sji = cmk(0, 0);
+  for (int l = 0; l < ba; ++l) {
+    const double va = s.VF[at(pa + l * ba + i, c, s.Cpad)].x;
+    double2 x = cmk(0, 0), y = cmk(0, 0);
+    for (int m = 0; m < bb; ++m) {
+      const double2 d = D[l * bb + m], r = Rh[m * ba + l];
+      if (d.x == 0.0 && d.y == 0.0 && r.x == 0.0 && r.y == 0.0) continue;
+      const double vb = s.VF[at(pb + m * bb + j, c, s.Cpad)].x;
+      x.x = fma(d.x, vb, x.x), x.y = fma(d.y, vb, x.y);
+      y.x = fma(r.x, vb, y.x), y.y = fma(r.y, vb, y.y);
     }
-  for (int r = 0; r < ba; ++r)
-    for (int q = 0; q < bb; ++q) {
-      double2 acc = cmk(0, 0);
-      for (int l = 0; l < ba; ++l) acc = cfma(cmk(s.VF[at(pa + l * ba + r, c, s.Cpad)].x, 0.0), X[l * bb + q], acc);
-      Do[r * bb + q] = acc;
-    }
-  // sig0_ba = V_b^T (rho_ba V_a)   (bb x ba)
-  for (int m = 0; m < bb; ++m)
-    for (int r = 0; r < ba; ++r) {
-      double2 acc = cmk(0, 0);
-      for (int l = 0; l < ba; ++l) {
-        double2 d = Rh[m * ba + l];
-        if (d.x == 0.0 && d.y == 0.0) continue;
-        acc = cfma(d, cmk(s.VF[at(pa + l * ba + r, c, s.Cpad)].x, 0.0), acc);
-      }
-      X[m * ba + r] = acc;
-    }
-  const double z = s.dt * kPi2;
-  for (int i = 0; i < ba; ++i)
-    for (int j = 0; j < bb; ++j) {
-      double2 sg = cmk(0, 0);
-      for (int m = 0; m < bb; ++m) sg = cfma(cmk(s.VF[at(pb + m * bb + j, c, s.Cpad)].x, 0.0), X[m * ba + i], sg);
-      double2 A = cmul(Do[i * bb + j], sg);
-      if (A.x * A.x + A.y * A.y <= 1.0e-10) A = cmk(0, 0);
-      double si, ci, sj, cj;
-      sincos(z * s.L[at(s.boff[a] + i, c, s.Cpad)].x, &si, &ci);
-      sincos(z * s.L[at(s.boff[b] + j, c, s.Cpad)].x, &sj, &cj);
-      const double2 B = cmul(cmk(ci, si), cmk(cj, -sj));  // conj(e_i) e_j
-      const int e = e0 + i * bb + j;
-      double2 g = A;
-      for (int p = 0; p < s.n; ++p) {
-        s.G[at(p * s.ne + e, c, s.Cpad)] = g;
-        g = cmul(g, B);
-      }
-      // g = A B^ns now; Z_j = (B^ns)^j
-      double2 bn = cmk(1, 0);
-      for (int p = 0; p < s.n; ++p) bn = cmul(bn, B);
-      double2 zj = cmk(1, 0);
-      for (int j2 = 0; j2 < s.J; ++j2) {
-        s.Z[at(j2 * s.ne + e, c, s.Cpad)] = zj;
-        zj = cmul(zj, bn);
-      }
-    }
+    dij.x = fma(va, x.x, dij.x), dij.y = fma(va, x.y, dij.y);
+    sji.x = fma(va, y.x, sji.x), sji.y = fma(va, y.y, sji.y);
+  }
+  double2 A = cmul(dij, sji);
+  if (A.x * A.x + A.y * A.y <= 1.0e-10) A = cmk(0, 0);
+  double2 B, g = cmk(1, 0);
+  sincos(th, &B.y, &B.x);
+  const int p0 = ch * kStaticRun, p1 = min(s.n, p0 + kStaticRun);
+  if (p0) sincos(double(p0) * th, &g.y, &g.x);
+  g = cmul(A, g);
+  for (int p = p0; p < p1; ++p) {
+    s.G[at(p * s.ne + e, c, s.Cpad)] = g;
+    g = cmul(g, B);
+  }
 }
 
 // One thread per (crystallite, block k, step i): U_i = V diag(chop(e^{-i 2pi tau L})) V^T
@@ -1737,9 +1730,9 @@ __global__ void __launch_bounds__(kThreads) k_fave(DevSys s) {
   // z = exp(i n tau w)
   double2 z = cexp(cmk(-nt * w.y, nt * w.x));
   if (tile == 0) {
-    for (int j = 0; j < s.J; ++j) {
-      double2 zj = cexp(cmk(-double(j) * nt * w.y, double(j) * nt * w.x));
-      s.Z[at(j * s.ne + e, c, s.Cpad)] = zj;
+    for (int m = 0; m < pair_rows(s.J); ++m) {
+      const double pw = pair_power(s.J, m);
+      s.Z[at(m * s.ne + e, c, s.Cpad)] = cexp(cmk(-pw * nt * w.y, pw * nt * w.x));
     }
   }
   // Three phases over i for the tile p0..p0+PT-1: all j = i+p < n (no wrap), the mixed
@@ -1947,8 +1940,8 @@ __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
   const C *Qb = Bufs<C>::Q(s), *Rb = Bufs<C>::R(s);
   const double nt = double(n) * s.tau;
   // per crystallite of the group: w_rs = chop((l_r - l_s)/(i n tau), 1e-10), z = e^{i n tau w},
-  // and the powers z^j of the FID reconstruction.  FP64 form: four powers per thread, one
-  // cexp and three products (error a few ulp).  Single-precision form (the powers are stored
+  // and the powers of the FID reconstruction (FP64 form: pair_power's; mixed form: z^j).  FP64
+  // form: four powers per thread, one cexp and three products (error a few ulp).  Single-precision form (the powers are stored
   // as float): the exponent of z^j in FP64, then z_pow_f per power (after the first pass).
   constexpr bool kF = std::is_same<C, float2>::value;
   __shared__ float4 zexp[CG];
@@ -1967,18 +1960,19 @@ __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
     }
   } else {
     constexpr int kZrun = 4;
-    const int nzr = (s.J + 1 + kZrun - 1) / kZrun;
+    const int mr = pair_rows(s.J), nzr = (mr + kZrun - 1) / kZrun;
     for (int idx = threadIdx.x; idx < CG * nzr; idx += blockDim.x) {
-      const int cc = idx % CG, j0 = (idx / CG) * kZrun, c = c0 + cc;
+      const int cc = idx % CG, m0 = (idx / CG) * kZrun, c = c0 + cc;
       if (c >= s.C) continue;
       double2 d = csub(s.L[at(s.erg[e], c, s.Cpad)], s.L[at(s.esg[e], c, s.Cpad)]);
       double2 w = cmk(chop1(d.y / nt, 1e-10), chop1(-d.x / nt, 1e-10));
       const double2 z1 = cexp(cmk(-nt * w.y, nt * w.x));
-      double2 zj = cexp(cmk(-double(j0) * nt * w.y, double(j0) * nt * w.x));
-      for (int j = j0; j < min(j0 + kZrun, s.J + 1); ++j) {
-        if (j == s.J) zc[cc] = cvt<C>(z1);
-        else Bufs<C>::Z(s)[at(j * s.ne + e, c, s.Cpad)] = cvt<C>(zj);
-        zj = cmul(zj, z1);
+      const double pw = pair_power(s.J, m0);
+      double2 zm = cexp(cmk(-pw * nt * w.y, pw * nt * w.x));
+      if (m0 == 0) zc[cc] = cvt<C>(z1);
+      for (int m = m0; m < min(m0 + kZrun, mr); ++m) {
+        Bufs<C>::Z(s)[at(m * s.ne + e, c, s.Cpad)] = cvt<C>(zm);
+        zm = cmul(zm, z1);
       }
     }
   }
@@ -2156,75 +2150,82 @@ static size_t fave_twist_bytes(const DevSys &s, int cg) {
 #include "bl_huge.cuh"
 #include "bl_tc.cuh"
 
-constexpr int kFidJT = 4, kFidPT = 4;
-
-// One thread per (crystallite, tile of kFidJT j's, tile of kFidPT p's); lanes are
-// 32 consecutive crystallites, reduced with the powder weights by warp shuffles.
-template <class C, int JT = kFidJT, int PT = kFidPT>
-__global__ void __launch_bounds__(kThreads) k_fid(DevSys s) {
-  long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  int c = int(tid % s.Cpad);
-  long rest = tid / s.Cpad;
-  int npt = (s.gper + PT - 1) / PT, njt = (s.J + JT - 1) / JT;
-  if (rest >= long(npt) * njt) return;  // warp-uniform: whole warp leaves together
-  int pt = int(rest % npt), jt = int(rest / npt);
-  int p0 = pt * PT, j0 = jt * JT;
-  C acc[JT][PT];
+// FID terms of the FP64 form: fid[j gper + p] = sum_c w_c sum_e z_e^j G_p(e).  The FP64 pipe
+// bounds it, so the j's are taken in pairs about the middle of their range: with G' = w z^((J-1)/2) G
+// and z^m = cos + i sin (|z| = 1), the four real sums of cos G'x, sin G'y, cos G'y and sin G'x give
+// both z^m G' and z^-m G' (sum and difference, formed once at the end): four FMAs for two
+// complex terms instead of eight, plus one product by the middle power per (element, p, row
+// tile).  A warp takes 32 consecutive crystallites and a JT x PT tile of (m, p); W warps share
+// a tile's elements (W from the element count alone) and add up in shared memory.  The warp's
+// 4 JT PT sums over its lanes go by halving exchanges (each lane ends with two of them: 62 adds
+// instead of 5 per sum).  A crystallite's terms are summed in the same order alone and in a
+// batch.  Measured, before (4 x 4 tiles of plain complex products, all lanes reducing every
+// sum) -> after: 4 spins, 3722 crystallites, 2048 points 3.07 -> 1.80 ms; 7 spins, 144
+// crystallites (113 CTAs) 11.3 -> 3.55 ms; a pair, 1154 crystallites, 0.070 -> 0.033 ms.
+template <int JT, int PT>
+__global__ void __launch_bounds__(256) k_fid_pair(DevSys s, int W) {
+  constexpr int V = (4 * JT * PT + 31) / 32 * 32;
+  extern __shared__ double fps[];  // [warp][V]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, er = warp % W;
+  const int mr = pair_rows(s.J), nmt = (mr + JT - 1) / JT, npt = (s.gper + PT - 1) / PT;
+  const long tile = long(blockIdx.x) * (blockDim.x / 32 / W) + warp / W;
+  const bool valid = tile < long(s.Cpad / 32) * npt * nmt;
+  const int m0 = int(tile % nmt) * JT, p0 = int(tile / nmt % npt) * PT, g = int(tile / nmt / npt);
+  const int c = g * 32 + lane;
+  double acc[V];
 #pragma unroll
-  for (int a = 0; a < JT; ++a)
+  for (int x = 0; x < V; ++x) acc[x] = 0.0;
+  if (valid && c < s.C) {
+    const double wc = s.w[c] * s.scale;
+    const int e1 = int(long(s.ne) * (er + 1) / W);
+    for (int e = int(long(s.ne) * er / W); e < e1; ++e) {
+      double2 zm[JT], gp[PT];
+      const double2 zc = cscale(s.Z[at((mr - 1) * s.ne + e, c, s.Cpad)], wc);
 #pragma unroll
-    for (int b = 0; b < PT; ++b) acc[a][b] = mkc<C>(0, 0);
-  const C *Zb = Bufs<C>::Z(s), *Gb = Bufs<C>::G(s);
-  // Partial sums over chunks of kFidChunk elements in C, folded into FP64 accumulators:
-  // in single precision this keeps the summation error at ~sqrt(chunk) eps instead of
-  // ~sqrt(ne) eps (ne reaches 10^4 for 8 spins); in FP64 it changes nothing.
-  constexpr int kFidChunk = 32;
-  double2 acc64[JT][PT];
+      for (int a = 0; a < JT; ++a) zm[a] = m0 + a < mr ? s.Z[at((m0 + a) * s.ne + e, c, s.Cpad)] : cmk(0, 0);
 #pragma unroll
-  for (int a = 0; a < JT; ++a)
+      for (int b = 0; b < PT; ++b) gp[b] = p0 + b < s.gper ? s.G[at((p0 + b) * s.ne + e, c, s.Cpad)] : cmk(0, 0);
 #pragma unroll
-    for (int b = 0; b < PT; ++b) acc64[a][b] = cmk(0, 0);
-  if (c < s.C) {
-    for (int e0 = 0; e0 < s.ne; e0 += kFidChunk) {
-      const int e1 = min(s.ne, e0 + kFidChunk);
-      for (int e = e0; e < e1; ++e) {
-        C zj[JT], gp[PT];
+      for (int b = 0; b < PT; ++b) {
+        const double2 q = cmul(zc, gp[b]);
 #pragma unroll
-        for (int a = 0; a < JT; ++a)
-          zj[a] = (j0 + a < s.J) ? Zb[at((j0 + a) * s.ne + e, c, s.Cpad)] : mkc<C>(0, 0);
-#pragma unroll
-        for (int b = 0; b < PT; ++b)
-          gp[b] = (p0 + b < s.gper) ? Gb[at((p0 + b) * s.ne + e, c, s.Cpad)] : mkc<C>(0, 0);
-#pragma unroll
-        for (int a = 0; a < JT; ++a)
-#pragma unroll
-          for (int b = 0; b < PT; ++b) acc[a][b] = cfma(zj[a], gp[b], acc[a][b]);
-      }
-#pragma unroll
-      for (int a = 0; a < JT; ++a)
-#pragma unroll
-        for (int b = 0; b < PT; ++b) {
-          acc64[a][b] = cadd(acc64[a][b], todbl(acc[a][b]));
-          acc[a][b] = mkc<C>(0, 0);
+        for (int a = 0; a < JT; ++a) {
+          double *v = acc + 4 * (a * PT + b);
+          v[0] = fma(zm[a].x, q.x, v[0]);
+          v[1] = fma(zm[a].y, q.y, v[1]);
+          v[2] = fma(zm[a].x, q.y, v[2]);
+          v[3] = fma(zm[a].y, q.x, v[3]);
         }
+      }
     }
   }
-  double wc = (c < s.C) ? s.w[c] * s.scale : 0.0;
-  int lane = threadIdx.x & 31;
-  int wglob = s.warp_base + c / 32;
+  // sum x of the tile over the warp's lanes ends in lane x / (V / 32)
 #pragma unroll
-  for (int a = 0; a < JT; ++a)
+  for (int o = 16, half = V / 2; o > 0; o >>= 1, half >>= 1) {
+    const bool up = lane & o;
 #pragma unroll
-    for (int b = 0; b < PT; ++b) {
-      double2 v = cscale(acc64[a][b], wc);  // powder weight and the warp sum in FP64
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-      }
-      int k = (j0 + a) * s.gper + p0 + b;
-      if (lane == 0 && p0 + b < s.gper && k < s.npts) s.partial[size_t(wglob) * s.npts + k] = v;
+    for (int x = 0; x < half; ++x) {
+      const double send = up ? acc[x] : acc[x + half], keep = up ? acc[x + half] : acc[x];
+      acc[x] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
+  }
+#pragma unroll
+  for (int r = 0; r < V / 32; ++r) fps[warp * V + lane * (V / 32) + r] = acc[r];
+  __syncthreads();
+  if (!valid) return;
+  const double *t0 = fps + (warp - er) * V;  // the tile's sums, one row per warp
+  for (int x = er * 32 + lane; x < JT * PT; x += 32 * W) {
+    const int m = m0 + x / PT, p = p0 + x % PT;
+    if (m >= mr || p >= s.gper) continue;
+    double v[4] = {0, 0, 0, 0};
+    for (int w = 0; w < W; ++w)
+      for (int q = 0; q < 4; ++q) v[q] += t0[w * V + 4 * x + q];
+    const int jp = (s.J % 2 ? (s.J - 1) / 2 : s.J / 2) + m, jm = s.J - 1 - jp;
+    double2 *row = s.partial + size_t(s.warp_base + g) * s.npts;
+    const long kp = long(jp) * s.gper + p, km = long(jm) * s.gper + p;
+    if (kp < s.npts) row[kp] = cmk(v[0] - v[1], v[2] + v[3]);
+    if (jm != jp && km < s.npts) row[km] = cmk(v[0] + v[1], v[2] - v[3]);
+  }
 }
 
 // Point-to-point FID terms, one thread per (crystallite, element (r,s)).
@@ -2235,9 +2236,10 @@ __global__ void __launch_bounds__(kThreads) k_fid(DevSys s) {
 //   i = j' sub - 1, m = q' + 1   (m_tot = 0: i = n - 1, m = 0).
 // Point p = j b + k has m_tot = p f: its i depends on k only and m grows by f per j, so
 // G[k] = Q_{i_k}(r,s) R(s,r) e^{i m_k d} and Z[j] = e^{i j f d} (d = th_s - th_r) feed
-// k_fid's fid[j b + k] = sum_e Z[j] G[k].  The chunk products are never formed: the
+// the FID terms' fid[j b + k] = sum_e Z[j] G[k].  The chunk products are never formed: the
 // reference's PropReduce (examples/qmsims/MMMQMAS/propreduce.cc:455-521) builds every
-// dwell propagator from shared sub-products; here the Floquet powers replace them.
+// dwell propagator from shared sub-products; here the Floquet powers replace them.  (FP64
+// form: Z holds the powers that k_fid_pair takes instead.)
 template <class C>
 __global__ void __launch_bounds__(kThreads) k_p2p_elems(DevSys s) {
   long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -2276,14 +2278,16 @@ __global__ void __launch_bounds__(kThreads) k_p2p_elems(DevSys s) {
   double2 z1;
   sincos(double(s.pf) * d, &z1.y, &z1.x);
   double2 zj = cmk(1, 0);
-  for (int j = 0; j < s.J; ++j) {
-    if ((j & 63) == 0 && j) sincos(double(j) * double(s.pf) * d, &zj.y, &zj.x);
+  constexpr bool kPair = std::is_same<C, double2>::value;  // k_fid_pair's powers in the FP64 form
+  const int nz = kPair ? pair_rows(s.J) : s.J;
+  for (int j = 0; j < nz; ++j) {
+    const double pw = kPair ? pair_power(s.J, j) : double(j);
+    if ((j & 63) == 0 && pw != 0.0) sincos(pw * double(s.pf) * d, &zj.y, &zj.x);
     Bufs<C>::Z(s)[at(j * s.ne + e, c, s.Cpad)] = cvt<C>(zj);
     zj = cmul(zj, z1);
   }
 }
 
-// Compensated (Kahan) sum of the warp partials in fixed order: deterministic.
 // Mixed form: the FID terms as a tiled product.  fid[j gper + p] = sum_c w_c sum_e
 // z_e^j(c) G_p(e, c) is a product with K = (crystallite, element); one CTA takes a group of
 // 32 crystallites (one warp of the batch layout), a range of the elements (ft_r ranges, a
@@ -2404,17 +2408,30 @@ __global__ void __launch_bounds__(kFtThreads) k_fid_tiled(DevSys s) {
     }
 }
 
-__global__ void k_reduce(const double2 *__restrict__ partial, int nw, int npts, double2 *__restrict__ fid) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= npts) return;
+// Compensated (Kahan) sum of the warp partials in a fixed order: warp g of a block sums rows g,
+// g + kRedGroups, ... of 32 points; the first warp adds the groups' sums and compensations in
+// order.  One thread per point over every row was a serial chain of loads (37 rows, 1024
+// points: 27 us on 4 CTAs; now 16 us; 1872 rows, 2048 points 75 -> 22 us).
+constexpr int kRedGroups = 16;
+__global__ void __launch_bounds__(32 * kRedGroups) k_reduce(const double2 *__restrict__ partial, int nw, int npts,
+                                                           double2 *__restrict__ fid) {
+  __shared__ double2 sum[kRedGroups][32], comp[kRedGroups][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
   double sx = 0, sy = 0, cx = 0, cy = 0;
-  for (int w = 0; w < nw; ++w) {
-    double2 v = partial[size_t(w) * npts + k];
+  auto add = [&](double2 v) {
     double yx = v.x - cx, tx = sx + yx;
     cx = (tx - sx) - yx, sx = tx;
     double yy = v.y - cy, ty = sy + yy;
     cy = (ty - sy) - yy, sy = ty;
+  };
+  if (k < npts) {
+#pragma unroll 4
+    for (int w = g; w < nw; w += kRedGroups) add(partial[size_t(w) * npts + k]);
   }
+  sum[g][lane] = make_double2(sx, sy), comp[g][lane] = make_double2(-cx, -cy);
+  __syncthreads();
+  if (g != 0 || k >= npts) return;
+  for (int t = 1; t < min(kRedGroups, nw); ++t) add(sum[t][lane]), add(comp[t][lane]);
   fid[k] = make_double2(sx, sy);
 }
 
@@ -3303,7 +3320,7 @@ static void launch_block_kernels(JobImpl &J, DevSys &s, int stage) {
       if (s.nseg > 1) ++J.launches;
       break;
     case 2:
-      if (B == 1) {
+      if constexpr (B == 1) {
         k_floquet<B><<<grid_for(Cp * nl), kThreads, 0, st>>>(s, bl, nl);
       } else {  // B lanes per matrix, 32/B matrices per warp
         const long warps = (Cp * nl + (32 / B) - 1) / (32 / B);
@@ -3595,28 +3612,36 @@ static void launch_stage(JobImpl &J, DevSys &s, int stage) {
 static void mark_begin(JobImpl &J, int stage);
 static void mark_end(JobImpl &J, int stage, int nlaunch);
 
-// k_fid with a (j, p) register tile of about 16 accumulators whose p-width wastes the least of
-// the period gper (a point-to-point period of 9 takes 3-wide tiles instead of 4-wide)
-template <int JT, int PT, class C>
-static void launch_fid_tile(const DevSys &s, long Cp, int Jn, cudaStream_t st) {
-  const int npt = (s.gper + PT - 1) / PT, njt = (Jn + JT - 1) / JT;
-  k_fid<C, JT, PT><<<grid_for(Cp * npt * njt), kThreads, 0, st>>>(s);
+// k_fid_pair with the (m, p) tile that needs the fewest FP64 operations over the padded range.
+template <int JT, int PT>
+static void launch_fid_tile(const DevSys &s, long groups, int W, cudaStream_t st) {
+  const long tiles = groups * ((pair_rows(s.J) + JT - 1) / JT) * ((s.gper + PT - 1) / PT);
+  const int warps = std::max(4, W), per = warps / W;
+  constexpr int V = (4 * JT * PT + 31) / 32 * 32;
+  k_fid_pair<JT, PT><<<unsigned((tiles + per - 1) / per), 32 * warps, sizeof(double) * V * warps, st>>>(s, W);
 }
-template <class C>
-static void launch_fid(const DevSys &s, long Cp, int Jn, cudaStream_t st) {
-  int pt = kFidPT;
-  if (s.gper % kFidPT != 0 && s.gper < 64) {
-    int waste = 1 << 30;
-    for (int w = kFidPT; w >= 1; --w) {
-      const int ws = (s.gper + w - 1) / w * w - s.gper;
-      if (ws < waste) waste = ws, pt = w;
-    }
+static void launch_fid(const DevSys &s, long Cp, cudaStream_t st) {
+  // warps per tile: about 8 elements each, at most 8 (a function of the element count alone)
+  const int W = s.ne < 16 ? 1 : s.ne < 32 ? 2 : s.ne < 256 ? 4 : 8;
+  static const int shape[][2] = {{8, 2}, {7, 2}, {6, 2}, {5, 3}, {4, 4}, {3, 5}, {2, 8}, {1, 8}};
+  int best = 0;
+  double cost = 1e300;
+  for (int t = 0; t < 8; ++t) {
+    const int JT = shape[t][0], PT = shape[t][1];
+    const double n = double((pair_rows(s.J) + JT - 1) / JT) * double((s.gper + PT - 1) / PT);
+    const double x = n * ((4.0 * JT * PT + 4.0 * PT + 2.0) * (double(s.ne) / W + 1.0) + 4.0 * JT * PT);
+    if (x < cost) cost = x, best = t;
   }
-  switch (pt) {
-    case 1: launch_fid_tile<16, 1, C>(s, Cp, Jn, st); break;
-    case 2: launch_fid_tile<8, 2, C>(s, Cp, Jn, st); break;
-    case 3: launch_fid_tile<5, 3, C>(s, Cp, Jn, st); break;
-    default: launch_fid_tile<kFidJT, kFidPT, C>(s, Cp, Jn, st); break;
+  const long groups = Cp / 32;
+  switch (best) {
+    case 0: launch_fid_tile<8, 2>(s, groups, W, st); break;
+    case 1: launch_fid_tile<7, 2>(s, groups, W, st); break;
+    case 2: launch_fid_tile<6, 2>(s, groups, W, st); break;
+    case 3: launch_fid_tile<5, 3>(s, groups, W, st); break;
+    case 4: launch_fid_tile<4, 4>(s, groups, W, st); break;
+    case 5: launch_fid_tile<3, 5>(s, groups, W, st); break;
+    case 6: launch_fid_tile<2, 8>(s, groups, W, st); break;
+    default: launch_fid_tile<1, 8>(s, groups, W, st); break;
   }
 }
 
@@ -3682,7 +3707,7 @@ void Job::run() {
     mark_end(J, 4, J.launches - qr_before);
     mark_begin(J, 5);
     if (J.is_static && J.ne > 0) {
-      k_static_elems<<<grid_for(Cp * J.npq), kThreads, 0, st>>>(s);
+      k_static_elems<<<grid_for(Cp * J.ne * ((J.n + kStaticRun - 1) / kStaticRun + 1)), kThreads, 0, st>>>(s);
       ++J.launches;
     } else if (J.p2p && J.ne > 0) {
       if (s.mixed) k_p2p_elems<float2><<<grid_for(Cp * J.ne), kThreads, 0, st>>>(s);
@@ -3719,8 +3744,7 @@ void Job::run() {
       ++J.launches;
     }
     mark_end(J, 5, J.ne > 0 ? 1 : 0);
-    // k_fid writes every (warp, k) of this batch, so partials need no clearing; it exits
-    // per warp, and rows it does not cover (p >= n or k >= npts) do not exist
+    // every (row, k) of this batch is written, so partials need no clearing
     mark_begin(J, 6);
     if (s.mixed) {
       const unsigned npr = unsigned((s.gper + 4 * s.ft_pt - 1) / (4 * s.ft_pt));
@@ -3728,14 +3752,14 @@ void Job::run() {
       k_fid_tiled<<<dim3(unsigned(Cp / 32), npr * njr, unsigned(s.ft_r)), kFtThreads,
                     fid_tiled_smem(s.ft_jt, s.ft_pt), st>>>(s);
     } else {
-      launch_fid<double2>(s, Cp, J.J, st);
+      launch_fid(s, Cp, st);
     }
     ++J.launches;
     mark_end(J, 6, 1);
   }
   mark_begin(J, 7);
   // only warps that hold crystallites: the sum is then independent of the batch size
-  k_reduce<<<(J.P.npts + 255) / 256, 256, 0, st>>>(J.partial.p, (J.Ceff + 31) / 32 * (J.mixed ? J.ft_r : 1),
+  k_reduce<<<(J.P.npts + 31) / 32, 32 * kRedGroups, 0, st>>>(J.partial.p, (J.Ceff + 31) / 32 * (J.mixed ? J.ft_r : 1),
                                                     J.P.npts, J.fid.p);
   ++J.launches;
   mark_end(J, 7, 1);
