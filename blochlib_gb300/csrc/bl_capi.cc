@@ -62,7 +62,7 @@ bl_status guarded(F &&f) {
 
 bl::CMatrix load_op(const double *m, int N) {
   bl::CMatrix M(N);
-  for (size_t i = 0; i < M.a.size(); ++i) M.a[i] = bl::cplx(m[2 * i], m[2 * i + 1]);
+  std::memcpy(static_cast<void *>(M.a.data()), m, M.a.size() * sizeof(bl::cplx));  // interleaved (re, im), as std::complex
   return M;
 }
 
@@ -376,37 +376,35 @@ static void release_region(bl_ctx *ctx) {
 static bool fid_in_region(bl_ctx *ctx, const bl::SpinSystem &s, const bl::Powder &pw, const bl::CMatrix &ro,
                           const bl::CMatrix &det, const bl::FidParams &p, double *fid_out, double *sw_out) {
   std::lock_guard<std::mutex> lock(ctx->mu);
-  size_t lo = 0, full = 0;
-  bl::job_bytes(ctx->c.device, s, pw, ro, det, p, &lo, &full);
   if (cudaSetDevice(ctx->c.device) != cudaSuccess) return false;
-  size_t fr = 0, tot = 0;
-  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
-  const size_t budget = ctx->c.hbm_budget ? ctx->c.hbm_budget : size_t(0.6 * double(fr + ctx->region_bytes));
-  const size_t want = std::min(full, budget);
-  if (want < lo) {  // not one batch: give the region's memory back to a job of its own
-    if (ctx->region) cudaFree(ctx->region);
-    ctx->region = nullptr, ctx->region_bytes = 0;
-    return false;
-  }
-  if (want > ctx->region_bytes) {
-    if (ctx->region) cudaFree(ctx->region);
-    ctx->region = nullptr, ctx->region_bytes = 0;
-    if (cudaMalloc(&ctx->region, want) != cudaSuccess) {
-      cudaGetLastError();
-      ctx->region = nullptr;
-      return false;
+  // asked once, when the job is planned: the region as it stands when the whole powder fits it
+  // (no look at the free memory then), else grown to what the budget allows
+  auto region = [ctx](size_t lo, size_t full, size_t *bytes) -> void * {
+    if (ctx->region && ctx->region_bytes >= full) {
+      *bytes = ctx->region_bytes;
+      return ctx->region;
     }
-    ctx->region_bytes = want;
-  }
-  const size_t saved = ctx->c.hbm_budget;  // job_in_region sets the budget of the region
-  struct Restore {
-    bl::Context &c;
-    size_t v;
-    ~Restore() { c.hbm_budget = v; }
-  } restore{ctx->c, saved};
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return nullptr;
+    const size_t budget = ctx->c.hbm_budget ? ctx->c.hbm_budget : size_t(0.6 * double(fr + ctx->region_bytes));
+    const size_t want = std::min(full, budget);
+    if (want < lo || want > ctx->region_bytes) {
+      if (ctx->region) cudaFree(ctx->region);
+      ctx->region = nullptr, ctx->region_bytes = 0;
+      if (want < lo) return nullptr;  // not one batch: a job of its own reports the error
+      if (cudaMalloc(&ctx->region, want) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->region = nullptr;
+        return nullptr;
+      }
+      ctx->region_bytes = want;
+    }
+    *bytes = ctx->region_bytes;
+    return ctx->region;
+  };
   std::unique_ptr<bl::Job> job;
   try {
-    job = bl::job_in_region(ctx->c, ctx->region, ctx->region_bytes, s, pw, ro, det, p);
+    job = bl::job_in_asked_region(ctx->c, region, s, pw, ro, det, p);
   } catch (const bl::Error &e) {
     if (e.code == BL_ERR_NOMEM) return false;  // more than the planned bytes: a job of its own
     throw;

@@ -2409,8 +2409,8 @@ __global__ void __launch_bounds__(kFtThreads) k_fid_tiled(DevSys s) {
 }
 
 // Compensated (Kahan) sum of the warp partials in a fixed order: warp g of a block sums rows g,
-// g + kRedGroups, ... of 32 points; the first warp adds the groups' sums and compensations in
-// order.  One thread per point over every row was a serial chain of loads (37 rows, 1024
+// g + G, ... of 32 points (G groups of at least four rows); the first warp adds the groups' sums
+// and compensations in order.  One thread per point over every row was a serial chain of loads (37 rows, 1024
 // points: 27 us on 4 CTAs; now 16 us; 1872 rows, 2048 points 75 -> 22 us).
 constexpr int kRedGroups = 16;
 __global__ void __launch_bounds__(32 * kRedGroups) k_reduce(const double2 *__restrict__ partial, int nw, int npts,
@@ -2424,15 +2424,45 @@ __global__ void __launch_bounds__(32 * kRedGroups) k_reduce(const double2 *__res
     double yy = v.y - cy, ty = sy + yy;
     cy = (ty - sy) - yy, sy = ty;
   };
-  if (k < npts) {
+  const int G = min(kRedGroups, (nw + 3) / 4);
+  if (k < npts && g < G) {
 #pragma unroll 4
-    for (int w = g; w < nw; w += kRedGroups) add(partial[size_t(w) * npts + k]);
+    for (int w = g; w < nw; w += G) add(partial[size_t(w) * npts + k]);
   }
   sum[g][lane] = make_double2(sx, sy), comp[g][lane] = make_double2(-cx, -cy);
   __syncthreads();
   if (g != 0 || k >= npts) return;
-  for (int t = 1; t < min(kRedGroups, nw); ++t) add(sum[t][lane]), add(comp[t][lane]);
+  double2 cs = make_double2(0, 0);  // the other groups' compensations: below an ulp of the sums
+  for (int t = 1; t < G; ++t) add(sum[t][lane]), cs = cadd(cs, comp[t][lane]);
+  add(cs);
   fid[k] = make_double2(sx, sy);
+}
+
+// A non-zero of the packed term operators: element idx of the (term, packed block index) table.
+struct TermEntry {
+  int idx, pad;
+  double v;
+};
+// The dense term tables (zeroed before) from their non-zeros; Tdf may be null.
+__global__ void __launch_bounds__(kThreads) k_scatter_terms(const TermEntry *__restrict__ t, int n, double *T, float2 *Tdf) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= n) return;
+  T[t[x].idx] = t[x].v;
+  if (Tdf) Tdf[t[x].idx] = dfv_of(t[x].v);
+}
+// R_powder(phi, theta, gamma) (the 3-angle Cartesian rotation, space_ten.cc:578-618) of every
+// crystallite, batch-major [batch][element][c], from the angles [phi | theta | gamma].
+__global__ void __launch_bounds__(kThreads) k_orient(const double *__restrict__ ang, int all, int Cb, double *Rp) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= all) return;
+  double sa, ca, sb, cb, sg, cg;
+  sincos(ang[x], &sa, &ca), sincos(ang[all + x], &sb, &cb), sincos(ang[2 * all + x], &sg, &cg);
+  double *R = Rp + size_t(x / Cb) * 9 * Cb + x % Cb;
+  const double m[9] = {ca * cb * cg - sa * sg, sa * cb * cg + ca * sg, -sb * cg,
+                       -ca * cb * sg - sa * cg, -sa * cb * sg + ca * cg, sb * sg,
+                       ca * sb, sa * sb, cb};
+#pragma unroll
+  for (int e = 0; e < 9; ++e) R[size_t(e) * Cb] = m[e];
 }
 
 inline unsigned grid_for(long threads) { return unsigned((threads + kThreads - 1) / kThreads); }
@@ -2441,10 +2471,13 @@ inline unsigned grid_for(long threads) { return unsigned((threads + kThreads - 1
 
 // ------------------------------------------------------------------ host side
 Context::~Context() {
+  for (auto e : join_ev) cudaEventDestroy(e);
+  for (auto a : aux) cudaStreamDestroy(a);
+  if (fork_ev) cudaEventDestroy(fork_ev);
+  if (stage_ev) cudaEventDestroy(stage_ev);
+  if (stage) cudaFreeHost(stage);
   if (stream) cudaStreamDestroy(stream);
 }
-
-static thread_local size_t *g_upload_counter = nullptr;  // set while a Job uploads its inputs
 
 // Bump allocator over a caller-provided device region.  The allocation-free entry point
 // (powder_fid_noalloc) and job_in_region install one while they build a Job.
@@ -2455,6 +2488,8 @@ struct ScratchArena {
   bool aux_streams = false;  // the Job may create its own streams (not on the allocation-free path)
 };
 static thread_local ScratchArena *g_arena = nullptr;
+// Set by job_in_asked_region: the constructor asks it for the region once the job is planned.
+static thread_local const RegionFn *g_region = nullptr;
 // Set by job_bytes: the Job constructor records its memory plan here and returns before
 // touching the device.
 struct JobSizing {
@@ -2489,14 +2524,58 @@ struct DevBuf {
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
   DevBuf(DevBuf &&o) noexcept : p(o.p), n(o.n), owned(o.owned) { o.p = nullptr, o.n = 0; }
-  void upload(const std::vector<T> &v, cudaStream_t st) {
-    alloc(v.size());
-    if (!v.empty()) CUDA_OK(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-    if (g_upload_counter) *g_upload_counter += v.size() * sizeof(T);
-  }
   ~DevBuf() {
     if (p && owned) cudaFree(p);
   }
+};
+
+// The job's inputs and tables: gathered on the host at 256-byte offsets, then one device
+// buffer and one copy (forty copies of a few hundred bytes each took most of a small call).
+class Uploads {
+ public:
+  template <class T>
+  void add(DevBuf<T> &buf, const std::vector<T> &v) {
+    const size_t off = (host_.size() + 255) & ~size_t(255), bytes = v.size() * sizeof(T);
+    buf.n = v.size();
+    if (v.empty()) return;
+    host_.resize(off + bytes);
+    std::memcpy(host_.data() + off, v.data(), bytes);
+    total_ += bytes;
+    DevBuf<T> *b = &buf;
+    set_.push_back([b, off](unsigned char *base) { b->p = reinterpret_cast<T *>(base + off), b->owned = false; });
+  }
+  // enqueues the copy on the context's stream and sets every added buffer's address in `dev`;
+  // the pinned buffer is used unless the job may not allocate (pinned == false)
+  void flush(Context &ctx, DevBuf<unsigned char> &dev, bool pinned) {
+    if (host_.empty()) return;
+    dev.alloc(host_.size());
+    std::lock_guard<std::mutex> lock(ctx.mu);
+    const void *src = host_.data();
+    if (pinned && host_.size() <= Context::kMaxStage) {
+      if (ctx.stage_ev) CUDA_OK(cudaEventSynchronize(ctx.stage_ev));  // the last copy out of it has ended
+      else CUDA_OK(cudaEventCreateWithFlags(&ctx.stage_ev, cudaEventDisableTiming));
+      if (ctx.stage_bytes < host_.size()) {
+        if (ctx.stage) CUDA_OK(cudaFreeHost(ctx.stage));
+        ctx.stage = nullptr, ctx.stage_bytes = 0;
+        size_t want = size_t(256) << 10;
+        while (want < host_.size()) want *= 2;
+        CUDA_OK(cudaMallocHost(&ctx.stage, want));
+        ctx.stage_bytes = want;
+      }
+      std::memcpy(ctx.stage, host_.data(), host_.size());
+      src = ctx.stage;
+    }
+    // (a pageable copy returns once its source has been read)
+    CUDA_OK(cudaMemcpyAsync(dev.p, src, host_.size(), cudaMemcpyHostToDevice, ctx.stream));
+    if (src == ctx.stage) CUDA_OK(cudaEventRecord(ctx.stage_ev, ctx.stream));
+    for (auto &f : set_) f(dev.p);
+  }
+  size_t bytes() const { return total_; }
+
+ private:
+  std::vector<unsigned char> host_;
+  std::vector<std::function<void(unsigned char *)>> set_;
+  size_t total_ = 0;
 };
 
 struct JobImpl {
@@ -2524,7 +2603,9 @@ struct JobImpl {
   DevBuf<double2> big_cv;
   DevBuf<int> bs, boff, bpoff, qa, qb, qoff, doff, ra, rb, roff, rhooff, eq, erev, er, erg, esg, status, srp, seo;
   std::vector<DevBuf<int>> blist;
-  DevBuf<double> pas, iscale, Tk, Hc, Rp_all, t0_all, w_all;
+  DevBuf<unsigned char> tables;  // the one buffer behind the uploaded inputs and tables
+  DevBuf<double> pas, iscale, Tk, Hc, angles, Rp_all, t0_all, w_all;
+  DevBuf<TermEntry> tk_entries;  // large systems: the term operators' non-zeros, scattered into Tk
   DevBuf<int> ikind;
   int has2 = 0;  // second-order quadrupolar terms present
   int p2p = 0, pb = 1, pf = 1, psub = 1;  // point-to-point FID: base, factor, steps per chunk
@@ -2543,8 +2624,6 @@ struct JobImpl {
   DevBuf<unsigned long long> tcf;  // the two tensor-flop counters
   std::vector<size_t> usl_off;  // per block index: byte offset of its region (large blocks)
   int mixed = 0;
-  DevBuf<double> Rp_b, t0_b, w_b;
-  std::vector<double> h_Rp, h_t0, h_w;  // all virtual crystallites (C * gammaloop)
   int Ceff = 0;
   double flops = 0;
   int launches = 0;
@@ -2559,26 +2638,81 @@ struct JobImpl {
   };
   std::vector<Mark> marks;
   int evnext = 0;
-  // streams on which the large blocks of one stage run side by side (fork/join on the
-  // context stream), so that their one-CTA-per-crystallite launches fill the SMs together
+  // the context's streams on which the large blocks of one stage run side by side (fork/join
+  // on the context stream), so that their one-CTA-per-crystallite launches fill the SMs together
   std::vector<cudaStream_t> aux;
   cudaEvent_t fork_ev = nullptr;
   std::vector<cudaEvent_t> join_ev;
   ~JobImpl() {
     for (auto &e : evpool) cudaEventDestroy(e);
-    for (auto &e : join_ev) cudaEventDestroy(e);
-    if (fork_ev) cudaEventDestroy(fork_ev);
-    for (auto &a : aux) cudaStreamDestroy(a);
   }
   double cos_rotb = 1, sin_rotb = 0;
   DevSys base{};
 };
 
-static bool any_nonzero(const CMatrix &M, const BlockLayout &L, int a, int b) {
-  for (int r = 0; r < L.size[a]; ++r)
-    for (int s = 0; s < L.size[b]; ++s)
-      if (M(L.perm[L.off[a] + r], L.perm[L.off[b] + s]) != cplx(0, 0)) return true;
-  return false;
+// Device bytes outside the batch-sized work buffers: tables, per-crystallite inputs (11
+// doubles each, padded by up to one batch), warp partials and the FID.
+static size_t fixed_bytes(const Powder &pw, const FidParams &p) {
+  long n = p.wr != 0.0 ? long(std::floor(p.sw / p.wr + 0.5)) : 1;
+  long g = (n >= 1 && n <= 10) ? std::max(1L, 10 / n) : 1;
+  size_t ceff = size_t(pw.size()) * size_t(g) + 32;
+  // warp partials: up to kFtR rows per warp in the mixed form (k_fid_tiled's element ranges)
+  return (size_t(8) << 20) + 2 * ceff * 11 * sizeof(double) +
+         (ceff / 32 + 1) * size_t(p.precision == 1 ? kFtR : 1) * size_t(std::max(p.npts, 0)) * sizeof(double2);
+}
+
+// Bytes of a planned job with one warp (32) of crystallites per batch and with all of them in one.
+static void planned_bytes(const JobSizing &plan, const Powder &pw, const FidParams &p, size_t *min_bytes,
+                          size_t *full_bytes) {
+  // work buffers are carved with 256-byte alignment: allow for it on each of ~40 buffers
+  const size_t fixed = fixed_bytes(pw, p) + 40 * 256 + plan.extra + plan.tables;
+  if (min_bytes) *min_bytes = fixed + plan.per_c * 32;
+  if (full_bytes) *full_bytes = fixed + plan.per_c * size_t(plan.cpad);
+}
+
+static float2 df_split(double v) {
+  const float h = float(v);
+  return make_float2(h, float(v - double(h)));
+}
+// term operators of up to this many elements in all go up dense
+constexpr size_t kDenseTerms = size_t(1) << 15;
+
+// Which block pairs (a, b) of M hold a non-zero: one pass over M.
+static std::vector<char> nonzero_blocks(const CMatrix &M, const BlockLayout &L) {
+  const size_t nb = L.size.size();
+  std::vector<char> f(nb * nb, 0);
+  for (int r = 0; r < M.n; ++r)
+    for (int c = 0; c < M.n; ++c)
+      if (M(r, c) != cplx(0, 0)) f[size_t(L.block_of[L.inv[r]]) * nb + size_t(L.block_of[L.inv[c]])] = 1;
+  return f;
+}
+
+// Every kernel with dynamic shared memory may take all that its static part leaves (once per
+// context: the limit is the same for every job, whatever runs beside it).
+static void ready_kernels(Context &ctx) {
+  std::lock_guard<std::mutex> lock(ctx.mu);
+  if (ctx.kernels_ready) return;
+  int most = 0;
+  CUDA_OK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx.device));
+  auto all = [&](const void *f) {
+    cudaFuncAttributes a;
+    CUDA_OK(cudaFuncGetAttributes(&a, f));
+    CUDA_OK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(a.sharedSizeBytes)));
+  };
+  for (const void *f :
+       {(const void *)k_big_step, (const void *)k_big_step_df, (const void *)k_big_dyson<1>,
+        (const void *)k_big_dyson<2>, (const void *)k_big_dyson_df<1>, (const void *)k_big_dyson_df<2>,
+        (const void *)k_tc_step, (const void *)k_tc_step_stk, (const void *)k_tc_dyson, (const void *)k_tc_dyson_stk,
+        (const void *)k_big_seg_frame<false>, (const void *)k_big_seg_frame<true>,
+        (const void *)k_big_eigframe<1, double2>, (const void *)k_big_eigframe<2, double2>,
+        (const void *)k_big_eigframe4, (const void *)k_big_floquet, (const void *)k_huge_floquet,
+        (const void *)k_big_qr<1, float2>, (const void *)k_big_qr<2, float2>, (const void *)k_big_qr<1, double2>,
+        (const void *)k_big_qr<2, double2>, (const void *)k_fave_fft<8, double2>, (const void *)k_fave_fft<4, double2>,
+        (const void *)k_fave_fft<2, double2>, (const void *)k_fave_fft<1, double2>, (const void *)k_fave_fft<8, float2>,
+        (const void *)k_fave_fft<4, float2>, (const void *)k_fave_fft<2, float2>, (const void *)k_fave_fft<1, float2>,
+        (const void *)k_fid_tiled})
+    all(f);
+  ctx.kernels_ready = true;
 }
 
 Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &ro_in, const CMatrix &det_in,
@@ -2697,11 +2831,15 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
       }
   // rf phases: the engine propagates the real H' = R^H H R, so rho and det enter as R^H X R
   // (under an rf schedule each step's U is turned back into the lab frame instead)
-  const CMatrix ro = sched ? ro_in : sys.to_frame(ro_in), det = sched ? det_in : sys.to_frame(det_in);
+  const bool turned = !sched && !sys.frame().empty();
+  CMatrix ro_t, det_t;
+  if (turned) ro_t = sys.to_frame(ro_in), det_t = sys.to_frame(det_in);
+  const CMatrix &ro = turned ? ro_t : ro_in, &det = turned ? det_t : det_in;
   if (J.is_static) J.rosym = 0;  // the static FID always transforms rho itself
   // Hamiltonian terms, packed per block
   const int nhc = sched ? J.pb : 1;
-  std::vector<double> pas, isc, Tk, Hc(size_t(L.S2) * nhc, 0.0);
+  std::vector<double> pas, isc, Hc(size_t(L.S2) * nhc, 0.0);
+  std::vector<TermEntry> Tnz;  // non-zeros of the packed operators, term by term
   auto pack = [&](const std::vector<double> &M, double *dst) {
     for (int k = 0; k < nb; ++k)
       for (int r = 0; r < L.size[k]; ++r)
@@ -2721,14 +2859,22 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   const auto &ints = sys.interactions();
   const double Bf = sys.bfield();
   std::vector<int> ikind;
-  auto add_term = [&](const Interaction &I, int kind, double scale, const std::vector<double> &op) {
+  auto entry = [&](int r, int c, double v) {
+    const int pr = L.inv[r], pc = L.inv[c], k = L.block_of[pr];
+    Tnz.push_back({J.nint * L.S2 + L.poff[k] + (pr - L.off[k]) * L.size[k] + (pc - L.off[k]), 0, v});
+  };
+  auto add_term = [&](const Interaction &I, int kind, double scale, size_t kk) {
     pas.insert(pas.end(), {I.pas[0][0], I.pas[0][1], I.pas[0][2], I.pas[1][1], I.pas[1][2], I.pas[2][2]});
     isc.push_back(scale);
     ikind.push_back(kind);
     if (!g_sizing) {
-      size_t o = Tk.size();
-      Tk.resize(o + L.S2);
-      pack(op, Tk.data() + o);
+      if (kind == 0) {
+        for (const auto &e : sys.h_nonzeros()[kk]) entry(e.r, e.c, e.v);
+      } else {  // the second-order operators are diagonal
+        const auto &op = kind == 1 ? sys.h_ops_q4()[kk] : sys.h_ops_q2()[kk];
+        for (int r = 0; r < N; ++r)
+          if (op[size_t(r) * N + r] != 0.0) entry(r, r, op[size_t(r) * N + r]);
+      }
     }
     ++J.nint;
   };
@@ -2738,11 +2884,11 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     const bool quad = I.kind == 'Q';
     const bool first_only = !quad || I.order == 1 || std::fabs(Bf) <= 1e-12;
     const bool second_only = !first_only && I.order == 2;
-    if (!second_only) add_term(I, 0, I.op_scale, sys.h_ops()[kk]);
+    if (!second_only) add_term(I, 0, I.op_scale, kk);
     if (!first_only) {
       const double s2 = I.op_scale * I.op_scale / (Bf * isotope_rel_freq(sys.isotopes()[I.s1]));
-      add_term(I, 1, s2, sys.h_ops_q4()[kk]);
-      add_term(I, 2, -s2, sys.h_ops_q2()[kk]);
+      add_term(I, 1, s2, kk);
+      add_term(I, 2, -s2, kk);
     }
   }
   J.has2 = std::any_of(ikind.begin(), ikind.end(), [](int k) { return k != 0; }) ? 1 : 0;
@@ -2750,9 +2896,11 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   std::vector<int> qa, qb, qoff, doff, ra, rb, roff, rhooff;
   std::vector<double2> Dblk, Rhoblk;
   std::vector<std::vector<int>> qpair(nb, std::vector<int>(nb, -1)), rpair(nb, std::vector<int>(nb, -1));
+  const std::vector<char> det_nz = nonzero_blocks(det, L),
+                          ro_nz = J.rosym ? std::vector<char>() : nonzero_blocks(ro, L);
   for (int a = 0; a < nb; ++a)
     for (int b = 0; b < nb; ++b) {
-      if (any_nonzero(det, L, a, b)) {
+      if (det_nz[size_t(a) * nb + b]) {
         qpair[a][b] = int(qa.size());
         qa.push_back(a), qb.push_back(b), qoff.push_back(J.nq), doff.push_back(int(Dblk.size()));
         for (int r = 0; r < L.size[a]; ++r)
@@ -2762,7 +2910,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
           }
         J.nq += L.size[a] * L.size[b];
       }
-      if (!J.rosym && any_nonzero(ro, L, a, b)) {
+      if (!J.rosym && ro_nz[size_t(a) * nb + b]) {
         rpair[a][b] = int(ra.size());
         ra.push_back(a), rb.push_back(b), roff.push_back(J.nr), rhooff.push_back(int(Rhoblk.size()));
         for (int r = 0; r < L.size[a]; ++r)
@@ -2811,16 +2959,6 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   J.C = pw.size();
   J.Ceff = J.C * J.gammaloop;
   const double d2r = kPi / 180.0;
-  for (int c = 0; c < J.C; ++c) {
-    double R[3][3];
-    rotation3(pw.phi[c], pw.theta[c], pw.gamma[c], R);  // setPowderAngles(phi, theta, gamma)
-    for (int q = 0; q < J.gammaloop; ++q) {
-      for (int a = 0; a < 3; ++a)
-        for (int b = 0; b < 3; ++b) J.h_Rp.push_back(R[a][b]);
-      J.h_t0.push_back(q == 0 ? tmin : tmin + kPi2 * double(q) / double(J.gammaloop * J.n) / p.wr);
-      J.h_w.push_back(pw.weight[c]);
-    }
-  }
   J.cos_rotb = std::cos(p.rotb_deg * d2r);
   J.sin_rotb = std::sin(p.rotb_deg * d2r);
   // batch size from the memory budget
@@ -2871,19 +3009,40 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
       huge_fixed = J.huge_ws_bytes + size_t(J.huge_items) * (sizeof(double) * (J.nint + 1) + sizeof(int)) + 4096;
     }
   }
-  if (g_sizing) {
-    g_sizing->per_c = per_c;
-    g_sizing->cpad = cpad_all;
-    g_sizing->extra = huge_fixed;
-    // Tk and Hc (per chunk), their double-float copies in the mixed form, the D and rho
-    // blocks, the rf frames, and 256-byte alignment per buffer
+  JobSizing plan;
+  plan.per_c = per_c;
+  plan.cpad = cpad_all;
+  plan.extra = huge_fixed;
+  {  // Tk and Hc (per chunk), their double-float copies in the mixed form, the D and rho
+     // blocks, the rf frames, and 256-byte alignment per buffer
     const size_t tk = size_t(J.nint) * L.S2, hc = size_t(L.S2) * (sched ? J.pb : 1);
-    g_sizing->tables = (tk + hc) * sizeof(double) * ((p.precision == 1 && !J.is_static) ? 2 : 1) +
-                       (Dblk.size() + Rhoblk.size()) * sizeof(double2) + size_t(N) * J.pb * sizeof(double2) +
-                       64 * 256;
+    plan.tables = (tk + hc) * sizeof(double) * ((p.precision == 1 && !J.is_static) ? 2 : 1) +
+                  (Dblk.size() + Rhoblk.size()) * sizeof(double2) + size_t(N) * J.pb * sizeof(double2) + 64 * 256;
+  }
+  if (g_sizing) {
+    *g_sizing = plan;
     return;
   }
   size_t budget = ctx.hbm_budget;
+  ScratchArena asked;
+  struct ArenaScope {
+    bool on = false;
+    ScratchArena *prev = nullptr;
+    ~ArenaScope() {
+      if (on) g_arena = prev;
+    }
+  } arena_scope;
+  if (g_region) {
+    size_t lo = 0, full = 0, bytes = 0;
+    planned_bytes(plan, pw, p, &lo, &full);
+    asked.base = static_cast<char *>((*g_region)(lo, full, &bytes));
+    const size_t fixed = fixed_bytes(pw, p);
+    if (!asked.base || fixed >= bytes) throw Error(4, "job does not fit its device region");
+    asked.cap = bytes, asked.label = "device region given to the job", asked.aux_streams = true;
+    arena_scope.prev = g_arena, arena_scope.on = true;
+    g_arena = &asked;
+    budget = bytes - fixed;
+  }
   if (!budget) {  // default: 60% of the device memory free when the job is created
     size_t fr = 0, tot = 0;
     CUDA_OK(cudaMemGetInfo(&fr, &tot));
@@ -2907,27 +3066,34 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   }
   // per huge block: squarings enough for every step, from a rotation-free bound on
   // ||2 pi tau H||_inf (|a_k| <= ||PAS'_k||_F); the kernels skip items that need fewer
-  for (int k : J.huge_blocks) {
-    const int b = L.size[k], bp = L.poff[k];
-    double nrm = 0;
-    for (int r = 0; r < b; ++r) {
-      double rs = 0;
-      for (int q = 0; q < b; ++q) {
-        double v = 0;  // the largest constant part over the chunks of an rf schedule
-        for (int kc = 0; kc < nhc; ++kc) v = std::max(v, std::fabs(Hc[size_t(kc) * L.S2 + bp + r * b + q]));
-        for (int kk = 0; kk < J.nint; ++kk) {
-          const double *Pa = pas.data() + 6 * kk;
-          const double fro = std::sqrt(Pa[0] * Pa[0] + Pa[3] * Pa[3] + Pa[5] * Pa[5] +
-                                       2 * (Pa[1] * Pa[1] + Pa[2] * Pa[2] + Pa[4] * Pa[4]));
-          // |r_ij| <= ||PAS'||_F: first order |a| <= fro, second order |a| <= 2 fro^2
-          const double amax = ikind[kk] == 0 ? fro : 2.0 * fro * fro;
-          v += std::fabs(isc[kk]) * amax * std::fabs(Tk[size_t(kk) * L.S2 + bp + r * b + q]);
+  std::vector<double> row_bound;  // per permuted row: largest constant part plus the terms' bounds
+  if (!J.huge_blocks.empty()) {
+    row_bound.assign(N, 0.0);
+    for (int k : J.huge_blocks)
+      for (int r = 0; r < L.size[k]; ++r)
+        for (int q = 0; q < L.size[k]; ++q) {
+          double v = 0;  // the largest over the chunks of an rf schedule
+          for (int kc = 0; kc < nhc; ++kc)
+            v = std::max(v, std::fabs(Hc[size_t(kc) * L.S2 + L.poff[k] + r * L.size[k] + q]));
+          row_bound[L.off[k] + r] += v;
         }
-        rs += v;
-      }
-      nrm = std::max(nrm, rs);
+    std::vector<int> row_of(L.S2);
+    for (int k = 0; k < nb; ++k)
+      for (int e = 0; e < L.size[k] * L.size[k]; ++e) row_of[L.poff[k] + e] = L.off[k] + e / L.size[k];
+    for (const TermEntry &e : Tnz) {
+      const int kk = e.idx / L.S2;
+      const double *Pa = pas.data() + 6 * kk;
+      const double fro = std::sqrt(Pa[0] * Pa[0] + Pa[3] * Pa[3] + Pa[5] * Pa[5] +
+                                   2 * (Pa[1] * Pa[1] + Pa[2] * Pa[2] + Pa[4] * Pa[4]));
+      // |r_ij| <= ||PAS'||_F: first order |a| <= fro, second order |a| <= 2 fro^2
+      const double amax = ikind[kk] == 0 ? fro : 2.0 * fro * fro;
+      row_bound[row_of[e.idx % L.S2]] += std::fabs(isc[kk]) * amax * std::fabs(e.v);
     }
-    nrm *= J.tau * kPi2 * (1.0 + 1e-12);  // margin over the device's rounding of the same sum
+  }
+  for (int k : J.huge_blocks) {
+    double nrm = 0;
+    for (int r = 0; r < L.size[k]; ++r) nrm = std::max(nrm, row_bound[L.off[k] + r]);
+    nrm *= J.tau * kPi2 * (1.0 + 1e-10);  // margin over the rounding of either side's sums
     int q = 0;
     if (nrm > 0.5) {
       std::frexp(nrm / 0.5, &q);
@@ -2941,11 +3107,6 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     if (!J.big_blocks.empty() && J.nint > kMaxInt)
       throw Error(5, "more than " + std::to_string(kMaxInt) + " anisotropic interactions");
     const size_t csz = J.mixed ? sizeof(float2) : sizeof(double2);
-    size_t smem_step = 0, smem_mat = 0, smem_qr[2] = {0, 0};
-    for (int k : J.big_blocks) {
-      smem_step = std::max(smem_step, big_step_smem(L.size[k]));
-      smem_mat = std::max(smem_mat, sizeof(double2) * 2 * size_t(L.size[k]) * L.size[k]);
-    }
     // Q/R pairs with a big block: M_ab's non-zeros by row, and the W_b column chunk that
     // keeps W_a, W_b and X within half the shared memory (two CTAs per SM) where it can
     for (int pr = 0; pr < J.npq + J.npr; ++pr) {
@@ -2977,103 +3138,73 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
       }
       J.big_pairs.push_back(P);
       J.big_rp_off.push_back(rp_off);
-      const size_t sm = J.mixed ? big_qr_smem<float2>(ba, bb, w) : big_qr_smem<double2>(ba, bb, w);
-      smem_qr[big_nt(ba, w) - 1] = std::max(smem_qr[big_nt(ba, w) - 1], sm);
-    }
-    if (!g_sizing) {
-      auto attr = [](const void *f, size_t bytes) {
-        if (bytes) CUDA_OK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-      };
-      attr((const void *)k_big_step, smem_step);
-      attr((const void *)k_big_dyson<1>, smem_mat);
-      attr((const void *)k_big_dyson<2>, smem_mat);
-      attr((const void *)k_big_step_df, smem_step);  // 5 b^2 float2 <= the FP64 step's 5 or 7 b^2 doubles
-      attr((const void *)k_big_dyson_df<1>, smem_mat);
-      attr((const void *)k_big_dyson_df<2>, smem_mat);
-      if (J.tc) {
-        size_t sm_step = 0, sm_dy = 0;
-        for (int k : J.big_blocks)
-          if (L.size[k] >= tc::kMinB)
-            sm_step = std::max(sm_step, tc_step_smem(L.size[k])), sm_dy = std::max(sm_dy, tc_dyson_smem(L.size[k]));
-        attr((const void *)k_tc_step, sm_step);
-        attr((const void *)k_tc_dyson, sm_dy);
-        attr((const void *)k_tc_dyson_stk, tc_dyson_stk_smem(64));
-        attr((const void *)k_tc_step_stk, tc_step_stk_smem(64));
-      }
-      attr((const void *)k_big_eigframe<1, double2>, smem_mat);
-      attr((const void *)k_big_eigframe<2, double2>, smem_mat);
-      attr((const void *)k_big_seg_frame<false>, smem_mat);
-      attr((const void *)k_big_seg_frame<true>, smem_mat);
-      attr((const void *)k_big_eigframe4, smem_mat);
-      attr((const void *)k_big_floquet, smem_mat + (J.mixed ? smem_mat / 4 : 0));  // + b^2 float2 (K)
-      size_t smem_hf = 0;
-      for (int k : J.huge_blocks) smem_hf = std::max(smem_hf, huge_floquet_smem(L.size[k]));
-      if (smem_hf > (size_t(48) << 10)) attr((const void *)k_huge_floquet, smem_hf);
-      if (J.mixed) {
-        attr((const void *)k_big_qr<1, float2>, smem_qr[0]);
-        attr((const void *)k_big_qr<2, float2>, smem_qr[1]);
-      } else {
-        attr((const void *)k_big_qr<1, double2>, smem_qr[0]);
-        attr((const void *)k_big_qr<2, double2>, smem_qr[1]);
-      }
     }
   }
-  if (!g_sizing && !J.big_blocks.empty() && (!g_arena || g_arena->aux_streams)) {
-    const int naux = int(std::min<size_t>(4, std::max(J.big_blocks.size(), J.big_pairs.size())));
-    CUDA_OK(cudaEventCreateWithFlags(&J.fork_ev, cudaEventDisableTiming));
-    for (int a = 0; a < naux; ++a) {
+  ready_kernels(ctx);
+  if (!J.big_blocks.empty() && (!g_arena || g_arena->aux_streams)) {
+    const size_t naux = std::min<size_t>(4, std::max(J.big_blocks.size(), J.big_pairs.size()));
+    std::lock_guard<std::mutex> lock(ctx.mu);
+    if (!ctx.fork_ev) CUDA_OK(cudaEventCreateWithFlags(&ctx.fork_ev, cudaEventDisableTiming));
+    while (ctx.join_ev.size() < naux) {
       cudaStream_t x;
       cudaEvent_t e;
-      CUDA_OK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-      J.aux.push_back(x);
+      if (ctx.aux.size() == ctx.join_ev.size()) {
+        CUDA_OK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+        ctx.aux.push_back(x);
+      }
       CUDA_OK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      J.join_ev.push_back(e);
+      ctx.join_ev.push_back(e);
     }
+    J.aux.assign(ctx.aux.begin(), ctx.aux.begin() + std::ptrdiff_t(naux));
+    J.join_ev.assign(ctx.join_ev.begin(), ctx.join_ev.begin() + std::ptrdiff_t(naux));
+    J.fork_ev = ctx.fork_ev;
   }
   J.blist.resize(kMaxBlock + 1);
   cudaStream_t st = ctx.stream;
-  g_upload_counter = &J.h2d;
-  struct CounterReset {
-    ~CounterReset() { g_upload_counter = nullptr; }
-  } counter_reset;
-  for (int b = 1; b <= kMaxBlock; ++b) J.blist[b].upload(J.blocks_by_size[b], st);
-  J.bs.upload(L.size, st), J.boff.upload(L.off, st), J.bpoff.upload(L.poff, st);
-  J.qa.upload(qa, st), J.qb.upload(qb, st), J.qoff.upload(qoff, st), J.doff.upload(doff, st);
-  J.ra.upload(ra, st), J.rb.upload(rb, st), J.roff.upload(roff, st), J.rhooff.upload(rhooff, st);
-  J.eq.upload(eq, st), J.erev.upload(erev, st), J.er.upload(er, st), J.erg.upload(erg, st), J.esg.upload(esg, st);
-  J.srp.upload(srp, st), J.seo.upload(seo, st);
-  J.big_rp.upload(big_rp_h, st), J.big_ci.upload(big_ci_h, st), J.big_cv.upload(big_cv_h, st);
-  for (size_t t = 0; t < J.big_pairs.size(); ++t)
-    J.big_pairs[t].rp = J.big_rp.p + J.big_rp_off[t], J.big_pairs[t].ci = J.big_ci.p, J.big_pairs[t].cv = J.big_cv.p;
-  for (size_t t = 0; t < J.huge_pairs.size(); ++t)
-    J.huge_pairs[t].rp = J.big_rp.p + J.huge_rp_off[t], J.huge_pairs[t].ci = J.big_ci.p,
-    J.huge_pairs[t].cv = J.big_cv.p;
-  J.pas.upload(pas, st), J.iscale.upload(isc, st), J.Tk.upload(Tk, st), J.Hc.upload(Hc, st);
+  Uploads up;
+  for (int b = 1; b <= kMaxBlock; ++b) up.add(J.blist[b], J.blocks_by_size[b]);
+  up.add(J.bs, L.size), up.add(J.boff, L.off), up.add(J.bpoff, L.poff);
+  up.add(J.qa, qa), up.add(J.qb, qb), up.add(J.qoff, qoff), up.add(J.doff, doff);
+  up.add(J.ra, ra), up.add(J.rb, rb), up.add(J.roff, roff), up.add(J.rhooff, rhooff);
+  up.add(J.eq, eq), up.add(J.erev, erev), up.add(J.er, er), up.add(J.erg, erg), up.add(J.esg, esg);
+  up.add(J.srp, srp), up.add(J.seo, seo);
+  up.add(J.big_rp, big_rp_h), up.add(J.big_ci, big_ci_h), up.add(J.big_cv, big_cv_h);
+  up.add(J.pas, pas), up.add(J.iscale, isc), up.add(J.Hc, Hc);
+  // the packed operators: dense from the host while they are small, else their non-zeros go up
+  // and k_scatter_terms fills the (zeroed) dense tables (9 spins: 17.5 MB in each precision, 45
+  // terms of 768 non-zeros)
+  const bool df_tables = p.precision == 1 && !J.is_static;
+  const size_t tk_n = size_t(J.nint) * L.S2;
+  const bool scatter = tk_n > kDenseTerms;
+  if (scatter) {
+    up.add(J.tk_entries, Tnz);
+  } else {
+    std::vector<double> Tk(tk_n, 0.0);
+    for (const TermEntry &e : Tnz) Tk[size_t(e.idx)] = e.v;
+    up.add(J.Tk, Tk);
+    if (df_tables) {
+      std::vector<float2> t(tk_n);
+      for (size_t x = 0; x < tk_n; ++x) t[x] = df_split(Tk[x]);
+      up.add(J.Tk_df, t);
+    }
+  }
   if (p.precision == 1 && !J.is_static) {  // hi, lo splits for the mixed form's double-float step
-    auto split = [](const std::vector<double> &v) {
-      std::vector<float2> o(v.size());
-      for (size_t x = 0; x < v.size(); ++x) {
-        const float h = float(v[x]);
-        o[x] = make_float2(h, float(v[x] - double(h)));
-      }
-      return o;
-    };
-    J.Tk_df.upload(split(Tk), st);
-    J.Hc_df.upload(split(Hc), st);
+    std::vector<float2> h(Hc.size());
+    for (size_t x = 0; x < Hc.size(); ++x) h[x] = df_split(Hc[x]);
+    up.add(J.Hc_df, h);
     if (J.tc) {
-      std::vector<int> ptr(size_t(L.S2) + 1, 0), term;
-      std::vector<float2> val;
-      for (size_t e = 0; e < size_t(L.S2); ++e) {
-        ptr[e] = int(term.size());
-        for (int kk = 0; kk < J.nint; ++kk) {
-          const double v = Tk[size_t(kk) * L.S2 + e];
-          if (v != 0.0) {
-            const float h = float(v);
-            term.push_back(kk), val.push_back(make_float2(h, float(v - double(h))));
-          }
+      // by element, terms ascending: a counting pass, then the entries in term order
+      std::vector<int> ptr(size_t(L.S2) + 1, 0), term(Tnz.size());
+      std::vector<float2> val(Tnz.size());
+      for (const TermEntry &e : Tnz) ++ptr[size_t(e.idx % L.S2) + 1];
+      for (int e = 0; e < L.S2; ++e) ptr[size_t(e) + 1] += ptr[e];
+      {
+        std::vector<int> at(ptr.begin(), ptr.end() - 1);
+        for (const TermEntry &e : Tnz) {
+          const int x = at[e.idx % L.S2]++;
+          term[x] = e.idx / L.S2, val[x] = df_split(e.v);
         }
       }
-      ptr[L.S2] = int(term.size());
       // per block, its elements by descending term count (ties in element order): the
       // step's H build visits them in this order, so a warp's lanes walk similar lengths
       std::vector<int> order(size_t(L.S2), 0);
@@ -3085,8 +3216,8 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
           return ptr[bp + x + 1] - ptr[bp + x] > ptr[bp + y + 1] - ptr[bp + y];
         });
       }
-      J.tk_ptr.upload(ptr, st), J.tk_term.upload(term, st), J.tk_val.upload(val, st);
-      J.tk_order.upload(order, st);
+      up.add(J.tk_ptr, ptr), up.add(J.tk_term, term), up.add(J.tk_val, val);
+      up.add(J.tk_order, order);
     }
   }
   if (sched) {  // per chunk: the rf frame of each permuted index (1 where a chunk has none)
@@ -3099,25 +3230,76 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
         if (f.empty()) continue;
         for (int x = 0; x < N; ++x) fr[size_t(kc) * N + x] = make_double2(f[L.perm[x]].real(), f[L.perm[x]].imag());
       }
-      J.frames.upload(fr, st);
+      up.add(J.frames, fr);
     }
   }
-  J.ikind.upload(ikind, st);
-  J.Dblk.upload(Dblk, st), J.Rhoblk.upload(Rhoblk, st);
-  J.status.upload(std::vector<int>(1, 0), st);
-  // per-crystallite inputs, all batches, transposed to [item][c] per batch at run time
-  // (stored here already in batch-major, crystallite-fastest order)
+  up.add(J.ikind, ikind);
+  up.add(J.Dblk, Dblk), up.add(J.Rhoblk, Rhoblk);
+  // per-crystallite inputs, batch-major and crystallite-fastest: the powder angles (k_orient
+  // forms the rotations), start times and weights, expanded by the gamma loop
+  // (compute.h:294-306: fid summed over q)
   {
-    std::vector<double> Rp(size_t(J.nbatch) * 9 * J.Cb, 0.0), t0(size_t(J.nbatch) * J.Cb, 0.0),
-        w(size_t(J.nbatch) * J.Cb, 0.0);
-    for (int cg = 0; cg < J.Ceff; ++cg) {
-      int bi = cg / J.Cb, c = cg % J.Cb;
-      for (int x = 0; x < 9; ++x) Rp[(size_t(bi) * 9 + x) * J.Cb + c] = J.h_Rp[size_t(cg) * 9 + x];
-      t0[size_t(bi) * J.Cb + c] = J.h_t0[cg];
-      w[size_t(bi) * J.Cb + c] = J.h_w[cg];
-    }
-    J.Rp_all.upload(Rp, st), J.t0_all.upload(t0, st), J.w_all.upload(w, st);
+    const size_t all = size_t(J.nbatch) * J.Cb;
+    std::vector<double> ang(3 * all, 0.0), t0(all, 0.0), w(all, 0.0);
+    for (int c = 0; c < J.C; ++c)
+      for (int q = 0; q < J.gammaloop; ++q) {
+        const size_t cg = size_t(c) * J.gammaloop + q;  // batches are Cb apart: its own place too
+        ang[cg] = pw.phi[c], ang[all + cg] = pw.theta[c], ang[2 * all + cg] = pw.gamma[c];
+        t0[cg] = q == 0 ? tmin : tmin + kPi2 * double(q) / double(J.gammaloop * J.n) / p.wr;
+        w[cg] = pw.weight[c];
+      }
+    up.add(J.angles, ang), up.add(J.t0_all, t0), up.add(J.w_all, w);
   }
+  // FFT length of the Fave correlation: n itself when it is a power of two (twisted circular
+  // correlation; FP64 form only, its twist factors are FP64 work), else the power of two >= 2n
+  // (zero-padded linear correlation, the single-precision transforms of the mixed form)
+  DevSys &s = J.base;
+  if (!J.p2p) {
+    s.fave_twist = (!J.mixed && J.n >= 8 && (J.n & (J.n - 1)) == 0) ? 1 : 0;
+    s.logM = 1;
+    while ((1 << s.logM) < (s.fave_twist ? J.n : 2 * J.n)) ++s.logM;
+    s.M = 1 << s.logM;
+    // FFT correlation up to M = 4096 (its shared-memory tile is M * max(1, 2048/M) * 32 B)
+    if (p.fave_method == 2 && s.M > 4096) throw Error(5, "FFT Fave supports at most 2048 steps per period");
+    s.fave_method = (p.fave_method != 1 && s.M <= 4096) ? 1 : 0;
+    if (J.mixed && !s.fave_method) throw Error(5, "the mixed form needs the FFT correlation (at most 2048 steps)");
+    if (s.fave_method) {
+      std::vector<double2> tw(s.M / 2);
+      for (int k = 0; k < s.M / 2; ++k) {
+        double a = kPi2 * double(k) / double(s.M);
+        tw[k] = make_double2(std::cos(a), -std::sin(a));
+      }
+      if (J.mixed) {
+        std::vector<float2> twf(tw.size());
+        for (size_t k = 0; k < tw.size(); ++k) twf[k] = make_float2(float(tw[k].x), float(tw[k].y));
+        up.add(J.twf, twf);
+      } else {
+        up.add(J.tw, tw);
+      }
+    }
+  } else {  // no Fave: the point-to-point terms come from Q/R and the Floquet phases
+    s.fave_twist = 0, s.logM = 0, s.M = 0, s.fave_method = 0;
+  }
+  up.flush(ctx, J.tables, !g_arena || g_arena->aux_streams);
+  J.h2d = up.bytes();
+  s.tw = J.tw.p, s.twf = J.twf.p;
+  for (size_t t = 0; t < J.big_pairs.size(); ++t)
+    J.big_pairs[t].rp = J.big_rp.p + J.big_rp_off[t], J.big_pairs[t].ci = J.big_ci.p, J.big_pairs[t].cv = J.big_cv.p;
+  for (size_t t = 0; t < J.huge_pairs.size(); ++t)
+    J.huge_pairs[t].rp = J.big_rp.p + J.huge_rp_off[t], J.huge_pairs[t].ci = J.big_ci.p,
+    J.huge_pairs[t].cv = J.big_cv.p;
+  if (scatter) {
+    J.Tk.alloc(tk_n);
+    CUDA_OK(cudaMemsetAsync(J.Tk.p, 0, tk_n * sizeof(double), st));
+    if (df_tables) {
+      J.Tk_df.alloc(tk_n);
+      CUDA_OK(cudaMemsetAsync(J.Tk_df.p, 0, tk_n * sizeof(float2), st));
+    }
+    k_scatter_terms<<<grid_for(long(Tnz.size())), kThreads, 0, st>>>(J.tk_entries.p, int(Tnz.size()), J.Tk.p, J.Tk_df.p);
+  }
+  J.Rp_all.alloc(size_t(J.nbatch) * 9 * J.Cb);
+  k_orient<<<grid_for(long(J.nbatch) * J.Cb), kThreads, 0, st>>>(J.angles.p, J.nbatch * J.Cb, J.Cb, J.Rp_all.p);
+  CUDA_OK(cudaGetLastError());
   size_t Cb = J.Cb;
   J.U.alloc(std::max<size_t>(1, nsteps * L.S2 * Cb));
   J.A.alloc(std::max<size_t>(1, nsteps * L.S2 * Cb));
@@ -3140,9 +3322,11 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     J.hsq.alloc(size_t(J.huge_items));
     J.hsqmax.alloc(1);
   }
-  J.fid.alloc(p.npts);
+  // the FID, then the status word and the two tensor-flop counters: one read brings them all
+  J.fid.alloc(size_t(p.npts) + 2);
+  J.status.p = reinterpret_cast<int *>(J.fid.p + p.npts), J.status.n = 1, J.status.owned = false;
+  J.tcf.p = reinterpret_cast<unsigned long long *>(J.fid.p + p.npts + 1), J.tcf.n = 2, J.tcf.owned = false;
   if (use_fk) J.fkc.alloc(size_t(J.n) * J.nint * Cb);
-  J.tcf.alloc(2);
   if (J.tc && usl_per_c) {
     J.usl.alloc(usl_per_c * Cb);
     size_t off = 0;
@@ -3152,8 +3336,6 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
         off += nsteps * tc::slab_bytes(L.size[k]) * Cb;
       }
   }
-  CUDA_OK(cudaMemsetAsync(J.partial.p, 0, J.partial.n * sizeof(double2), st));
-  CUDA_OK(cudaStreamSynchronize(st));
   // algorithmic flop count (one complex MAC = 8 flop; eigh counted as 32 b^3, the
   // Floquet eig as 100 b^3)
   double S3 = 0;
@@ -3195,48 +3377,8 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   J.flops = 0;
   for (double f : J.stage_fl) J.flops += f;
   // static part of the device description
-  DevSys &s = J.base;
   s.n = J.n, s.npts = p.npts, s.N = N, s.nb = nb, s.S2 = L.S2, s.nint = J.nint, s.nq = J.nq, s.nr = J.nr;
   s.ne = J.ne, s.J = J.J, s.rosym = J.rosym, s.step_method = p.step_method;
-  // FFT length: n itself when it is a power of two (twisted circular correlation; FP64 form
-  // only, its twist factors are FP64 work), else the power of two >= 2n (zero-padded linear
-  // correlation, the single-precision transforms of the mixed form)
-  if (!J.p2p) {
-    s.fave_twist = (!J.mixed && J.n >= 8 && (J.n & (J.n - 1)) == 0) ? 1 : 0;
-    s.logM = 1;
-    while ((1 << s.logM) < (s.fave_twist ? J.n : 2 * J.n)) ++s.logM;
-    s.M = 1 << s.logM;
-    // FFT correlation up to M = 4096 (its shared-memory tile is M * max(1, 2048/M) * 32 B)
-    if (p.fave_method == 2 && s.M > 4096) throw Error(5, "FFT Fave supports at most 2048 steps per period");
-    s.fave_method = (p.fave_method != 1 && s.M <= 4096) ? 1 : 0;
-    if (J.mixed && !s.fave_method) throw Error(5, "the mixed form needs the FFT correlation (at most 2048 steps)");
-    {
-      std::vector<double2> tw(s.M / 2);
-      for (int k = 0; k < s.M / 2; ++k) {
-        double a = kPi2 * double(k) / double(s.M);
-        tw[k] = make_double2(std::cos(a), -std::sin(a));
-      }
-      std::vector<float2> twf(tw.size());
-      for (size_t k = 0; k < tw.size(); ++k) twf[k] = make_float2(float(tw[k].x), float(tw[k].y));
-      g_upload_counter = &J.h2d;
-      J.tw.upload(tw, st);
-      J.twf.upload(twf, st);
-      g_upload_counter = nullptr;
-      s.tw = J.tw.p;
-      s.twf = J.twf.p;
-      // one cap for every job (jobs on other threads launch these kernels concurrently): the
-      // largest M (4096, for 2048 steps) with its twist tables
-      const size_t shm_max = sizeof(double2) * 4096 * 2 + sizeof(double2) * 2 * (8 + 4096 / 8);
-      for (auto f : {k_fave_fft<8, double2>, k_fave_fft<4, double2>, k_fave_fft<2, double2>, k_fave_fft<1, double2>,
-                     k_fave_fft<8, float2>, k_fave_fft<4, float2>, k_fave_fft<2, float2>, k_fave_fft<1, float2>})
-        CUDA_OK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm_max)));
-    }
-    CUDA_OK(cudaFuncSetAttribute(k_fid_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(fid_tiled_smem(kFtJmax / 4, kFtThreads))));
-  } else {  // no Fave: the point-to-point terms come from Q/R and the Floquet phases
-    s.fave_twist = 0, s.logM = 0, s.M = 0, s.fave_method = 0;
-    s.tw = nullptr, s.twf = nullptr;
-  }
   s.tau = J.tau, s.wr = p.wr, s.sin_rotb = J.sin_rotb, s.cos_rotb = J.cos_rotb;
   s.is_static = J.is_static, s.dt = J.dt, s.srp = J.srp.p, s.seo = J.seo.p;
   s.scale = J.is_static ? 1.0 : double(1. / double(J.n / (J.rosym ? 2 : 1)));
@@ -3656,8 +3798,7 @@ void Job::run() {
     J.evpool.resize(size_t(2) * Job::kStages * (J.nbatch + 1));
     for (auto &e : J.evpool) CUDA_OK(cudaEventCreate(&e));
   }
-  CUDA_OK(cudaMemsetAsync(J.status.p, 0, sizeof(int), st));
-  CUDA_OK(cudaMemsetAsync(J.tcf.p, 0, 2 * sizeof(unsigned long long), st));
+  CUDA_OK(cudaMemsetAsync(J.status.p, 0, 2 * sizeof(double2), st));  // the status word and the tensor-flop counters
   for (int bi = 0; bi < J.nbatch; ++bi) {
     DevSys s = J.base;
     int c0 = bi * J.Cb;
@@ -3796,10 +3937,12 @@ static void mark_end(JobImpl &J, int stage, int nlaunch) {
 
 void Job::read(double *fid_out) {
   JobImpl &J = *d_;
-  CUDA_OK(cudaMemcpyAsync(fid_out, J.fid.p, sizeof(double2) * J.P.npts, cudaMemcpyDeviceToHost, J.ctx->stream));
-  int status = 0;
-  CUDA_OK(cudaMemcpyAsync(&status, J.status.p, sizeof(int), cudaMemcpyDeviceToHost, J.ctx->stream));
+  std::vector<double2> host(size_t(J.P.npts) + 1);  // the FID and the status word behind it
+  CUDA_OK(cudaMemcpyAsync(host.data(), J.fid.p, sizeof(double2) * host.size(), cudaMemcpyDeviceToHost, J.ctx->stream));
   CUDA_OK(cudaStreamSynchronize(J.ctx->stream));
+  std::memcpy(fid_out, host.data(), sizeof(double2) * J.P.npts);
+  int status = 0;
+  std::memcpy(&status, host.data() + J.P.npts, sizeof(int));
   if (status & (kNoConvergeStep | kNoConvergeFloquet))
     throw Error(7, "an eigen-decomposition did not converge within its sweep limit");
   if (status & kSingularCayley) throw Error(7, "singular Cayley transform in the Floquet eigen-decomposition");
@@ -4008,17 +4151,6 @@ static char *noalloc_base() {
   return static_cast<char *>(ptr);
 }
 
-// Device bytes outside the batch-sized work buffers: tables, per-crystallite inputs (11
-// doubles each, padded by up to one batch), warp partials and the FID.
-static size_t fixed_bytes(const Powder &pw, const FidParams &p) {
-  long n = p.wr != 0.0 ? long(std::floor(p.sw / p.wr + 0.5)) : 1;
-  long g = (n >= 1 && n <= 10) ? std::max(1L, 10 / n) : 1;
-  size_t ceff = size_t(pw.size()) * size_t(g) + 32;
-  // warp partials: up to kFtR rows per warp in the mixed form (k_fid_tiled's element ranges)
-  return (size_t(8) << 20) + 2 * ceff * 11 * sizeof(double) +
-         (ceff / 32 + 1) * size_t(p.precision == 1 ? kFtR : 1) * size_t(std::max(p.npts, 0)) * sizeof(double2);
-}
-
 void job_bytes(int device, const SpinSystem &sys, const Powder &pw, const CMatrix &ro, const CMatrix &det,
                const FidParams &p, size_t *min_bytes, size_t *full_bytes) {
   Context ctx;
@@ -4030,10 +4162,7 @@ void job_bytes(int device, const SpinSystem &sys, const Powder &pw, const CMatri
     ~Scope() { g_sizing = prev; }
   } scope(&plan);
   Job job(ctx, sys, pw, ro, det, p);
-  // work buffers are carved with 256-byte alignment: allow for it on each of ~40 buffers
-  size_t fixed = fixed_bytes(pw, p) + 40 * 256 + plan.extra + plan.tables;
-  if (min_bytes) *min_bytes = fixed + plan.per_c * 32;
-  if (full_bytes) *full_bytes = fixed + plan.per_c * size_t(plan.cpad);
+  planned_bytes(plan, pw, p, min_bytes, full_bytes);
 }
 
 void powder_fid_noalloc(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &ro, const CMatrix &det,
@@ -4063,8 +4192,10 @@ void powder_fid_noalloc(Context &ctx, const SpinSystem &sys, const Powder &pw, c
   arena.base = noalloc_base();
   arena.cap = kNoAllocScratch;
   Context view;  // same device and stream; budget = what the scratch leaves for work buffers
+  ready_kernels(ctx);
   view.device = ctx.device;
   view.stream = ctx.stream;
+  view.kernels_ready = true;
   view.hbm_budget = kNoAllocScratch - (fixed - plan.extra);  // the Job sets the workspace (extra) aside itself
   struct Release {
     Context &c;
@@ -4086,6 +4217,17 @@ void powder_fid_noalloc(Context &ctx, const SpinSystem &sys, const Powder &pw, c
                          " MiB static device scratch of the allocation-free entry point: " + e.what());
     throw;
   }
+}
+
+std::unique_ptr<Job> job_in_asked_region(Context &ctx, const RegionFn &region, const SpinSystem &sys, const Powder &pw,
+                                         const CMatrix &ro, const CMatrix &det, const FidParams &p) {
+  CUDA_OK(cudaSetDevice(ctx.device));
+  struct Scope {
+    const RegionFn *prev;
+    explicit Scope(const RegionFn *r) : prev(g_region) { g_region = r; }
+    ~Scope() { g_region = prev; }
+  } scope(&region);
+  return std::unique_ptr<Job>(new Job(ctx, sys, pw, ro, det, p));
 }
 
 // A resident Job whose every device buffer lives in [base, base + bytes): the serving loop

@@ -3,7 +3,9 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -42,6 +44,26 @@ struct Context {
   size_t hbm_budget = 0;  // bytes the engine may hold for one job's work buffers
                           // (0: 60% of the device memory free when the job is created)
   cudaStream_t stream = nullptr;
+  // Made by the first job that needs them and kept for the context's later jobs, which may be
+  // built and run from several threads: mu guards them while a job is built.
+  //   aux, join_ev, fork_ev  streams on which the large blocks of one stage run side by side
+  //                          (fork / join on the context stream); a later record of an event
+  //                          only makes its waits later, so jobs may share them
+  //   stage                  pinned buffer through which a job's inputs go up in one copy
+  //                          (at most kMaxStage bytes are kept; larger inputs go pageable);
+  //                          stage_ev marks the end of the last copy out of it
+  //   kernels_ready          the kernels' shared-memory limits are set on this device context
+  static constexpr size_t kMaxStage = size_t(16) << 20;
+  std::mutex mu;
+  std::vector<cudaStream_t> aux;
+  std::vector<cudaEvent_t> join_ev;
+  cudaEvent_t fork_ev = nullptr, stage_ev = nullptr;
+  void *stage = nullptr;
+  size_t stage_bytes = 0;
+  bool kernels_ready = false;
+  Context() {}
+  Context(const Context &) = delete;
+  Context &operator=(const Context &) = delete;
   ~Context();
 };
 
@@ -103,6 +125,13 @@ size_t noalloc_scratch_bytes();
 // *full_bytes with all crystallites in one batch.  Plans the job on the host only.
 void job_bytes(int device, const SpinSystem &sys, const Powder &pw, const CMatrix &ro, const CMatrix &det,
                const FidParams &p, size_t *min_bytes, size_t *full_bytes);
+
+// A Job whose device buffers are all carved from a region that `region` returns: it is asked
+// once, when the job is planned, with the bytes job_bytes would give, and answers with the base
+// and size of a region of at least *min* bytes, or a null base (the call then throws code 4).
+using RegionFn = std::function<void *(size_t min_bytes, size_t full_bytes, size_t *bytes)>;
+std::unique_ptr<Job> job_in_asked_region(Context &ctx, const RegionFn &region, const SpinSystem &sys, const Powder &pw,
+                                         const CMatrix &ro, const CMatrix &det, const FidParams &p);
 
 // A Job whose device buffers are all carved from [base, base + bytes) (no allocation).
 std::unique_ptr<Job> job_in_region(Context &ctx, void *base, size_t bytes, const SpinSystem &sys, const Powder &pw,

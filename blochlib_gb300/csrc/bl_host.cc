@@ -355,17 +355,23 @@ void SpinSystem::build() {
   size_t NN = size_t(N_) * N_;
   hc_.assign(NN, 0.0);
   hops_.clear();
+  hnz_.clear();
   hq4_.assign(ints_.size(), {});
   hq2_.assign(ints_.size(), {});
   const double inv_r3 = 1.0 / std::pow(3., 0.5), r3 = std::pow(3., 0.5);
   for (auto &it : ints_) {
     std::vector<double> T(NN, 0.0);
+    std::vector<NonZero> nz;
+    auto put = [&](long r, long c, double v) {
+      T[size_t(r) * N_ + c] = v;
+      if (v != 0.0) nz.push_back({int(r), int(c), v});
+    };
     if (it.kind == 'C') {
       // a*Iz + (1/sqrt3 Iz)(-sqrt3 iso)   (csa.cc:289-329, spin_ten.cc:211-236)
       const std::vector<double> Iz = iz_diag(it.s1);
       for (int k = 0; k < N_; ++k) {
         double z = Iz[k];
-        T[size_t(k) * N_ + k] = z;
+        put(k, k, z);
         if (it.iso != 0) hc_[size_t(k) * N_ + k] += (inv_r3 * z) * (-r3 * it.iso);
       }
     } else if (it.kind == 'D') {
@@ -373,12 +379,12 @@ void SpinSystem::build() {
       if (iso_[it.s1] == iso_[it.s2]) {
         double f = std::pow(1. / 6., 0.5);
         pair_terms(it.s1, it.s2, [&](long r, long c, double xx, double yy, double zz) {
-          T[size_t(r) * N_ + c] = f * (2.0 * zz - xx - yy);
+          put(r, c, f * (2.0 * zz - xx - yy));
         });
       } else {
         double f = std::pow(4. / 6., 0.5);
         pair_terms(it.s1, it.s2, [&](long r, long c, double, double, double zz) {
-          T[size_t(r) * N_ + c] = f * zz;
+          put(r, c, f * zz);
         });
       }
     } else if (it.kind == 'J') {
@@ -399,13 +405,14 @@ void SpinSystem::build() {
       const double q = spin;
       for (int k = 0; k < N_; ++k) {
         double z = Iz[k];
-        T[size_t(k) * N_ + k] = 3.0 * (z * z);
+        put(k, k, 3.0 * (z * z));
         // T_QuadTotal: Iz 2 (-8 Iz^2 - 1 + 4 I(I+1)) (rank 2), Iz 2 (-2 Iz^2 - 1 + 2 I(I+1)) (rank 4)
         hq2_[ki][size_t(k) * N_ + k] = (z * 2.0) * ((-8.0 * (z * z) - 1.0) + 4.0 * q * (q + 1));
         hq4_[ki][size_t(k) * N_ + k] = (z * 2.0) * ((-2.0 * (z * z) - 1.0) + 2.0 * q * (q + 1));
       }
     }
-    hops_.push_back(T);
+    hops_.push_back(std::move(T));
+    hnz_.push_back(std::move(nz));
   }
   // rf fields (PulseData::Pulse, pulsedata.cc:110-125): per isotope the sum of its fields
   // amp e^{i phase}; the real axis goes into hc_, a phase off it into the frame
@@ -475,18 +482,16 @@ void SpinSystem::build() {
     while (parent[x] != x) x = parent[x] = parent[parent[x]];
     return x;
   };
-  auto scan = [&](const std::vector<double> &M) {  // row by row: both triangles
-    for (int r = 0; r < N_; ++r) {
-      const double *row = M.data() + size_t(r) * N_;
-      for (int c = 0; c < N_; ++c)
-        if (c != r && row[c] != 0.0) {
-          int a = find(r), b = find(c);
-          if (a != b) parent[std::max(a, b)] = std::min(a, b);
-        }
-    }
+  auto link = [&](int r, int c) {
+    if (r == c) return;
+    const int a = find(r), b = find(c);
+    if (a != b) parent[std::max(a, b)] = std::min(a, b);
   };
-  scan(hc_);
-  for (auto &T : hops_) scan(T);
+  for (int r = 0; r < N_; ++r)
+    for (int c = 0; c < N_; ++c)
+      if (hc_[size_t(r) * N_ + c] != 0.0) link(r, c);
+  for (const auto &nz : hnz_)
+    for (const NonZero &e : nz) link(e.r, e.c);
   std::map<int, std::vector<int>> comps;
   for (int s = 0; s < N_; ++s) comps[find(s)].push_back(s);
   BlockLayout &L = layout_;

@@ -96,6 +96,13 @@ class SpinSystem {
   // orientation-dependent interaction (index matches interactions(); zero for J).
   const std::vector<double> &h_const() const { return hc_; }  // N*N real, row-major
   const std::vector<std::vector<double>> &h_ops() const { return hops_; }
+  // the non-zeros of each h_ops() matrix (Zeeman indices, row by row): a job packs its terms
+  // from these instead of walking the dense matrices
+  struct NonZero {
+    int r, c;
+    double v;
+  };
+  const std::vector<std::vector<NonZero>> &h_nonzeros() const { return hnz_; }
   // second-order quadrupolar spin operators of each quadrupole (empty for other kinds):
   // T_QuadTotal(rank 4) and (rank 2) of spin_ten.cc:364-375, both diagonal
   const std::vector<std::vector<double>> &h_ops_q4() const { return hq4_; }
@@ -126,6 +133,7 @@ class SpinSystem {
   std::vector<Interaction> ints_;
   std::vector<double> hc_;
   std::vector<std::vector<double>> hops_, hq4_, hq2_;
+  std::vector<std::vector<NonZero>> hnz_;
   double bfield_ = 0;
   std::vector<RfField> rf_;
   std::vector<cplx> frame_;
