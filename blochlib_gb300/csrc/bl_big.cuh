@@ -396,6 +396,7 @@ __global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_eigframe(DevSys s,
 // non-zeros of M_ab (D or rho) by row: row l holds entries [rp[l], rp[l+1]) of (ci, cv).
 struct BigPair {
   int a, b, off, nitems, isq, wchunk;
+  int e2;  // |M_ab W_b| <= 2^e2: the larger of M_ab's row and column sums
   const int *rp, *ci;
   const double2 *cv;
 };

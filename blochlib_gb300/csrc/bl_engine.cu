@@ -238,7 +238,7 @@ struct DevSys {
   int clay;
   // Segments of the Dyson products: nseg = ceil(n / kSegLen); blocks up to seg_max are segmented
   // (none when nseg == 1).  See seg_E.
-  int nseg, seg_max;
+  int nseg, seg_max, seg_from;  // (and blocks from seg_from on, the batched-product path's)
 };
 
 // Precision-dependent arrays: W (eigenframe; in place over A in FP64), Q, R, G, Z, twiddles.
@@ -530,10 +530,11 @@ __device__ __forceinline__ size_t at(int item, int c, int Cpad) { return size_t(
 // n = 128, FP64 1.83 -> 1.33 and 1.14 -> 1.23 ms (the latter FP64-issue bound before too); one
 // 3-spin crystallite, n = 64, Dyson 0.151 -> 0.061 ms.
 // E_s and V_s live in the U buffer, which is dead once a block's segments are done: E_{s+1} in
-// the slots of step s (the same block's items), V_s as float2 (mixed form) from step nseg + s;
-// the FP64 form writes V_s over E_s.
+// the slots of step s (the same block's items), V_s as float2 (mixed form) from step nseg + s, or
+// over E_s in the FP64 form; the batched-product path (bl_huge.cuh) keeps V_s as FP64 from step
+// 2 nseg + s (3 nseg <= n).
 constexpr int kSegLen = 16;
-__device__ __forceinline__ bool segmented(const DevSys &s, int b) { return b <= s.seg_max; }
+__device__ __forceinline__ bool segmented(const DevSys &s, int b) { return b <= s.seg_max || b >= s.seg_from; }
 __device__ __forceinline__ double2 *seg_E(const DevSys &s, int t) { return s.U + size_t(t) * s.S2 * s.Cpad; }
 __device__ __forceinline__ float2 *seg_Vf(const DevSys &s, int t) {
   return reinterpret_cast<float2 *>(s.U + size_t(s.nseg + t) * s.S2 * s.Cpad);
@@ -2149,6 +2150,7 @@ static size_t fave_twist_bytes(const DevSys &s, int cg) {
 #include "bl_big.cuh"
 #include "bl_huge.cuh"
 #include "bl_tc.cuh"
+#include "bl_xs.cuh"
 
 // FID terms of the FP64 form: fid[j gper + p] = sum_c w_c sum_e z_e^j G_p(e).  The FP64 pipe
 // bounds it, so the j's are taken in pairs about the middle of their range: with G' = w z^((J-1)/2) G
@@ -2596,8 +2598,8 @@ struct JobImpl {
   size_t huge_ws_bytes = 0;                      // workspace of the huge-block products
   int huge_items = 0;                            // largest chunk of exponential items
   DevBuf<double2> huge_ws;
-  DevBuf<double> hfk, hsc;
-  DevBuf<int> hsq, hsqmax;
+  DevBuf<double> hfk;
+  DevBuf<int> hsq;
   std::vector<size_t> big_rp_off, huge_rp_off;   // each pair's row pointers in big_rp
   DevBuf<int> big_rp, big_ci;                    // non-zeros of M_ab by row, all big pairs
   DevBuf<double2> big_cv;
@@ -2710,7 +2712,9 @@ static void ready_kernels(Context &ctx) {
         (const void *)k_big_qr<2, double2>, (const void *)k_fave_fft<8, double2>, (const void *)k_fave_fft<4, double2>,
         (const void *)k_fave_fft<2, double2>, (const void *)k_fave_fft<1, double2>, (const void *)k_fave_fft<8, float2>,
         (const void *)k_fave_fft<4, float2>, (const void *)k_fave_fft<2, float2>, (const void *)k_fave_fft<1, float2>,
-        (const void *)k_fid_tiled})
+        (const void *)k_fid_tiled, (const void *)k_xs_gemm<true, 6, false, double2>,
+        (const void *)k_xs_gemm<true, 7, false, double2>, (const void *)k_xs_gemm<true, 7, true, double2>,
+        (const void *)k_xs_gemm<false, 6, false, double>, (const void *)k_xs_gemm<false, 7, false, double>})
     all(f);
   ctx.kernels_ready = true;
 }
@@ -3130,7 +3134,20 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
         if (csz * (size_t(ba) * ba + size_t(bb + ba) * w) <= (size_t(113) << 10) || w <= 8) break;
         ++nch;
       }
-      BigPair P{a, b, isq ? qoff[pr] : roff[pr - J.npq], isq ? J.nq : J.nr, isq ? 1 : 0, w, nullptr, nullptr, nullptr};
+      double most = 1e-300;  // largest row or column sum of |M_ab|
+      std::vector<double> col(bb, 0.0);
+      for (int l = 0; l < ba; ++l) {
+        double row = 0;
+        for (int m = 0; m < bb; ++m) {
+          const double v = std::hypot(M[l * bb + m].x, M[l * bb + m].y);
+          row += v, col[m] += v;
+        }
+        most = std::max(most, row);
+      }
+      for (double v : col) most = std::max(most, v);
+      int e2 = 0;
+      std::frexp(most, &e2);  // most < 2^e2
+      BigPair P{a, b, isq ? qoff[pr] : roff[pr - J.npq], isq ? J.nq : J.nr, isq ? 1 : 0, w, e2, nullptr, nullptr, nullptr};
       if (std::max(ba, bb) > kMaxBigBlock) {  // k_huge_mx + k_huge_zgemm
         J.huge_pairs.push_back(P);
         J.huge_rp_off.push_back(rp_off);
@@ -3318,9 +3335,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   if (J.huge_ws_bytes) {
     J.huge_ws.alloc(J.huge_ws_bytes / sizeof(double2));
     J.hfk.alloc(size_t(J.huge_items) * std::max(J.nint, 1));
-    J.hsc.alloc(size_t(J.huge_items));
     J.hsq.alloc(size_t(J.huge_items));
-    J.hsqmax.alloc(1);
   }
   // the FID, then the status word and the two tensor-flop counters: one read brings them all
   J.fid.alloc(size_t(p.npts) + 2);
@@ -3426,6 +3441,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   // the tensor-core blocks (mixed form) keep one chain per crystallite
   s.nseg = J.is_static ? 1 : (J.n + kSegLen - 1) / kSegLen;
   s.seg_max = s.nseg > 1 ? (J.tc ? tc::kMinB - 1 : kMaxBigBlock) : 0;
+  s.seg_from = s.nseg > 1 ? kMaxBigBlock + 1 : 1 << 30;
 }
 
 Job::~Job() {}
@@ -3514,6 +3530,34 @@ static HMat<T> ws_mat(T *p, long j0, long mat, int C, int ld) {
 }
 static unsigned tiles(int m, int n) { return unsigned(((m + kHT - 1) / kHT) * ((n + kHT - 1) / kHT)); }
 
+// Products O = op(A) B of `items` items from j0 on: exact digit slices on the tensor cores
+// (bl_xs.cuh) where their sums stay exact (K' = 2k <= 512 digits; the mixed form, which needs
+// 2^-44, always), else FP64 tiles.  |A| <= 2^ea, |B| <= 2^eb.
+static void huge_mm(JobImpl &J, const DevSys &s, cudaStream_t st, bool conjA, HMat<const double2> A,
+                    HMat<const double2> B, HMat<double2> O, int m, int n, int k, int Cb, long j0, int items, int ea,
+                    int eb) {
+  const unsigned tx = unsigned(((m + 63) / 64) * ((n + xs::kN - 1) / xs::kN));
+  const XsReal none{};
+  if (s.mixed) {
+    k_xs_gemm<true, 6, false, double2><<<dim3(tx, unsigned(items)), xs::kThreadsXs, xs::smem<6>(), st>>>(
+        A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
+  } else if (2 * k <= 512) {
+    if (conjA)
+      k_xs_gemm<true, 7, true, double2><<<dim3(tx, unsigned(items)), xs::kThreadsXs, xs::smem<7>(), st>>>(
+          A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
+    else
+      k_xs_gemm<true, 7, false, double2><<<dim3(tx, unsigned(items)), xs::kThreadsXs, xs::smem<7>(), st>>>(
+          A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
+  } else if (conjA) {
+    k_huge_zgemm<double2, true, double2, double2, double2>
+        <<<dim3(tiles(m, n), unsigned(items)), kHThreads, 0, st>>>(A, B, O, m, n, k, Cb, j0, 1.0);
+  } else {
+    k_huge_zgemm<double2, false, double2, double2, double2>
+        <<<dim3(tiles(m, n), unsigned(items)), kHThreads, 0, st>>>(A, B, O, m, n, k, Cb, j0, 1.0);
+  }
+  ++J.launches;
+}
+
 // U_i of huge block k for every (crystallite, step): symmetric Paterson-Stockmeyer.
 static void huge_step(JobImpl &J, DevSys &s, size_t kh) {
   const int k = J.huge_blocks[kh], b = J.L.size[k], bp = J.L.poff[k];
@@ -3522,38 +3566,51 @@ static void huge_step(JobImpl &J, DevSys &s, size_t kh) {
   cudaStream_t st = J.ctx->stream;
   double *ws = reinterpret_cast<double *>(J.huge_ws.p);
   const unsigned ge = unsigned((bb + 255) / 256), tm = unsigned((b + kHT - 1) / kHT), gs = tm * (tm + 1) / 2;
+  const unsigned gx = unsigned(((b + 127) / 128) * ((b + xs::kN - 1) / xs::kN));
   for (long j0 = 0; j0 < total; j0 += per) {
     const int items = int(std::min(per, total - j0));
-    auto sym = [&](int a, int bsl, int o, int akind, double alpha, int round, bool low, double c0, double c1,
-                   double c2, double c3) {
-      SymArgs g{ws, J.hsc.p, J.hsq.p, bb, b, a, bsl, o, akind, alpha, round, low ? 1 : 0, c0, c1, c2, c3};
-      if (s.mixed) k_huge_sym_df<<<dim3(gs, unsigned(items)), kHThreads, 0, st>>>(g);
-      else k_huge_sym<<<dim3(gs, unsigned(items)), kHThreads, 0, st>>>(g);
+    auto sym = [&](int a, int bsl, int o, double alpha, int round, bool low, double c0, double c1, double c2,
+                   double c3) {
+      if (s.mixed || b <= 512) {
+        const long cs = kHugeSlots * bb;
+        const HMat<const double> A{ws + a * bb, 0, 0, b, 1, cs}, B{ws + bsl * bb, 0, 0, b, 1, cs};
+        const HMat<double> O{ws + o * bb, 0, 0, b, 1, cs};
+        const XsReal ep{low ? 1 : 0, alpha, c0, c1, c2, c3, ws + bb, ws + 2 * bb, ws + 3 * bb,
+                        round >= 0 ? J.hsq.p : nullptr, round};
+        if (s.mixed)
+          k_xs_gemm<false, 6, false, double><<<dim3(gx, unsigned(items)), xs::kThreadsXs, xs::smem<6>(), st>>>(
+              A, B, O, b, b, b, 1 << 30, 0, 0, 0, ep, s.status);
+        else
+          k_xs_gemm<false, 7, false, double><<<dim3(gx, unsigned(items)), xs::kThreadsXs, xs::smem<7>(), st>>>(
+              A, B, O, b, b, b, 1 << 30, 0, 0, 0, ep, s.status);
+      } else {
+        SymArgs g{ws, J.hsq.p, bb, b, a, bsl, o, alpha, round, low ? 1 : 0, c0, c1, c2, c3};
+        k_huge_sym<<<dim3(gs, unsigned(items)), kHThreads, 0, st>>>(g);
+      }
       ++J.launches;
     };
     k_huge_fk<<<unsigned((items + 127) / 128), 128, 0, st>>>(s, j0, items, J.hfk.p);
     k_huge_hbuild<<<dim3(ge, unsigned(items)), 256, 0, st>>>(s, bp, b, J.hfk.p, ws, j0);
-    CUDA_OK(cudaMemsetAsync(J.hsqmax.p, 0, sizeof(int), st));
-    k_huge_norm<<<unsigned(items), 256, 0, st>>>(ws, b, s.tau * kPi2, J.hsc.p, J.hsq.p, J.hsqmax.p);
+    k_huge_norm<<<unsigned(items), 256, 0, st>>>(ws, b, s.tau * kPi2, J.hsq.p);
     J.launches += 3;
-    sym(0, 0, 1, 1, 1.0, -1, false, 0, 0, 0, 0);  // Y = sc^2 H H
-    sym(1, 1, 2, 0, 1.0, -1, false, 0, 0, 0, 0);  // Y^2
-    sym(2, 1, 3, 0, 1.0, -1, false, 0, 0, 0, 0);  // Y^3
-    sym(2, 2, 4, 0, 1.0, -1, false, 0, 0, 0, 0);  // Y^4
+    sym(0, 0, 1, 1.0, -1, false, 0, 0, 0, 0);  // Y = X X
+    sym(1, 1, 2, 1.0, -1, false, 0, 0, 0, 0);  // Y^2
+    sym(2, 1, 3, 1.0, -1, false, 0, 0, 0, 0);  // Y^3
+    sym(2, 2, 4, 1.0, -1, false, 0, 0, 0, 0);  // Y^4
     // cos X = C(Y), coefficients (-1)^j/(2j)!;  sin X = X S(Y), (-1)^j/(2j+1)!
     k_huge_low<<<dim3(ge, unsigned(items)), 256, 0, st>>>(ws, b, 1.0 / 40320, -1.0 / 3628800, 1.0 / 479001600,
                                                           -1.0 / 87178291200.0);
-    sym(4, 5, 6, 0, 1.0, -1, true, 1.0, -1.0 / 2, 1.0 / 24, -1.0 / 720);  // R = cos X
+    sym(4, 5, 6, 1.0, -1, true, 1.0, -1.0 / 2, 1.0 / 24, -1.0 / 720);  // R = cos X
     k_huge_low<<<dim3(ge, unsigned(items)), 256, 0, st>>>(ws, b, 1.0 / 362880, -1.0 / 39916800,
                                                           1.0 / 6227020800.0, -1.0 / 1307674368000.0);
-    sym(4, 5, 3, 0, 1.0, -1, true, 1.0, -1.0 / 6, 1.0 / 120, -1.0 / 5040);  // S(Y) over Y^3
-    sym(0, 3, 1, 2, 1.0, -1, false, 0, 0, 0, 0);                            // I = -sc H S
+    sym(4, 5, 3, 1.0, -1, true, 1.0, -1.0 / 6, 1.0 / 120, -1.0 / 5040);  // S(Y) over Y^3
+    sym(0, 3, 1, -1.0, -1, false, 0, 0, 0, 0);                           // I = -X S
     J.launches += 2;
     // squarings: the host bound for the block; each item skips the rounds it does not need
     for (int t = 0; t < J.huge_sq[kh]; ++t) {
-      sym(6, 6, 2, 0, 1.0, t, false, 0, 0, 0, 0);
-      sym(1, 1, 4, 0, 1.0, t, false, 0, 0, 0, 0);
-      sym(6, 1, 5, 0, 2.0, t, false, 0, 0, 0, 0);
+      sym(6, 6, 2, 1.0, t, false, 0, 0, 0, 0);
+      sym(1, 1, 4, 1.0, t, false, 0, 0, 0, 0);
+      sym(6, 1, 5, 2.0, t, false, 0, 0, 0, 0);
       k_huge_sqcomb<<<dim3(ge, unsigned(items)), 256, 0, st>>>(ws, b, J.hsq.p, t);
       ++J.launches;
     }
@@ -3562,24 +3619,32 @@ static void huge_step(JobImpl &J, DevSys &s, size_t kh) {
   }
 }
 
-// A_{i+1} = U_i A_i for huge block k, one product launch per step.
+// The segments' products P_i = U_i P_{i-1} of huge block k (step t of every segment in one
+// launch), then the chain E_{s+1} = P_last(s) E_s; without segments the one chain of all steps.
 static void huge_dyson(JobImpl &J, DevSys &s, size_t kh) {
-  const int k = J.huge_blocks[kh], b = J.L.size[k], bp = J.L.poff[k];
-  const long bb = long(b) * b;
+  const int k = J.huge_blocks[kh], b = J.L.size[k], bp = J.L.poff[k], n = J.n;
+  const unsigned ge = unsigned((long(b) * b + 255) / 256);
+  const int len = s.nseg > 1 ? kSegLen : n;
   cudaStream_t st = J.ctx->stream;
-  k_huge_copy_u0<<<dim3(unsigned((bb + 255) / 256), unsigned(s.C)), 256, 0, st>>>(s, bp, b);
+  const size_t step = size_t(s.S2) * s.Cpad;
+  k_huge_copy<<<dim3(ge, unsigned(s.C), unsigned(s.nseg)), 256, 0, st>>>(s, s.U, s.A, 0, 0, len, bp, b);
   ++J.launches;
-  const auto U = item_mat<const double2>(s.U, bp, s.S2, b, s.Cpad);
-  const auto Ain = item_mat<const double2>(s.A, long(bp) - s.S2, s.S2, b, s.Cpad);
-  const auto Aout = item_mat<double2>(s.A, bp, s.S2, b, s.Cpad);
-  for (int i = 1; i < J.n; ++i) {
-    if (s.mixed)  // double-float products, FP64 storage
-      k_huge_zgemm_df<<<dim3(tiles(b, b), unsigned(s.C)), kHThreads, 0, st>>>(U, Ain, Aout, b, b, b, s.C,
-                                                                              long(i) * s.C, 1.0);
-    else
-      k_huge_zgemm<double2, false, double2, double2, double2>
-          <<<dim3(tiles(b, b), unsigned(s.C)), kHThreads, 0, st>>>(U, Ain, Aout, b, b, b, s.C, long(i) * s.C, 1.0);
-    ++J.launches;
+  for (int t = 1; t < len; ++t) {
+    const int segs = (n - t + len - 1) / len;  // segments that have a step t
+    const auto U = item_mat<const double2>(s.U + t * step, bp, long(len) * s.S2, b, s.Cpad);
+    const auto Ain = item_mat<const double2>(s.A + (t - 1) * step, bp, long(len) * s.S2, b, s.Cpad);
+    const auto Aout = item_mat<double2>(s.A + t * step, bp, long(len) * s.S2, b, s.Cpad);
+    for (int g0 = 0; g0 < segs * s.C; g0 += kHugeMaxItems)
+      huge_mm(J, s, st, false, U, Ain, Aout, b, b, b, s.C, g0, std::min(kHugeMaxItems, segs * s.C - g0), 0, 0);
+  }
+  if (s.nseg <= 1) return;
+  k_huge_copy<<<dim3(ge, unsigned(s.C), 1), 256, 0, st>>>(s, s.A, s.U, std::min(len, n) - 1, 0, 0, bp, b);
+  ++J.launches;
+  for (int t = 1; t < s.nseg; ++t) {
+    const auto P = item_mat<const double2>(s.A + (std::min((t + 1) * len, n) - 1) * step, bp, 0, b, s.Cpad);
+    const auto Ein = item_mat<const double2>(s.U + (t - 1) * step, bp, 0, b, s.Cpad);
+    const auto Eout = item_mat<double2>(s.U + t * step, bp, 0, b, s.Cpad);
+    huge_mm(J, s, st, false, P, Ein, Eout, b, b, b, s.C, 0, s.C, 0, 0);
   }
 }
 
@@ -3614,32 +3679,47 @@ static void huge_floquet_all(JobImpl &J, DevSys &s) {
   }
 }
 
-// W_i = A_{i+1} V_F for huge block k: straight into W in the mixed form; through the
-// workspace and back over A in FP64 (a product may not overwrite its own operand).
+// W_i = A_{i+1} V_F = P_i V_s for huge block k, segment by segment (V_s = E_s V_F first):
+// straight into W in the mixed form; through the workspace and back over A in FP64 (a product
+// may not overwrite its own operand).
 static void huge_eigframe(JobImpl &J, DevSys &s, size_t kh) {
   const int k = J.huge_blocks[kh], b = J.L.size[k], bp = J.L.poff[k];
-  const long bb = long(b) * b, total = long(s.C) * J.n;
+  const long bb = long(b) * b;
   cudaStream_t st = J.ctx->stream;
-  const auto A = item_mat<const double2>(s.A, bp, s.S2, b, s.Cpad);
-  const auto V = item_mat<const double2>(s.VF, bp, 0, b, s.Cpad);
-  if (s.mixed) {
-    const auto W = item_mat<float2>(s.Wf, bp, s.S2, b, s.Cpad);
-    for (long j0 = 0; j0 < total; j0 += kHugeMaxItems) {
-      const int items = int(std::min<long>(kHugeMaxItems, total - j0));
-      k_huge_zgemm<float2, false, double2, double2, float2>
-          <<<dim3(tiles(b, b), unsigned(items)), kHThreads, 0, st>>>(A, V, W, b, b, b, s.C, j0, 1.0);
+  const size_t step = size_t(s.S2) * s.Cpad;
+  double2 *Vseg = s.U + size_t(2 * s.nseg) * step;  // V_s at step slot 2 nseg + s
+  if (s.nseg > 1) {
+    const auto E = item_mat<const double2>(s.U, bp, s.S2, b, s.Cpad);  // E_{sl+1}
+    const auto V = item_mat<const double2>(s.VF, bp, 0, b, s.Cpad);
+    const auto O = item_mat<double2>(Vseg + step, bp, s.S2, b, s.Cpad);
+    const int items = s.C * (s.nseg - 1);
+    for (int g0 = 0; g0 < items; g0 += kHugeMaxItems)
+      huge_mm(J, s, st, false, E, V, O, b, b, b, s.C, g0, std::min(kHugeMaxItems, items - g0), 0, 0);
+  }
+  const int len = s.nseg > 1 ? kSegLen : J.n;
+  for (int seg = 0; seg < s.nseg; ++seg) {
+    const int i0 = seg * len, i1 = std::min(J.n, i0 + len);
+    const auto V = item_mat<const double2>(seg ? Vseg + seg * step : s.VF, bp, 0, b, s.Cpad);
+    const auto A = item_mat<const double2>(s.A, bp, s.S2, b, s.Cpad);
+    const long total = long(s.C) * i1;
+    if (s.mixed) {
+      const auto W = item_mat<float2>(s.Wf, bp, s.S2, b, s.Cpad);
+      for (long j0 = long(s.C) * i0; j0 < total; j0 += kHugeMaxItems) {
+        const int items = int(std::min<long>(kHugeMaxItems, total - j0));
+        k_huge_zgemm<float2, false, double2, double2, float2>
+            <<<dim3(tiles(b, b), unsigned(items)), kHThreads, 0, st>>>(A, V, W, b, b, b, s.C, j0, 1.0);
+        ++J.launches;
+      }
+      continue;
+    }
+    const long per = std::min<long>(kHugeMaxItems, long(J.huge_ws_bytes / (sizeof(double2) * bb)));
+    for (long j0 = long(s.C) * i0; j0 < total; j0 += per) {
+      const int items = int(std::min(per, total - j0));
+      const auto O = ws_mat<double2>(J.huge_ws.p, j0, bb, s.C, b);
+      huge_mm(J, s, st, false, A, V, O, b, b, b, s.C, j0, items, 0, 0);
+      k_huge_copy_back<<<dim3(unsigned((bb + 255) / 256), unsigned(items)), 256, 0, st>>>(s, J.huge_ws.p, bp, b, j0);
       ++J.launches;
     }
-    return;
-  }
-  const long per = std::min<long>(kHugeMaxItems, long(J.huge_ws_bytes / (sizeof(double2) * bb)));
-  for (long j0 = 0; j0 < total; j0 += per) {
-    const int items = int(std::min(per, total - j0));
-    const auto O = ws_mat<double2>(J.huge_ws.p, j0, bb, s.C, b);
-    k_huge_zgemm<double2, false, double2, double2, double2>
-        <<<dim3(tiles(b, b), unsigned(items)), kHThreads, 0, st>>>(A, V, O, b, b, b, s.C, j0, 1.0);
-    k_huge_copy_back<<<dim3(unsigned((bb + 255) / 256), unsigned(items)), 256, 0, st>>>(s, J.huge_ws.p, bp, b, j0);
-    J.launches += 2;
   }
 }
 
@@ -3657,9 +3737,14 @@ static void huge_qr(JobImpl &J, DevSys &s, const BigPair &P, C *Wbuf, C *out) {
     const int items = int(std::min(per, total - j0));
     k_huge_mx<C><<<dim3(unsigned((ne + 255) / 256), unsigned(items)), 256, 0, st>>>(s, P, j0, ws);
     const auto X = ws_mat<const C>(ws, j0, ne, s.C, bb);
-    k_huge_zgemm<C, true, C, C, C><<<dim3(tiles(ba, bb), unsigned(items)), kHThreads, 0, st>>>(Wa, X, O, ba, bb, ba,
-                                                                                             s.C, j0, 1.0);
-    J.launches += 2;
+    ++J.launches;
+    if constexpr (std::is_same<C, double2>::value) {
+      huge_mm(J, s, st, true, Wa, X, O, ba, bb, ba, s.C, j0, items, 0, P.e2);
+    } else {
+      k_huge_zgemm<C, true, C, C, C><<<dim3(tiles(ba, bb), unsigned(items)), kHThreads, 0, st>>>(Wa, X, O, ba, bb, ba,
+                                                                                               s.C, j0, 1.0);
+      ++J.launches;
+    }
   }
 }
 

@@ -9,7 +9,8 @@
 //   step       k_huge_fk, k_huge_hbuild, k_huge_norm, k_huge_sym x 7, k_huge_low, squarings,
 //              k_huge_store_u: the same symmetric Paterson-Stockmeyer exponential as
 //              k_big_step, over a chunk of (crystallite, step) items at a time
-//   Dyson      k_huge_zgemm per step (A_{i+1} = U_i A_i), A_1 = U_0 by k_huge_copy_u0
+//   Dyson      products per step of all segments at once (A_{i+1} = U_i A_i), then the chain over
+//              the segments' last products; k_huge_copy starts each
 //   Floquet    k_huge_floquet: floquet_cta with its two b x b matrices in global memory
 //   eigenframe k_huge_zgemm (A_{i+1} V_F) into the workspace, copied back in FP64
 //   Q/R        k_huge_mx (X = M_ab W_b from M's non-zeros) and k_huge_zgemm (W_a^H X)
@@ -91,70 +92,20 @@ __global__ void __launch_bounds__(kHThreads) k_huge_zgemm(HMat<const TA> A, HMat
     }
 }
 
-// The mixed form's Dyson product for huge blocks: O = alpha A B (FP64 storage, as
-// k_huge_zgemm<double2>) with double-float arithmetic on the FP32 pipe: operands split into
-// hi + lo floats as they are staged, each output a compensated complex dot product (cdf_mac),
-// rounded to FP64 once at the end (~2^-44 relative against FP64's 2^-53).
-__global__ void __launch_bounds__(kHThreads) k_huge_zgemm_df(HMat<const double2> A, HMat<const double2> B,
-                                                            HMat<double2> O, int m, int n, int k, int Cb, long j0,
-                                                            double alpha) {
-  __shared__ float4 As[kHK][kHT + 1], Bs[kHK][kHT + 1];
-  const long g = j0 + blockIdx.y;
-  const int c = int(g % Cb), sl = int(g / Cb);
-  const int tn = (n + kHT - 1) / kHT;
-  const int r0 = (blockIdx.x / tn) * kHT, q0 = (blockIdx.x % tn) * kHT;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  CdfAcc acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = CdfAcc{{0.f, 0.f}, {0.f, 0.f}};
-  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int k0 = 0; k0 < k; k0 += kHK) {
-    for (int idx = threadIdx.x; idx < kHT * kHK; idx += kHThreads) {
-      const int rr = idx / kHK, kk = idx % kHK, r = r0 + rr, l = k0 + kk;
-      As[kk][rr] = (r < m && l < k) ? df_store(A(c, sl, r, l)) : z4;
-      const int kb = idx / kHT, qq = idx % kHT, lb = k0 + kb, q = q0 + qq;
-      Bs[kb][qq] = (lb < k && q < n) ? df_store(B(c, sl, lb, q)) : z4;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < kHK; ++kk) {
-      float4 a[4], b[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) a[t] = As[kk][ty + 16 * t], b[t] = Bs[kk][tx + 16 * t];
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) cdf_mac(acc[x][y], a[x], b[y]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int y = 0; y < 4; ++y) {
-      const int r = r0 + ty + 16 * x, q = q0 + tx + 16 * y;
-      if (r < m && q < n) O(c, sl, r, q) = cscale(df_load(cdf_fin(acc[x][y])), alpha);
-    }
-}
-
 // Arguments of k_huge_sym: workspace of kHugeSlots real b x b matrices per item (slot t of
-// item j at ws + (j*kHugeSlots + t)*bb) and per-item scale sc_j = 2 pi tau 2^-sq_j.
+// item j at ws + (j*kHugeSlots + t)*bb).
 struct SymArgs {
   double *ws;
-  const double *sc;
   const int *sq;
   long bb;
   int b, a, bsl, o;  // operand and output slots
-  int akind;         // alpha: 0 -> alpha, 1 -> sc_j^2, 2 -> -sc_j
   double alpha;
   int round;         // >= 0: squaring round, items with sq_j <= round are skipped
   int low;           // epilogue adds c0 I + c1 Y + c2 Y2 + c3 Y3 (slots 1, 2, 3)
   double c0, c1, c2, c3;
 };
 
-// O = alpha_j A B (+ low terms) for commuting real symmetric A, B of item j (blockIdx.y):
+// O = alpha A B (+ low terms) for commuting real symmetric A, B of item j (blockIdx.y):
 // upper-triangle tiles only, each value stored at (r, q) and (q, r).  The low terms are read
 // at the upper element only, so S may overwrite Y3 in place.
 __global__ void __launch_bounds__(kHThreads) k_huge_sym(SymArgs g) {
@@ -169,8 +120,7 @@ __global__ void __launch_bounds__(kHThreads) k_huge_sym(SymArgs g) {
   const double *A = base + g.a * g.bb, *B = base + g.bsl * g.bb;
   double *O = base + g.o * g.bb;
   const double *Y = base + g.bb, *Y2 = base + 2 * g.bb, *Y3 = base + 3 * g.bb;
-  const double scj = g.sc[j];
-  const double alpha = g.akind == 0 ? g.alpha : (g.akind == 1 ? scj * scj : -scj);
+  const double alpha = g.alpha;
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
   double acc[4][4];
 #pragma unroll
@@ -211,65 +161,6 @@ __global__ void __launch_bounds__(kHThreads) k_huge_sym(SymArgs g) {
     }
 }
 
-// k_huge_sym with double-float arithmetic (the mixed form): FP64 workspace, operands split
-// into hi + lo floats as they are staged, compensated dot products, the FP64 epilogue of
-// k_huge_sym (scale, low terms, mirrored store).
-__global__ void __launch_bounds__(kHThreads) k_huge_sym_df(SymArgs g) {
-  __shared__ float2 As[kHK][kHT + 1], Bs[kHK][kHT + 1];
-  const int j = blockIdx.y;
-  if (g.round >= 0 && g.sq[j] <= g.round) return;
-  const int b = g.b, tm = (b + kHT - 1) / kHT;
-  int ti, tj;
-  sym_tile(blockIdx.x, tm, ti, tj);
-  const int r0 = ti * kHT, q0 = tj * kHT;
-  double *base = g.ws + long(j) * kHugeSlots * g.bb;
-  const double *A = base + g.a * g.bb, *B = base + g.bsl * g.bb;
-  double *O = base + g.o * g.bb;
-  const double *Y = base + g.bb, *Y2 = base + 2 * g.bb, *Y3 = base + 3 * g.bb;
-  const double scj = g.sc[j];
-  const double alpha = g.akind == 0 ? g.alpha : (g.akind == 1 ? scj * scj : -scj);
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  DfAcc acc[4][4];
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int y = 0; y < 4; ++y) acc[x][y] = DfAcc{0.f, 0.f};
-  const float2 z2 = make_float2(0.f, 0.f);
-  for (int k0 = 0; k0 < b; k0 += kHK) {
-    for (int idx = threadIdx.x; idx < kHT * kHK; idx += kHThreads) {
-      const int rr = idx / kHK, kk = idx % kHK, r = r0 + rr, l = k0 + kk;
-      As[kk][rr] = (r < b && l < b) ? dfv_of(A[long(r) * b + l]) : z2;
-      const int kb = idx / kHT, qq = idx % kHT, lb = k0 + kb, q = q0 + qq;
-      Bs[kb][qq] = (lb < b && q < b) ? dfv_of(B[long(lb) * b + q]) : z2;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < kHK; ++kk) {
-      float2 a[4], bv[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) a[t] = As[kk][ty + 16 * t], bv[t] = Bs[kk][tx + 16 * t];
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) df_dot(acc[x][y], a[x].x, a[x].y, bv[y].x, bv[y].y);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int x = 0; x < 4; ++x)
-#pragma unroll
-    for (int y = 0; y < 4; ++y) {
-      const int r = r0 + ty + 16 * x, q = q0 + tx + 16 * y;
-      if (r >= b || q >= b || r > q) continue;  // upper triangle (r > q only on diagonal tiles)
-      const long e = long(r) * b + q;
-      const float2 d = df_fin(acc[x][y]);
-      double v = alpha * (double(d.x) + double(d.y));
-      if (g.low) v += fma(g.c3, Y3[e], fma(g.c2, Y2[e], fma(g.c1, Y[e], r == q ? g.c0 : 0.0)));
-      O[e] = v;
-      if (r != q) O[long(q) * b + r] = v;
-    }
-}
-
 // Interaction coefficients f_k = scale_k (M PAS'_k M^T)_22 of items g = j0 + j, as in
 // build_h.
 __global__ void k_huge_fk(DevSys s, long j0, int items, double *fk) {
@@ -300,14 +191,14 @@ __global__ void k_huge_hbuild(DevSys s, int bp, int b, const double *fk, double 
   ws[long(j) * kHugeSlots * bb + e] = h;
 }
 
-// Per item: ||2 pi tau H||_inf -> squarings sq_j (so that the scaled norm is <= 1/2) and
-// sc_j = 2 pi tau 2^-sq_j; the largest sq of the launch into *sq_max.
-__global__ void __launch_bounds__(256) k_huge_norm(const double *ws, int b, double tp, double *sc, int *sq,
-                                                   int *sq_max) {
+// Per item: ||2 pi tau H||_inf -> squarings sq_j (so that the scaled norm is <= 1/2), and
+// X = 2 pi tau 2^-sq_j H in place.
+__global__ void __launch_bounds__(256) k_huge_norm(double *ws, int b, double tp, int *sq) {
   __shared__ double red[256];
+  __shared__ double sc_s;
   const long bb = long(b) * b;
   const int j = blockIdx.x;
-  const double *X = ws + long(j) * kHugeSlots * bb;
+  double *X = ws + long(j) * kHugeSlots * bb;
   double m = 0;
   for (int r = threadIdx.x; r < b; r += blockDim.x) {
     double rs = 0;
@@ -325,10 +216,11 @@ __global__ void __launch_bounds__(256) k_huge_norm(const double *ws, int b, doub
       frexp(nrm / 0.5, &q);
       q = min(q, 60);
     }
-    sc[j] = ldexp(tp, -q);
+    sc_s = ldexp(tp, -q);
     sq[j] = q;
-    atomicMax(sq_max, q);
   }
+  __syncthreads();
+  for (long e = threadIdx.x; e < bb; e += blockDim.x) X[e] *= sc_s;
 }
 
 // T (slot 5) = c0 I + c1 Y + c2 Y2 + c3 Y3, every item.
@@ -364,13 +256,14 @@ __global__ void k_huge_store_u(DevSys s, const double *ws, int bp, int bo, int b
   s.U[(size_t(i) * s.S2 + bp + e) * s.Cpad + c] = u;
 }
 
-// A_1 = U_0 for block (bp, b), crystallite blockIdx.y.
-__global__ void k_huge_copy_u0(DevSys s, int bp, int b) {
+// dst = src for block (bp, b), crystallite blockIdx.y, segment blockIdx.z: step slots src0 + z
+// stride of one [item][c] buffer to dst0 + z stride of another.
+__global__ void k_huge_copy(DevSys s, const double2 *src, double2 *dst, int src0, int dst0, int stride, int bp, int b) {
   const long bb = long(b) * b, e = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y;
+  const int c = blockIdx.y, z = blockIdx.z;
   if (e >= bb) return;
-  const size_t a0 = (size_t(bp) + e) * s.Cpad + c;
-  s.A[a0] = s.U[a0];
+  const size_t x = (size_t(bp) + e) * s.Cpad + c, step = size_t(s.S2) * s.Cpad;
+  dst[size_t(dst0 + z * stride) * step + x] = src[size_t(src0 + z * stride) * step + x];
 }
 
 // W of item g = j0 + blockIdx.y = workspace (contiguous b x b per item), back over A in the

@@ -1,0 +1,301 @@
+// Batched exact-slice products on the tensor cores for matrices that live in HBM, included by
+// bl_engine.cu after bl_huge.cuh and bl_tc.cuh: O = A B for FP64 operands, real or complex, of
+// any size, one 128-row output tile per CTA.
+//
+// An operand (|x| <= 2^e, e given per operand) becomes a fixed-point integer x 2^(8S-1-e),
+// written as S balanced base-256 digits q_j (exact in BF16), and the product takes the digit
+// pairs with i + j <= top level into one FP32 accumulator per level in tensor memory.  A
+// level's sums are integers below 2^24 (rows and columns of norm ~1, K' <= 512 digits long),
+// so the tensor core's FP32 accumulation is exact; the epilogue joins the levels in 64-bit
+// integers and rounds once to FP64, without touching the FP64 pipe.
+//   S = 7 (FP64 form): levels 0..7, the last two in one accumulator: 34 pairs, operand rounding
+//     2^-56 and dropped levels below 2^-60 for |O| ~ 1: at or below a 252-term FP64 dot product;
+//   S = 6 (mixed form): levels 0..5, 21 pairs, dropped levels ~2^-44, the size of the compensated
+//     double-float sums they take the place of.
+// Why: GB300 issues 2 FP64 FMAs per clock and SM (a 126 x 126 complex product: 3.9 M clocks on
+// one SM; ~0.9 M in double-float on the FP32 pipe), while the 34 BF16 products of a 64 x 64 x 16
+// complex chunk take ~2200 clocks of the tensor pipe and the digit conversions of its operands
+// about 1100 of the integer and FP32 pipes, which run beside it.
+//
+// Complex operands are interleaved in place: complex row r is rows 2r (re) and 2r+1 (im) of the
+// M = 128 tile, complex k is K entries 2k, 2k+1: A(r, l) = a + ib fills [[a, -b], [b, a]] and
+// B(l, n) = c + id the pair (c, d), so one real product per tile gives re and im in adjacent
+// tensor-memory lanes, and four complex elements are one 16-byte core-matrix row.
+// Pipeline: 16 warps convert K chunks of 32 entries into two shared-memory buffers (K-major, no
+// swizzle, 8-row groups padded by 16 bytes), one warp issues the products of a full buffer;
+// every wait is bounded (tc::wait_parity).
+namespace xs {
+
+constexpr int kConv = 512;           // converting threads (16 warps), then the issuing warp
+constexpr int kThreadsXs = kConv + 32;
+constexpr int kN = 64;               // output columns per tile
+constexpr int kK = 32;               // K entries (16 complex) per chunk
+constexpr int kGroup = kK * 16 + 16; // bytes of an 8-row group (tc::sbo_bytes(kK))
+constexpr int kPlaneA = 16 * kGroup, kPlaneB = 8 * kGroup;
+template <int S>
+__host__ __device__ constexpr int buf_bytes() { return S * (kPlaneA + kPlaneB); }
+template <int S>
+__host__ __device__ constexpr size_t smem() { return 2 * size_t(buf_bytes<S>()) + 1024; }
+// rows of the output per tile
+__host__ __device__ constexpr int tile_rows(bool cplx) { return cplx ? 64 : 128; }
+
+__device__ __forceinline__ void arrive(uint64_t *mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::saddr(mbar)) : "memory");
+}
+__device__ __forceinline__ void init(uint64_t *mbar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc::saddr(mbar)), "r"(count));
+}
+
+// round(x 2^(8S-1-e)) plus the digit bias (128 in every digit but the first), on the integer
+// pipe: the mantissa with its leading bit at 63, shifted right once.  bad: set when x is not
+// finite or |x| >= 2^(e+1).
+template <int S>
+__device__ __forceinline__ long long fixed(double x, int e, bool &bad) {
+  constexpr unsigned long long kBias = 0x0080808080808080ull & ((1ull << (8 * (S - 1))) - 1);
+  const unsigned hi = unsigned(__double2hiint(x)), lo = unsigned(__double2loint(x));
+  const int ex = int(hi >> 20) & 0x7ff;
+  bad = bad || ex > 1023 + e;
+  // |x| = m 2^(ex - 1086) with m's leading bit at 63 (zeros and denormals: too small to matter)
+  const unsigned mh = 0x80000000u | (hi << 11) | (lo >> 21), ml = lo << 11;
+  const int sh = max(1086 - (8 * S - 1) + e - ex - 1, 0);  // one less than the whole shift
+  const unsigned long long m = sh < 64 ? ((unsigned long long)mh << 32) | ml : 0ull;
+  const unsigned long long v = ((m >> (sh & 63)) + 1) >> 1;
+  return (long long)kBias + ((int)hi < 0 ? -(long long)v : (long long)v);
+}
+// digit j of a biased fixed-point value, times 2^-8j, as a float (exact)
+template <int S>
+__device__ __forceinline__ float digit(long long w, int j) {
+  const float sc = __uint_as_float(uint32_t(127 - 8 * j) << 23);
+  if (j == 0)  // -256 .. 256
+    return __fadd_rn(__int_as_float(0x4B000200 + int(w >> (8 * (S - 1)))), -8389120.f);
+  const int byte = S - 1 - j;
+  const uint32_t word = byte < 4 ? uint32_t(w) : uint32_t((unsigned long long)w >> 32);
+  const float f = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u + uint32_t(byte & 3)));  // 2^23 + byte
+  return __fmaf_rn(f, sc, -8388736.f * sc);
+}
+// two floats that are exact in BF16, packed (a in the low half)
+__device__ __forceinline__ uint32_t pack(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632u);
+}
+
+// v 2^(e - 61) rounded to FP64, on the integer pipe
+__device__ __forceinline__ double join(long long v, int e) {
+  const unsigned sign = unsigned((unsigned long long)v >> 32) & 0x80000000u;
+  const unsigned long long u = v < 0 ? (unsigned long long)-v : (unsigned long long)v;
+  const int lz = __clzll((long long)u);
+  // leading bit at 62, rounded to 53 bits; a carry out of the rounding moves into the exponent
+  const unsigned long long m = ((u << lz) >> 1) + (1ull << 9);
+  const unsigned long long r = ((unsigned long long)(unsigned)(1023 + 2 - lz + e - 1) << 52) + (m >> 10);
+  return u ? __hiloint2double(int(unsigned(r >> 32) | sign), int(unsigned(r))) : 0.0;
+}
+
+}  // namespace xs
+
+// Epilogue of a real product (the step exponential): adds c0 I + c1 Y + c2 Y2 + c3 Y3 of the item
+// when low != 0; items whose squarings are done (sq[item] <= round) are skipped.
+struct XsReal {
+  int low;
+  double alpha, c0, c1, c2, c3;
+  const double *Y, *Y2, *Y3;  // item 0's matrices; item stride is the output's
+  const int *sq;
+  int round;
+};
+
+// O = op(A) B for items g = j0 + blockIdx.y (op(A) = A^H when CONJ_A, A then stored k x m; a real
+// A is symmetric and read down its columns, as B is).
+// |A| <= 2^ea, |B| <= 2^eb.  A non-finite or larger operand makes the tile NaN.
+template <bool CPLX, int S, bool CONJ_A, class T>
+__global__ void __launch_bounds__(xs::kThreadsXs, 1)
+    k_xs_gemm(HMat<const T> A, HMat<const T> B, HMat<T> O, int m, int n, int k, int Cb, long j0, int ea, int eb,
+              XsReal ep, int *status) {
+  using namespace xs;
+  constexpr int kLev = S == 7 ? 7 : 6;   // accumulators
+  constexpr int kTop = S == 7 ? 7 : 5;   // highest digit level taken
+  constexpr int TM = tile_rows(CPLX);
+  extern __shared__ __align__(1024) unsigned char xsm[];
+  __shared__ uint32_t tbase;
+  __shared__ __align__(8) uint64_t full[2], empty[2], done;
+  __shared__ int failed, bad_s;
+  if (!CPLX && ep.sq && ep.sq[blockIdx.y] <= ep.round) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const long g = j0 + blockIdx.y;
+  const int c = int(g % Cb), sl = int(g / Cb);
+  const int tn = (n + kN - 1) / kN;
+  const int r0 = int(blockIdx.x / tn) * TM, q0 = int(blockIdx.x % tn) * kN;
+  const int rows = min(TM, m - r0), cols = min(kN, n - q0), N16 = (cols + 15) / 16 * 16;
+  const int kc = CPLX ? kK / 2 : kK;  // source k per chunk
+  const int nch = (k + kc - 1) / kc;
+  unsigned char *base = xsm + ((1024 - (tc::saddr(xsm) & 1023)) & 1023);
+  if (warp == 0) tc::tmem_alloc(&tbase, 512);
+  if (tid == 0) {
+    init(&full[0], kConv), init(&full[1], kConv), init(&empty[0], 1), init(&empty[1], 1), init(&done, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;");
+    failed = 0, bad_s = 0;
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tbase;
+  bool ok = true;
+  if (warp < kConv / 32) {
+    bool bad = false;
+    constexpr int U = 8;  // K entries per unit: one 16-byte core-matrix row (4 complex)
+    // units of a chunk: A rows x 4 k groups, then B columns x 4 k groups; rows (columns) fastest
+    const int nA = rows * 4, nU = nA + cols * 4;
+    // the products that read chunk ch's buffer two chunks ago have ended
+    auto released = [&](int ch) -> bool {
+      if (ch < 2 || tc::wait_parity(&empty[ch & 1], uint32_t((ch / 2 - 1) & 1))) return true;
+      failed = 1;
+      return false;
+    };
+    for (int ch = 0; ch < nch; ++ch) {
+      const int buf = ch & 1;
+      unsigned char *sa = base + buf * buf_bytes<S>(), *sb = sa + S * kPlaneA;
+      bool waited = false;
+      for (int u = tid; u < nU; u += kConv) {
+        const bool isA = u < nA;
+        const int x = isA ? u % rows : (u - nA) % cols, kg = isA ? u / rows : (u - nA) / cols;
+        const int l0 = ch * kc + kg * (kc / 4);
+        double v[U];
+        // source entry t of the unit at p + t d (A runs along its rows, or down its columns when
+        // it is conjugate-transposed or symmetric; B down its columns)
+        const bool down = !isA || CONJ_A || !CPLX;
+        const T *p = isA ? (down ? &A(c, sl, l0, r0 + x) : &A(c, sl, r0 + x, l0)) : &B(c, sl, l0, q0 + x);
+        const long d = isA ? (down ? A.ld * A.es : A.es) : B.ld * B.es;
+#pragma unroll
+        for (int t = 0; t < (CPLX ? 4 : 8); ++t) {
+          if constexpr (CPLX) {
+            double2 z = make_double2(0.0, 0.0);
+            if (l0 + t < k) z = p[t * d];
+            v[2 * t] = z.x, v[2 * t + 1] = CONJ_A && isA ? -z.y : z.y;
+          } else {
+            v[t] = l0 + t < k ? p[t * d] : 0.0;
+          }
+        }
+        long long w[U];
+#pragma unroll
+        for (int t = 0; t < U; ++t) w[t] = fixed<S>(v[t], isA ? ea : eb, bad);
+        if (!waited) {
+          waited = true;
+          if (!(ok = released(ch))) break;
+        }
+        const int row = isA ? (CPLX ? 2 * x : x) : x;
+        unsigned char *dst = (isA ? sa : sb) + (row >> 3) * kGroup + kg * 128 + (row & 7) * 16;
+        const int plane = isA ? kPlaneA : kPlaneB;
+#pragma unroll
+        for (int j = 0; j < S; ++j) {
+          float f[U];
+#pragma unroll
+          for (int t = 0; t < U; ++t) f[t] = digit<S>(w[t], j);
+          uint4 p = make_uint4(pack(f[0], f[1]), pack(f[2], f[3]), pack(f[4], f[5]), pack(f[6], f[7]));
+          if (CPLX && isA) {  // row 2x: (a, -b); row 2x + 1: (b, a)
+            const uint4 q = make_uint4(pack(f[1], f[0]), pack(f[3], f[2]), pack(f[5], f[4]), pack(f[7], f[6]));
+            *reinterpret_cast<uint4 *>(dst + j * plane + 16) = q;
+            p.x ^= 0x80000000u, p.y ^= 0x80000000u, p.z ^= 0x80000000u, p.w ^= 0x80000000u;
+          }
+          *reinterpret_cast<uint4 *>(dst + j * plane) = p;
+        }
+      }
+      // a thread without units waits too: it must not arrive for this chunk before the last one
+      // of the same buffer is through
+      if (!waited) ok = released(ch);
+      if (!ok) break;
+      tc::fence_smem_async();
+      arrive(&full[buf]);
+    }
+    if (bad) bad_s = 1;
+    if (ok && !tc::wait_parity(&done, 0)) failed = 1;
+  } else if (lane == 0) {
+    const uint32_t id = tc::idesc_bf16(N16, false);
+    for (int ch = 0; ch < nch; ++ch) {
+      const int buf = ch & 1;
+      if (!tc::wait_parity(&full[buf], uint32_t((ch / 2) & 1))) {
+        failed = 1;
+        break;
+      }
+      tc::fence_after();
+      const uint32_t a = tc::saddr(base + buf * buf_bytes<S>()), b = a + S * kPlaneA;
+      // the last chunk's K entries beyond k are zeros; a whole 16-entry half of them is skipped
+      const int ks = (ch == nch - 1 && (k - ch * kc) * (CPLX ? 2 : 1) <= 16) ? 1 : 2;
+#pragma unroll 1
+      for (int lev = 0; lev <= kTop; ++lev) {
+        const uint32_t d = tmem + uint32_t(min(lev, kLev - 1) * kN);
+        for (int i = max(0, lev - (S - 1)); i <= min(lev, S - 1); ++i) {
+          const int j = lev - i;
+          const bool first = ch == 0 && lev < kLev && i == max(0, lev - (S - 1));
+          for (int kk = 0; kk < ks; ++kk)
+            tc::mma(d, tc::sdesc(a + i * kPlaneA + kk * 256, kK), tc::sdesc(b + j * kPlaneB + kk * 256, kK), id,
+                    first && kk == 0 ? 0u : 1u);
+        }
+      }
+      tc::commit(&empty[buf]);
+    }
+    tc::commit(&done);
+  }
+  __syncwarp();
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const bool fine = failed == 0;
+  if (fine && warp < kConv / 32) {
+    const bool nan = bad_s != 0;
+    const int q4 = warp & 3, L = 32 * q4 + lane;  // tensor-memory lane: tile row
+    const int live = CPLX ? 2 * rows : rows;
+    if (32 * q4 < live) {  // warp-uniform
+      for (int c0 = 8 * (warp >> 2); c0 < cols; c0 += 32) {
+        float a[kLev][8];
+        const uint32_t ta = tmem + (uint32_t(32 * q4) << 16) + uint32_t(c0);
+#pragma unroll
+        for (int l = 0; l < kLev; ++l) tc::ld8(ta + uint32_t(l * kN), a[l]);
+        tc::wait_ld();
+        double d[8];
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          int I[7];
+#pragma unroll
+          for (int l = 0; l < kLev; ++l) I[l] = __float2int_rn(a[l][t] * __uint_as_float(uint32_t(127 + 8 * l) << 23));
+          // sum of I_l 2^(-14-8l) in units of 2^-61 (|sum| < 2: level 0 to 2 fit 32 bits)
+          long long v = (long long)((I[0] << 16) + (I[1] << 8) + I[2]) << 31;
+          v += (long long)I[3] * (1 << 23);
+          v += (long long)I[4] * (1 << 15);
+          v += (long long)I[5] * (1 << 7);
+          if constexpr (kLev == 7) v += I[6] >> 1;
+          d[t] = nan ? __longlong_as_double(0x7FF8000000000000ll) : join(v, ea + eb);
+        }
+        if constexpr (CPLX) {
+          const bool odd = L & 1;
+          const int r = r0 + (L >> 1);
+#pragma unroll
+          for (int t = 0; t < 8; t += 2) {
+            const double send = odd ? d[t] : d[t + 1];
+            const double got = __shfl_xor_sync(0xffffffffu, send, 1);
+            const int q = q0 + c0 + t + (odd ? 1 : 0);
+            if (L < live && q < n) O(c, sl, r, q) = odd ? make_double2(got, d[t + 1]) : make_double2(d[t], got);
+          }
+        } else {
+          const int r = r0 + L;
+          if (L < live) {
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+              const int q = q0 + c0 + t;
+              if (q >= n) continue;
+              double v = ep.alpha == 1.0 ? d[t] : ep.alpha * d[t];
+              if (ep.low) {
+                const long e = long(c) * O.cs + long(r) * O.ld + q;
+                v += fma(ep.c3, ep.Y3[e], fma(ep.c2, ep.Y2[e], fma(ep.c1, ep.Y[e], r == q ? ep.c0 : 0.0)));
+              }
+              O(c, sl, r, q) = v;
+            }
+          }
+        }
+      }
+    }
+  } else if (!fine) {
+    if (tid == 0) atomicOr(status, kTcTimeout);
+    tc::wait_parity(&done, 0);  // bounded: let products in flight drain before TMEM is freed
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  if (warp == 0) tc::tmem_free(tmem, 512);
+}
