@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(1024) k_big_step(DevSys s, int k) {
     double h = Hcb[e];
     for (int kk = 0; kk < s.nint; ++kk) {
       const double t = s.Tk[size_t(kk) * s.S2 + bp + e];
-      if (t != 0.0) h = fma(fk[kk], t, h);
+      if (nonzero(t)) h = fma(fk[kk], t, h);
     }
     X[e] = h;
   }
@@ -399,7 +399,10 @@ struct BigPair {
   int e2;  // |M_ab W_b| <= 2^e2: the larger of M_ab's row and column sums
   const int *rp, *ci;
   const double2 *cv;
+  const float2 *cvf;  // mixed form: cv in single precision (a conversion is an FP64-pipe instruction)
 };
+__device__ __forceinline__ double2 pair_coef(const BigPair &P, int j, double2) { return __ldg(P.cv + j); }
+__device__ __forceinline__ float2 pair_coef(const BigPair &P, int j, float2) { return __ldg(P.cvf + j); }
 
 // Shared memory of k_big_qr: W_a, a column chunk of W_b and of X = M_ab W_b.
 template <class C>
@@ -432,7 +435,7 @@ __global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_qr(DevSys s, BigPa
       const int l = e / wc, q = e % wc;
       C x = mkc<C>(0, 0);
       for (int j = __ldg(bp2.rp + l); j < __ldg(bp2.rp + l + 1); ++j)
-        x = cfma(cvt<C>(__ldg(bp2.cv + j)), Wb[__ldg(bp2.ci + j) * wc + q], x);
+        x = cfma(pair_coef(bp2, j, C()), Wb[__ldg(bp2.ci + j) * wc + q], x);
       X[e] = x;
     }
     __syncthreads();

@@ -86,6 +86,13 @@ __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
 }
 __device__ __forceinline__ double chop1(double v, double eps) { return fabs(v) < eps ? 0.0 : v; }
 
+// v != 0.0 on the integer pipe: an FP64 comparison costs as much as an FP64 FMA, and the skips
+// over an operator's structural zeros test every element
+__device__ __forceinline__ bool nonzero(double v) {
+  return ((unsigned(__double2hiint(v)) << 1) | unsigned(__double2loint(v))) != 0u;
+}
+__device__ __forceinline__ bool nonzero(double2 v) { return nonzero(v.x) || nonzero(v.y); }
+
 // Single-precision twins for the mixed-precision form (same names, float2 arguments).
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
@@ -655,7 +662,7 @@ __device__ __forceinline__ void build_h_at(const DevSys &s, int c, double sp, do
 #pragma unroll
       for (int q = 0; q < B; ++q) {
         const double t = T[p * B + q];  // same for every lane: the skip is warp-uniform
-        if (t != 0.0) h[p][q] = fma(f, t, h[p][q]);
+        if (nonzero(t)) h[p][q] = fma(f, t, h[p][q]);
       }
   }
 }
@@ -696,7 +703,7 @@ __device__ __forceinline__ void build_h(const DevSys &s, int c, int i, int bp, d
 #pragma unroll
         for (int q = 0; q < B; ++q) {
           const double t = T[p * B + q];
-          if (t != 0.0) h[p][q] = fma(f, t, h[p][q]);
+          if (nonzero(t)) h[p][q] = fma(f, t, h[p][q]);
         }
     }
     return;
@@ -770,7 +777,7 @@ __global__ void __launch_bounds__(kThreads) k_static_elems(DevSys s) {
     double2 x = cmk(0, 0), y = cmk(0, 0);
     for (int m = 0; m < bb; ++m) {
       const double2 d = D[l * bb + m], r = Rh[m * ba + l];
-      if (d.x == 0.0 && d.y == 0.0 && r.x == 0.0 && r.y == 0.0) continue;
+      if (!nonzero(d) && !nonzero(r)) continue;
       const double vb = s.VF[at(pb + m * bb + j, c, s.Cpad)].x;
       x.x = fma(d.x, vb, x.x), x.y = fma(d.y, vb, x.y);
       y.x = fma(r.x, vb, y.x), y.y = fma(r.y, vb, y.y);
@@ -1694,7 +1701,7 @@ __global__ void __launch_bounds__(kThreads) k_qr(DevSys s) {
   for (int l = 0; l < ba; ++l)
     for (int m = 0; m < bb; ++m) {
       double2 d2 = M[moff + l * bb + m];
-      if (d2.x == 0.0 && d2.y == 0.0) continue;
+      if (!nonzero(d2)) continue;
       const C d = cvt<C>(d2);
       for (int q = 0; q < bb; ++q) X[l * bb + q] = cfma(d, W[at(pb + m * bb + q, c, s.Cpad)], X[l * bb + q]);
     }
@@ -2603,6 +2610,7 @@ struct JobImpl {
   std::vector<size_t> big_rp_off, huge_rp_off;   // each pair's row pointers in big_rp
   DevBuf<int> big_rp, big_ci;                    // non-zeros of M_ab by row, all big pairs
   DevBuf<double2> big_cv;
+  DevBuf<float2> big_cvf;
   DevBuf<int> bs, boff, bpoff, qa, qb, qoff, doff, ra, rb, roff, rhooff, eq, erev, er, erg, esg, status, srp, seo;
   std::vector<DevBuf<int>> blist;
   DevBuf<unsigned char> tables;  // the one buffer behind the uploaded inputs and tables
@@ -3147,7 +3155,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
       for (double v : col) most = std::max(most, v);
       int e2 = 0;
       std::frexp(most, &e2);  // most < 2^e2
-      BigPair P{a, b, isq ? qoff[pr] : roff[pr - J.npq], isq ? J.nq : J.nr, isq ? 1 : 0, w, e2, nullptr, nullptr, nullptr};
+      BigPair P{a, b, isq ? qoff[pr] : roff[pr - J.npq], isq ? J.nq : J.nr, isq ? 1 : 0, w, e2, nullptr, nullptr, nullptr, nullptr};
       if (std::max(ba, bb) > kMaxBigBlock) {  // k_huge_mx + k_huge_zgemm
         J.huge_pairs.push_back(P);
         J.huge_rp_off.push_back(rp_off);
@@ -3186,6 +3194,11 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   up.add(J.eq, eq), up.add(J.erev, erev), up.add(J.er, er), up.add(J.erg, erg), up.add(J.esg, esg);
   up.add(J.srp, srp), up.add(J.seo, seo);
   up.add(J.big_rp, big_rp_h), up.add(J.big_ci, big_ci_h), up.add(J.big_cv, big_cv_h);
+  if (J.mixed) {
+    std::vector<float2> f(big_cv_h.size());
+    for (size_t x = 0; x < f.size(); ++x) f[x] = make_float2(float(big_cv_h[x].x), float(big_cv_h[x].y));
+    up.add(J.big_cvf, f);
+  }
   up.add(J.pas, pas), up.add(J.iscale, isc), up.add(J.Hc, Hc);
   // the packed operators: dense from the host while they are small, else their non-zeros go up
   // and k_scatter_terms fills the (zeroed) dense tables (9 spins: 17.5 MB in each precision, 45
@@ -3301,10 +3314,11 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   J.h2d = up.bytes();
   s.tw = J.tw.p, s.twf = J.twf.p;
   for (size_t t = 0; t < J.big_pairs.size(); ++t)
-    J.big_pairs[t].rp = J.big_rp.p + J.big_rp_off[t], J.big_pairs[t].ci = J.big_ci.p, J.big_pairs[t].cv = J.big_cv.p;
+    J.big_pairs[t].rp = J.big_rp.p + J.big_rp_off[t], J.big_pairs[t].ci = J.big_ci.p, J.big_pairs[t].cv = J.big_cv.p,
+    J.big_pairs[t].cvf = J.big_cvf.p;
   for (size_t t = 0; t < J.huge_pairs.size(); ++t)
     J.huge_pairs[t].rp = J.big_rp.p + J.huge_rp_off[t], J.huge_pairs[t].ci = J.big_ci.p,
-    J.huge_pairs[t].cv = J.big_cv.p;
+    J.huge_pairs[t].cv = J.big_cv.p, J.huge_pairs[t].cvf = J.big_cvf.p;
   if (scatter) {
     J.Tk.alloc(tk_n);
     CUDA_OK(cudaMemsetAsync(J.Tk.p, 0, tk_n * sizeof(double), st));

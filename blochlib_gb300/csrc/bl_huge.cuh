@@ -186,7 +186,7 @@ __global__ void k_huge_hbuild(DevSys s, int bp, int b, const double *fk, double 
   const double *f = fk + long(j) * s.nint;
   for (int kk = 0; kk < s.nint; ++kk) {
     const double t = s.Tk[size_t(kk) * s.S2 + bp + e];
-    if (t != 0.0) h = fma(f[kk], t, h);
+    if (nonzero(t)) h = fma(f[kk], t, h);
   }
   ws[long(j) * kHugeSlots * bb + e] = h;
 }
@@ -290,7 +290,7 @@ __global__ void k_huge_mx(DevSys s, BigPair P, long j0, C *ws) {
   const int l = int(e / bb), q = int(e % bb);
   const C *W = Bufs<C>::W(s) + size_t(i) * s.S2 * s.Cpad;
   C x = mkc<C>(0, 0);
-  for (int t = P.rp[l]; t < P.rp[l + 1]; ++t) x = cfma(cvt<C>(P.cv[t]), W[at(pb + P.ci[t] * bb + q, c, s.Cpad)], x);
+  for (int t = P.rp[l]; t < P.rp[l + 1]; ++t) x = cfma(pair_coef(P, t, C()), W[at(pb + P.ci[t] * bb + q, c, s.Cpad)], x);
   ws[long(j) * ne + e] = x;
 }
 
