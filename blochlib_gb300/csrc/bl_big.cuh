@@ -189,12 +189,10 @@ __global__ void __launch_bounds__(1024) k_big_step(DevSys s, int k) {
   __syncthreads();
   double *X = bsm;
   const double *Hcb = hc_of(s, i) + bp;
-  for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+  for (int x = threadIdx.x; x < bb; x += blockDim.x) {  // each element's own terms, longest first
+    const int e = s.tk_order[bp + x];
     double h = Hcb[e];
-    for (int kk = 0; kk < s.nint; ++kk) {
-      const double t = s.Tk[size_t(kk) * s.S2 + bp + e];
-      if (nonzero(t)) h = fma(fk[kk], t, h);
-    }
+    for (int t = s.tk_ptr[bp + e]; t < s.tk_ptr[bp + e + 1]; ++t) h = fma(fk[s.tk_term[t]], s.tk_val64[t], h);
     X[e] = h;
   }
   __syncthreads();
@@ -831,12 +829,11 @@ __global__ void __launch_bounds__(1024) k_big_step_df(DevSys s, int k) {
   __syncthreads();
   float2 *X = reinterpret_cast<float2 *>(bsd), *P = X + bb, *Q = P + bb, *R = Q + bb, *I = R + bb;
   const float2 *Hcb = s.Hc_df + (s.hc_chunks ? size_t(i / s.psub) * s.S2 : 0) + bp;
-  for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+  for (int x = threadIdx.x; x < bb; x += blockDim.x) {  // each element's own terms, longest first
+    const int e = s.tk_order[bp + x];
     float2 h = Hcb[e];
-    for (int kk = 0; kk < s.nint; ++kk) {
-      const float2 t = s.Tk_df[size_t(kk) * s.S2 + bp + e];
-      if (t.x != 0.f) h = dfv_add(h, dfv_mul(fk[kk], t));
-    }
+    for (int t = s.tk_ptr[bp + e]; t < s.tk_ptr[bp + e + 1]; ++t)
+      h = dfv_add(h, dfv_mul(fk[s.tk_term[t]], s.tk_val[t]));
     X[e] = h;
   }
   __syncthreads();

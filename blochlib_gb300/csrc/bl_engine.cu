@@ -188,7 +188,7 @@ __device__ __forceinline__ float4 cdf_fin(const CdfAcc &a) {
 // ------------------------------------------------------------------ job description
 struct DevSys {
   int C, Cpad, n, npts, N, nb, S2, nint, nq, nr, ne, J, rosym, step_method;
-  int M, logM, fave_method;  // FFT length for the Fave correlation; 0 direct, 1 FFT
+  int M, logM, fftq, fave_method;  // FFT length M = fftq 2^logM of the Fave correlation; 0 direct, 1 FFT
   int fave_twist;            // 1: M == n, circular correlation of the twisted sequences
   int is_static;             // static powder FID (oneFID.h:292-336): dt = 1/sw, n = p-period
   int gper;                  // period of the FID split fid[j*gper + p] (n, or the p2p base)
@@ -198,7 +198,7 @@ struct DevSys {
   int floq32;
   double dt;
   const int *srp, *seo;      // per D pair (a,b): the rho pair (b,a) and first element, or -1
-  const double2 *tw;         // exp(-2 pi i k / M), k < M/2
+  const double2 *tw;         // exp(-2 pi i k / M), k < M
   double tau, wr, sin_rotb, cos_rotb, scale;
   // per block
   const int *bs, *boff, *bpoff;
@@ -212,10 +212,12 @@ struct DevSys {
   // double-float copies for the mixed form's step (hi, lo): term operators, constant parts,
   // and fk_df = 1 when k_coef stores the coefficients as float2 in fk's slots
   const float2 *Tk_df, *Hc_df;
-  // the same operators by element for the tensor-core step: element e (packed block index)
-  // holds entries [tk_ptr[e], tk_ptr[e+1]) of (term, double-float value), terms ascending
+  // the same operators by element for the blocks above kMaxBlock: element e (packed block index)
+  // holds entries [tk_ptr[e], tk_ptr[e+1]) of (term, value in FP64 and double-float), terms
+  // ascending; tk_order: each block's elements by descending term count
   const int *tk_ptr, *tk_term, *tk_order;
   const float2 *tk_val;
+  const double *tk_val64;
   int fk_df;
   float2 tpdf;  // 2 pi tau as double-float
   const int *ikind;  // per term: 0 first order, 1 / 2 second-order quadrupolar (c4 / c2)
@@ -1806,18 +1808,31 @@ __global__ void __launch_bounds__(kThreads) k_fave(DevSys s) {
   }
 }
 
-// Radix-2 decimation-in-time FFT (negative exponent) of CG interleaved sequences of length
-// M = 2^logM held in shared memory as X[i * CG + cc], input in bit-reversed order, output in
-// natural order.  tw[k] = exp(-2 pi i k / (M twm)), k < M twm / 2 (twm = 2: a half-length
-// transform on the table of the full length).  Stage st pairs the points i and i + 2^st of
-// each block of 2^(st+1) with twiddle tw[(i mod 2^st) (M >> (st+1)) twm]; stages 0 and 1
-// multiply by 1 and -i only.  The stages run in passes of up to three: a thread holds the
-// 2^LR points of one group in registers and applies LR stages to them, so a pass costs one
-// shared-memory round trip and one barrier, and every point sees the same butterflies in
-// the same order as stage by stage (the result does not depend on the grouping).
+// Decimation-in-time FFT (negative exponent) of CG interleaved sequences of length M = q 2^a,
+// q = 1, 3 or 5, held in shared memory as X[i * CG + cc]: q transforms of length 2^a (radix 2,
+// segment r holding the points q m + r in bit-reversed order of m), then one combining pass of
+// radix q; output in natural order.  tw[k] = exp(-2 pi i k / (M twm)), k < M twm (twm = 2: a
+// half-length transform on the table of the full length).  The radix-2 stages run in passes of up
+// to three: a thread holds the 2^LR points of one group in registers and applies LR stages to
+// them, so a pass costs one shared-memory round trip and one barrier, and every point sees the
+// same butterflies in the same order as stage by stage (the result does not depend on the
+// grouping).  In FP64 the butterflies bound the kernel: a +- t d takes six FMAs (a + t d by four,
+// a - t d = 2a - (a + t d) by two) instead of four multiplies or FMAs and four additions.
 
-// Stages st .. st+LR-1 on x[k] = point (group base) + pos + k 2^st, pos < 2^st.
-template <class C, int LR>
+// a + w d and a - w d
+__device__ __forceinline__ void butterfly(double2 &a, double2 &d, double2 w) {
+  const double2 u = cmk(fma(w.x, d.x, fma(-w.y, d.y, a.x)), fma(w.x, d.y, fma(w.y, d.x, a.y)));
+  d = cmk(fma(2.0, a.x, -u.x), fma(2.0, a.y, -u.y));
+  a = u;
+}
+__device__ __forceinline__ void butterfly(float2 &a, float2 &d, float2 w) {
+  const float2 t = cmul(w, d), a0 = a;
+  a = cadd(a0, t), d = csub(a0, t);
+}
+
+// Stages st .. st+LR-1 on x[k] = point (group base) + pos + k 2^st, pos < 2^st.  HALF: the odd
+// points are zero before stage 0.
+template <class C, int LR, bool HALF = false>
 __device__ __forceinline__ void fft_regs(C (&x)[1 << LR], int st, int pos, int M, const C *__restrict__ tw,
                                          int twm) {
 #pragma unroll
@@ -1828,23 +1843,26 @@ __device__ __forceinline__ void fft_regs(C (&x)[1 << LR], int st, int pos, int M
       if ((k >> l) & 1) continue;
       const int k1 = k + (1 << l);
       const int p = pos + ((k & ((1 << l) - 1)) << st);  // position within the half block
-      const C a = x[k], d = x[k1];
-      C t = d;
-      if (sl == 1) {
-        if (p) t.x = d.y, t.y = -d.x;
-      } else if (sl > 1) {
-        t = cmul(tw[p * tstride * twm], d);
+      if (HALF && l == 0) {
+        x[k1] = x[k];
+      } else if (sl <= 1) {
+        const C a = x[k], d = x[k1];
+        C t = d;
+        if (sl == 1 && p) t.x = d.y, t.y = -d.x;
+        x[k] = cadd(a, t), x[k1] = csub(a, t);
+      } else {
+        butterfly(x[k], x[k1], tw[p * tstride * twm]);
       }
-      x[k] = cadd(a, t), x[k1] = csub(a, t);
     }
   }
 }
 
-// One pass of LR stages from st over X (and Y), in place; ends with a barrier.
+// One pass of LR stages from st over the q 2^a points of X (and Y), in place; ends with a
+// barrier.  M2 = 2^a; the twiddles of its transforms are every (q twm)-th of the table.
 template <int CG, class C, int LR>
-__device__ void fft_pass(C *X, C *Y, int M, int st, const C *__restrict__ tw, int twm) {
+__device__ void fft_pass(C *X, C *Y, int M2, int q, int st, const C *__restrict__ tw, int twm) {
   constexpr int R = 1 << LR;
-  const int h = 1 << st, items = (M >> LR) * CG;
+  const int h = 1 << st, items = (M2 >> LR) * q * CG;
   for (int idx = threadIdx.x; idx < items; idx += blockDim.x) {
     const int cc = idx % CG, b = idx / CG;
     const int pos = b & (h - 1), grp = b >> st;
@@ -1854,7 +1872,7 @@ __device__ void fft_pass(C *X, C *Y, int M, int st, const C *__restrict__ tw, in
       C x[R];
 #pragma unroll
       for (int k = 0; k < R; ++k) x[k] = V[base + k * h * CG];
-      fft_regs<C, LR>(x, st, pos, M, tw, twm);
+      fft_regs<C, LR>(x, st, pos, M2, tw, q * twm);
 #pragma unroll
       for (int k = 0; k < R; ++k) V[base + k * h * CG] = x[k];
     }
@@ -1862,37 +1880,108 @@ __device__ void fft_pass(C *X, C *Y, int M, int st, const C *__restrict__ tw, in
   __syncthreads();
 }
 
-// Stages st0 .. logM-1 in passes of three (the last pass two or one).
-template <int CG, class C>
-__device__ void fft_dit(C *X, C *Y, int M, int logM, const C *__restrict__ tw, int twm = 1, int st0 = 0) {
-  int st = st0;
-  for (; st + 3 <= logM; st += 3) fft_pass<CG, C, 3>(X, Y, M, st, tw, twm);
-  if (logM - st == 2) fft_pass<CG, C, 2>(X, Y, M, st, tw, twm);
-  else if (logM - st == 1) fft_pass<CG, C, 1>(X, Y, M, st, tw, twm);
+// q-point DFT in place, q odd: the pairs x_r +- x_(q-r) against cos and sin
+template <int Q, class C>
+__device__ __forceinline__ void dft_odd(C (&x)[Q]) {
+  using R = decltype(C::x);
+  constexpr int H = (Q - 1) / 2;
+  // cos and sin of 2 pi j / Q
+  constexpr double c3[2] = {1.0, -0.5}, s3[2] = {0.0, 0.86602540378443864676};
+  constexpr double c5[3] = {1.0, 0.30901699437494742410, -0.80901699437494742410};
+  constexpr double s5[3] = {0.0, 0.95105651629515357212, 0.58778525229247312917};
+  C p[H + 1], m[H + 1], y[Q];
+#pragma unroll
+  for (int r = 1; r <= H; ++r) p[r] = cadd(x[r], x[Q - r]), m[r] = csub(x[r], x[Q - r]);
+  y[0] = x[0];
+#pragma unroll
+  for (int r = 1; r <= H; ++r) y[0] = cadd(y[0], p[r]);
+#pragma unroll
+  for (int s = 1; s <= H; ++s) {
+    C a = x[0], b = mkc<C>(0, 0);  // X_s = a - i b, X_(Q-s) = a + i b
+#pragma unroll
+    for (int r = 1; r <= H; ++r) {
+      const int j = (r * s) % Q, f = j <= H ? j : Q - j;
+      const R c = R(Q == 3 ? c3[f % 2] : c5[f % 3]), sn = R((j <= H ? 1.0 : -1.0) * (Q == 3 ? s3[f % 2] : s5[f % 3]));
+      a.x = fma(c, p[r].x, a.x), a.y = fma(c, p[r].y, a.y);
+      b.x = fma(sn, m[r].x, b.x), b.y = fma(sn, m[r].y, b.y);
+    }
+    y[s].x = a.x + b.y, y[s].y = a.y - b.x;
+    y[Q - s].x = a.x - b.y, y[Q - s].y = a.y + b.x;
+  }
+#pragma unroll
+  for (int s = 0; s < Q; ++s) x[s] = y[s];
 }
 
-// The first pass (stages 0..2, logM >= 3) fused with the load: point (bit-reversed position)
-// j of column cc is load(natural index brev(j), cc, x, y); the transformed groups go to X
-// (and Y when it is given).  Ends with a barrier; fft_dit(..., st0 = 3) continues.
-template <int CG, class C, class F>
-__device__ void fft_first_pass(C *X, C *Y, int M, int logM, const C *__restrict__ tw, int twm, F &&load) {
-  const int items = (M >> 3) * CG;
+// The combining pass: X[k + 2^a s] = sum_r W^(rk) e^(-2 pi i rs / Q) (segment r)[k].
+template <int CG, int Q, class C>
+__device__ void fft_combine(C *X, C *Y, int M2, const C *__restrict__ tw, int twm) {
+  for (int idx = threadIdx.x; idx < M2 * CG; idx += blockDim.x) {
+    const int k = idx / CG;
+    for (int w = 0; w < (Y ? 2 : 1); ++w) {
+      C *V = w ? Y : X;
+      C x[Q];
+      x[0] = V[idx];
+#pragma unroll
+      for (int r = 1; r < Q; ++r) x[r] = cmul(tw[r * k * twm], V[r * M2 * CG + idx]);
+      dft_odd<Q>(x);
+#pragma unroll
+      for (int t = 0; t < Q; ++t) V[t * M2 * CG + idx] = x[t];
+    }
+  }
+  __syncthreads();
+}
+
+// Stages st0 .. a-1 in passes of three (the last pass two or one), then the combining pass.
+template <int CG, class C>
+__device__ void fft_dit(C *X, C *Y, int a, int q, const C *__restrict__ tw, int twm = 1, int st0 = 0) {
+  const int M2 = 1 << a;
+  int st = st0;
+  for (; st + 3 <= a; st += 3) fft_pass<CG, C, 3>(X, Y, M2, q, st, tw, twm);
+  if (a - st == 2) fft_pass<CG, C, 2>(X, Y, M2, q, st, tw, twm);
+  else if (a - st == 1) fft_pass<CG, C, 1>(X, Y, M2, q, st, tw, twm);
+  if (q == 3) fft_combine<CG, 3>(X, Y, M2, tw, twm);
+  else if (q == 5) fft_combine<CG, 5>(X, Y, M2, tw, twm);
+}
+
+// natural index of the point stored at position x: segment x >> a, bit-reversed within it
+__device__ __forceinline__ int fft_index(int x, int a, int q) {
+  const int m = a ? int(__brev(unsigned(x & ((1 << a) - 1))) >> (32 - a)) : 0;
+  return q * m + (x >> a);
+}
+
+// The first pass (stages 0..2, a >= 3) fused with the load: position j of column cc is
+// load(natural index, cc, x, y); the transformed groups go to X (and Y when it is given).  HALF:
+// the upper half of the sequence is zero (the odd points of every group).  Ends with a barrier;
+// fft_dit(..., st0 = 3) continues.
+template <int CG, bool HALF, class C, class F>
+__device__ void fft_first_pass(C *X, C *Y, int a, int q, const C *__restrict__ tw, int twm, F &&load) {
+  const int items = ((1 << a) >> 3) * q * CG;
   for (int idx = threadIdx.x; idx < items; idx += blockDim.x) {
     const int cc = idx % CG, grp = idx / CG;
     C x[8], y[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int i = int(__brev(unsigned(grp * 8 + k)) >> (32 - logM));
-      load(i, cc, x[k], y[k]);
-    }
-    fft_regs<C, 3>(x, 0, 0, M, tw, twm);
+    for (int k = 0; k < 8; ++k)
+      if (!HALF || !(k & 1)) load(fft_index(grp * 8 + k, a, q), cc, x[k], y[k]);
+    fft_regs<C, 3, HALF>(x, 0, 0, 1 << a, tw, q * twm);
 #pragma unroll
     for (int k = 0; k < 8; ++k) X[(grp * 8 + k) * CG + cc] = x[k];
     if (Y) {
-      fft_regs<C, 3>(y, 0, 0, M, tw, twm);
+      fft_regs<C, 3, HALF>(y, 0, 0, 1 << a, tw, q * twm);
 #pragma unroll
       for (int k = 0; k < 8; ++k) Y[(grp * 8 + k) * CG + cc] = y[k];
     }
+  }
+  __syncthreads();
+}
+// The first pass where a < 3: plain loads into position.
+template <int CG, class C, class F>
+__device__ void fft_load(C *X, C *Y, int a, int q, F &&load) {
+  for (int idx = threadIdx.x; idx < (q << a) * CG; idx += blockDim.x) {
+    const int cc = idx % CG, x = idx / CG;
+    C u, v;
+    load(fft_index(x, a, q), cc, u, v);
+    X[idx] = u;
+    if (Y) Y[idx] = v;
   }
   __syncthreads();
 }
@@ -1919,7 +2008,7 @@ __device__ __forceinline__ float2 z_pow_f(float4 e, int j) {
 
 // Fave by FFT.  One CTA per (element e, group of CG crystallites).  With q zero outside
 // [0, n), Lin_d = sum_i q_{i+d} r_i for |d| < n is the linear cross-correlation, obtained
-// from zero-padded transforms of length M >= 2n:  Lin = IFFT(FFT(q) . conj(FFT(conj r))).
+// from zero-padded transforms of length M = 2^a, 3 2^a or 5 2^a >= 2n:  Lin = IFFT(FFT(q) . conj(FFT(conj r))).
 // Then G_p = Lin_p + z Lin_{p-n} (the same G as k_fave).  When r = conj(q) (rho = (D+D^H)/2
 // and D has no block pair (b,a) for this element) the product is |FFT(q)|^2 and the second
 // forward transform is skipped.
@@ -1933,7 +2022,7 @@ __device__ __forceinline__ float2 z_pow_f(float4 e, int j) {
 template <int CG, class C>
 __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
   extern __shared__ __align__(16) unsigned char fsm_raw[];
-  const int M = s.M, logM = s.logM, n = s.n;
+  const int M = s.M, la = s.logM, q5 = s.fftq, n = s.n;  // M = q5 2^la
   C *X = reinterpret_cast<C *>(fsm_raw), *Y = X + size_t(M) * CG;
   // twist tables per column: zeta^b (b < 8), zeta^8a (a < M/8), and those of zeta^-1
   double2 *tp1 = reinterpret_cast<double2 *>(Y + size_t(M) * CG), *tp8 = tp1 + 8 * CG;
@@ -2039,19 +2128,9 @@ __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
   };
   const C *tw = Bufs<C>::tw(s);
   C *Yf = autoc ? nullptr : Y;
-  if (logM >= 3) {
-    fft_first_pass<CG, C>(X, Yf, M, logM, tw, 1, load);
-  } else {
-    for (int idx = threadIdx.x; idx < M * CG; idx += blockDim.x) {
-      const int cc = idx % CG, i = idx / CG;
-      const int ri = int(__brev(unsigned(i)) >> (32 - logM));
-      C q, y;
-      load(i, cc, q, y);
-      X[ri * CG + cc] = q;
-      if (!autoc) Y[ri * CG + cc] = y;
-    }
-    __syncthreads();
-  }
+  if (la < 3) fft_load<CG>(X, Yf, la, q5, load);
+  else if (twist) fft_first_pass<CG, false>(X, Yf, la, q5, tw, 1, load);
+  else fft_first_pass<CG, true>(X, Yf, la, q5, tw, 1, load);  // q is zero from n <= M/2 on
   if constexpr (kF) {  // z^j, j < J, and z itself (the exponents were written before the first pass's barrier)
     for (int idx = threadIdx.x; idx < CG * (s.J + 1); idx += blockDim.x) {
       const int cc = idx % CG, j = idx / CG, c = c0 + cc;
@@ -2060,32 +2139,23 @@ __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
       else Bufs<C>::Z(s)[at(j * s.ne + e, c, s.Cpad)] = z_pow_f(zexp[cc], j);
     }
   }
-  fft_dit<CG, C>(X, Yf, M, logM, tw, 1, logM >= 3 ? 3 : 0);
+  fft_dit<CG, C>(X, Yf, la, q5, tw, 1, la >= 3 ? 3 : 0);
   // Inverse transform by a forward one: conj(FFT(x))/M.  Autocorrelation: the spectrum
   // S = |FFT q|^2 is real, so its transform takes one of half length on z_k = S_2k + i S_2k+1
   // (each column on its own, so a crystallite's result does not depend on its neighbours):
   // with Z = FFT_{M/2}(z), E_p = (Z_p + conj Z_-p)/2, O_p = (Z_p - conj Z_-p)/(2i),
   // FFT(S)_p = E_p + w^p O_p and FFT(S)_{p+M/2} = E_p - w^p O_p, w = exp(-2 pi i / M).
   const int Mh = M / 2;
-  const bool half = autoc && M >= 4;
+  const bool half = autoc && la >= 2;
   const C *twb = tw;
   if (half) {
     auto spow = [&](int k, int cc, C &zo, C &) {
       const C xe = X[(2 * k) * CG + cc], xo = X[(2 * k + 1) * CG + cc];
       zo = mkc<C>(xe.x * xe.x + xe.y * xe.y, xo.x * xo.x + xo.y * xo.y);
     };
-    if (logM - 1 >= 3) {
-      fft_first_pass<CG, C>(Y, nullptr, Mh, logM - 1, twb, 2, spow);
-    } else {
-      for (int idx = threadIdx.x; idx < Mh * CG; idx += blockDim.x) {
-        const int cc = idx % CG, k = idx / CG;
-        C z, u;
-        spow(k, cc, z, u);
-        Y[int(__brev(unsigned(k)) >> (33 - logM)) * CG + cc] = z;
-      }
-      __syncthreads();
-    }
-    fft_dit<CG, C>(Y, nullptr, Mh, logM - 1, twb, 2, logM - 1 >= 3 ? 3 : 0);
+    if (la - 1 >= 3) fft_first_pass<CG, false>(Y, (C *)nullptr, la - 1, q5, twb, 2, spow);
+    else fft_load<CG>(Y, (C *)nullptr, la - 1, q5, spow);
+    fft_dit<CG, C>(Y, nullptr, la - 1, q5, twb, 2, la - 1 >= 3 ? 3 : 0);
   } else {
     // conj of the cross spectrum, in place in X (same index read and written)
     for (int idx = threadIdx.x; idx < M * CG; idx += blockDim.x) {
@@ -2095,22 +2165,15 @@ __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
     }
     __syncthreads();
     auto fromX = [&](int f, int cc, C &xo, C &) { xo = X[f * CG + cc]; };
-    if (logM >= 3) {
-      fft_first_pass<CG, C>(Y, nullptr, M, logM, tw, 1, fromX);
-    } else {
-      for (int idx = threadIdx.x; idx < M * CG; idx += blockDim.x) {
-        const int cc = idx % CG, f = idx / CG;
-        Y[int(__brev(unsigned(f)) >> (32 - logM)) * CG + cc] = X[idx];
-      }
-      __syncthreads();
-    }
-    fft_dit<CG, C>(Y, nullptr, M, logM, tw, 1, logM >= 3 ? 3 : 0);
+    if (la >= 3) fft_first_pass<CG, false>(Y, (C *)nullptr, la, q5, tw, 1, fromX);
+    else fft_load<CG>(Y, (C *)nullptr, la, q5, fromX);
+    fft_dit<CG, C>(Y, nullptr, la, q5, tw, 1, la >= 3 ? 3 : 0);
   }
   // transform of column cc at frequency p
   auto spec = [&](int p, int cc) -> C {
     if (!half) return Y[p * CG + cc];
-    const int q = p & (Mh - 1);
-    const C zp = Y[q * CG + cc], zm = cconj(Y[((Mh - q) & (Mh - 1)) * CG + cc]);
+    const int q = p < Mh ? p : p - Mh;
+    const C zp = Y[q * CG + cc], zm = cconj(Y[(q ? Mh - q : 0) * CG + cc]);
     const C ev = cscale(cadd(zp, zm), 0.5), d = csub(zp, zm);
     const C wo = cmul(twb[q], mkc<C>(0.5 * d.y, -0.5 * d.x));
     return p < Mh ? cadd(ev, wo) : csub(ev, wo);
@@ -2121,7 +2184,7 @@ __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
     for (int idx = threadIdx.x; idx < Mh * CG; idx += blockDim.x) {
       const int cc = idx % CG, q = idx / CG, c = c0 + cc;
       if (c >= s.C) continue;
-      const C zp = Y[q * CG + cc], zm = cconj(Y[((Mh - q) & (Mh - 1)) * CG + cc]);
+      const C zp = Y[q * CG + cc], zm = cconj(Y[(q ? Mh - q : 0) * CG + cc]);
       const C ev = cscale(cadd(zp, zm), 0.5), d = csub(zp, zm);
       const C wo = cmul(twb[q], mkc<C>(0.5 * d.y, -0.5 * d.x));
 #pragma unroll
@@ -2599,7 +2662,11 @@ struct JobImpl {
   std::vector<std::vector<int>> blocks_by_size;  // size -> list of block indices (size <= kMaxBlock)
   std::vector<int> big_blocks;                   // blocks kMaxBlock < b <= kMaxBigBlock
   std::vector<BigPair> big_pairs;                // Q/R pairs whose largest block is one of those
-  std::vector<int> huge_blocks;                  // blocks larger than kMaxBigBlock
+  // blocks on the batched products (bl_huge.cuh, bl_xs.cuh): those above kMaxBigBlock, and in the
+  // FP64 form those from kXsMin64 on (xs_from: the smallest)
+  std::vector<int> huge_blocks;
+  int xs_from = 0;
+  bool side = false;  // some blocks run on the auxiliary streams
   std::vector<int> huge_sq;                      // per huge block: squarings that bound every step's
   std::vector<BigPair> huge_pairs;               // Q/R pairs with a huge block
   size_t huge_ws_bytes = 0;                      // workspace of the huge-block products
@@ -2622,8 +2689,9 @@ struct JobImpl {
   DevBuf<double> fkc;                      // k_coef's term coefficients (small blocks)
   DevBuf<double2> frames;                  // rf schedule: per chunk frame (permuted index)
   DevBuf<float2> Tk_df, Hc_df;             // mixed form: double-float operators and constant parts
-  DevBuf<int> tk_ptr, tk_term, tk_order;  // tensor-core step: the operators' non-zeros by element
+  DevBuf<int> tk_ptr, tk_term, tk_order;  // blocks above kMaxBlock: the operators' non-zeros by element
   DevBuf<float2> tk_val;
+  DevBuf<double> tk_val64;
   DevBuf<double2> Dblk, Rhoblk;
   DevBuf<double2> U, A, VF, Lb, Q, R, G, Z, partial, fid, tw;
   DevBuf<float2> Wf, Qf, Rf, Gf, Zf, twf;  // mixed-precision form
@@ -2680,6 +2748,23 @@ static void planned_bytes(const JobSizing &plan, const Powder &pw, const FidPara
   if (full_bytes) *full_bytes = fixed + plan.per_c * size_t(plan.cpad);
 }
 
+// Length q 2^a of Fave's transforms: n itself when twisted (n a power of two), else the length
+// >= 2n of least work, per point 3 FP64 operations a radix-2 stage, about 7 for a radix-3 and 10 for
+// a radix-5 combining pass (n = 157: 320 points instead of 512).  Lengths of at most 4096 stay
+// there: a power of two is always tried.
+static void fave_length(int n, bool twist, int &q, int &a) {
+  q = 1, a = 1;
+  while ((1 << a) < (twist ? n : 2 * n)) ++a;
+  if (twist) return;
+  double best = double(1 << a) * 3.0 * a;
+  for (int t : {3, 5}) {
+    int b = 2;
+    while ((t << b) < 2 * n) ++b;
+    const double cost = double(t << b) * (3.0 * b + (t == 3 ? 7.0 : 10.0));
+    if (cost < best && (t << b) < (1 << a)) best = cost, q = t, a = b;
+  }
+}
+
 static float2 df_split(double v) {
   const float h = float(v);
   return make_float2(h, float(v - double(h)));
@@ -2687,6 +2772,11 @@ static float2 df_split(double v) {
 // term operators of up to this many elements in all go up dense
 constexpr size_t kDenseTerms = size_t(1) << 15;
 
+// Smallest block on the batched products in the FP64 form: 7 spins (blocks 21 and 35), 144
+// crystallites, n = 120: Dyson 14.6 -> 7.3 ms, eigenframe 14.3 -> 8.7, Q/R 13.3 -> 9.1 against the
+// FP64 tiles of k_big_*; below 20 a block fills less than a third of the 64-row tile.  The step stays
+// in k_big_step (18.5 ms there, 42 ms as batched products: seven matrices per item through HBM).
+constexpr int kXsMin64 = 20;
 // Which block pairs (a, b) of M hold a non-zero: one pass over M.
 static std::vector<char> nonzero_blocks(const CMatrix &M, const BlockLayout &L) {
   const size_t nb = L.size.size();
@@ -2988,6 +3078,24 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   // from k_coef, no rf schedule): the U slab of every (step, large block)
   J.tc = J.mixed && use_fk && p.step_method == 1 && !sched;
   size_t usl_per_c = 0;
+  // FP64 form: blocks from kXsMin64 on take the batched products too (Dyson, eigenframe, Q/R),
+  // with the buffer of the FID terms G, idle until Fave, as their workspace; where 32 crystallites'
+  // G would not hold two items of each use they stay with k_big_* (a rule on the job's shape, not
+  // on its crystallites)
+  int xs_from = kMaxBigBlock + 1;
+  if (!J.mixed && !J.is_static) {
+    size_t need = 0;
+    for (int k = 0; k < nb; ++k)
+      if (L.size[k] >= kXsMin64 && L.size[k] <= kMaxBigBlock)
+        need = std::max(need, sizeof(double2) * size_t(L.size[k]) * L.size[k]);
+    for (int pr = 0; pr < J.npq + J.npr; ++pr) {
+      const bool isq = pr < J.npq;
+      const int ba = L.size[isq ? qa[pr] : ra[pr - J.npq]], bb = L.size[isq ? qb[pr] : rb[pr - J.npq]];
+      need = std::max(need, sizeof(double2) * size_t(ba) * bb);
+    }
+    if (L.max_block <= kMaxBigBlock && size_t(J.n) * J.ne * sizeof(double2) * 32 >= 2 * need + 4096) xs_from = kXsMin64;
+  }
+  J.xs_from = xs_from;
   if (J.tc) {
     J.usl_off.assign(nb, 0);
     for (int k = 0; k < nb; ++k)
@@ -3073,7 +3181,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   J.blocks_by_size.assign(kMaxBlock + 1, {});
   for (int k = 0; k < nb; ++k) {
     if (L.size[k] <= kMaxBlock) J.blocks_by_size[L.size[k]].push_back(k);
-    else if (L.size[k] <= kMaxBigBlock) J.big_blocks.push_back(k);
+    else if (L.size[k] < xs_from) J.big_blocks.push_back(k);
     else J.huge_blocks.push_back(k);
   }
   // per huge block: squarings enough for every step, from a rotation-free bound on
@@ -3116,7 +3224,8 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   std::vector<int> big_rp_h, big_ci_h;
   std::vector<double2> big_cv_h;
   if (!J.big_blocks.empty() || !J.huge_blocks.empty()) {
-    if (!J.big_blocks.empty() && J.nint > kMaxInt)
+    if (std::any_of(L.size.begin(), L.size.end(), [](int b) { return b > kMaxBlock && b <= kMaxBigBlock; }) &&
+        J.nint > kMaxInt)
       throw Error(5, "more than " + std::to_string(kMaxInt) + " anisotropic interactions");
     const size_t csz = J.mixed ? sizeof(float2) : sizeof(double2);
     // Q/R pairs with a big block: M_ab's non-zeros by row, and the W_b column chunk that
@@ -3156,7 +3265,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
       int e2 = 0;
       std::frexp(most, &e2);  // most < 2^e2
       BigPair P{a, b, isq ? qoff[pr] : roff[pr - J.npq], isq ? J.nq : J.nr, isq ? 1 : 0, w, e2, nullptr, nullptr, nullptr, nullptr};
-      if (std::max(ba, bb) > kMaxBigBlock) {  // k_huge_mx + k_huge_zgemm
+      if (std::max(ba, bb) >= xs_from) {  // k_huge_mx + a product
         J.huge_pairs.push_back(P);
         J.huge_rp_off.push_back(rp_off);
         continue;
@@ -3166,8 +3275,9 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     }
   }
   ready_kernels(ctx);
-  if (!J.big_blocks.empty() && (!g_arena || g_arena->aux_streams)) {
-    const size_t naux = std::min<size_t>(4, std::max(J.big_blocks.size(), J.big_pairs.size()));
+  J.side = !J.big_blocks.empty() || (xs_from <= kMaxBigBlock && !J.huge_blocks.empty());
+  if (J.side && (!g_arena || g_arena->aux_streams)) {
+    const size_t naux = std::min<size_t>(4, std::max({J.big_blocks.size(), J.big_pairs.size(), J.huge_blocks.size()}));
     std::lock_guard<std::mutex> lock(ctx.mu);
     if (!ctx.fork_ev) CUDA_OK(cudaEventCreateWithFlags(&ctx.fork_ev, cudaEventDisableTiming));
     while (ctx.join_ev.size() < naux) {
@@ -3222,33 +3332,36 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     std::vector<float2> h(Hc.size());
     for (size_t x = 0; x < Hc.size(); ++x) h[x] = df_split(Hc[x]);
     up.add(J.Hc_df, h);
-    if (J.tc) {
-      // by element, terms ascending: a counting pass, then the entries in term order
-      std::vector<int> ptr(size_t(L.S2) + 1, 0), term(Tnz.size());
-      std::vector<float2> val(Tnz.size());
-      for (const TermEntry &e : Tnz) ++ptr[size_t(e.idx % L.S2) + 1];
-      for (int e = 0; e < L.S2; ++e) ptr[size_t(e) + 1] += ptr[e];
-      {
-        std::vector<int> at(ptr.begin(), ptr.end() - 1);
-        for (const TermEntry &e : Tnz) {
-          const int x = at[e.idx % L.S2]++;
-          term[x] = e.idx / L.S2, val[x] = df_split(e.v);
-        }
+  }
+  if (L.max_block > kMaxBlock) {
+    // by element, terms ascending: a counting pass, then the entries in term order
+    std::vector<int> ptr(size_t(L.S2) + 1, 0), term(Tnz.size());
+    std::vector<float2> val(df_tables ? Tnz.size() : 0);
+    std::vector<double> val64(Tnz.size());
+    for (const TermEntry &e : Tnz) ++ptr[size_t(e.idx % L.S2) + 1];
+    for (int e = 0; e < L.S2; ++e) ptr[size_t(e) + 1] += ptr[e];
+    {
+      std::vector<int> at(ptr.begin(), ptr.end() - 1);
+      for (const TermEntry &e : Tnz) {
+        const int x = at[e.idx % L.S2]++;
+        term[x] = e.idx / L.S2, val64[x] = e.v;
+        if (df_tables) val[x] = df_split(e.v);
       }
-      // per block, its elements by descending term count (ties in element order): the
-      // step's H build visits them in this order, so a warp's lanes walk similar lengths
-      std::vector<int> order(size_t(L.S2), 0);
-      for (size_t kb = 0; kb < L.size.size(); ++kb) {
-        const int b = L.size[kb], bp = L.poff[kb];
-        int *o = order.data() + bp;
-        for (int e = 0; e < b * b; ++e) o[e] = e;
-        std::stable_sort(o, o + b * b, [&](int x, int y) {
-          return ptr[bp + x + 1] - ptr[bp + x] > ptr[bp + y + 1] - ptr[bp + y];
-        });
-      }
-      up.add(J.tk_ptr, ptr), up.add(J.tk_term, term), up.add(J.tk_val, val);
-      up.add(J.tk_order, order);
     }
+    // per block, its elements by descending term count (ties in element order): the
+    // step's H build visits them in this order, so a warp's lanes walk similar lengths
+    std::vector<int> order(size_t(L.S2), 0);
+    for (size_t kb = 0; kb < L.size.size(); ++kb) {
+      const int b = L.size[kb], bp = L.poff[kb];
+      int *o = order.data() + bp;
+      std::vector<int> first(size_t(J.nint) + 2, 0);  // by term count, the largest first
+      auto bucket = [&](int e) { return size_t(J.nint - (ptr[bp + e + 1] - ptr[bp + e])); };
+      for (int e = 0; e < b * b; ++e) ++first[bucket(e) + 1];
+      for (int t = 0; t <= J.nint; ++t) first[size_t(t) + 1] += first[size_t(t)];
+      for (int e = 0; e < b * b; ++e) o[first[bucket(e)]++] = e;
+    }
+    up.add(J.tk_ptr, ptr), up.add(J.tk_term, term), up.add(J.tk_val, val), up.add(J.tk_val64, val64);
+    up.add(J.tk_order, order);
   }
   if (sched) {  // per chunk: the rf frame of each permuted index (1 where a chunk has none)
     bool any = false;
@@ -3286,16 +3399,15 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   DevSys &s = J.base;
   if (!J.p2p) {
     s.fave_twist = (!J.mixed && J.n >= 8 && (J.n & (J.n - 1)) == 0) ? 1 : 0;
-    s.logM = 1;
-    while ((1 << s.logM) < (s.fave_twist ? J.n : 2 * J.n)) ++s.logM;
-    s.M = 1 << s.logM;
+    fave_length(J.n, s.fave_twist != 0, s.fftq, s.logM);
+    s.M = s.fftq << s.logM;
     // FFT correlation up to M = 4096 (its shared-memory tile is M * max(1, 2048/M) * 32 B)
     if (p.fave_method == 2 && s.M > 4096) throw Error(5, "FFT Fave supports at most 2048 steps per period");
     s.fave_method = (p.fave_method != 1 && s.M <= 4096) ? 1 : 0;
     if (J.mixed && !s.fave_method) throw Error(5, "the mixed form needs the FFT correlation (at most 2048 steps)");
     if (s.fave_method) {
-      std::vector<double2> tw(s.M / 2);
-      for (int k = 0; k < s.M / 2; ++k) {
+      std::vector<double2> tw(s.M);
+      for (int k = 0; k < s.M; ++k) {
         double a = kPi2 * double(k) / double(s.M);
         tw[k] = make_double2(std::cos(a), -std::sin(a));
       }
@@ -3308,7 +3420,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
       }
     }
   } else {  // no Fave: the point-to-point terms come from Q/R and the Floquet phases
-    s.fave_twist = 0, s.logM = 0, s.M = 0, s.fave_method = 0;
+    s.fave_twist = 0, s.logM = 0, s.M = 0, s.fftq = 1, s.fave_method = 0;
   }
   up.flush(ctx, J.tables, !g_arena || g_arena->aux_streams);
   J.h2d = up.bytes();
@@ -3346,7 +3458,10 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     J.Q.alloc(nQ), J.R.alloc(nR), J.G.alloc(nG), J.Z.alloc(nZ);
   }
   J.partial.alloc(size_t(J.nwarps_total) * (J.mixed ? J.ft_r : 1) * p.npts);
-  if (J.huge_ws_bytes) {
+  if (!J.huge_blocks.empty() && xs_from <= kMaxBigBlock) {  // the workspace lies in G
+    J.huge_ws_bytes = J.G.n * sizeof(double2);
+    J.huge_ws.p = J.G.p, J.huge_ws.n = J.G.n, J.huge_ws.owned = false;
+  } else if (J.huge_ws_bytes) {
     J.huge_ws.alloc(J.huge_ws_bytes / sizeof(double2));
     J.hfk.alloc(size_t(J.huge_items) * std::max(J.nint, 1));
     J.hsq.alloc(size_t(J.huge_items));
@@ -3388,9 +3503,9 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     // (two when r = conj(q), three otherwise), 8 M for the spectrum product, 8 n for G
     // (length n with 6 flop per twisted point when n is a power of two, else length >= 2n)
     const bool twist = !J.mixed && J.n >= 8 && (J.n & (J.n - 1)) == 0;
-    int lm = 1;
-    while ((1 << lm) < (twist ? J.n : 2 * J.n)) ++lm;
-    double M = double(1 << lm), fftf = 5.0 * M * lm;
+    int fq = 1, lm = 1;
+    fave_length(J.n, twist, fq, lm);
+    double M = double(fq << lm), fftf = 5.0 * M * std::log2(M);
     bool fft = p.fave_method != 1 && M <= 4096;
     double per = 0;
     for (int e = 0; e < J.ne; ++e) {
@@ -3426,7 +3541,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   s.hc_chunks = sched ? J.pb : 0;
   s.frames = J.frames.n ? J.frames.p : nullptr;
   s.Tk_df = J.Tk_df.p, s.Hc_df = J.Hc_df.p;
-  s.tk_ptr = J.tk_ptr.p, s.tk_term = J.tk_term.p, s.tk_val = J.tk_val.p, s.tk_order = J.tk_order.p;
+  s.tk_ptr = J.tk_ptr.p, s.tk_term = J.tk_term.p, s.tk_val = J.tk_val.p, s.tk_val64 = J.tk_val64.p, s.tk_order = J.tk_order.p;
   s.fk_df = (J.mixed && p.step_method == 1 && use_fk) ? 1 : 0;
   {
     const double tp = J.tau * kPi2;
@@ -3603,8 +3718,9 @@ static void huge_step(JobImpl &J, DevSys &s, size_t kh) {
       }
       ++J.launches;
     };
-    k_huge_fk<<<unsigned((items + 127) / 128), 128, 0, st>>>(s, j0, items, J.hfk.p);
-    k_huge_hbuild<<<dim3(ge, unsigned(items)), 256, 0, st>>>(s, bp, b, J.hfk.p, ws, j0);
+    const bool own_fk = !s.fk || s.fk_df;  // k_coef's coefficients are absent or split into floats
+    if (own_fk) k_huge_fk<<<unsigned((items + 127) / 128), 128, 0, st>>>(s, j0, items, J.hfk.p);
+    k_huge_hbuild<<<dim3(ge, unsigned(items)), 256, 0, st>>>(s, bp, b, own_fk ? J.hfk.p : nullptr, ws, j0);
     k_huge_norm<<<unsigned(items), 256, 0, st>>>(ws, b, s.tau * kPi2, J.hsq.p);
     J.launches += 3;
     sym(0, 0, 1, 1.0, -1, false, 0, 0, 0, 0);  // Y = X X
@@ -3635,11 +3751,10 @@ static void huge_step(JobImpl &J, DevSys &s, size_t kh) {
 
 // The segments' products P_i = U_i P_{i-1} of huge block k (step t of every segment in one
 // launch), then the chain E_{s+1} = P_last(s) E_s; without segments the one chain of all steps.
-static void huge_dyson(JobImpl &J, DevSys &s, size_t kh) {
+static void huge_dyson(JobImpl &J, DevSys &s, size_t kh, cudaStream_t st) {
   const int k = J.huge_blocks[kh], b = J.L.size[k], bp = J.L.poff[k], n = J.n;
   const unsigned ge = unsigned((long(b) * b + 255) / 256);
   const int len = s.nseg > 1 ? kSegLen : n;
-  cudaStream_t st = J.ctx->stream;
   const size_t step = size_t(s.S2) * s.Cpad;
   k_huge_copy<<<dim3(ge, unsigned(s.C), unsigned(s.nseg)), 256, 0, st>>>(s, s.U, s.A, 0, 0, len, bp, b);
   ++J.launches;
@@ -3767,7 +3882,7 @@ static void launch_stage(JobImpl &J, DevSys &s, int stage) {
     k_coef<<<grid_for(long(s.Cpad) * s.n), kThreads, 0, J.ctx->stream>>>(s, J.fkc.p);
     ++J.launches;
   }
-  if (!J.big_blocks.empty()) fork(J);
+  if (J.side) fork(J);
   launch_block_kernels<1>(J, s, stage);
   launch_block_kernels<2>(J, s, stage);
   launch_block_kernels<3>(J, s, stage);
@@ -3839,15 +3954,33 @@ static void launch_stage(JobImpl &J, DevSys &s, int stage) {
   // large blocks on the auxiliary streams
   for (size_t kh = 0; kh < J.huge_blocks.size(); ++kh) {
     switch (stage) {
-      case 0: huge_step(J, s, kh); break;
-      case 1: huge_dyson(J, s, kh); break;
+      case 0:
+        if (J.xs_from <= kMaxBigBlock) {  // one fused kernel keeps its seven matrices in shared memory
+          const int k = J.huge_blocks[kh], b = J.L.size[k];
+          k_big_step<<<unsigned(s.C) * unsigned(s.n), unsigned((big_sym_tiles(b) + 31) / 32 * 32), big_step_smem(b),
+                       aux_stream(J, J.big_blocks.size() + kh)>>>(s, k);
+          ++J.launches;
+        } else {
+          huge_step(J, s, kh);
+        }
+        break;
+      case 1:  // (no workspace: the blocks run side by side)
+        huge_dyson(J, s, kh, J.xs_from <= kMaxBigBlock ? aux_stream(J, J.big_blocks.size() + kh) : J.ctx->stream);
+        break;
       case 2:
-        if (kh == 0) huge_floquet_all(J, s);
+        if (J.xs_from <= kMaxBigBlock) {  // fits shared memory
+          const int k = J.huge_blocks[kh], b = J.L.size[k];
+          k_big_floquet<<<unsigned(s.C), kBigThreads, sizeof(double2) * 2 * size_t(b) * b,
+                          aux_stream(J, J.big_blocks.size() + kh)>>>(s, k);
+          ++J.launches;
+        } else if (kh == 0) {
+          huge_floquet_all(J, s);
+        }
         break;
       case 3: huge_eigframe(J, s, kh); break;
     }
   }
-  if (!J.big_blocks.empty()) join(J);
+  if (J.side) join(J);
 }
 
 static void mark_begin(JobImpl &J, int stage);
@@ -3955,7 +4088,7 @@ void Job::run() {
       ++J.launches;
     } else if (J.ne > 0) {
       if (s.fave_method == 1) {
-        int cg = std::max(1, std::min(8, 2048 / s.M));
+        int cg = s.M <= 256 ? 8 : s.M <= 512 ? 4 : s.M <= 1024 ? 2 : 1;
         const size_t shm = sizeof(double2) * size_t(s.M) * cg * 2 + fave_twist_bytes(s, cg);
         const size_t shmf = sizeof(float2) * size_t(s.M) * cg * 2 + fave_twist_bytes(s, cg);
         unsigned grid = unsigned(J.ne) * unsigned(Cp / cg);

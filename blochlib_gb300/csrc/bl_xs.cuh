@@ -21,13 +21,14 @@
 // M = 128 tile, complex k is K entries 2k, 2k+1: A(r, l) = a + ib fills [[a, -b], [b, a]] and
 // B(l, n) = c + id the pair (c, d), so one real product per tile gives re and im in adjacent
 // tensor-memory lanes, and four complex elements are one 16-byte core-matrix row.
-// Pipeline: 16 warps convert K chunks of 32 entries into two shared-memory buffers (K-major, no
+// Pipeline: 31 warps convert K chunks of 32 entries into two shared-memory buffers (K-major, no
 // swizzle, 8-row groups padded by 16 bytes), one warp issues the products of a full buffer;
 // every wait is bounded (tc::wait_parity).
 namespace xs {
 
-constexpr int kConv = 512;           // converting threads (16 warps), then the issuing warp
-constexpr int kThreadsXs = kConv + 32;
+constexpr int kConv = 992;           // converting threads (31 warps), then the issuing warp: 32
+constexpr int kThreadsXs = kConv + 32;  // resident warps hide the integer chains' latency
+                                        // (with 544 threads the issue slots were 43 % busy)
 constexpr int kN = 64;               // output columns per tile
 constexpr int kK = 32;               // K entries (16 complex) per chunk
 constexpr int kGroup = kK * 16 + 16; // bytes of an 8-row group (tc::sbo_bytes(kK))
@@ -72,6 +73,15 @@ __device__ __forceinline__ float digit(long long w, int j) {
   const uint32_t word = byte < 4 ? uint32_t(w) : uint32_t((unsigned long long)w >> 32);
   const float f = __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u + uint32_t(byte & 3)));  // 2^23 + byte
   return __fmaf_rn(f, sc, -8388736.f * sc);
+}
+// warp-wide: 4 consecutive 32-bit columns of this thread's tensor-memory lane
+__device__ __forceinline__ void ld4(uint32_t taddr, float (&v)[4]) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[j]);
 }
 // two floats that are exact in BF16, packed (a in the low half)
 __device__ __forceinline__ uint32_t pack(float a, float b) {
@@ -237,20 +247,36 @@ __global__ void __launch_bounds__(xs::kThreadsXs, 1)
   __syncthreads();
   tc::fence_after();
   const bool fine = failed == 0;
-  if (fine && warp < kConv / 32) {
+  if (fine) {
     const bool nan = bad_s != 0;
     const int q4 = warp & 3, L = 32 * q4 + lane;  // tensor-memory lane: tile row
-    const int live = CPLX ? 2 * rows : rows;
-    if (32 * q4 < live) {  // warp-uniform
-      for (int c0 = 8 * (warp >> 2); c0 < cols; c0 += 32) {
-        float a[kLev][8];
+    const int live = CPLX ? 2 * rows : rows, c8 = 8 * (warp >> 2);
+    if (32 * q4 < live && c8 < cols) {  // warp-uniform
+#pragma unroll 1
+      for (int c0 = c8; c0 < c8 + 8; c0 += 4) {
+        float a[kLev][4];
         const uint32_t ta = tmem + (uint32_t(32 * q4) << 16) + uint32_t(c0);
 #pragma unroll
-        for (int l = 0; l < kLev; ++l) tc::ld8(ta + uint32_t(l * kN), a[l]);
-        tc::wait_ld();
-        double d[8];
+        for (int l = 0; l < kLev; ++l) ld4(ta + uint32_t(l * kN), a[l]);
+        double add[4] = {0, 0, 0, 0};
+        if constexpr (!CPLX) {  // the low terms, loaded together before anything is stored
+          if (ep.low && L < live) {
+            double y[3][4];
+            const int r = r0 + L;
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
+            for (int t = 0; t < 4; ++t) {
+              const long e = long(c) * O.cs + long(r) * O.ld + min(q0 + c0 + t, n - 1);
+              y[0][t] = ep.Y[e], y[1][t] = ep.Y2[e], y[2][t] = ep.Y3[e];
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+              add[t] = fma(ep.c3, y[2][t], fma(ep.c2, y[1][t], fma(ep.c1, y[0][t], r == q0 + c0 + t ? ep.c0 : 0.0)));
+          }
+        }
+        tc::wait_ld();
+        double d[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
           int I[7];
 #pragma unroll
           for (int l = 0; l < kLev; ++l) I[l] = __float2int_rn(a[l][t] * __uint_as_float(uint32_t(127 + 8 * l) << 23));
@@ -266,31 +292,24 @@ __global__ void __launch_bounds__(xs::kThreadsXs, 1)
           const bool odd = L & 1;
           const int r = r0 + (L >> 1);
 #pragma unroll
-          for (int t = 0; t < 8; t += 2) {
+          for (int t = 0; t < 4; t += 2) {
             const double send = odd ? d[t] : d[t + 1];
             const double got = __shfl_xor_sync(0xffffffffu, send, 1);
             const int q = q0 + c0 + t + (odd ? 1 : 0);
             if (L < live && q < n) O(c, sl, r, q) = odd ? make_double2(got, d[t + 1]) : make_double2(d[t], got);
           }
-        } else {
-          const int r = r0 + L;
-          if (L < live) {
+        } else if (L < live) {
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const int q = q0 + c0 + t;
-              if (q >= n) continue;
-              double v = ep.alpha == 1.0 ? d[t] : ep.alpha * d[t];
-              if (ep.low) {
-                const long e = long(c) * O.cs + long(r) * O.ld + q;
-                v += fma(ep.c3, ep.Y3[e], fma(ep.c2, ep.Y2[e], fma(ep.c1, ep.Y[e], r == q ? ep.c0 : 0.0)));
-              }
-              O(c, sl, r, q) = v;
-            }
+          for (int t = 0; t < 4; ++t) {
+            const int q = q0 + c0 + t;
+            double v = ep.alpha == 1.0 ? d[t] : ep.alpha * d[t];
+            if (ep.low) v += add[t];
+            if (q < n) O(c, sl, r0 + L, q) = v;
           }
         }
       }
     }
-  } else if (!fine) {
+  } else {
     if (tid == 0) atomicOr(status, kTcTimeout);
     tc::wait_parity(&done, 0);  // bounded: let products in flight drain before TMEM is freed
   }
