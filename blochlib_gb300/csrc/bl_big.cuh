@@ -164,8 +164,9 @@ __host__ __device__ constexpr size_t big_step_smem(int b) {
 // (||X||_inf <= 1/2) by its Taylor polynomial, then sq squarings.  Blocks above kBigPSMax
 // sum the series term by term up to the degree taylor_degree gives for the step's norm.
 // Blocks up to kBigPSMax evaluate the polynomial as cos X = C(Y), sin X = X S(Y), Y = X^2,
-// C and S of degree 7 in Y by Paterson-Stockmeyer with Y^4 (Y, Y^2, Y^3, Y^4, C, S, X S:
-// 7 real products); larger blocks accumulate the terms one product at a time (14).  All
+// C and S by Paterson-Stockmeyer with the power of Y that the step's degree needs (5 to 7 real
+// products; always 7 before: 5 spins, 320 crystallites, n = 157, step 2.58 -> 2.18 ms); larger
+// blocks accumulate the terms one product at a time (up to 14).  All
 // factors are polynomials in X, hence symmetric and commuting: products are symmetric
 // and only their upper triangles are computed (cta_mm_sym).
 __global__ void __launch_bounds__(1024) k_big_step(DevSys s, int k) {
@@ -229,30 +230,38 @@ __global__ void __launch_bounds__(1024) k_big_step(DevSys s, int k) {
     __syncthreads();
     cta_mm_sym(Y, Y, Y2, b, 1.0);
     __syncthreads();
-    cta_mm_sym(Y2, Y, Y3, b, 1.0);
-    cta_mm_sym(Y2, Y2, Y4, b, 1.0);
-    // c0 I + c1 Y + c2 Y^2 + c3 Y^3 at element e; cos: (-1)^j / (2j)!, sin: (-1)^j / (2j+1)!
-    auto low = [&](double c0, double c1, double c2, double c3, int e) {
-      const double d = (e / b == e % b) ? c0 : 0.0;
-      return fma(c3, Y3[e], fma(c2, Y2[e], fma(c1, Y[e], d)));
-    };
+    // the polynomials to the degree this step's norm needs (cos X: nterms / 2 in Y), at the fewest
+    // products: powers up to Y^2 serve degree 4 (5 products in all), Y^3 degree 6 (6), Y^4
+    // degree 7 (7).  P(Y) = low(Y) + top(Y) Y^m, top evaluated into T.
+    const int m = nterms <= 9 ? 2 : nterms <= 13 ? 3 : 4;
+    double *Ym = m == 2 ? Y2 : m == 3 ? Y3 : Y4;
+    if (m >= 3) cta_mm_sym(Y2, Y, Y3, b, 1.0);
+    if (m == 4) cta_mm_sym(Y2, Y2, Y4, b, 1.0);
     __syncthreads();
-    for (int e = threadIdx.x; e < bb; e += blockDim.x)
-      T[e] = low(1.0 / 40320, -1.0 / 3628800, 1.0 / 479001600, -1.0 / 87178291200.0, e);
-    __syncthreads();
-    cta_mm_sym(Y4, T, R, b, 1.0,
-                [&](int e, double v) { return v + low(1.0, -1.0 / 2, 1.0 / 24, -1.0 / 720, e); });
-    __syncthreads();
-    for (int e = threadIdx.x; e < bb; e += blockDim.x)
-      T[e] = low(1.0 / 362880, -1.0 / 39916800, 1.0 / 6227020800.0, -1.0 / 1307674368000.0, e);
-    __syncthreads();
-    // S(Y) over Y3 in place: element e's epilogue reads Y3[e] before the same thread writes it
-    cta_mm_sym(Y4, T, Y3, b, 1.0,
-                [&](int e, double v) { return v + low(1.0, -1.0 / 6, 1.0 / 120, -1.0 / 5040, e); });
-    __syncthreads();
+    double *S = m == 4 ? Y3 : Y4;  // S(Y): over Y^3 in place when Y^4 is the factor (element e's
+                                   // epilogue reads Y3[e] before the same thread writes it)
+    for (int pass = 0; pass < 2; ++pass) {
+      const bool sn = pass == 1;
+      auto cf = [&](int j) { return sn ? sin_coef(j) : cos_coef(j); };
+      const double t0 = cf(m), t1 = cf(m + 1), t2 = cf(m + 2), t3 = m >= 3 ? cf(m + 3) : 0.0;
+      const double l0 = cf(0), l1 = cf(1), l2 = cf(2), l3 = cf(3);
+      for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+        double v = fma(t2, Y2[e], fma(t1, Y[e], (e / b == e % b) ? t0 : 0.0));
+        if (m >= 3) v = fma(t3, Y3[e], v);
+        T[e] = v;
+      }
+      __syncthreads();
+      cta_mm_sym(Ym, T, sn ? S : R, b, 1.0, [&](int e, double v) {
+        v += fma(l1, Y[e], (e / b == e % b) ? l0 : 0.0);
+        if (m >= 3) v = fma(l2, Y2[e], v);
+        if (m == 4) v = fma(l3, Y3[e], v);
+        return v;
+      });
+      __syncthreads();
+    }
     I = Y;  // -sin X = -X S(Y)
-    cta_mm_sym(X, Y3, I, b, -1.0);
-    F0 = Y2, F1 = Y4, F2 = T;
+    cta_mm_sym(X, S, I, b, -1.0);
+    F0 = Y2, F1 = S == Y4 ? Y3 : Y4, F2 = T;
   } else {
     double *P = X + bb, *Q = P + bb;
     R = Q + bb, I = R + bb;
@@ -456,22 +465,17 @@ struct FloqWork {
   float2 *Kf;  // MIX: b x b single-precision K
 };
 
-// The parallel Jacobi sweeps of floquet_cta over K (Xk, element type KC) with V (Mm, FP64)
-// accumulating the rotations; returns convergence.  KC = double2: the FP64 form.  KC =
-// float2 (mixed form): K in single precision, the sweeps stop one sweep after
-// off(K)^2 <= 1e-10 diag(K)^2, and each rotation is scaled to c^2 + |s|^2 = 1 in FP64
-// before V takes it, so that V stays unitary to FP64 rounding.
-template <class KC>
-__device__ bool floquet_sweeps(KC *Xk, double2 *Mm, int b, int max_sweeps, const FloqWork &wk) {
-  using R = decltype(KC::x);
-  constexpr bool F32 = sizeof(R) == sizeof(float);
+// The parallel Jacobi sweeps of floquet_cta over K (Xk) with V (Mm) accumulating the rotations;
+// returns convergence.  The angles come from single precision and each rotation is scaled to
+// c^2 + |s|^2 = 1 in FP64, as in lanes_sweeps.
+__device__ bool floquet_sweeps(double2 *Xk, double2 *Mm, int b, int max_sweeps, const FloqWork &wk) {
   auto rot = [&](int t, int q) -> double2 & { return wk.rot[2 * t + q]; };
   auto rpair = [&](int t, int q) -> int & { return wk.rpair[2 * t + q]; };
   double *red = wk.red;
   const int bb = b * b;
   const int bq = b + (b & 1);  // players in the round-robin (one dummy when b is odd)
   const int np = bq / 2;
-  bool conv = false, polish = false;
+  bool conv = false;
   const int nw = (blockDim.x + 31) / 32, wid = threadIdx.x >> 5, lid = threadIdx.x & 31;
   for (int sweep = 0; sweep < max_sweeps && !conv; ++sweep) {
     // off(K)^2 and diag(K)^2: FP64 sums per thread, a fixed shuffle tree per warp, the warps'
@@ -479,7 +483,7 @@ __device__ bool floquet_sweeps(KC *Xk, double2 *Mm, int b, int max_sweeps, const
     double off = 0, dg = 0;
     for (int e = threadIdx.x; e < bb; e += blockDim.x) {
       const int r = e / b, q = e % b;
-      const double2 v = todbl(Xk[e]);
+      const double2 v = Xk[e];
       if (r < q) off += v.x * v.x + v.y * v.y;
       else if (r == q) dg += v.x * v.x;
     }
@@ -498,14 +502,7 @@ __device__ bool floquet_sweeps(KC *Xk, double2 *Mm, int b, int max_sweeps, const
     __syncthreads();
     const double offs = red[2 * nw], dgs = red[2 * nw + 1];
     __syncthreads();
-    if (F32) {  // offs, dgs are the same in every thread: polish too
-      const bool small = offs <= 1e-10 * dgs || offs == 0.0;
-      if (small && (polish || offs == 0.0)) {
-        conv = true;
-        break;
-      }
-      polish = polish || small;
-    } else if (offs <= 1e-34 * dgs || offs == 0.0) {
+    if (offs <= 1e-34 * dgs || offs <= 1e-60) {
       conv = true;
       break;
     }
@@ -520,23 +517,20 @@ __device__ bool floquet_sweeps(KC *Xk, double2 *Mm, int b, int max_sweeps, const
         rpair(t, 0) = p, rpair(t, 1) = q;
         rot(t, 0) = cmk(1, 0), rot(t, 1) = cmk(0, 0);
         if (q < b) {
-          const KC hpq = Xk[p * b + q];
-          const R ab = hypot(hpq.x, hpq.y);
-          if (ab != R(0)) {
-            const R phx = hpq.x / ab, phy = hpq.y / ab;
-            const R theta = R(0.5) * (Xk[q * b + q].x - Xk[p * b + p].x) / ab;
-            R tt;
-            if (fabs(theta) > R(F32 ? 1e18 : 1e100)) tt = R(0.5) / theta;  // theta^2 stays finite
-            else tt = copysign(R(1), theta) / (fabs(theta) + sqrt(fma(theta, theta, R(1))));
-            const R cc = rsqrt(fma(tt, tt, R(1)));
-            double cd = cc;
-            double2 sd = cmk(double(phx * (tt * cc)), double(phy * (tt * cc)));
-            if (F32) {
-              const double nn = 1.0 / sqrt(fma(cd, cd, fma(sd.x, sd.x, sd.y * sd.y)));
-              cd *= nn, sd = cscale(sd, nn);
-            }
-            rot(t, 0) = cmk(cd, 0.0);
-            rot(t, 1) = sd;
+          const float hx = float(Xk[p * b + q].x), hy = float(Xk[p * b + q].y);
+          const float ab = hypotf(hx, hy);
+          if (ab != 0.f) {
+            const float theta = 0.5f * float(Xk[q * b + q].x - Xk[p * b + p].x) / ab;
+            float tt;
+            if (fabsf(theta) > 1e18f) tt = 0.5f / theta;  // theta^2 stays finite
+            else tt = copysignf(1.f, theta) / (fabsf(theta) + sqrtf(fmaf(theta, theta, 1.f)));
+            const float cf = rsqrtf(fmaf(tt, tt, 1.f)), ts = tt * cf / ab;
+            const double cd = cf;
+            const double2 sd = cmk(hx * ts, hy * ts);
+            const double d = fma(cd, cd, fma(sd.x, sd.x, fma(sd.y, sd.y, -1.0)));
+            const double nn = fma(fma(0.375, d, -0.5), d, 1.0);
+            rot(t, 0) = cmk(cd * nn, 0.0);
+            rot(t, 1) = cscale(sd, nn);
           }
         }
       }
@@ -549,33 +543,23 @@ __device__ bool floquet_sweeps(KC *Xk, double2 *Mm, int b, int max_sweeps, const
         if (q >= b) continue;
         const double cc = rot(t, 0).x;
         const double2 sp = rot(t, 1), spc = cconj(sp);
-        if (rest < b) {
-          const R ccr = R(cc);
-          const KC spr = cxm(R(sp.x), R(sp.y)), spcr = cxm(R(spc.x), R(spc.y));
-          const KC xkp = Xk[kk * b + p], xkq = Xk[kk * b + q];
-          Xk[kk * b + p] = csub(cscale(xkp, ccr), cmul(spcr, xkq));
-          Xk[kk * b + q] = cadd(cmul(spr, xkp), cscale(xkq, ccr));
-        } else {
-          const double2 xkp = Mm[kk * b + p], xkq = Mm[kk * b + q];
-          Mm[kk * b + p] = csub(cscale(xkp, cc), cmul(spc, xkq));
-          Mm[kk * b + q] = cadd(cmul(sp, xkp), cscale(xkq, cc));
-        }
+        double2 *Z = rest < b ? Xk : Mm;
+        const double2 xkp = Z[kk * b + p], xkq = Z[kk * b + q];
+        Z[kk * b + p] = csub(cscale(xkp, cc), cmul(spc, xkq));
+        Z[kk * b + q] = cadd(cmul(sp, xkp), cscale(xkq, cc));
       }
       __syncthreads();
-      // rows p, q of K:  K <- G^H K; a non-trivial rotation then zeroes K_pq, K_qp and the
-      // imaginary parts of K_pp, K_qq (written by the items of columns p and q)
+      // rows p, q of K:  K <- G^H K, the diagonal kept real
       for (int e = threadIdx.x; e < np * b; e += blockDim.x) {
         const int t = e / b, kk = e % b;
         const int p = rpair(t, 0), q = rpair(t, 1);
         if (q >= b) continue;
-        const R cc = R(rot(t, 0).x);
-        const KC sp = cxm(R(rot(t, 1).x), R(rot(t, 1).y)), spc = cconj(sp);
-        const KC xpk = Xk[p * b + kk], xqk = Xk[q * b + kk];
-        KC np_ = csub(cscale(xpk, cc), cmul(sp, xqk)), nq_ = cadd(cmul(spc, xpk), cscale(xqk, cc));
-        if ((kk == p || kk == q) && !(rot(t, 1).x == 0.0 && rot(t, 1).y == 0.0)) {
-          if (kk == p) np_.y = R(0), nq_ = cxm(R(0), R(0));
-          else np_ = cxm(R(0), R(0)), nq_.y = R(0);
-        }
+        const double cc = rot(t, 0).x;
+        const double2 sp = rot(t, 1), spc = cconj(sp);
+        const double2 xpk = Xk[p * b + kk], xqk = Xk[q * b + kk];
+        double2 np_ = csub(cscale(xpk, cc), cmul(sp, xqk)), nq_ = cadd(cmul(spc, xpk), cscale(xqk, cc));
+        if (kk == p) np_.y = 0.0;
+        if (kk == q) nq_.y = 0.0;
         Xk[p * b + kk] = np_;
         Xk[q * b + kk] = nq_;
       }
@@ -585,12 +569,9 @@ __device__ bool floquet_sweeps(KC *Xk, double2 *Mm, int b, int max_sweeps, const
   return conv;
 }
 
-// sweeps0 < kMaxSweeps: the first pass only locates the spectrum (that many sweeps); the
-// second pass, with -1 in the widest gap of those eigenphases, always follows.  DFA: A_n is
-// double-float (mixed form).  K32: the sweeps run over a single-precision K (wk.Kf); the
-// eigenvalues stay FP64 Rayleigh quotients, whose error is quadratic in V's.
-template <bool DFA, bool K32>
-__device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk, int sweeps0 = kMaxSweeps) {
+// DFA: A_n is double-float (mixed form).
+template <bool DFA>
+__device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk) {
   constexpr bool dfA = DFA;
   __shared__ int piv_s;
   __shared__ double a_s;
@@ -678,16 +659,8 @@ __device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk, int swee
     __syncthreads();
     for (int e = threadIdx.x; e < b; e += blockDim.x) Xk[e * b + e].y = 0.0;
     __syncthreads();
-    const int max_sweeps = pass == 0 ? sweeps0 : kMaxSweeps;
-    bool conv;
-    if (K32) {
-      for (int e = threadIdx.x; e < bb; e += blockDim.x) wk.Kf[e] = make_float2(float(Xk[e].x), float(Xk[e].y));
-      __syncthreads();
-      conv = floquet_sweeps<float2>(wk.Kf, Mm, b, max_sweeps, wk);
-    } else {
-      conv = floquet_sweeps<double2>(Xk, Mm, b, max_sweeps, wk);
-    }
-    if (!conv && max_sweeps == kMaxSweeps) atomicOr(s.status, kNoConvergeFloquet);
+    const bool conv = floquet_sweeps(Xk, Mm, b, kMaxSweeps, wk);
+    if (!conv) atomicOr(s.status, kNoConvergeFloquet);
     // Rayleigh quotients lam_r = v_r^H U v_r
     for (int r = threadIdx.x; r < b; r += blockDim.x) {
       double2 acc = cmk(0, 0);
@@ -746,9 +719,9 @@ __global__ void __launch_bounds__(kBigThreads) k_big_floquet(DevSys s, int k) {
     floquet_cta_df(s, k, blockIdx.x, FloqWork{bsc, bsc + b * b, rot, fv, lam, rpair, red,
                                               reinterpret_cast<float2 *>(bsc + 2 * b * b)});
   } else if (s.mixed) {
-    floquet_cta<true, false>(s, k, blockIdx.x, FloqWork{bsc, bsc + b * b, rot, fv, lam, rpair, red, nullptr});
+    floquet_cta<true>(s, k, blockIdx.x, FloqWork{bsc, bsc + b * b, rot, fv, lam, rpair, red, nullptr});
   } else {
-    floquet_cta<false, false>(s, k, blockIdx.x, FloqWork{bsc, bsc + b * b, rot, fv, lam, rpair, red, nullptr});
+    floquet_cta<false>(s, k, blockIdx.x, FloqWork{bsc, bsc + b * b, rot, fv, lam, rpair, red, nullptr});
   }
 }
 
@@ -757,8 +730,10 @@ __global__ void __launch_bounds__(kBigThreads) k_big_floquet(DevSys s, int k) {
 // hi, lo; complex elements float4 = re.hi, im.hi, re.lo, im.lo), with the same tiling as the
 // FP64 kernels and sums as compensated dot products.
 
-// C = alpha A B for symmetric commuting A, B (upper tiles, mirrored), double-float.
-__device__ void cta_mm_sym_df(const float2 *A, const float2 *B, float2 *C, int m, float2 alpha) {
+// C = ep(e, A B) for symmetric commuting A, B (upper tiles, mirrored; e the upper element),
+// double-float.
+template <class EP>
+__device__ void cta_mm_sym_df(const float2 *A, const float2 *B, float2 *C, int m, EP ep) {
   const int tm = (m + 1) / 2;
   for (int t = threadIdx.x; t < big_sym_tiles(m); t += blockDim.x) {
     int ti, tj;
@@ -774,7 +749,7 @@ __device__ void cta_mm_sym_df(const float2 *A, const float2 *B, float2 *C, int m
       df_dot(c11, a1.x, a1.y, b1.x, b1.y);
     }
     auto put = [&](int i, int j, const DfAcc &v) {
-      const float2 x = dfv_mul(alpha, df_fin(v));
+      const float2 x = ep(i * m + j, df_fin(v));
       C[i * m + j] = x;
       if (i != j) C[j * m + i] = x;
     };
@@ -787,22 +762,26 @@ __device__ void cta_mm_sym_df(const float2 *A, const float2 *B, float2 *C, int m
   }
 }
 
-// 1/k for the Taylor terms, double-float
-static_assert(kTaylorTerms == 15, "inv_df covers the terms 2..15");
-__device__ __forceinline__ float2 inv_df(int kt) {
-  switch (kt) {
-    case 2: return dfv_const(1.0 / 2); case 3: return dfv_const(1.0 / 3); case 4: return dfv_const(1.0 / 4);
-    case 5: return dfv_const(1.0 / 5); case 6: return dfv_const(1.0 / 6); case 7: return dfv_const(1.0 / 7);
-    case 8: return dfv_const(1.0 / 8); case 9: return dfv_const(1.0 / 9); case 10: return dfv_const(1.0 / 10);
-    case 11: return dfv_const(1.0 / 11); case 12: return dfv_const(1.0 / 12); case 13: return dfv_const(1.0 / 13);
-    case 14: return dfv_const(1.0 / 14); default: return dfv_const(1.0 / 15);
-  }
-}
+// coefficients of cos X = sum c_j Y^j and sin X = X sum s_j Y^j (Y = X^2), double-float
+__constant__ float2 kCosDf[8] = {dfv_const(cos_coef(0)), dfv_const(cos_coef(1)), dfv_const(cos_coef(2)),
+                                 dfv_const(cos_coef(3)), dfv_const(cos_coef(4)), dfv_const(cos_coef(5)),
+                                 dfv_const(cos_coef(6)), dfv_const(cos_coef(7))};
+__constant__ float2 kInvDf[8] = {dfv_const(1.0),     dfv_const(1.0),     dfv_const(1.0 / 2), dfv_const(1.0 / 3),
+                                 dfv_const(1.0 / 4), dfv_const(1.0 / 5), dfv_const(1.0 / 6), dfv_const(1.0 / 7)};
+__constant__ float2 kSinDf[8] = {dfv_const(sin_coef(0)), dfv_const(sin_coef(1)), dfv_const(sin_coef(2)),
+                                 dfv_const(sin_coef(3)), dfv_const(sin_coef(4)), dfv_const(sin_coef(5)),
+                                 dfv_const(sin_coef(6)), dfv_const(sin_coef(7))};
 
 __host__ __device__ constexpr size_t big_step_df_smem(int b) { return sizeof(float2) * 5 * size_t(b) * size_t(b); }
 
 // One CTA per (crystallite, step): the large block's U_i in double-float: H from the hi/lo
-// tables, the series term by term to the degree taylor_degree gives at 2^-40, squarings.
+// tables, cos X and sin X to the degree K that taylor_degree gives at 2^-40 by
+// Paterson-Stockmeyer in Y^2 (Y = X^2): the degree-2 chunks c_2j + c_2j+1 Y (the highest one with
+// c_2j+2 Y^2 where the degree is even) by Horner's rule, so degree 2 of C or S takes no product
+// own, 4 one, 6 two; K = 9 takes 5 products where the series term by term takes 8 (8
+// spins, 1154 crystallites, n = 200, blocks of 28: all steps 193 -> 180 ms; up to K = 7 the series
+// is kept, 6 spins at n = 231 took 7.87 ms by it and 8.12 this way).  The sine comes first, so that X's
+// buffer is free for the cosine: five b x b buffers as before.
 __global__ void __launch_bounds__(1024) k_big_step_df(DevSys s, int k) {
   extern __shared__ __align__(16) unsigned char bsd[];
   __shared__ float2 fk[kMaxInt];
@@ -859,39 +838,85 @@ __global__ void __launch_bounds__(1024) k_big_step_df(DevSys s, int k) {
   __syncthreads();
   const float2 sc = scl;
   const int sq = nsq, K = nterms;
-  for (int e = threadIdx.x; e < bb; e += blockDim.x) {
-    const float2 x = dfv_mul(sc, X[e]);
-    X[e] = x, P[e] = x;
-    R[e] = make_float2((e / b == e % b) ? 1.f : 0.f, 0.f);
-    I[e] = make_float2(-x.x, -x.y);
-  }
+  const auto keep = [](int, float2 v) { return v; };
+  float2 *Y = R, *Y2 = I, *A = P, *B = Q;  // and X
+  for (int e = threadIdx.x; e < bb; e += blockDim.x) X[e] = dfv_mul(sc, X[e]);
   __syncthreads();
-  for (int kt = 2; kt <= K; ++kt) {
-    cta_mm_sym_df(P, X, Q, b, inv_df(kt));
-    __syncthreads();
-    const int m4 = kt & 3;
+  float2 *F[3];  // the three buffers that do not hold the result
+  if (K <= 7) {  // few terms: the series, one product a term (the chunks' sums would cost one product)
     for (int e = threadIdx.x; e < bb; e += blockDim.x) {
-      const float2 v = Q[e], nv = make_float2(-v.x, -v.y);
-      if (m4 == 2) R[e] = dfv_add(R[e], nv);
-      else if (m4 == 3) I[e] = dfv_add(I[e], v);
-      else if (m4 == 0) R[e] = dfv_add(R[e], v);
-      else I[e] = dfv_add(I[e], nv);
+      const float2 x = X[e];
+      P[e] = x, R[e] = make_float2((e / b == e % b) ? 1.f : 0.f, 0.f), I[e] = make_float2(-x.x, -x.y);
     }
-    float2 *t = P;
-    P = Q, Q = t;
     __syncthreads();
+    for (int kt = 2; kt <= K; ++kt) {
+      const float2 ik = kInvDf[kt];
+      const int m4 = kt & 3;
+      cta_mm_sym_df(P, X, Q, b, [&](int, float2 v) { return dfv_mul(ik, v); });
+      __syncthreads();
+      for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+        const float2 v = Q[e], nv = make_float2(-v.x, -v.y);
+        if (m4 == 2) R[e] = dfv_add(R[e], nv);
+        else if (m4 == 3) I[e] = dfv_add(I[e], v);
+        else if (m4 == 0) R[e] = dfv_add(R[e], v);
+        else I[e] = dfv_add(I[e], nv);
+      }
+      float2 *t = P;
+      P = Q, Q = t;
+      __syncthreads();
+    }
+    F[0] = P, F[1] = Q, F[2] = X;
+  } else {
+  cta_mm_sym_df(X, X, Y, b, keep);
+  __syncthreads();
+  cta_mm_sym_df(Y, Y, Y2, b, keep);
+  __syncthreads();
+  // sum_j coef_j Y^j, j <= d, in buffer u or v; returns which
+  auto poly = [&](const float2 *coef, int d, float2 *u, float2 *v) -> float2 * {
+    const int top = d >= 2 && d % 2 == 0 ? d / 2 - 1 : d / 2;  // chunk that starts the recurrence
+    const float2 zero = make_float2(0.f, 0.f);
+    const float2 c0 = coef[2 * top], c1 = 2 * top + 1 <= d ? coef[2 * top + 1] : zero,
+                 c2 = 2 * top + 2 <= d ? coef[2 * top + 2] : zero;
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+      float2 x = dfv_mul(c1, Y[e]);
+      if (2 * top + 2 <= d) x = dfv_add(x, dfv_mul(c2, Y2[e]));
+      u[e] = e / b == e % b ? dfv_add(x, c0) : x;
+    }
+    __syncthreads();
+    for (int t = top - 1; t >= 0; --t) {
+      const float2 l0 = coef[2 * t], l1 = coef[2 * t + 1];
+      cta_mm_sym_df(Y2, u, v, b, [&](int e, float2 x) {
+        x = dfv_add(x, dfv_mul(l1, Y[e]));
+        return e / b == e % b ? dfv_add(x, l0) : x;
+      });
+      __syncthreads();
+      float2 *w = u;
+      u = v, v = w;
+    }
+    return u;
+  };
+  {
+    float2 *S = poly(kSinDf, (K - 1) / 2, A, B);
+    I = S == A ? B : A;  // -sin X = -X S(Y)
+    cta_mm_sym_df(X, S, I, b, [](int, float2 v) { return make_float2(-v.x, -v.y); });
+    __syncthreads();
+    R = poly(kCosDf, K / 2, X, S);
   }
-  // squarings: (R + iI)^2 = (RR - II) + i 2RI, in P, Q, X
-  for (int t = 0; t < sq; ++t) {
-    cta_mm_sym_df(R, R, P, b, make_float2(1.f, 0.f));
-    cta_mm_sym_df(I, I, Q, b, make_float2(1.f, 0.f));
-    cta_mm_sym_df(R, I, X, b, make_float2(2.f, 0.f));
-    __syncthreads();
-    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
-      const float2 q = Q[e];
-      R[e] = dfv_add(P[e], make_float2(-q.x, -q.y)), I[e] = X[e];
+  F[0] = Y, F[1] = Y2, F[2] = R == X ? (I == A ? B : A) : X;
+  }
+  // squarings: (R + iI)^2 = (RR - II) + i 2RI, in the three other buffers
+  {
+    for (int t = 0; t < sq; ++t) {
+      cta_mm_sym_df(R, R, F[0], b, keep);
+      cta_mm_sym_df(I, I, F[1], b, keep);
+      cta_mm_sym_df(R, I, F[2], b, [](int, float2 v) { return make_float2(2.f * v.x, 2.f * v.y); });
+      __syncthreads();
+      for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+        const float2 q = F[1][e];
+        R[e] = dfv_add(F[0][e], make_float2(-q.x, -q.y)), I[e] = F[2][e];
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
   double2 *Ub = s.U + size_t(i) * s.S2 * s.Cpad;
   float4 *U4 = reinterpret_cast<float4 *>(Ub);
@@ -1280,16 +1305,27 @@ __device__ void floquet_cta_df(const DevSys &s, int k, int c, FloqWork wk, bool 
 }
 
 // ------------------------------------------------------------------ mixed form, 4 x 4 tiles
-// The mixed form's single-precision eigenframe with 4 x 4 output tiles per thread: 8 shared-memory loads per 16 complex multiply-adds (the 2 x 2 tiles of
-// cta_mm_cplx_regs take 4 per 4), one tile per thread (blocks up to 74: at most 19 x 19
-// tiles).  Same operands and the same sum per output element, in the same order.
+// The mixed form's single-precision eigenframe and Q/R: 4 x 4 output tiles per thread, operands
+// read as 16-byte vectors (two complex elements), 8 shared-memory vectors per 32 complex
+// multiply-adds (the 2 x 2 tiles of cta_mm_cplx_regs take 32 8-byte loads for them), one tile per
+// thread (blocks up to 74: at most 19 x 19 tiles).  Leading dimensions are multiples of four, so
+// that a tile's vectors stay inside its rows; what lies beyond an operand only enters outputs that
+// are not stored.  Same operands and the same sum per output element, in the same order, as with
+// the 2 x 2 tiles.  Measured on 8 spins, 1154 crystallites, n = 200: eigenframe 59.8 -> 42.9 ms,
+// Q/R 71.8 -> 62.6 ms.
 __host__ __device__ constexpr int big4_tiles(int m, int n) { return ((m + 3) / 4) * ((n + 3) / 4); }
 __host__ __device__ constexpr int big4_threads(int m, int n) { return (big4_tiles(m, n) + 31) / 32 * 32; }
+__host__ __device__ constexpr int up4(int x) { return (x + 3) / 4 * 4; }
 
-// acc (this thread's tile; zero when it has none) = op(A) B, op = ^H if CONJ_A
-template <bool CONJ_A>
-__device__ __forceinline__ void cta_mm_cplx4(const float2 *A, int lda, const float2 *B, int ldb, int m, int n, int k,
-                                             float2 (&acc)[4][4]) {
+__device__ __forceinline__ void ld_c2(const float2 *p, float2 &a, float2 &b) {
+  const float4 v = *reinterpret_cast<const float4 *>(p);
+  a = make_float2(v.x, v.y), b = make_float2(v.z, v.w);
+}
+
+// acc (this thread's tile) = A B: A row-major m x k (lda even, column k zero when k is odd), B
+// row-major k x n (ldb a multiple of four, row k zero when k is odd)
+__device__ __forceinline__ void cta_mm4(const float2 *A, int lda, const float2 *B, int ldb, int m, int n, int k,
+                                        float2 (&acc)[4][4]) {
   const int tm = (m + 3) / 4, tn = (n + 3) / 4, t = threadIdx.x;
 #pragma unroll
   for (int a = 0; a < 4; ++a)
@@ -1297,19 +1333,43 @@ __device__ __forceinline__ void cta_mm_cplx4(const float2 *A, int lda, const flo
     for (int b = 0; b < 4; ++b) acc[a][b] = make_float2(0.f, 0.f);
   if (t >= tm * tn) return;
   const int i0 = (t / tn) * 4, j0 = (t % tn) * 4;
-  int ii[4], jj[4];
+  const float2 *ap[4];
 #pragma unroll
-  for (int a = 0; a < 4; ++a) ii[a] = min(i0 + a, m - 1), jj[a] = min(j0 + a, n - 1);
-  for (int l = 0; l < k; ++l) {
+  for (int a = 0; a < 4; ++a) ap[a] = A + min(i0 + a, m - 1) * lda;
+  const float2 *bp = B + j0;
+  for (int l = 0; l < k; l += 2, bp += 2 * ldb) {
+    float2 av[4][2], bv[2][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) ld_c2(ap[a] + l, av[a][0], av[a][1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) ld_c2(bp + h * ldb, bv[h][0], bv[h][1]), ld_c2(bp + h * ldb + 2, bv[h][2], bv[h][3]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = cfma(av[a][h], bv[h][b], acc[a][b]);
+  }
+}
+// acc = A^H B, A row-major k x m (lda a multiple of four)
+__device__ __forceinline__ void cta_mm4_h(const float2 *A, int lda, const float2 *B, int ldb, int m, int n, int k,
+                                          float2 (&acc)[4][4]) {
+  const int tm = (m + 3) / 4, tn = (n + 3) / 4, t = threadIdx.x;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = make_float2(0.f, 0.f);
+  if (t >= tm * tn) return;
+  const float2 *ap = A + (t / tn) * 4, *bp = B + (t % tn) * 4;
+#pragma unroll 2
+  for (int l = 0; l < k; ++l, ap += lda, bp += ldb) {
     float2 av[4], bv[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) av[a] = CONJ_A ? cconj(A[l * lda + ii[a]]) : A[ii[a] * lda + l];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) bv[b] = B[l * ldb + jj[b]];
+    ld_c2(ap, av[0], av[1]), ld_c2(ap + 2, av[2], av[3]);
+    ld_c2(bp, bv[0], bv[1]), ld_c2(bp + 2, bv[2], bv[3]);
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = cfma(av[a], bv[b], acc[a][b]);
+      for (int b = 0; b < 4; ++b) acc[a][b] = cfmaconj(av[a], bv[b], acc[a][b]);
   }
 }
 template <class F>
@@ -1325,26 +1385,73 @@ __device__ __forceinline__ void cta_tiles4_store(int m, int n, const float2 (&ac
 }
 
 // One CTA per (crystallite, kSegLen steps): W_i = A_{i+1} V_F = P_i V_s (mixed form: high parts
-// of the double-float A, single-precision V and W), 4 x 4 tiles.
+// of the double-float A, single-precision V and W).
+__host__ __device__ constexpr size_t big_eigframe4_smem(int b) {
+  return sizeof(float2) * (size_t(b + 1) * up4(b) + size_t(b) * ((b + 1) / 2 * 2));
+}
 __global__ void __launch_bounds__(384) k_big_eigframe4(DevSys s, int k) {
   extern __shared__ __align__(16) unsigned char bsr4[];
   const int c = blockIdx.x % s.C, i0 = int(blockIdx.x / s.C) * kSegLen, i1 = min(s.n, i0 + kSegLen);
-  const int b = s.bs[k], bp = s.bpoff[k], bb = b * b;
-  float2 *Vs = reinterpret_cast<float2 *>(bsr4), *As = Vs + bb;
+  const int b = s.bs[k], bp = s.bpoff[k], bb = b * b, lv = up4(b), la = (b + 1) / 2 * 2;
+  float2 *Vs = reinterpret_cast<float2 *>(bsr4), *As = Vs + (b + 1) * lv;
   const bool seg = segmented(s, b);
   for (int e = threadIdx.x; e < bb; e += blockDim.x)
-    Vs[e] = frame_elem<float2>(s, seg, i0, seg ? big_at(s, b, bp, e, c) : at(bp + e, c, s.Cpad));
+    Vs[(e / b) * lv + e % b] = frame_elem<float2>(s, seg, i0, seg ? big_at(s, b, bp, e, c) : at(bp + e, c, s.Cpad));
+  for (int e = threadIdx.x; e < lv; e += blockDim.x) Vs[b * lv + e] = make_float2(0.f, 0.f);
+  if (la > b)
+    for (int r = threadIdx.x; r < b; r += blockDim.x) As[r * la + b] = make_float2(0.f, 0.f);
   float2 acc[4][4];
   for (int i = i0; i < i1; ++i) {
     const float4 *Ab4 = reinterpret_cast<const float4 *>(s.A + size_t(i) * s.S2 * s.Cpad);
     float2 *Wb = s.Wf + size_t(i) * s.S2 * s.Cpad;
     for (int e = threadIdx.x; e < bb; e += blockDim.x) {
       const float4 v = Ab4[big_at(s, b, bp, e, c)];
-      As[e] = make_float2(v.x, v.y);
+      As[(e / b) * la + e % b] = make_float2(v.x, v.y);
     }
     __syncthreads();
-    cta_mm_cplx4<false>(As, b, Vs, b, b, b, b, acc);
+    cta_mm4(As, la, Vs, lv, b, b, b, acc);
     cta_tiles4_store(b, b, acc, [&](int r, int q, float2 v) { Wb[big_at(s, b, bp, r * b + q, c)] = v; });
+    __syncthreads();
+  }
+}
+
+// k_big_qr in single precision for row blocks from kQr4Min on: W_a, a column chunk of W_b and of X =
+// M_ab W_b in shared memory, loaded by asynchronous copies, a warp per row.  Smaller row blocks
+// stay with the 2 x 2 tiles: 20 x 20 has 25 tiles of 4 x 4, one warp (6 spins: 2.01 ms by 2 x 2, 2.65
+// by 4 x 4).
+constexpr int kQr4Min = 40;
+__host__ __device__ constexpr size_t big_qr4_smem(int ba, int bb, int w) {
+  return sizeof(float2) * (size_t(ba) * up4(ba) + size_t(bb) * w + size_t(ba) * up4(w));
+}
+__global__ void __launch_bounds__(384) k_big_qr4(DevSys s, BigPair P) {
+  extern __shared__ __align__(16) unsigned char bsr4[];
+  const int c = blockIdx.x % s.C, i = blockIdx.x / s.C;
+  const int ba = s.bs[P.a], bb = s.bs[P.b], pa = s.bpoff[P.a], pb = s.bpoff[P.b];
+  const int w = P.wchunk, la = up4(ba), lx = up4(w);
+  const float2 *W = s.Wf + size_t(i) * s.S2 * s.Cpad;
+  float2 *Wa = reinterpret_cast<float2 *>(bsr4), *X = Wa + ba * la, *Wb = X + ba * lx;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;  // a warp per row
+  for (int r = warp; r < ba; r += nw)
+    for (int q = lane; q < ba; q += 32) cp_async8(&Wa[r * la + q], &W[big_at(s, ba, pa, r * ba + q, c)], 8);
+  float2 *ob = (P.isq ? s.Qf : s.Rf) + size_t(i) * P.nitems * s.Cpad;
+  float2 acc[4][4];
+  for (int q0 = 0; q0 < bb; q0 += w) {
+    const int wc = min(w, bb - q0);
+    for (int r = warp; r < bb; r += nw)
+      for (int q = lane; q < wc; q += 32) cp_async8(&Wb[r * w + q], &W[big_at(s, bb, pb, r * bb + q0 + q, c)], 8);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int l = warp; l < ba; l += nw) {
+      const int j0 = __ldg(P.rp + l), j1 = __ldg(P.rp + l + 1);
+      for (int q = lane; q < wc; q += 32) {
+        float2 x = make_float2(0.f, 0.f);
+        for (int j = j0; j < j1; ++j) x = cfma(pair_coef(P, j, x), Wb[__ldg(P.ci + j) * w + q], x);
+        X[l * lx + q] = x;
+      }
+    }
+    __syncthreads();
+    cta_mm4_h(Wa, la, X, lx, ba, wc, ba, acc);
+    cta_tiles4_store(ba, wc, acc, [&](int r, int q, float2 v) { ob[at(P.off + r * bb + q0 + q, c, s.Cpad)] = v; });
     __syncthreads();
   }
 }

@@ -185,6 +185,13 @@ __device__ __forceinline__ float4 cdf_fin(const CdfAcc &a) {
   return make_float4(r.x, m.x, r.y, m.y);
 }
 
+// 8-byte asynchronous copy global -> shared (cp.async); src_bytes 0 writes zeros
+__device__ __forceinline__ void cp_async8(void *dst, const void *src, int src_bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src),
+               "r"(src_bytes)
+               : "memory");
+}
+
 // ------------------------------------------------------------------ job description
 struct DevSys {
   int C, Cpad, n, npts, N, nb, S2, nint, nq, nr, ne, J, rosym, step_method;
@@ -238,7 +245,8 @@ struct DevSys {
   float2 *Wf, *Qf, *Rf, *Gf, *Zf;
   const float2 *twf;
   int warp_base;  // global warp index of this batch's first crystallite
-  int ft_jt, ft_pt, ft_r;  // k_fid_tiled: thread rows (4 j each), columns (4 p each), element ranges
+  // k_fid_tiled: thread rows (4 j each), columns (4 p each), element ranges, groups per CTA
+  int ft_jt, ft_pt, ft_r, ft_sub;
   int *status;
   unsigned long long *tc_flops;  // [2]: BF16 tensor flops issued by the step and Dyson kernels
   // 1: in the mixed form, A and W of the large blocks (kMaxBlock < b <= kMaxBigBlock) are
@@ -669,8 +677,56 @@ __device__ __forceinline__ void build_h_at(const DevSys &s, int c, double sp, do
   }
 }
 
-// Term coefficients of step i for every crystallite, once per (crystallite, step): the
-// small-block step kernels of all blocks read them instead of each recomputing them.
+// Fourier coefficients of the first-order terms over the rotor phase, one thread per (term,
+// crystallite): with the rows R_0, R_1, R_2 of R_powder and A_ij = R_i PAS' R_j, the rotor row
+// (sin phi sin b, -cos phi sin b, cos b) gives
+//   a(phi) = f0 + f1 cos phi + f2 sin phi + f3 cos 2 phi + f4 sin 2 phi.
+__global__ void __launch_bounds__(kThreads) k_term_series(DevSys s, double *series) {
+  const long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int c = int(tid % s.Cpad), kk = int(tid / s.Cpad);
+  if (kk >= s.nint || c >= s.C) return;
+  double R[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) R[i][j] = s.Rp[at(3 * i + j, c, s.Cpad)];
+  const double *P = s.pas + 6 * kk;
+  const double a00 = pas_form(P, R[0], R[0]), a01 = pas_form(P, R[0], R[1]), a02 = pas_form(P, R[0], R[2]),
+               a11 = pas_form(P, R[1], R[1]), a12 = pas_form(P, R[1], R[2]), a22 = pas_form(P, R[2], R[2]);
+  const double sc = s.iscale[kk], ss = s.sin_rotb * s.sin_rotb * sc, s2 = 2.0 * s.sin_rotb * s.cos_rotb * sc;
+  double *f = series + at(5 * kk, c, s.Cpad);
+  f[0] = fma(0.5 * ss, a00 + a11, s.cos_rotb * s.cos_rotb * sc * a22);
+  f[size_t(1) * s.Cpad] = -s2 * a12;
+  f[size_t(2) * s.Cpad] = s2 * a02;
+  f[size_t(3) * s.Cpad] = 0.5 * ss * (a11 - a00);
+  f[size_t(4) * s.Cpad] = -ss * a01;
+}
+
+// Term coefficients for every crystallite and step, once for all blocks.  Where every term is
+// first order and the crystallites start together (phase: cos, sin of phi and 2 phi per step,
+// from the host), a thread takes one term of one crystallite over kCoefRun steps: four FMAs a
+// coefficient from its Fourier series, against a sincos per step and about 20 FP64 operations per
+// coefficient otherwise (4 spins, 3722 crystallites, n = 128: the step stage 1.19 -> 1.08 ms).
+constexpr int kCoefRun = 16;
+__global__ void __launch_bounds__(kThreads) k_coef_series(DevSys s, const double *__restrict__ series,
+                                                         const double *__restrict__ phase, double *fk) {
+  const long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int c = int(tid % s.Cpad), kk = int(tid / s.Cpad % s.nint), i0 = int(tid / s.Cpad / s.nint) * kCoefRun;
+  if (i0 >= s.n || c >= s.C) return;
+  double f[5];
+#pragma unroll
+  for (int t = 0; t < 5; ++t) f[t] = series[at(5 * kk + t, c, s.Cpad)];
+  float2 *fk2 = reinterpret_cast<float2 *>(fk);
+  const int i1 = min(s.n, i0 + kCoefRun);
+  for (int i = i0; i < i1; ++i) {
+    const double2 p1 = *reinterpret_cast<const double2 *>(phase + 4 * i), p2 = *reinterpret_cast<const double2 *>(phase + 4 * i + 2);
+    const double v = fma(f[4], p2.y, fma(f[3], p2.x, fma(f[2], p1.y, fma(f[1], p1.x, f[0]))));
+    if (s.fk_df) fk2[at(i * s.nint + kk, c, s.Cpad)] = dfv_of(v);
+    else fk[at(i * s.nint + kk, c, s.Cpad)] = v;
+  }
+}
+
+// The same, step by step, for second-order terms or crystallites that start apart.
 __global__ void __launch_bounds__(kThreads) k_coef(DevSys s, double *fk) {
   long tid = long(blockIdx.x) * blockDim.x + threadIdx.x;
   const int c = int(tid % s.Cpad), i = int(tid / s.Cpad);
@@ -1299,20 +1355,234 @@ template <> struct LaneCx<float> { using type = float2; };
 __device__ __forceinline__ double2 cxm(double r, double i) { return make_double2(r, i); }
 __device__ __forceinline__ float2 cxm(float r, float i) { return make_float2(r, i); }
 
-//
-// T = double: the FP64 form.  T = float (mixed form): the Cayley transform and the sweeps
-// over K in single precision; the sweeps stop one sweep after off(K)^2 <= 1e-10 diag(K)^2
-// (quadratic convergence takes that to the float floor).  V accumulates the rotations in FP64,
-// each scaled to exact unitarity first: the FID's reconstruction takes V^-1 = V^H, which a
-// single-precision V (unitary to ~1e-7 per rotation) breaks by more than 1e-6.  The
-// eigenvalues stay FP64 Rayleigh quotients of the double-float A_n: their error is quadratic
-// in V's, so the phases that the FID carries over npts points keep FP64 accuracy.
+// K = Hermitian part of i (I+W)^{-1} (I-W), W = ea U, for the group's matrix (lane r holds row r):
+// Gaussian elimination with partial pivoting (first largest |M[i][k]|, i >= k) and back
+// substitution in T.  Returns kSingularCayley for a zero pivot; soft: such pivots (and those
+// below 1e-7, which single precision cannot tell from zero) are replaced by 1e-7 instead.
+template <int B, class T>
+__device__ __forceinline__ int lanes_cayley(const LaneGroup<B> &g, int r, const double2 (&U)[B], double2 ea,
+                                            typename LaneCx<T>::type (&K)[B], bool soft) {
+  using CT = typename LaneCx<T>::type;
+  int st = 0;
+  CT M[B], X[B];
+#pragma unroll
+  for (int q = 0; q < B; ++q) {
+    const double id = (q == r) ? 1.0 : 0.0;
+    if constexpr (sizeof(T) == sizeof(float)) {
+      const float2 w = cmul(cvt<float2>(ea), cvt<float2>(U[q]));
+      M[q] = cxm(T(id) + w.x, w.y), X[q] = cxm(T(id) - w.x, -w.y);
+    } else {
+      const double2 w = cmul(ea, U[q]);
+      M[q] = cxm(T(id + w.x), T(w.y)), X[q] = cxm(T(id - w.x), T(-w.y));
+    }
+  }
+#pragma unroll
+  for (int kc = 0; kc < B; ++kc) {
+    const T m2 = (r >= kc) ? M[kc].x * M[kc].x + M[kc].y * M[kc].y : T(-1);
+    int piv = kc;
+    T best = g.shfl(m2, kc);
+#pragma unroll
+    for (int i = kc + 1; i < B; ++i) {
+      const T v = g.shfl(m2, i);
+      if (v > best) best = v, piv = i;
+    }
+    if (best == T(0) && !soft) st |= kSingularCayley;
+    const int src = (r == kc) ? piv : (r == piv ? kc : r);
+#pragma unroll
+    for (int q = 0; q < B; ++q) M[q] = g.shfl(M[q], src), X[q] = g.shfl(X[q], src);
+    if (soft && best < T(1e-14) && r == kc) M[kc] = cxm(T(1e-7), T(0));
+    CT Mk[B], Xk[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q) Mk[q] = g.shfl(M[q], kc), Xk[q] = g.shfl(X[q], kc);
+    if (r > kc) {
+      const CT f = cmul(M[kc], cdiv(cxm(T(1), T(0)), Mk[kc]));
+#pragma unroll
+      for (int q = kc; q < B; ++q) M[q] = csub(M[q], cmul(f, Mk[q]));
+#pragma unroll
+      for (int q = 0; q < B; ++q) X[q] = csub(X[q], cmul(f, Xk[q]));
+    }
+  }
+  // back substitution, row kc on lane kc from the final rows below it
+#pragma unroll
+  for (int kc = B - 1; kc >= 0; --kc) {
+    CT acc[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q) acc[q] = X[q];
+#pragma unroll
+    for (int i = kc + 1; i < B; ++i) {
+      const CT mki = M[i];  // M[kc][i] on lane kc
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const CT xiq = g.shfl(X[q], i);
+        acc[q] = csub(acc[q], cmul(mki, xiq));
+      }
+    }
+    if (r == kc) {
+      const CT inv = cdiv(cxm(T(1), T(0)), M[kc]);
+#pragma unroll
+      for (int q = 0; q < B; ++q) X[q] = cmul(acc[q], inv);
+    }
+  }
+  // Hermitian part of i X (row r needs column r of X: X[q][r] from lane q)
+#pragma unroll
+  for (int q = 0; q < B; ++q) {
+    CT xqr = cxm(T(0), T(0));
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+      const CT v = g.shfl(X[t], q);
+      if (t == r) xqr = v;
+    }
+    const CT krq = cxm(-X[q].y, X[q].x), kqr = cxm(-xqr.y, xqr.x);
+    K[q] = cscale(cadd(krq, cconj(kqr)), T(0.5));
+    if (q == r) K[q].y = T(0);
+  }
+  return st;
+}
+
+// Parallel (round-robin) complex Jacobi sweeps over K, at most `sweeps`; with VEC, V (FP64)
+// accumulates the rotations from the identity.  The rotation angles come from single precision
+// in both forms (an FP64 hypot, three divisions and two square roots per rotation were more than
+// half of the kernel's FP64 instructions): a rotation that misses its angle by 1e-7 of it leaves
+// 1e-7 of the element, which the next sweep removes, so the sweep count stays.  Each rotation is
+// scaled to c^2 + |s|^2 = 1 in FP64 (n^-1/2 = 1 - d/2 + 3 d^2/8 for n = 1 + d, d ~ 1e-7), so V
+// stays unitary to FP64 rounding; K takes the scaled rotation in FP64 and the single-precision
+// one otherwise.  T = double stops at off(K)^2 <= 1e-34 diag(K)^2 (or 1e-60: K = tan(phase / 2), so
+// what is left is far below any phase); T = float one sweep after 1e-10 diag(K)^2 (quadratic
+// convergence takes that to the float floor).
+template <int B, class T, bool VEC>
+__device__ __forceinline__ bool lanes_sweeps(const LaneGroup<B> &g, int r, typename LaneCx<T>::type (&K)[B],
+                                             double2 (&V)[B], int sweeps) {
+  using CT = typename LaneCx<T>::type;
+  constexpr bool F32 = sizeof(T) == sizeof(float);
+  constexpr int BQ = B + (B & 1), NP = BQ / 2;  // round-robin players (one dummy when B is odd)
+  if (VEC) {
+#pragma unroll
+    for (int q = 0; q < B; ++q) V[q] = cmk(q == r ? 1.0 : 0.0, 0.0);
+  }
+  bool polish = false;
+  for (int sweep = 0; sweep < sweeps; ++sweep) {
+    T off = 0, dg = 0;
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      if (q > r) off += K[q].x * K[q].x + K[q].y * K[q].y;
+      if (q == r) dg += K[q].x * K[q].x;
+    }
+    T offs = 0, dgs = 0;
+#pragma unroll
+    for (int t = 0; t < B; ++t) offs += g.shfl(off, t), dgs += g.shfl(dg, t);
+    if (F32) {
+      const bool small = offs <= T(1e-10) * dgs || offs == T(0);
+      if (small && (polish || offs == T(0))) return true;
+      polish = polish || small;
+    } else if (offs <= T(1e-34) * dgs || offs <= T(1e-60)) {
+      return true;
+    }
+#pragma unroll
+    for (int round = 0; round < BQ - 1; ++round) {
+      // this lane's pair (mp, mq) of the round, or none
+      int mp = r, mq = r;
+      bool paired = false;
+#pragma unroll
+      for (int t = 0; t < NP; ++t) {
+        const int j1 = t, j2 = BQ - 1 - t;
+        int p = j1 == 0 ? 0 : 1 + (j1 - 1 + round) % (BQ - 1);
+        int q = j2 == 0 ? 0 : 1 + (j2 - 1 + round) % (BQ - 1);
+        if (p > q) { const int x = p; p = q; q = x; }
+        if (q < B && (r == p || r == q)) mp = p, mq = q, paired = true;
+      }
+      // the pair's rotation, computed identically by both of its lanes from K[p][q]
+      // (lane p's entry q), K[p][p] and K[q][q]
+      CT own_q = cxm(T(0), T(0)), own_d = cxm(T(0), T(0));
+#pragma unroll
+      for (int q2 = 0; q2 < B; ++q2) {
+        if (q2 == mq) own_q = K[q2];
+        if (q2 == r) own_d = K[q2];
+      }
+      const CT hpq = g.shfl(own_q, mp);
+      const T kpp = g.shfl(own_d.x, mp), kqq = g.shfl(own_d.x, mq);
+      float cf = 1.f, sx = 0.f, sy = 0.f;
+      if (paired) {
+        const float hx = float(hpq.x), hy = float(hpq.y);
+        const float ab = hypotf(hx, hy);
+        if (ab != 0.f) {
+          const float theta = 0.5f * float(kqq - kpp) / ab;
+          float tt;
+          if (fabsf(theta) > 1e18f) tt = 0.5f / theta;  // theta^2 stays finite
+          else tt = copysignf(1.f, theta) / (fabsf(theta) + sqrtf(fmaf(theta, theta, 1.f)));
+          cf = rsqrtf(fmaf(tt, tt, 1.f));
+          const float ts = tt * cf / ab;
+          sx = hx * ts, sy = hy * ts;
+        }
+      }
+      double cd = cf;
+      double2 sd = cmk(sx, sy);
+      if (VEC || !F32) {
+        const double d = fma(cd, cd, fma(sd.x, sd.x, fma(sd.y, sd.y, -1.0)));
+        const double nn = fma(fma(0.375, d, -0.5), d, 1.0);
+        cd *= nn, sd = cscale(sd, nn);
+      }
+      T cs;
+      CT sp;
+      if constexpr (F32) cs = cf, sp = cxm(sx, sy);
+      else cs = cd, sp = sd;
+      // columns p, q of K and V for every pair: K <- K G, V <- V G, G = [[c, sp], [-conj(sp), c]]
+#pragma unroll
+      for (int t = 0; t < NP; ++t) {
+        const int j1 = t, j2 = BQ - 1 - t;
+        int p = j1 == 0 ? 0 : 1 + (j1 - 1 + round) % (BQ - 1);
+        int q = j2 == 0 ? 0 : 1 + (j2 - 1 + round) % (BQ - 1);
+        if (p > q) { const int x = p; p = q; q = x; }
+        if (q >= B) continue;
+        const T cst = g.shfl(cs, p);
+        const CT spt = g.shfl(sp, p), spc = cconj(spt);
+        const CT kp = K[p], kq = K[q];
+        K[p] = csub(cscale(kp, cst), cmul(spc, kq));
+        K[q] = cadd(cmul(spt, kp), cscale(kq, cst));
+        if (VEC) {
+          double ct;
+          double2 st;
+          if constexpr (F32) ct = g.shfl(cd, p), st = g.shfl(sd, p);
+          else ct = cst, st = spt;
+          const double2 vp = V[p], vq = V[q];
+          V[p] = csub(cscale(vp, ct), cmul(cconj(st), vq));
+          V[q] = cadd(cmul(st, vp), cscale(vq, ct));
+        }
+      }
+      // rows p, q of K: K <- G^H K, as row = alpha row_p + beta row_q in every lane
+      // (lane p: cs, -sp; lane q: conj(sp), cs; a lane without a pair keeps its row)
+      const bool isp = paired && r == mp;
+      const CT al = isp ? cxm(cs, T(0)) : cconj(sp), be = isp ? cxm(-sp.x, -sp.y) : cxm(cs, T(0));
+#pragma unroll
+      for (int q2 = 0; q2 < B; ++q2) {
+        const CT kpk = g.shfl(K[q2], mp), kqk = g.shfl(K[q2], mq);
+        if (paired) {
+          // one of alpha, beta is real: the products differ between the lanes of a pair
+          const CT u = isp ? kpk : kqk, v = isp ? kqk : kpk, sg = isp ? be : al;
+          K[q2] = cadd(cscale(u, cs), cmul(sg, v));
+          if (q2 == r) K[q2].y = T(0);
+        }
+      }
+    }
+  }
+  return false;
+}
+
+// T = double: the FP64 form.  T = float (mixed form): the Cayley transform and the sweeps over K
+// in single precision, V in FP64 (the FID's reconstruction takes V^-1 = V^H, which a
+// single-precision V, unitary to ~1e-7 per rotation, breaks by more than 1e-6).  The eigenvalues
+// are FP64 Rayleigh quotients in both: their error is quadratic in V's, so the phases that the
+// FID carries over npts points keep FP64 accuracy.
+// The shift a has to keep every |1 + e^{ia} lambda| well above zero.  Phases near 0 (A_n near I, as
+// under fast spinning) take a = 1/2; otherwise -1 goes into the widest gap of the spectrum, found
+// by a single-precision pass without vectors (K's eigenvalues are tan((theta + a) / 2)) where a
+// full first pass found it before.  A second pass follows only if the first turns out badly
+// conditioned after all.  Measured, with the single-precision angles: a 4-block under rf, 677
+// crystallites, FP64 215 -> 100 us; 4 spins, 3722 crystallites, FP64 0.78 -> 0.58 ms, mixed 0.34 ->
+// 0.20 ms; one 3-spin crystallite 89 -> 63 us.
 template <int B, class T>
 __global__ void __launch_bounds__(kThreads) k_floquet_lanes(DevSys s, const int *__restrict__ blist, int nblist) {
   using CT = typename LaneCx<T>::type;
-  constexpr bool F32 = sizeof(T) == sizeof(float);
   constexpr int GPW = 32 / B;             // matrices per warp
-  constexpr int BQ = B + (B & 1), NP = BQ / 2;  // round-robin players (one dummy when B is odd)
   const int lane = threadIdx.x & 31;
   const long warp = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int gi = lane / B, r = lane % B;
@@ -1326,192 +1596,52 @@ __global__ void __launch_bounds__(kThreads) k_floquet_lanes(DevSys s, const int 
   const double2 *An = period_prop(s, B);
   const float4 *An4 = reinterpret_cast<const float4 *>(An);  // mixed form: double-float A
   double2 U[B], lam[B], V[B];  // V accumulates in FP64 in both forms
-  CT K[B];
 #pragma unroll
   for (int q = 0; q < B; ++q)
     U[q] = s.mixed ? df_load(An4[at(bp + r * B + q, c, s.Cpad)]) : An[at(bp + r * B + q, c, s.Cpad)];
   int st = 0;
   double a = 0.5;
+  float dev = 0.f;  // |A_n - I|_F^2
+#pragma unroll
+  for (int q = 0; q < B; ++q) {
+    const float2 u = cvt<float2>(U[q]);
+    dev = fmaf(u.y, u.y, fmaf(u.x - (q == r ? 1.f : 0.f), u.x - (q == r ? 1.f : 0.f), dev));
+  }
+  float devs = 0.f;
+#pragma unroll
+  for (int t = 0; t < B; ++t) devs += g.shfl(dev, t);
+  if (devs > 1.44f) {  // some phase may exceed 1.3: where to put -1, in single precision
+    float2 Kf[B];
+    lanes_cayley<B, float>(g, r, U, cmk(0.87758256189037271612, 0.47942553860420300027), Kf, true);  // e^{i/2}
+    lanes_sweeps<B, float, false>(g, r, Kf, V, 12);
+    float own = 0.f;
+#pragma unroll
+    for (int q = 0; q < B; ++q)
+      if (q == r) own = 2.f * atanf(Kf[q].x) - 0.5f;
+    if (own < -3.14159265f) own += 6.28318531f;
+    float th[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q) th[q] = g.shfl(own, q);
+#pragma unroll
+    for (int i = 1; i < B; ++i)
+#pragma unroll
+      for (int j = i; j > 0; --j)
+        if (th[j - 1] > th[j]) { const float x = th[j]; th[j] = th[j - 1]; th[j - 1] = x; }
+    float best = -1.f, mid = 0.f;
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      const float lo = th[q], hi = (q + 1 < B) ? th[q + 1] : th[0] + 6.28318531f;
+      if (hi - lo > best) best = hi - lo, mid = 0.5f * (lo + hi);
+    }
+    if (best > 0.f) a = kPi - double(mid);  // (not a number: the first shift stays)
+  }
   for (int pass = 0; pass < 2; ++pass) {
     double sa, ca;
     sincos(a, &sa, &ca);
     const double2 ea = cmk(ca, sa);
-    CT M[B], X[B];
-#pragma unroll
-    for (int q = 0; q < B; ++q) {
-      const double2 w = cmul(ea, U[q]);
-      const double id = (q == r) ? 1.0 : 0.0;
-      M[q] = cxm(T(id + w.x), T(w.y));
-      X[q] = cxm(T(id - w.x), T(-w.y));
-    }
-    // Gaussian elimination with partial pivoting (first largest |M[i][k]|, i >= k): M X' = X
-#pragma unroll
-    for (int kc = 0; kc < B; ++kc) {
-      const T m2 = (r >= kc) ? M[kc].x * M[kc].x + M[kc].y * M[kc].y : T(-1);
-      int piv = kc;
-      T best = g.shfl(m2, kc);
-#pragma unroll
-      for (int i = kc + 1; i < B; ++i) {
-        const T v = g.shfl(m2, i);
-        if (v > best) best = v, piv = i;
-      }
-      if (best == T(0)) st |= kSingularCayley;
-      const int src = (r == kc) ? piv : (r == piv ? kc : r);
-#pragma unroll
-      for (int q = 0; q < B; ++q) M[q] = g.shfl(M[q], src), X[q] = g.shfl(X[q], src);
-      CT Mk[B], Xk[B];
-#pragma unroll
-      for (int q = 0; q < B; ++q) Mk[q] = g.shfl(M[q], kc), Xk[q] = g.shfl(X[q], kc);
-      if (r > kc) {
-        const CT f = cmul(M[kc], cdiv(cxm(T(1), T(0)), Mk[kc]));
-#pragma unroll
-        for (int q = kc; q < B; ++q) M[q] = csub(M[q], cmul(f, Mk[q]));
-#pragma unroll
-        for (int q = 0; q < B; ++q) X[q] = csub(X[q], cmul(f, Xk[q]));
-      }
-    }
-    // back substitution, row kc on lane kc from the final rows below it
-#pragma unroll
-    for (int kc = B - 1; kc >= 0; --kc) {
-      CT acc[B];
-#pragma unroll
-      for (int q = 0; q < B; ++q) acc[q] = X[q];
-#pragma unroll
-      for (int i = kc + 1; i < B; ++i) {
-        const CT mki = M[i];  // M[kc][i] on lane kc
-#pragma unroll
-        for (int q = 0; q < B; ++q) {
-          const CT xiq = g.shfl(X[q], i);
-          acc[q] = csub(acc[q], cmul(mki, xiq));
-        }
-      }
-      if (r == kc) {
-        const CT inv = cdiv(cxm(T(1), T(0)), M[kc]);
-#pragma unroll
-        for (int q = 0; q < B; ++q) X[q] = cmul(acc[q], inv);
-      }
-    }
-    // K = Hermitian part of i X (row r needs column r of X: X[q][r] from lane q), V = I
-#pragma unroll
-    for (int q = 0; q < B; ++q) {
-      CT xqr = cxm(T(0), T(0));
-#pragma unroll
-      for (int t = 0; t < B; ++t) {
-        const CT v = g.shfl(X[t], q);
-        if (t == r) xqr = v;
-      }
-      const CT krq = cxm(-X[q].y, X[q].x), kqr = cxm(-xqr.y, xqr.x);
-      K[q] = cscale(cadd(krq, cconj(kqr)), T(0.5));
-      V[q] = cmk(q == r ? 1.0 : 0.0, 0.0);
-    }
-#pragma unroll
-    for (int q = 0; q < B; ++q)
-      if (q == r) K[q].y = T(0);
-    bool conv = false, polish = false;
-    for (int sweep = 0; sweep < kMaxSweeps && !conv; ++sweep) {
-      T off = 0, dg = 0;
-#pragma unroll
-      for (int q = 0; q < B; ++q) {
-        if (q > r) off += K[q].x * K[q].x + K[q].y * K[q].y;
-        if (q == r) dg += K[q].x * K[q].x;
-      }
-      T offs = 0, dgs = 0;
-#pragma unroll
-      for (int t = 0; t < B; ++t) offs += g.shfl(off, t), dgs += g.shfl(dg, t);
-      if (F32) {
-        const bool small = offs <= T(1e-10) * dgs || offs == T(0);
-        if (small && (polish || offs == T(0))) {
-          conv = true;
-          break;
-        }
-        polish = polish || small;
-      } else if (offs <= 1e-34 * dgs || offs == 0.0) {
-        conv = true;
-        break;
-      }
-#pragma unroll
-      for (int round = 0; round < BQ - 1; ++round) {
-        // this lane's pair (mp, mq) of the round, or none
-        int mp = r, mq = r;
-        bool paired = false;
-#pragma unroll
-        for (int t = 0; t < NP; ++t) {
-          const int j1 = t, j2 = BQ - 1 - t;
-          int p = j1 == 0 ? 0 : 1 + (j1 - 1 + round) % (BQ - 1);
-          int q = j2 == 0 ? 0 : 1 + (j2 - 1 + round) % (BQ - 1);
-          if (p > q) { const int x = p; p = q; q = x; }
-          if (q < B && (r == p || r == q)) mp = p, mq = q, paired = true;
-        }
-        // the pair's rotation, computed identically by both of its lanes from K[p][q]
-        // (lane p's entry q), K[p][p] and K[q][q]
-        CT own_q = cxm(T(0), T(0)), own_d = cxm(T(0), T(0));
-#pragma unroll
-        for (int q2 = 0; q2 < B; ++q2) {
-          if (q2 == mq) own_q = K[q2];
-          if (q2 == r) own_d = K[q2];
-        }
-        const CT hpq = g.shfl(own_q, mp);
-        const T kpp = g.shfl(own_d.x, mp), kqq = g.shfl(own_d.x, mq);
-        T cs = T(1);
-        CT sp = cxm(T(0), T(0));
-        if (paired) {
-          const T ab = hypot(hpq.x, hpq.y);
-          if (ab != T(0)) {
-            const CT ph = cxm(hpq.x / ab, hpq.y / ab);
-            const T theta = T(0.5) * (kqq - kpp) / ab;
-            T tt;
-            if (fabs(theta) > T(F32 ? 1e18 : 1e100)) tt = T(0.5) / theta;  // theta^2 stays finite
-            else tt = copysign(T(1), theta) / (fabs(theta) + sqrt(fma(theta, theta, T(1))));
-            cs = rsqrt(fma(tt, tt, T(1)));
-            sp = cscale(ph, tt * cs);
-          }
-        }
-        // columns p, q of K and V for every pair: K <- K G, V <- V G, G = [[c, sp], [-conj(sp), c]]
-#pragma unroll
-        for (int t = 0; t < NP; ++t) {
-          const int j1 = t, j2 = BQ - 1 - t;
-          int p = j1 == 0 ? 0 : 1 + (j1 - 1 + round) % (BQ - 1);
-          int q = j2 == 0 ? 0 : 1 + (j2 - 1 + round) % (BQ - 1);
-          if (p > q) { const int x = p; p = q; q = x; }
-          if (q >= B) continue;
-          const T cst = g.shfl(cs, p);
-          const CT spt = g.shfl(sp, p), spc = cconj(spt);
-          const CT kp = K[p], kq = K[q];
-          K[p] = csub(cscale(kp, cst), cmul(spc, kq));
-          K[q] = cadd(cmul(spt, kp), cscale(kq, cst));
-          // V in FP64; a single-precision rotation is first scaled to c^2 + |s|^2 = 1 in FP64,
-          // so that V stays unitary to FP64 rounding
-          double cd = cst;
-          double2 sd = todbl(spt);
-          if (F32) {
-            const double nn = 1.0 / sqrt(fma(cd, cd, fma(sd.x, sd.x, sd.y * sd.y)));
-            cd *= nn, sd = cscale(sd, nn);
-          }
-          const double2 vp = V[p], vq = V[q];
-          V[p] = csub(cscale(vp, cd), cmul(cconj(sd), vq));
-          V[q] = cadd(cmul(sd, vp), cscale(vq, cd));
-        }
-        // rows p, q of K: K <- G^H K, as row = alpha row_p + beta row_q in every lane
-        // (lane p: cs, -sp; lane q: conj(sp), cs; a lane without a pair keeps its row)
-        const bool isp = paired && r == mp;
-        const CT al = !paired ? cxm(T(1), T(0)) : (isp ? cxm(cs, T(0)) : cconj(sp));
-        const CT be = !paired ? cxm(T(0), T(0)) : (isp ? cxm(-sp.x, -sp.y) : cxm(cs, T(0)));
-#pragma unroll
-        for (int q2 = 0; q2 < B; ++q2) {
-          const CT kpk = g.shfl(K[q2], mp), kqk = g.shfl(K[q2], mq);
-          if (paired) K[q2] = cadd(cmul(al, kpk), cmul(be, kqk));
-        }
-        if (paired && !(sp.x == T(0) && sp.y == T(0))) {
-          const int other = isp ? mq : mp;
-#pragma unroll
-          for (int q2 = 0; q2 < B; ++q2) {
-            if (q2 == other) K[q2] = cxm(T(0), T(0));
-            if (q2 == r) K[q2].y = T(0);
-          }
-        }
-      }
-    }
-    if (!conv) st |= kNoConvergeFloquet;
+    CT K[B];
+    st |= lanes_cayley<B, T>(g, r, U, ea, K, false);
+    if (!lanes_sweeps<B, T, true>(g, r, K, V, kMaxSweeps)) st |= kNoConvergeFloquet;
     // Rayleigh quotients lam_r = v_r^H U v_r (columns of V), in every lane
     double2 uv[B];
 #pragma unroll
@@ -2019,10 +2149,11 @@ __device__ __forceinline__ float2 z_pow_f(float4 e, int j) {
 // |zeta| = 1, and zeta = e^{i tau Re w} is used there: exact when the chop has zeroed Im w,
 // otherwise G_p carries z e^{-n tau Im w} in place of z on its wrapped part (relative error
 // at most n tau |Im w|).
-template <int CG, class C>
+// POW2: M is a power of two (fftq = 1).
+template <int CG, class C, bool POW2>
 __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
   extern __shared__ __align__(16) unsigned char fsm_raw[];
-  const int M = s.M, la = s.logM, q5 = s.fftq, n = s.n;  // M = q5 2^la
+  const int M = s.M, la = s.logM, q5 = POW2 ? 1 : s.fftq, n = s.n;  // M = q5 2^la
   C *X = reinterpret_cast<C *>(fsm_raw), *Y = X + size_t(M) * CG;
   // twist tables per column: zeta^b (b < 8), zeta^8a (a < M/8), and those of zeta^-1
   double2 *tp1 = reinterpret_cast<double2 *>(Y + size_t(M) * CG), *tp8 = tp1 + 8 * CG;
@@ -2129,7 +2260,7 @@ __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
   const C *tw = Bufs<C>::tw(s);
   C *Yf = autoc ? nullptr : Y;
   if (la < 3) fft_load<CG>(X, Yf, la, q5, load);
-  else if (twist) fft_first_pass<CG, false>(X, Yf, la, q5, tw, 1, load);
+  else if (twist || (kF && CG < 8)) fft_first_pass<CG, false>(X, Yf, la, q5, tw, 1, load);
   else fft_first_pass<CG, true>(X, Yf, la, q5, tw, 1, load);  // q is zero from n <= M/2 on
   if constexpr (kF) {  // z^j, j < J, and z itself (the exponents were written before the first pass's barrier)
     for (int idx = threadIdx.x; idx < CG * (s.J + 1); idx += blockDim.x) {
@@ -2369,36 +2500,42 @@ __global__ void __launch_bounds__(kThreads) k_p2p_elems(DevSys s) {
 // asynchronous copies (coalesced: crystallites are fastest in HBM; double-buffered, so the
 // next element's copies are in flight while this one is summed), and each thread updates its
 // tile with w_c scale z, accumulating one element in FP32 and folding it into double-float
-// (hi + lo) sums.  The CTA writes its tile to partial row (warp * ft_r + range); k_reduce
+// (hi + lo) sums.  ft_sub groups of 64 threads each take a part of the
+// range and add up their double-float sums in order (one or two 64-thread CTAs an SM before where
+// there are few elements or crystallites: 4 spins, 3722 crystallites 0.315 -> 0.274 ms; 9 spins, 32
+// crystallites 11.5 -> 4.1 ms; 8 spins, 1154 crystallites 26.6 -> 22.7 ms).  The CTA writes its tile to partial row (warp * ft_r + range); k_reduce
 // sums the rows of the populated warps in a fixed order.  Each output's summation order
 // (crystallites 0..31 per element, elements in order within a range) depends on neither
 // the tile shape nor the batch, so a crystallite's contribution does not depend on its
 // neighbours.
 constexpr int kFtThreads = 64, kFtR = 16, kFtJmax = 32;
-// 8-byte asynchronous copy global -> shared (cp.async); src_bytes 0 writes zeros
-__device__ __forceinline__ void cp_async8(void *dst, const void *src, int src_bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src),
-               "r"(src_bytes)
-               : "memory");
-}
 // Dynamic shared memory of k_fid_tiled: two buffers of 32 crystallites x (4 jt + 4 pt).
-static size_t fid_tiled_smem(int jt, int pt) { return sizeof(float2) * 2 * 32 * 4 * size_t(jt + pt); }
-__global__ void __launch_bounds__(kFtThreads) k_fid_tiled(DevSys s) {
+// Groups per CTA: as many as leave their buffers within 200 KB.
+static int fid_tiled_sub(int jt, int pt) { return jt + pt <= 24 ? 4 : jt + pt <= 48 ? 2 : 1; }
+static size_t fid_tiled_smem(int jt, int pt) {  // (at least the sums handed over at the end)
+  const int sub = fid_tiled_sub(jt, pt);
+  return std::max(sizeof(float2) * 2 * 32 * 4 * size_t(jt + pt) * sub, sizeof(float4) * 16 * kFtThreads * size_t(sub - 1));
+}
+__global__ void __launch_bounds__(kFtThreads * 4) k_fid_tiled(DevSys s) {
   extern __shared__ __align__(16) float2 ftsm[];
   const int JT = 4 * s.ft_jt, PT = 4 * s.ft_pt;
-  float2 *zs = ftsm, *gs = ftsm + 2 * 32 * JT;  // [buffer][c][j], [buffer][c][p]
+  const int sub = threadIdx.x / kFtThreads;
+  float2 *zs = ftsm + size_t(sub) * 2 * 32 * (JT + PT), *gs = zs + 2 * 32 * JT;  // [buffer][c][j], [buffer][c][p]
   __shared__ float ws[32];
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x % kFtThreads;
   const int g = blockIdx.x;  // group of 32 crystallites in this batch
   const int npr = (s.gper + PT - 1) / PT;
   const int pr = blockIdx.y % npr, jr = blockIdx.y / npr, er = blockIdx.z;
   const int p0 = pr * PT, j0 = jr * JT;
-  const int e_lo = int((long(s.ne) * er) / s.ft_r), e_hi = int((long(s.ne) * (er + 1)) / s.ft_r);
+  const int parts = s.ft_r * s.ft_sub, part = er * s.ft_sub + sub;
+  const int e_lo = int((long(s.ne) * part) / parts), e_hi = int((long(s.ne) * (part + 1)) / parts);
   const int c0 = g * 32;
-  if (tid < 32) {
+  if (threadIdx.x < 32) {
     const int c = c0 + tid;
     ws[tid] = c < s.C ? float(s.w[c] * s.scale) : 0.f;
   }
+  __syncthreads();
+  auto sub_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(sub + 1), "n"(kFtThreads) : "memory"); };
   const bool active = tid < s.ft_jt * s.ft_pt;
   const int jt = active ? tid / s.ft_pt : 0, pt = active ? tid % s.ft_pt : 0;  // j0 + 4 jt + a, p0 + 4 pt + b
   float2 acc[4][4];
@@ -2431,7 +2568,7 @@ __global__ void __launch_bounds__(kFtThreads) k_fid_tiled(DevSys s) {
     } else {
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-    __syncthreads();
+    sub_sync();
     if (active) {
 #pragma unroll
       for (int a = 0; a < 4; ++a)
@@ -2463,9 +2600,29 @@ __global__ void __launch_bounds__(kFtThreads) k_fid_tiled(DevSys s) {
           hi[a][b] = make_float2(x.x, y.x), lo[a][b] = make_float2(x.y, y.y);
         }
     }
-    __syncthreads();  // the next stage() overwrites this buffer
+    sub_sync();  // the next stage() overwrites this buffer
     buf ^= 1;
   }
+  // the sub-ranges' sums, added in order by the first group
+  __syncthreads();
+  float4 *hand = reinterpret_cast<float4 *>(ftsm);
+  if (sub > 0) {
+#pragma unroll
+    for (int x = 0; x < 16; ++x)
+      hand[((sub - 1) * 16 + x) * kFtThreads + tid] =
+          make_float4(hi[x / 4][x % 4].x, hi[x / 4][x % 4].y, lo[x / 4][x % 4].x, lo[x / 4][x % 4].y);
+  }
+  __syncthreads();
+  if (sub > 0) return;
+  for (int u = 0; u < s.ft_sub - 1; ++u)
+#pragma unroll
+    for (int x = 0; x < 16; ++x) {
+      const float4 v = hand[(u * 16 + x) * kFtThreads + tid];
+      const int a = x / 4, b = x % 4;
+      const float2 re = dfv_add(make_float2(hi[a][b].x, lo[a][b].x), make_float2(v.x, v.z));
+      const float2 im = dfv_add(make_float2(hi[a][b].y, lo[a][b].y), make_float2(v.y, v.w));
+      hi[a][b] = make_float2(re.x, im.x), lo[a][b] = make_float2(re.y, im.y);
+    }
   if (!active) return;
   const long row = long(s.warp_base + g) * s.ft_r + er;
 #pragma unroll
@@ -2686,7 +2843,8 @@ struct JobImpl {
   DevBuf<int> ikind;
   int has2 = 0;  // second-order quadrupolar terms present
   int p2p = 0, pb = 1, pf = 1, psub = 1;  // point-to-point FID: base, factor, steps per chunk
-  DevBuf<double> fkc;                      // k_coef's term coefficients (small blocks)
+  DevBuf<double> fkc;                      // the term coefficients of every step
+  DevBuf<double> phase;                    // per step: cos, sin of the rotor phase and of twice it
   DevBuf<double2> frames;                  // rf schedule: per chunk frame (permuted index)
   DevBuf<float2> Tk_df, Hc_df;             // mixed form: double-float operators and constant parts
   DevBuf<int> tk_ptr, tk_term, tk_order;  // blocks above kMaxBlock: the operators' non-zeros by element
@@ -2806,10 +2964,16 @@ static void ready_kernels(Context &ctx) {
         (const void *)k_big_seg_frame<false>, (const void *)k_big_seg_frame<true>,
         (const void *)k_big_eigframe<1, double2>, (const void *)k_big_eigframe<2, double2>,
         (const void *)k_big_eigframe4, (const void *)k_big_floquet, (const void *)k_huge_floquet,
-        (const void *)k_big_qr<1, float2>, (const void *)k_big_qr<2, float2>, (const void *)k_big_qr<1, double2>,
-        (const void *)k_big_qr<2, double2>, (const void *)k_fave_fft<8, double2>, (const void *)k_fave_fft<4, double2>,
-        (const void *)k_fave_fft<2, double2>, (const void *)k_fave_fft<1, double2>, (const void *)k_fave_fft<8, float2>,
-        (const void *)k_fave_fft<4, float2>, (const void *)k_fave_fft<2, float2>, (const void *)k_fave_fft<1, float2>,
+        (const void *)k_big_qr4, (const void *)k_big_qr<1, float2>, (const void *)k_big_qr<1, double2>,
+        (const void *)k_big_qr<2, double2>,
+        (const void *)k_fave_fft<8, double2, true>, (const void *)k_fave_fft<8, double2, false>,
+        (const void *)k_fave_fft<8, float2, true>, (const void *)k_fave_fft<8, float2, false>,
+        (const void *)k_fave_fft<4, double2, true>, (const void *)k_fave_fft<4, double2, false>,
+        (const void *)k_fave_fft<4, float2, true>, (const void *)k_fave_fft<4, float2, false>,
+        (const void *)k_fave_fft<2, double2, true>, (const void *)k_fave_fft<2, double2, false>,
+        (const void *)k_fave_fft<2, float2, true>, (const void *)k_fave_fft<2, float2, false>,
+        (const void *)k_fave_fft<1, double2, true>, (const void *)k_fave_fft<1, double2, false>,
+        (const void *)k_fave_fft<1, float2, true>, (const void *)k_fave_fft<1, float2, false>,
         (const void *)k_fid_tiled, (const void *)k_xs_gemm<true, 6, false, double2>,
         (const void *)k_xs_gemm<true, 7, false, double2>, (const void *)k_xs_gemm<true, 7, true, double2>,
         (const void *)k_xs_gemm<false, 6, false, double>, (const void *)k_xs_gemm<false, 7, false, double>})
@@ -3227,7 +3391,6 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     if (std::any_of(L.size.begin(), L.size.end(), [](int b) { return b > kMaxBlock && b <= kMaxBigBlock; }) &&
         J.nint > kMaxInt)
       throw Error(5, "more than " + std::to_string(kMaxInt) + " anisotropic interactions");
-    const size_t csz = J.mixed ? sizeof(float2) : sizeof(double2);
     // Q/R pairs with a big block: M_ab's non-zeros by row, and the W_b column chunk that
     // keeps W_a, W_b and X within half the shared memory (two CTAs per SM) where it can
     for (int pr = 0; pr < J.npq + J.npr; ++pr) {
@@ -3248,7 +3411,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
       int nch = 1, w = bb;
       for (;;) {
         w = (bb + nch - 1) / nch;
-        if (csz * (size_t(ba) * ba + size_t(bb + ba) * w) <= (size_t(113) << 10) || w <= 8) break;
+        if ((J.mixed ? big_qr4_smem(ba, bb, w) : big_qr_smem<double2>(ba, bb, w)) <= (size_t(113) << 10) || w <= 8) break;
         ++nch;
       }
       double most = 1e-300;  // largest row or column sum of |M_ab|
@@ -3422,6 +3585,15 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   } else {  // no Fave: the point-to-point terms come from Q/R and the Floquet phases
     s.fave_twist = 0, s.logM = 0, s.M = 0, s.fftq = 1, s.fave_method = 0;
   }
+  // (the series' 5 nint doubles per crystallite have to fit A: n S2 complex)
+  if (use_fk && !J.has2 && J.gammaloop == 1 && size_t(5) * J.nint <= 2 * nsteps * L.S2) {
+    std::vector<double> ph(size_t(4) * J.n);
+    for (int i = 0; i < J.n; ++i) {
+      const double t1 = tmin + double(i) * J.tau, t2 = t1 + J.tau, a = ((t2 - t1) / 2.0 + t1) * p.wr * kPi2;
+      ph[4 * i] = std::cos(a), ph[4 * i + 1] = std::sin(a), ph[4 * i + 2] = std::cos(2 * a), ph[4 * i + 3] = std::sin(2 * a);
+    }
+    up.add(J.phase, ph);
+  }
   up.flush(ctx, J.tables, !g_arena || g_arena->aux_streams);
   J.h2d = up.bytes();
   s.tw = J.tw.p, s.twf = J.twf.p;
@@ -3528,6 +3700,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   s.scale = J.is_static ? 1.0 : double(1. / double(J.n / (J.rosym ? 2 : 1)));
   s.gper = J.n, s.p2p = J.p2p, s.pb = J.pb, s.pf = J.pf, s.psub = J.psub;
   s.ft_jt = J.ft_jt, s.ft_pt = J.ft_pt, s.ft_r = J.ft_r;
+  s.ft_sub = fid_tiled_sub(J.ft_jt, J.ft_pt);
   if (J.p2p) {  // fid = sum_c w_c Tr(rho_c det) / Tr(det det^H)  (sequencerun_funcs.cc:624-645)
     double dd = 0;
     for (const auto &v : det.a) dd += std::norm(v);
@@ -3879,7 +4052,15 @@ static void huge_qr(JobImpl &J, DevSys &s, const BigPair &P, C *Wbuf, C *out) {
 
 static void launch_stage(JobImpl &J, DevSys &s, int stage) {
   if (stage == 0 && s.fk) {  // the small blocks' term coefficients, before the streams fork
-    k_coef<<<grid_for(long(s.Cpad) * s.n), kThreads, 0, J.ctx->stream>>>(s, J.fkc.p);
+    if (J.phase.n) {
+      // the series' few values per crystallite wait in A, which the Dyson stage writes later
+      k_term_series<<<grid_for(long(s.Cpad) * s.nint), kThreads, 0, J.ctx->stream>>>(s, reinterpret_cast<double *>(s.A));
+      k_coef_series<<<grid_for(long(s.Cpad) * s.nint * ((s.n + kCoefRun - 1) / kCoefRun)), kThreads, 0, J.ctx->stream>>>(
+          s, reinterpret_cast<const double *>(s.A), J.phase.p, J.fkc.p);
+      ++J.launches;
+    } else {
+      k_coef<<<grid_for(long(s.Cpad) * s.n), kThreads, 0, J.ctx->stream>>>(s, J.fkc.p);
+    }
     ++J.launches;
   }
   if (J.side) fork(J);
@@ -3941,7 +4122,7 @@ static void launch_stage(JobImpl &J, DevSys &s, int stage) {
           ++J.launches;
         }
         if (s.mixed) {
-          k_big_eigframe4<<<unsigned(s.C) * unsigned(s.nseg), unsigned(big4_threads(b, b)), sw, st>>>(s, k);
+          k_big_eigframe4<<<unsigned(s.C) * unsigned(s.nseg), unsigned(big4_threads(b, b)), big_eigframe4_smem(b), st>>>(s, k);
         } else {
           if (nt1) k_big_eigframe<1, double2><<<unsigned(s.C) * unsigned(s.nseg), th, sw, st>>>(s, k);
           else k_big_eigframe<2, double2><<<unsigned(s.C) * unsigned(s.nseg), th, sw, st>>>(s, k);
@@ -4019,6 +4200,17 @@ static void launch_fid(const DevSys &s, long Cp, cudaStream_t st) {
   }
 }
 
+template <int CG>
+static void launch_fave(const DevSys &s, unsigned grid, size_t smem, cudaStream_t st) {
+  if (s.mixed) {
+    if (s.fftq == 1) k_fave_fft<CG, float2, true><<<grid, 128, smem, st>>>(s);
+    else k_fave_fft<CG, float2, false><<<grid, 128, smem, st>>>(s);
+  } else {
+    if (s.fftq == 1) k_fave_fft<CG, double2, true><<<grid, 128, smem, st>>>(s);
+    else k_fave_fft<CG, double2, false><<<grid, 128, smem, st>>>(s);
+  }
+}
+
 void Job::run() {
   JobImpl &J = *d_;
   CUDA_OK(cudaSetDevice(J.ctx->device));
@@ -4061,9 +4253,10 @@ void Job::run() {
         const unsigned grid = unsigned(s.C) * unsigned(J.n), th = big_threads(ba, P.wchunk);
         const bool nt1 = big_nt(ba, P.wchunk) == 1;
         if (s.mixed) {
-          const size_t sm = big_qr_smem<float2>(ba, bb, P.wchunk);
-          if (nt1) k_big_qr<1, float2><<<grid, th, sm, st>>>(s, P);
-          else k_big_qr<2, float2><<<grid, th, sm, st>>>(s, P);
+          if (ba >= kQr4Min)
+            k_big_qr4<<<grid, unsigned(big4_threads(ba, P.wchunk)), big_qr4_smem(ba, bb, P.wchunk), st>>>(s, P);
+          else  // at most 20 x 37 tiles
+            k_big_qr<1, float2><<<grid, th, big_qr_smem<float2>(ba, bb, P.wchunk), st>>>(s, P);
         } else {
           const size_t sm = big_qr_smem<double2>(ba, bb, P.wchunk);
           if (nt1) k_big_qr<1, double2><<<grid, th, sm, st>>>(s, P);
@@ -4093,22 +4286,10 @@ void Job::run() {
         const size_t shmf = sizeof(float2) * size_t(s.M) * cg * 2 + fave_twist_bytes(s, cg);
         unsigned grid = unsigned(J.ne) * unsigned(Cp / cg);
         switch (cg) {
-          case 8:
-            if (s.mixed) k_fave_fft<8, float2><<<grid, 128, shmf, st>>>(s);
-            else k_fave_fft<8, double2><<<grid, 128, shm, st>>>(s);
-            break;
-          case 4:
-            if (s.mixed) k_fave_fft<4, float2><<<grid, 128, shmf, st>>>(s);
-            else k_fave_fft<4, double2><<<grid, 128, shm, st>>>(s);
-            break;
-          case 2:
-            if (s.mixed) k_fave_fft<2, float2><<<grid, 128, shmf, st>>>(s);
-            else k_fave_fft<2, double2><<<grid, 128, shm, st>>>(s);
-            break;
-          default:
-            if (s.mixed) k_fave_fft<1, float2><<<grid, 128, shmf, st>>>(s);
-            else k_fave_fft<1, double2><<<grid, 128, shm, st>>>(s);
-            break;
+          case 8: launch_fave<8>(s, grid, s.mixed ? shmf : shm, st); break;
+          case 4: launch_fave<4>(s, grid, s.mixed ? shmf : shm, st); break;
+          case 2: launch_fave<2>(s, grid, s.mixed ? shmf : shm, st); break;
+          default: launch_fave<1>(s, grid, s.mixed ? shmf : shm, st); break;
         }
       } else {
         int ntile = (J.n + kFavePT - 1) / kFavePT;
@@ -4122,7 +4303,7 @@ void Job::run() {
     if (s.mixed) {
       const unsigned npr = unsigned((s.gper + 4 * s.ft_pt - 1) / (4 * s.ft_pt));
       const unsigned njr = unsigned((J.J + 4 * s.ft_jt - 1) / (4 * s.ft_jt));
-      k_fid_tiled<<<dim3(unsigned(Cp / 32), npr * njr, unsigned(s.ft_r)), kFtThreads,
+      k_fid_tiled<<<dim3(unsigned(Cp / 32), npr * njr, unsigned(s.ft_r)), kFtThreads * unsigned(s.ft_sub),
                     fid_tiled_smem(s.ft_jt, s.ft_pt), st>>>(s);
     } else {
       launch_fid(s, Cp, st);

@@ -298,7 +298,6 @@ __global__ void k_huge_mx(DevSys s, BigPair P, long j0, C *ws) {
 }
 
 constexpr int kHugeFloqThreads = 1024;
-constexpr int kHugeFloqSweeps0 = 4;  // first pass: locate the spectrum only
 constexpr int kMaxHugeLaunch = 16;   // huge blocks per Floquet launch
 
 __host__ __device__ constexpr size_t huge_floquet_smem(int b) {
@@ -331,6 +330,5 @@ __global__ void __launch_bounds__(kHugeFloqThreads) k_huge_floquet(DevSys s, Hug
                             reinterpret_cast<float2 *>(Mm + 2 * size_t(b) * b)},
                    true);
   else
-    floquet_cta<false, false>(s, k, c, FloqWork{Mm, Mm + size_t(b) * b, rot, fv, lam, rpair, red, nullptr},
-                              kHugeFloqSweeps0);
+    floquet_cta<false>(s, k, c, FloqWork{Mm, Mm + size_t(b) * b, rot, fv, lam, rpair, red, nullptr});
 }
