@@ -151,36 +151,53 @@ __host__ __device__ constexpr int pow2_cols(int c) {
 // Four natural-scale slices of the double-float x = hi + lo (|x| <= ~1), as floats (each an
 // integer times 2^-8j, exact in BF16).  Each residual d_j is exact (a rounded multiple of the
 // previous one's ulp, below 1/2 in size); lo enters every stage through one FMA.
+// Rounding to an integer adds and subtracts 1.5 2^23 (round to nearest even, as rintf, for
+// |x| < 2^22): the conversion instruction behind rintf runs at an eighth of the FP32 rate, and four
+// of them per element were the epilogues' largest single cost.
+__device__ __forceinline__ float round_int(float x) { return __fsub_rn(__fadd_rn(x, 12582912.f), 12582912.f); }
 __device__ __forceinline__ void slice4f(float hi, float lo, float (&q)[4]) {
-  const float q0 = rintf(hi * 256.f);
+  const float q0 = round_int(hi * 256.f);
   const float d0 = __fmaf_rn(hi, 256.f, -q0);
-  const float q1 = rintf(__fmaf_rn(lo, 65536.f, d0 * 256.f));
+  const float q1 = round_int(__fmaf_rn(lo, 65536.f, d0 * 256.f));
   const float d1 = __fmaf_rn(d0, 256.f, -q1);
-  const float q2 = rintf(__fmaf_rn(lo, 16777216.f, d1 * 256.f));
+  const float q2 = round_int(__fmaf_rn(lo, 16777216.f, d1 * 256.f));
   const float d2 = __fmaf_rn(d1, 256.f, -q2);
-  const float q3 = rintf(__fmaf_rn(lo, 4294967296.f, d2 * 256.f));
+  const float q3 = round_int(__fmaf_rn(lo, 4294967296.f, d2 * 256.f));
   q[0] = q0, q[1] = q1 * 0x1p-8f, q[2] = q2 * 0x1p-16f, q[3] = q3 * 0x1p-24f;
 }
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {  // a in the low half (lower address)
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t *>(&v);
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {  // a in the low half; both exact in BF16
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632u);
 }
-// Slices of 8 consecutive elements (one core-matrix row) stored as one 16-byte vector per
-// plane: planes at base + l * plane_elems (BF16 units), row offset o (a multiple of 8).
-__device__ __forceinline__ void store_row8(__nv_bfloat16 *base, int plane_elems, int o, const float (&hi)[8],
-                                           const float (&lo)[8]) {
+// Slices of 8 consecutive elements (one core-matrix row): one 16-byte vector per plane.
+struct Row8 {
+  uint4 v[4];
+};
+__device__ __forceinline__ Row8 slice_row8(const float (&hi)[8], const float (&lo)[8]) {
   float q[8][4];
+  Row8 r;
 #pragma unroll
   for (int j = 0; j < 8; ++j) slice4f(hi[j], lo[j], q[j]);
 #pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    uint4 v;
-    v.x = pack_bf16(q[0][l], q[1][l]);
-    v.y = pack_bf16(q[2][l], q[3][l]);
-    v.z = pack_bf16(q[4][l], q[5][l]);
-    v.w = pack_bf16(q[6][l], q[7][l]);
-    *reinterpret_cast<uint4 *>(base + size_t(l) * plane_elems + o) = v;
-  }
+  for (int l = 0; l < 4; ++l)
+    r.v[l] = make_uint4(pack_bf16(q[0][l], q[1][l]), pack_bf16(q[2][l], q[3][l]), pack_bf16(q[4][l], q[5][l]),
+                        pack_bf16(q[6][l], q[7][l]));
+  return r;
+}
+// the slices of the negated elements (rounding to nearest even is symmetric)
+__device__ __forceinline__ Row8 negated(Row8 r) {
+#pragma unroll
+  for (int l = 0; l < 4; ++l)
+    r.v[l].x ^= 0x80008000u, r.v[l].y ^= 0x80008000u, r.v[l].z ^= 0x80008000u, r.v[l].w ^= 0x80008000u;
+  return r;
+}
+// planes at base + l * plane_elems (BF16 units), row offset o (a multiple of 8)
+__device__ __forceinline__ void put_row8(__nv_bfloat16 *base, int plane_elems, int o, const Row8 &r) {
+#pragma unroll
+  for (int l = 0; l < 4; ++l) *reinterpret_cast<uint4 *>(base + size_t(l) * plane_elems + o) = r.v[l];
+}
+__device__ __forceinline__ void store_row8(__nv_bfloat16 *base, int plane_elems, int o, const float (&hi)[8],
+                                           const float (&lo)[8]) {
+  put_row8(base, plane_elems, o, slice_row8(hi, lo));
 }
 // (hi, lo) of a + b + c for FP32 a, b (exact sums) and c: Knuth's two-sum twice
 __device__ __forceinline__ float2 sum3(float a, float b, float c) {
@@ -639,8 +656,9 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
         if (r < b && q < b) x = dfv_mul(sc, H[q * b + r]);
         hi[j] = x.x, lo[j] = x.y;
       }
-      tc::store_row8(XS, peS, tc::tix(r, c0, R), hi, lo);
-      tc::store_row8(XS, peS, tc::tix(R + r, c0, R), hi, lo);
+      const tc::Row8 x8 = tc::slice_row8(hi, lo);
+      tc::put_row8(XS, peS, tc::tix(r, c0, R), x8);
+      tc::put_row8(XS, peS, tc::tix(R + r, c0, R), x8);
     }
   }
   tc::fence_smem_async();
@@ -1073,7 +1091,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_dyson_stk(DevSys s, in
         tc::ld8(ta + uint32_t(2 * R), v2);
         tc::wait_ld();
         if (live) {
-          float h[8], l[8], nh[8], nl[8];
+          float h[8], l[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int n = c0 + j;
@@ -1084,12 +1102,13 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_dyson_stk(DevSys s, in
               float *e = Ab + 4 * big_at(s, b, bp, n * b + m, c) + (is_im ? 1 : 0);
               e[0] = v.x, e[2] = v.y;
             }
-            h[j] = v.x, l[j] = v.y, nh[j] = -v.x, nl[j] = -v.y;
+            h[j] = v.x, l[j] = v.y;
           }
+          const tc::Row8 row = tc::slice_row8(h, l);
           // re row m: A1 row m, A2 row R + m negated; im row m: A1 row R + m, A2 row m
-          tc::store_row8(A1, peA, tc::tix(is_im ? R + m : m, c0, R), h, l);
-          if (is_im) tc::store_row8(A2, peA, tc::tix(m, c0, R), h, l);
-          else tc::store_row8(A2, peA, tc::tix(R + m, c0, R), nh, nl);
+          tc::put_row8(A1, peA, tc::tix(is_im ? R + m : m, c0, R), row);
+          if (is_im) tc::put_row8(A2, peA, tc::tix(m, c0, R), row);
+          else tc::put_row8(A2, peA, tc::tix(R + m, c0, R), tc::negated(row));
         }
       }
     }
