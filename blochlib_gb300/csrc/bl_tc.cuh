@@ -148,35 +148,42 @@ __host__ __device__ constexpr int pow2_cols(int c) {
   return c <= 32 ? 32 : c <= 64 ? 64 : c <= 128 ? 128 : c <= 256 ? 256 : 512;
 }
 
-// Four natural-scale slices of the double-float x = hi + lo (|x| <= ~1), as floats (each an
-// integer times 2^-8j, exact in BF16).  Each residual d_j is exact (a rounded multiple of the
-// previous one's ulp, below 1/2 in size); lo enters every stage through one FMA.
-// Rounding to an integer adds and subtracts 1.5 2^23 (round to nearest even, as rintf, for
-// |x| < 2^22): the conversion instruction behind rintf runs at an eighth of the FP32 rate, and four
-// of them per element were the epilogues' largest single cost.
-__device__ __forceinline__ float round_int(float x) { return __fsub_rn(__fadd_rn(x, 12582912.f), 12582912.f); }
-__device__ __forceinline__ void slice4f(float hi, float lo, float (&q)[4]) {
-  const float q0 = round_int(hi * 256.f);
-  const float d0 = __fmaf_rn(hi, 256.f, -q0);
-  const float q1 = round_int(__fmaf_rn(lo, 65536.f, d0 * 256.f));
-  const float d1 = __fmaf_rn(d0, 256.f, -q1);
-  const float q2 = round_int(__fmaf_rn(lo, 16777216.f, d1 * 256.f));
-  const float d2 = __fmaf_rn(d1, 256.f, -q2);
-  const float q3 = round_int(__fmaf_rn(lo, 4294967296.f, d2 * 256.f));
-  q[0] = q0, q[1] = q1 * 0x1p-8f, q[2] = q2 * 0x1p-16f, q[3] = q3 * 0x1p-24f;
+// x rounded to a multiple of 2^-P (nearest even) for |x| < 2^(22-P): adding and subtracting
+// 1.5 2^(23-P) (the conversion instructions run below the FP32 rate).
+template <int P>
+__device__ __forceinline__ float round_at(float x) {
+  constexpr float kMagic = P == 0 ? 12582912.f : P == 8 ? 49152.f : P == 16 ? 192.f : 0.75f;
+  return __fsub_rn(__fadd_rn(x, kMagic), kMagic);
+}
+// Four natural-scale slices (times 256) of the value h + l in units of 2^-8, |h| <= 256: multiples
+// of 1, 2^-8, 2^-16 and 2^-24 of at most 8 bits each, exact in BF16.  h and l need not be
+// normalised (|l| < 2^-2): l enters below the first slice, where every difference is exact but
+// the one that takes it in, rounded at 2^-34 or below.
+__device__ __forceinline__ void slice4f(float h, float l, float (&q)[4]) {
+  q[0] = round_at<0>(h);
+  float d = __fsub_rn(h, q[0]);
+  q[1] = round_at<8>(__fadd_rn(d, l));
+  d = __fadd_rn(__fsub_rn(d, q[1]), l);
+  q[2] = round_at<16>(d);
+  q[3] = round_at<24>(__fsub_rn(d, q[2]));
 }
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {  // a in the low half; both exact in BF16
   return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632u);
 }
-// Slices of 8 consecutive elements (one core-matrix row): one 16-byte vector per plane.
+// Slices of 8 consecutive elements (one core-matrix row), given as slice4f takes them: one 16-byte
+// vector per plane.
 struct Row8 {
   uint4 v[4];
 };
-__device__ __forceinline__ Row8 slice_row8(const float (&hi)[8], const float (&lo)[8]) {
+// dj: the element (if any) to add 256 to, the diagonal of I
+__device__ __forceinline__ Row8 slice_row8(const float (&hi)[8], const float (&lo)[8], int dj = -1) {
   float q[8][4];
   Row8 r;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) slice4f(hi[j], lo[j], q[j]);
+  for (int j = 0; j < 8; ++j) {
+    slice4f(hi[j], lo[j], q[j]);
+    if (j == dj) q[j][0] += 256.f;
+  }
 #pragma unroll
   for (int l = 0; l < 4; ++l)
     r.v[l] = make_uint4(pack_bf16(q[0][l], q[1][l]), pack_bf16(q[2][l], q[3][l]), pack_bf16(q[4][l], q[5][l]),
@@ -199,15 +206,21 @@ __device__ __forceinline__ void store_row8(__nv_bfloat16 *base, int plane_elems,
                                            const float (&lo)[8]) {
   put_row8(base, plane_elems, o, slice_row8(hi, lo));
 }
-// (hi, lo) of a + b + c for FP32 a, b (exact sums) and c: Knuth's two-sum twice
-__device__ __forceinline__ float2 sum3(float a, float b, float c) {
-  float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-  float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-  const float s2 = __fadd_rn(s, c);
-  bb = __fsub_rn(s2, s);
-  e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(s2, bb)), __fsub_rn(c, bb)));
-  const float h = __fadd_rn(s2, e);
-  return make_float2(h, __fsub_rn(e, __fsub_rn(h, s2)));
+// The three accumulators of a product as s + e (a0: integers, a1: multiples of 2^-8 below 2^15, a2:
+// of size ~2^3), the sum a0 + a1 exact: where |a1| > |a0| the rounded sum itself is, so three
+// operations do in either case.  a2 only meets e, at its own rounding's size.
+__device__ __forceinline__ float2 join(float a0, float a1, float a2) {
+  const float s = __fadd_rn(a0, a1);
+  return make_float2(s, __fadd_rn(__fsub_rn(a1, __fsub_rn(s, a0)), a2));
+}
+// coef v for slice4f (not normalised), coef carrying the units (2^-16 to 2^-8: 2^8 less)
+__device__ __forceinline__ float2 scaled(float2 coef, float2 v) {
+  const float p = __fmul_rn(coef.x, v.x);
+  return make_float2(p, __fmaf_rn(coef.y, v.x, __fmaf_rn(coef.x, v.y, __fmaf_rn(coef.x, v.x, -p))));
+}
+__device__ __forceinline__ float2 normal(float2 v) {
+  const float h = __fadd_rn(v.x, v.y);
+  return make_float2(h, __fsub_rn(v.y, __fsub_rn(h, v.x)));
 }
 
 // Issues the 10 slice pairs of one real product into the three accumulators at TMEM column
@@ -233,9 +246,9 @@ __device__ __forceinline__ void issue_product(uint32_t tmem, uint32_t col, uint3
   issue_product(tmem, col, a, pl, b, pl, R, negA, accumulate);
 }
 
-// -1 / (k (k + 1)) as double-float for the Horner steps (k = 1 .. 31), folded at compile time
+// -2^-8 / (k (k + 1)) (the units of slice4f) as double-float for the Horner steps (k = 1 .. 31), folded at compile time
 // into constant memory (k is the same in every thread), so that no epilogue divides in FP64
-#define BL_HC(k) dfv_const(-1.0 / (double(k) * double((k) + 1)))
+#define BL_HC(k) dfv_const(-0x1p-8 / (double(k) * double((k) + 1)))
 __constant__ float2 kHornerCoef[32] = {BL_HC(1),  BL_HC(1),  BL_HC(2),  BL_HC(3),  BL_HC(4),  BL_HC(5),  BL_HC(6),
                                        BL_HC(7),  BL_HC(8),  BL_HC(9),  BL_HC(10), BL_HC(11), BL_HC(12), BL_HC(13),
                                        BL_HC(14), BL_HC(15), BL_HC(16), BL_HC(17), BL_HC(18), BL_HC(19), BL_HC(20),
@@ -396,7 +409,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
   {  // X slices into the first tile: one 8-column row chunk per thread and iteration, rows
      // fastest (a warp's 16-byte row stores fill whole row groups: no bank conflicts), H read
      // down its columns (H is symmetric, its (r, q) and (q, r) sums alike), contiguous
-    const float2 sc = scl;
+    const float2 sc = make_float2(scl.x * 256.f, scl.y * 256.f);
     const int nch = R * (R / 8);
     for (int t = tid; t < nch; t += kTcThreads) {
       const int r = t % R, c0 = (t / R) * 8;
@@ -422,10 +435,10 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
   bool ok = true;
   const int q4 = warp & 3;  // this warp's TMEM lane quarter
   // Epilogue of accumulator set `set` over this thread's row and its 8-column chunks
-  // (chunk index part, part + nparts, ...): out = diag I + coef P with
+  // (chunk index part, part + nparts, ...): out = (I if diag) + 2^-8 coef P with
   // P = 2^-16 (acc0 + acc1 + acc23), or with `second` P = P_set0 - P_set1 (the squaring's
-  // C^2 - S^2); slices into tile dst, zero padding.
-  auto epilogue = [&](int set, float2 coef, float diag, bool second, __nv_bfloat16 *dst, int part, int nparts) {
+  // C^2 - S^2, exact level by level); slices into tile dst, zero padding.
+  auto epilogue = [&](int set, float2 coef, bool diag, bool second, __nv_bfloat16 *dst, int part, int nparts) {
     const int r = 32 * q4 + lane;
     if (32 * q4 >= R) return;  // warp-uniform: no stored row in this lane quarter
     for (int c0 = 8 * part; c0 < R; c0 += 8 * nparts) {
@@ -441,25 +454,15 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
         tc::ld8(tb + uint32_t(2 * R), b2);
       }
       tc::wait_ld();
-      if (r < R) {
+      if (r < R) {  // (the operands' padding is zero, and so are its products)
         float hi[8], lo[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int q = c0 + j;
-          float2 v = make_float2(0.f, 0.f);
-          if (r < b && q < b) {
-            const float2 p = tc::sum3(a0[j], a1[j], a2[j]);
-            v = make_float2(p.x * 0x1p-16f, p.y * 0x1p-16f);
-            if (second) {
-              const float2 p2 = tc::sum3(b0[j], b1[j], b2[j]);
-              v = dfv_add(v, make_float2(-p2.x * 0x1p-16f, -p2.y * 0x1p-16f));
-            }
-            v = dfv_mul(coef, v);
-            if (r == q) v = dfv_add(v, make_float2(diag, 0.f));
-          }
+          const float2 v = tc::scaled(coef, second ? tc::join(a0[j] - b0[j], a1[j] - b1[j], a2[j] - b2[j])
+                                                   : tc::join(a0[j], a1[j], a2[j]));
           hi[j] = v.x, lo[j] = v.y;
         }
-        tc::store_row8(dst, pe, tc::tix(r, c0, R), hi, lo);
+        tc::put_row8(dst, pe, tc::tix(r, c0, R), tc::slice_row8(hi, lo, diag && r < b ? r - c0 : -1));
       }
     }
   };
@@ -469,7 +472,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
       const int r = t / (R / 8), c0 = (t % (R / 8)) * 8;
       float hi[8], lo[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) hi[j] = (r < b && r == c0 + j) ? 1.f : 0.f, lo[j] = 0.f;
+      for (int j = 0; j < 8; ++j) hi[j] = (r < b && r == c0 + j) ? 256.f : 0.f, lo[j] = 0.f;
       tc::store_row8(dst, pe, tc::tix(r, c0, R), hi, lo);
     }
   };
@@ -486,7 +489,8 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
     tc::fence_after();
     return all;
   };
-  auto hcoef = [](int kk) { return tc::horner_coef(kk); };  // -1/(k(k+1)), double-float
+  auto hcoef = [](int kk) { return tc::horner_coef(kk); };  // -1/(k(k+1)) in slice units
+  const float2 one = make_float2(0x1p-8f, 0.f);
   __nv_bfloat16 *X = Bf[0], *Y = Bf[1], *TC = Bf[2], *TS = Bf[3];
   const uint32_t aX = ba[0], aY = ba[1], aTC = ba[2], aTS = ba[3];
   // Y = X X, then the innermost Horner terms straight from Y (all 16 warps)
@@ -496,10 +500,10 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
   }
   if (!wait_all(0)) ok = false;
   if (ok) {
-    epilogue(0, make_float2(1.f, 0.f), 0.f, false, Y, warp >> 2, 4);
-    if (mC >= 1) epilogue(0, hcoef(2 * mC - 1), 1.f, false, TC, warp >> 2, 4);
+    epilogue(0, one, false, false, Y, warp >> 2, 4);
+    if (mC >= 1) epilogue(0, hcoef(2 * mC - 1), true, false, TC, warp >> 2, 4);
     else identity(TC);
-    if (mS >= 1) epilogue(0, hcoef(2 * mS), 1.f, false, TS, warp >> 2, 4);
+    if (mS >= 1) epilogue(0, hcoef(2 * mS), true, false, TS, warp >> 2, 4);
     sync_all();
   }
   // The two Horner chains, each in its own group of 8 warps (two per lane quarter) with its
@@ -531,14 +535,14 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
     while (j >= 1) {
       if (tid == leader) tc::issue_product(tmem, set_col[set], aY, aT, pl, R, false, false), tc::commit(&mbar[set]);
       if (!wait_grp(set)) break;
-      epilogue(set, hcoef(grp == 0 ? 2 * j - 1 : 2 * j), 1.f, false, T, gpart, 2);
+      epilogue(set, hcoef(grp == 0 ? 2 * j - 1 : 2 * j), true, false, T, gpart, 2);
       --j;
       sync_grp();
     }
     if (grp == 1 && mS >= 1 && gfail[1] == 0) {
       if (tid == leader) tc::issue_product(tmem, set_col[1], aX, aTS, pl, R, false, false), tc::commit(&mbar[1]);
       if (wait_grp(1)) {
-        epilogue(1, make_float2(1.f, 0.f), 0.f, false, X, gpart, 2);
+        epilogue(1, one, false, false, X, gpart, 2);
         sync_grp();
       }
     }
@@ -568,14 +572,14 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
       ok = false;
       break;
     }
-    epilogue(0, make_float2(1.f, 0.f), 0.f, true, fr[0], warp >> 2, 4);
+    epilogue(0, one, false, true, fr[0], warp >> 2, 4);
     sync_all();
     if (tid == 0) tc::issue_product(tmem, set_col[0], aC, aS, pl, R, false, false), tc::commit(&mbar[0]);
     if (!wait_all(0)) {
       ok = false;
       break;
     }
-    epilogue(0, make_float2(2.f, 0.f), 0.f, false, fr[1], warp >> 2, 4);
+    epilogue(0, make_float2(0x1p-7f, 0.f), false, false, fr[1], warp >> 2, 4);
     sync_all();
     Ct = fr[0], aC = fa[0], St = fr[1], aS = fa[1];
   }
@@ -644,7 +648,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
   const int mC = K / 2;  // C to X^(2 mC), S to X^(2 mC + 1)
   {  // X slices into both halves of XS: one 8-column row chunk per thread and iteration, rows
      // fastest, H read down its columns (as in k_tc_step)
-    const float2 sc = scl;
+    const float2 sc = make_float2(scl.x * 256.f, scl.y * 256.f);
     const int nch = R * (R / 8);
     for (int t = tid; t < nch; t += kTcThreads) {
       const int r = t % R, c0 = (t / R) * 8;
@@ -676,11 +680,11 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
     __nv_bfloat16 *dst;
     int pe, row0;
     float2 coef;
-    float diag;
+    bool diag;
   };
   // Epilogue of a stacked product (accumulator set 0): each live lane's row P (2^-16 times
-  // the three accumulator levels, double-float) goes out as coef P + diag I into the outputs
-  // of its half, as slices (row row0 + m of dst, plane stride pe), zero padding.
+  // the three accumulator levels) goes out as 2^-8 coef P (+ I if diag) into the outputs of its
+  // half, as slices (row row0 + m of dst, plane stride pe), zero padding.
   auto epi = [&](const Out *o0, int n0, const Out *o1, int n1) {
     if (32 * q4 >= 2 * R) return;  // warp-uniform: no stacked row in this lane quarter
     const Out *o = bot ? o1 : o0;
@@ -693,25 +697,18 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
       tc::ld8(ta + uint32_t(2 * R), a2);
       tc::wait_ld();
       if (!live || no == 0) continue;
-      float2 P[8];
+      float2 P[8];  // (the operands' padding is zero, and so are its products)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float2 p = tc::sum3(a0[j], a1[j], a2[j]);
-        P[j] = (m < b && c0 + j < b) ? make_float2(p.x * 0x1p-16f, p.y * 0x1p-16f) : make_float2(0.f, 0.f);
-      }
+      for (int j = 0; j < 8; ++j) P[j] = tc::join(a0[j], a1[j], a2[j]);
       for (int u = 0; u < no; ++u) {
         float hi[8], lo[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int q = c0 + j;
-          float2 v = make_float2(0.f, 0.f);
-          if (m < b && q < b) {
-            v = dfv_mul(o[u].coef, P[j]);
-            if (m == q) v = dfv_add(v, make_float2(o[u].diag, 0.f));
-          }
+          const float2 v = tc::scaled(o[u].coef, P[j]);
           hi[j] = v.x, lo[j] = v.y;
         }
-        tc::store_row8(o[u].dst, o[u].pe, tc::tix(o[u].row0 + m, c0, R), hi, lo);
+        tc::put_row8(o[u].dst, o[u].pe, tc::tix(o[u].row0 + m, c0, R),
+                     tc::slice_row8(hi, lo, o[u].diag && m < b ? m - c0 : -1));
       }
     }
   };
@@ -728,7 +725,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
     tc::fence_after();
     return all;
   };
-  const float2 one = make_float2(1.f, 0.f), zero = make_float2(0.f, 0.f);
+  const float2 one = make_float2(0x1p-8f, 0.f), zero = make_float2(0.f, 0.f);
   // Y = X X (top and bottom halves alike); Y to Yt (when a chain step follows), the first
   // Horner terms T_C = I + c Y (to T, or straight to Yt as C when no chain step follows) and
   // T_S = I + c' Y (to T's bottom half); c = 0 when the series stops at the identity
@@ -739,9 +736,9 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
   if (!wait_all(0)) ok = false;
   if (ok) {
     const float2 cC = mC >= 1 ? tc::horner_coef(2 * mC - 1) : zero, cS = mC >= 1 ? tc::horner_coef(2 * mC) : zero;
-    const Out top2[2] = {{Yt, pe, 0, one, 0.f}, {T, peS, 0, cC, 1.f}};
-    const Out top1[1] = {{Yt, pe, 0, cC, 1.f}};
-    const Out bot1[1] = {{T, peS, R, cS, 1.f}};
+    const Out top2[2] = {{Yt, pe, 0, one, false}, {T, peS, 0, cC, true}};
+    const Out top1[1] = {{Yt, pe, 0, cC, true}};
+    const Out bot1[1] = {{T, peS, R, cS, true}};
     if (mC >= 2) epi(top2, 2, bot1, 1);
     else epi(top1, 1, bot1, 1);
     sync_all();
@@ -757,8 +754,8 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
       ok = false;
       break;
     }
-    const Out top[1] = {{j > 1 ? T : Yt, j > 1 ? peS : pe, 0, tc::horner_coef(2 * j - 1), 1.f}};
-    const Out btm[1] = {{T, peS, R, tc::horner_coef(2 * j), 1.f}};
+    const Out top[1] = {{j > 1 ? T : Yt, j > 1 ? peS : pe, 0, tc::horner_coef(2 * j - 1), true}};
+    const Out btm[1] = {{T, peS, R, tc::horner_coef(2 * j), true}};
     epi(top, 1, btm, 1);
     sync_all();
   }
@@ -770,7 +767,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
     }
     if (!wait_all(0)) ok = false;
     if (ok) {
-      const Out btm[1] = {{Wt, pe, 0, one, 0.f}};
+      const Out btm[1] = {{Wt, pe, 0, one, false}};
       epi(nullptr, 0, btm, 1);
       sync_all();
     }
@@ -801,17 +798,8 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
         float hi[8], lo[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int q = c0 + j;
-          float2 v = make_float2(0.f, 0.f);
-          if (r < b && q < b) {
-            const float2 p = tc::sum3(a0[j], a1[j], a2[j]);
-            v = make_float2(p.x * 0x1p-16f, p.y * 0x1p-16f);
-            if (second) {
-              const float2 p2 = tc::sum3(b0[j], b1[j], b2[j]);
-              v = dfv_add(v, make_float2(-p2.x * 0x1p-16f, -p2.y * 0x1p-16f));
-            }
-            v = dfv_mul(coef, v);
-          }
+          const float2 v = tc::scaled(coef, second ? tc::join(a0[j] - b0[j], a1[j] - b1[j], a2[j] - b2[j])
+                                                   : tc::join(a0[j], a1[j], a2[j]));
           hi[j] = v.x, lo[j] = v.y;
         }
         tc::store_row8(dst, pe, tc::tix(r, c0, R), hi, lo);
@@ -842,7 +830,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
       ok = false;
       break;
     }
-    epi_sq(0, make_float2(2.f, 0.f), false, fr[1]);
+    epi_sq(0, make_float2(0x1p-7f, 0.f), false, fr[1]);
     sync_all();
     Ct = fr[0], aC = fa[0], St = fr[1], aS = fa[1];
   }
@@ -960,18 +948,17 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_dyson(DevSys s, int k,
         tc::ld8(ta + uint32_t(5 * R), i2);
         tc::wait_ld();
         if (m < R) {
-          float rh[8], rl[8], ih[8], il[8];
+          float rh[8], rl[8], ih[8], il[8];  // slice4f's units: the accumulators' times 2^-8
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int n = c0 + j;
-            float2 re = make_float2(0.f, 0.f), im = re;
+            const float2 re = tc::join(r0[j], r1[j], r2[j]), im = tc::join(i0[j], i1[j], i2[j]);
             if (m < b && n < b) {
-              const float2 pr = tc::sum3(r0[j], r1[j], r2[j]), pi = tc::sum3(i0[j], i1[j], i2[j]);
-              re = make_float2(pr.x * 0x1p-16f, pr.y * 0x1p-16f);
-              im = make_float2(pi.x * 0x1p-16f, pi.y * 0x1p-16f);
-              Ab[big_at(s, b, bp, n * b + m, c)] = make_float4(re.x, im.x, re.y, im.y);
+              const float2 nr = tc::normal(re), ni = tc::normal(im);
+              Ab[big_at(s, b, bp, n * b + m, c)] =
+                  make_float4(nr.x * 0x1p-16f, ni.x * 0x1p-16f, nr.y * 0x1p-16f, ni.y * 0x1p-16f);
             }
-            rh[j] = re.x, rl[j] = re.y, ih[j] = im.x, il[j] = im.y;
+            rh[j] = re.x * 0x1p-8f, rl[j] = re.y * 0x1p-8f, ih[j] = im.x * 0x1p-8f, il[j] = im.y * 0x1p-8f;
           }
           const int o = tc::tix(m, c0, R);
           tc::store_row8(Ar, pe, o, rh, rl);
@@ -1091,18 +1078,17 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_dyson_stk(DevSys s, in
         tc::ld8(ta + uint32_t(2 * R), v2);
         tc::wait_ld();
         if (live) {
-          float h[8], l[8];
+          float h[8], l[8];  // slice4f's units: the accumulators' times 2^-8
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int n = c0 + j;
-            float2 v = make_float2(0.f, 0.f);
+            const float2 v = tc::join(v0[j], v1[j], v2[j]);
             if (m < b && n < b) {
-              const float2 p = tc::sum3(v0[j], v1[j], v2[j]);
-              v = make_float2(p.x * 0x1p-16f, p.y * 0x1p-16f);
+              const float2 w = tc::normal(v);
               float *e = Ab + 4 * big_at(s, b, bp, n * b + m, c) + (is_im ? 1 : 0);
-              e[0] = v.x, e[2] = v.y;
+              e[0] = w.x * 0x1p-16f, e[2] = w.y * 0x1p-16f;
             }
-            h[j] = v.x, l[j] = v.y;
+            h[j] = v.x * 0x1p-8f, l[j] = v.y * 0x1p-8f;
           }
           const tc::Row8 row = tc::slice_row8(h, l);
           // re row m: A1 row m, A2 row R + m negated; im row m: A1 row R + m, A2 row m
