@@ -465,25 +465,63 @@ struct FloqWork {
   float2 *Kf;  // MIX: b x b single-precision K
 };
 
-// The parallel Jacobi sweeps of floquet_cta over K (Xk) with V (Mm) accumulating the rotations;
-// returns convergence.  The angles come from single precision and each rotation is scaled to
-// c^2 + |s|^2 = 1 in FP64, as in lanes_sweeps.
-__device__ bool floquet_sweeps(double2 *Xk, double2 *Mm, int b, int max_sweeps, const FloqWork &wk) {
-  auto rot = [&](int t, int q) -> double2 & { return wk.rot[2 * t + q]; };
+// q = e / d and r = e - q d without an integer division: the FP32 quotient is at most one off
+__device__ __forceinline__ int fdiv(int e, float invd, int d, int &r) {
+  int q = __float2int_rz(float(e) * invd);
+  r = e - q * d;
+  if (r < 0) --q, r += d;
+  if (r >= d) ++q, r -= d;
+  return q;
+}
+// (i, j) with i <= j < n of the e-th of n (n + 1) / 2 pairs: rows i and n-1-i share a line of n + 1
+__device__ __forceinline__ int tri_pair(int e, int n, float inv_n1, int &j) {
+  int col;
+  const int r = fdiv(e, inv_n1, n + 1, col);
+  if (col < n - r) {
+    j = r + col;
+    return r;
+  }
+  j = col - 1;
+  return n - 1 - r;
+}
+
+// c x - s y and s' x + c y of a rotation's two outputs
+template <class C, class T>
+__device__ __forceinline__ C rot_mix(T c, C x, C s, C y) {
+  C v;
+  v.x = fma(c, x.x, fma(s.x, y.x, -(s.y * y.y)));
+  v.y = fma(c, x.y, fma(s.x, y.y, s.y * y.x));
+  return v;
+}
+
+// The parallel Jacobi sweeps of floquet_cta over the Hermitian K with V accumulating the rotations;
+// returns convergence.  The angles come from single precision; in FP64 each rotation is scaled to
+// c^2 + |s|^2 = 1, as in lanes_sweeps.  A round's pairs are disjoint, so K <- G^H K G splits into
+// 2 x 2 blocks (pair t1's rows, pair t2's columns): only t1 <= t2 is computed and its conjugate
+// stored with it, 24 FP64 operations per element pair against 48 for columns then rows of the
+// whole of K, and one barrier less per round.
+template <class C>
+__device__ bool floquet_sweeps(C *K, C *V, int b, int max_sweeps, const FloqWork &wk) {
+  using T = decltype(C::x);
+  constexpr bool kF64 = sizeof(T) == 8;
+  C *rot = reinterpret_cast<C *>(wk.rot);  // per pair: (c, 0), (s e^{i ph})
   auto rpair = [&](int t, int q) -> int & { return wk.rpair[2 * t + q]; };
   double *red = wk.red;
   const int bb = b * b;
+  const float invb = 1.f / float(b);
   const int bq = b + (b & 1);  // players in the round-robin (one dummy when b is odd)
-  const int np = bq / 2;
-  bool conv = false;
+  const int np = bq / 2, nblk = np * (np + 1) / 2;
+  const float inv_np = 1.f / float(np), inv_np1 = 1.f / float(np + 1);
+  bool conv = false, polish = false;
   const int nw = (blockDim.x + 31) / 32, wid = threadIdx.x >> 5, lid = threadIdx.x & 31;
   for (int sweep = 0; sweep < max_sweeps && !conv; ++sweep) {
-    // off(K)^2 and diag(K)^2: FP64 sums per thread, a fixed shuffle tree per warp, the warps'
-    // sums added by one thread
-    double off = 0, dg = 0;
+    // off(K)^2 and diag(K)^2: sums per thread, a fixed shuffle tree per warp, the warps' sums
+    // added by one thread
+    T off = 0, dg = 0;
     for (int e = threadIdx.x; e < bb; e += blockDim.x) {
-      const int r = e / b, q = e % b;
-      const double2 v = Xk[e];
+      int q;
+      const int r = fdiv(e, invb, b, q);
+      const C v = K[e];
       if (r < q) off += v.x * v.x + v.y * v.y;
       else if (r == q) dg += v.x * v.x;
     }
@@ -502,10 +540,14 @@ __device__ bool floquet_sweeps(double2 *Xk, double2 *Mm, int b, int max_sweeps, 
     __syncthreads();
     const double offs = red[2 * nw], dgs = red[2 * nw + 1];
     __syncthreads();
-    if (offs <= 1e-34 * dgs || offs <= 1e-60) {
-      conv = true;
-      break;
+    if (kF64) {
+      conv = offs <= 1e-34 * dgs || offs <= 1e-60;
+    } else {  // single precision: once small, one more sweep reaches its rounding
+      const bool small = offs <= 1e-10 * dgs;
+      conv = (small && polish) || offs == 0.0;
+      polish = small;
     }
+    if (conv) break;
     for (int round = 0; round < bq - 1; ++round) {
       for (int t = threadIdx.x; t < np; t += blockDim.x) {
         auto player = [&](int j) { return j == 0 ? 0 : 1 + (j - 1 + round) % (bq - 1); };
@@ -515,58 +557,221 @@ __device__ bool floquet_sweeps(double2 *Xk, double2 *Mm, int b, int max_sweeps, 
           p = q, q = tmp;
         }
         rpair(t, 0) = p, rpair(t, 1) = q;
-        rot(t, 0) = cmk(1, 0), rot(t, 1) = cmk(0, 0);
+        C rc = mkc<C>(1, 0), rs = mkc<C>(0, 0);
         if (q < b) {
-          const float hx = float(Xk[p * b + q].x), hy = float(Xk[p * b + q].y);
+          const float hx = float(K[p * b + q].x), hy = float(K[p * b + q].y);
           const float ab = hypotf(hx, hy);
           if (ab != 0.f) {
-            const float theta = 0.5f * float(Xk[q * b + q].x - Xk[p * b + p].x) / ab;
+            const float theta = 0.5f * float(K[q * b + q].x - K[p * b + p].x) / ab;
             float tt;
             if (fabsf(theta) > 1e18f) tt = 0.5f / theta;  // theta^2 stays finite
             else tt = copysignf(1.f, theta) / (fabsf(theta) + sqrtf(fmaf(theta, theta, 1.f)));
             const float cf = rsqrtf(fmaf(tt, tt, 1.f)), ts = tt * cf / ab;
-            const double cd = cf;
-            const double2 sd = cmk(hx * ts, hy * ts);
-            const double d = fma(cd, cd, fma(sd.x, sd.x, fma(sd.y, sd.y, -1.0)));
-            const double nn = fma(fma(0.375, d, -0.5), d, 1.0);
-            rot(t, 0) = cmk(cd * nn, 0.0);
-            rot(t, 1) = cscale(sd, nn);
+            rc.x = cf;
+            rs = mkc<C>(hx * ts, hy * ts);
+            if (kF64) {
+              const T d = fma(rc.x, rc.x, fma(rs.x, rs.x, fma(rs.y, rs.y, T(-1))));
+              const T nn = fma(fma(T(0.375), d, T(-0.5)), d, T(1));
+              rc.x *= nn;
+              rs = cscale(rs, nn);
+            }
           }
         }
+        rot[2 * t] = rc, rot[2 * t + 1] = rs;
       }
       __syncthreads();
-      // columns p, q of K and V:  K <- K G, V <- V G  with G = [[c, sp], [-conj(sp), c]];
-      // the pair index runs fastest, so a warp's accesses stay within one row of K (or V)
-      for (int e = threadIdx.x; e < np * b * 2; e += blockDim.x) {
-        const int t = e % np, rest = e / np, kk = rest % b;
-        const int p = rpair(t, 0), q = rpair(t, 1);
-        if (q >= b) continue;
-        const double cc = rot(t, 0).x;
-        const double2 sp = rot(t, 1), spc = cconj(sp);
-        double2 *Z = rest < b ? Xk : Mm;
-        const double2 xkp = Z[kk * b + p], xkq = Z[kk * b + q];
-        Z[kk * b + p] = csub(cscale(xkp, cc), cmul(spc, xkq));
-        Z[kk * b + q] = cadd(cmul(sp, xkp), cscale(xkq, cc));
-      }
-      __syncthreads();
-      // rows p, q of K:  K <- G^H K, the diagonal kept real
-      for (int e = threadIdx.x; e < np * b; e += blockDim.x) {
-        const int t = e / b, kk = e % b;
-        const int p = rpair(t, 0), q = rpair(t, 1);
-        if (q >= b) continue;
-        const double cc = rot(t, 0).x;
-        const double2 sp = rot(t, 1), spc = cconj(sp);
-        const double2 xpk = Xk[p * b + kk], xqk = Xk[q * b + kk];
-        double2 np_ = csub(cscale(xpk, cc), cmul(sp, xqk)), nq_ = cadd(cmul(spc, xpk), cscale(xqk, cc));
-        if (kk == p) np_.y = 0.0;
-        if (kk == q) nq_.y = 0.0;
-        Xk[p * b + kk] = np_;
-        Xk[q * b + kk] = nq_;
+      // G = [[c, s], [-conj(s), c]] per pair: K's blocks, then the columns of V, the pair index
+      // fastest (a warp's accesses to V stay within one row)
+      for (int e = threadIdx.x; e < nblk + np * b; e += blockDim.x) {
+        if (e < nblk) {
+          int t2;
+          const int t1 = tri_pair(e, np, inv_np1, t2);
+          const int p1 = rpair(t1, 0), q1 = rpair(t1, 1), p2 = rpair(t2, 0), q2 = rpair(t2, 1);
+          const bool h1 = q1 < b, h2 = q2 < b;
+          const C zero = mkc<C>(0, 0);
+          C kpp = K[p1 * b + p2], kpq = h2 ? K[p1 * b + q2] : zero, kqp = h1 ? K[q1 * b + p2] : zero,
+            kqq = h1 && h2 ? K[q1 * b + q2] : zero;
+          {
+            const T c2 = rot[2 * t2].x;
+            const C s2 = rot[2 * t2 + 1], m2 = mkc<C>(-s2.x, s2.y);
+            const C x = rot_mix(c2, kpp, m2, kpq), y = rot_mix(c2, kqp, m2, kqq);
+            kpq = rot_mix(c2, kpq, s2, kpp), kqq = rot_mix(c2, kqq, s2, kqp);
+            kpp = x, kqp = y;
+          }
+          {
+            const T c1 = rot[2 * t1].x;
+            const C s1 = rot[2 * t1 + 1], m1 = mkc<C>(-s1.x, -s1.y), j1 = cconj(s1);
+            const C x = rot_mix(c1, kpp, m1, kqp), y = rot_mix(c1, kpq, m1, kqq);
+            kqp = rot_mix(c1, kqp, j1, kpp), kqq = rot_mix(c1, kqq, j1, kpq);
+            kpp = x, kpq = y;
+          }
+          if (t1 == t2) kpp.y = 0, kqq.y = 0, kqp = cconj(kpq);  // the diagonal stays real
+          K[p1 * b + p2] = kpp;
+          if (t1 != t2) K[p2 * b + p1] = cconj(kpp);
+          if (h2) K[p1 * b + q2] = kpq;
+          if (h2 && t1 != t2) K[q2 * b + p1] = cconj(kpq);
+          if (h1) K[q1 * b + p2] = kqp;
+          if (h1 && t1 != t2) K[p2 * b + q1] = cconj(kqp);
+          if (h1 && h2) K[q1 * b + q2] = kqq;
+          if (h1 && h2 && t1 != t2) K[q2 * b + q1] = cconj(kqq);
+        } else {
+          int t;
+          const int kk = fdiv(e - nblk, inv_np, np, t);
+          const int p = rpair(t, 0), q = rpair(t, 1);
+          if (q >= b) continue;
+          const T cc = rot[2 * t].x;
+          const C sp = rot[2 * t + 1];
+          const C vp = V[kk * b + p], vq = V[kk * b + q];
+          V[kk * b + p] = rot_mix(cc, vp, mkc<C>(-sp.x, sp.y), vq);
+          V[kk * b + q] = rot_mix(cc, vq, sp, vp);
+        }
       }
       __syncthreads();
     }
   }
   return conv;
+}
+
+// Start of the FP64 sweeps: K = V^H K0 V nearly diagonal (Xk) and its V, orthonormal in FP64 (Mm),
+// from the eigenvectors of K0 (Xk on entry) in single precision.  The FP64 pipe issues 2 FMAs per
+// clock and SM against 128 in FP32, and all sweeps but the last two only bring the off-diagonal
+// down to where single precision leaves it: those run in FP32 (K and V in Mm's two halves), V is
+// widened and orthonormalised by the Cholesky factor of its Gram matrix (which departs from one by
+// ~1e-6: the reciprocals are short series), and K0 is transformed: 11 b^3 FMAs against 12 b^3 for
+// each sweep that it saves (~5).  Where single precision does not deliver (not finite, or far from
+// orthonormal), V = I and the FP64 sweeps do all of the work.
+// Blocks below kFloqStartMin stay with FP64 sweeps alone (blocks of 10, 320 crystallites: 0.66 ms
+// against 0.73; blocks of 20 to 35, 7 spins, 144 crystallites: 8.5 -> 3.0 ms).
+constexpr int kFloqSweeps32 = 12, kFloqStartMin = 16;
+__device__ void floquet_start(double2 *Xk, double2 *Mm, int b, const FloqWork &wk) {
+  const int bb = b * b, nt = blockDim.x, tid = threadIdx.x;
+  const float invb = 1.f / float(b), invb1 = 1.f / float(b + 1);
+  constexpr int kPer = 4;  // elements per thread of a group in the products below
+  float2 *K32 = reinterpret_cast<float2 *>(Mm), *V32 = K32 + bb;
+  if (b < kFloqStartMin || b > kPer * nt) {
+    for (int e = tid; e < bb; e += nt) Mm[e] = cmk(e % (b + 1) == 0 ? 1.0 : 0.0, 0.0);
+    __syncthreads();
+    return;
+  }
+  for (int e = tid; e < bb; e += nt) {
+    K32[e] = make_float2(float(Xk[e].x), float(Xk[e].y));
+    V32[e] = make_float2(e % (b + 1) == 0 ? 1.f : 0.f, 0.f);
+  }
+  __syncthreads();
+  floquet_sweeps(K32, V32, b, kFloqSweeps32, wk);
+  __syncthreads();
+  // widen in place, upwards: element e's place ends below element e + 1 of V32
+  bool bad = false;
+  for (int e0 = 0; e0 < bb; e0 += nt) {
+    const int e = e0 + tid;
+    float2 v = make_float2(0.f, 0.f);
+    if (e < bb) v = V32[e];
+    bad = bad || !(fabsf(v.x) <= 2.f && fabsf(v.y) <= 2.f);
+    __syncthreads();
+    if (e < bb) Mm[e] = cmk(v.x, v.y);
+  }
+  bad = __syncthreads_or(bad);
+  // Gram matrix E of V: E_ij (i < j) in Xk's lower triangle (element j, i), E_ii in the diagonal's
+  // imaginary parts; K0 stays in the upper triangle
+  const int ntri = b * (b + 1) / 2;
+  for (int e = tid; e < ntri && !bad; e += nt) {
+    int j;
+    const int i = tri_pair(e, b, invb1, j);
+    double2 g = cmk(0, 0);
+    for (int r = 0; r < b; ++r) g = cfmaconj(Mm[r * b + i], Mm[r * b + j], g);
+    if (i == j) Xk[i * b + i].y = g.x;
+    else Xk[j * b + i] = g;
+    const double d = i == j ? g.x - 1.0 : g.x;
+    bad = !(fabs(d) <= 1e-4 && fabs(g.y) <= 1e-4);
+  }
+  bad = __syncthreads_or(bad);
+  // V <- V R^-1 with E = R^H R, right-looking: step k takes column k's part out of the columns
+  // above it, in V and in what is left of E; the columns' norms follow at the end
+  for (int k = 0; k < b - 1 && !bad; ++k) {
+    const double d = Xk[k * b + k].y - 1.0;
+    const double inv = fma(-d, fma(-d, fma(-d, fma(-d, 1.0, 1.0), 1.0), 1.0), 1.0);  // 1 / E_kk
+    const int w = b - 1 - k, nv = b * w, ng = w * (w + 1) / 2;
+    const float invw = 1.f / float(w), invw1 = 1.f / float(w + 1);
+    for (int e = tid; e < nv + ng; e += nt) {
+      if (e < nv) {
+        int j;
+        const int r = fdiv(e, invw, w, j);
+        j += k + 1;
+        const double2 f = cscale(Xk[j * b + k], -inv);
+        Mm[r * b + j] = cfma(Mm[r * b + k], f, Mm[r * b + j]);
+      } else {
+        int j;
+        const int i = k + 1 + tri_pair(e - nv, w, invw1, j);
+        j += k + 1;
+        const double2 f = cscale(Xk[j * b + k], -inv);
+        if (i == j) Xk[i * b + i].y = fma(Xk[i * b + k].x, f.x, fma(Xk[i * b + k].y, f.y, Xk[i * b + i].y));
+        else Xk[j * b + i] = cfmaconj(Xk[i * b + k], f, Xk[j * b + i]);
+      }
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < bb; e += nt) {
+    int q;
+    const int r = fdiv(e, invb, b, q);
+    if (bad) {
+      Mm[e] = cmk(r == q ? 1.0 : 0.0, 0.0);
+    } else {
+      const double d = Xk[q * b + q].y - 1.0;  // E_qq^-1/2
+      Mm[e] = cscale(Mm[e], fma(-d, fma(-d, fma(-d, 0.3125, 0.375), 0.5), 1.0));
+    }
+  }
+  __syncthreads();
+  auto mirror = [&]() {
+    for (int e = tid; e < ntri; e += nt) {
+      int j;
+      const int i = tri_pair(e, b, invb1, j);
+      if (i == j) Xk[i * b + i].y = 0.0;
+      else Xk[j * b + i] = cconj(Xk[i * b + j]);
+    }
+    __syncthreads();
+  };
+  mirror();
+  if (bad) return;
+  // Xk <- K0 V by groups of rows, then V^H (K0 V) by groups of columns, each in place
+  const int group = min(b, kPer * nt / b);
+  for (int r0 = 0; r0 < b; r0 += group) {
+    double2 acc[kPer];
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      acc[t] = cmk(0, 0);
+      int j;
+      const int e = tid + t * nt, r = r0 + fdiv(e, invb, b, j);
+      if (e < group * b && r < b)
+        for (int l = 0; l < b; ++l) acc[t] = cfma(Xk[r * b + l], Mm[l * b + j], acc[t]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      const int e = tid + t * nt;
+      if (e < group * b && r0 * b + e < bb) Xk[r0 * b + e] = acc[t];
+    }
+  }
+  __syncthreads();
+  for (int j0 = 0; j0 < b; j0 += group) {
+    double2 acc[kPer];
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      acc[t] = cmk(0, 0);
+      int i;
+      const int e = tid + t * nt, j = j0 + fdiv(e, invb, b, i);
+      if (e < group * b && j < b && i <= j)
+        for (int l = 0; l < b; ++l) acc[t] = cfmaconj(Mm[l * b + i], Xk[l * b + j], acc[t]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      int i;
+      const int e = tid + t * nt, j = j0 + fdiv(e, invb, b, i);
+      if (e < group * b && j < b && i <= j) Xk[i * b + j] = acc[t];
+    }
+  }
+  __syncthreads();
+  mirror();
 }
 
 // DFA: A_n is double-float (mixed form).
@@ -635,16 +840,18 @@ __device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk) {
       }
       __syncthreads();
     }
-    for (int kr = b - 1; kr >= 0; --kr) {  // back substitution, columns in parallel
+    for (int kr = b - 1; kr >= 0; --kr) {  // back substitution, all rows above at once
       const double2 inv = cdiv(cmk(1, 0), Mm[kr * b + kr]);
-      for (int j = threadIdx.x; j < b; j += blockDim.x) {
-        double2 acc = Xk[kr * b + j];
-        for (int r = kr + 1; r < b; ++r) acc = csub(acc, cmul(Mm[kr * b + r], Xk[r * b + j]));
-        Xk[kr * b + j] = cmul(acc, inv);
+      for (int j = threadIdx.x; j < b; j += blockDim.x) Xk[kr * b + j] = cmul(Xk[kr * b + j], inv);
+      __syncthreads();
+      for (int e = threadIdx.x; e < kr * b; e += blockDim.x) {
+        int j;
+        const int r = fdiv(e, 1.f / float(b), b, j);
+        Xk[e] = csub(Xk[e], cmul(Mm[r * b + kr], Xk[kr * b + j]));
       }
       __syncthreads();
     }
-    // K = Hermitian part of i X, in Xk; V = I in Mm
+    // K = Hermitian part of i X, in Xk
     for (int e = threadIdx.x; e < bb; e += blockDim.x) {
       const int r = e / b, q = e % b;
       if (r <= q) {
@@ -655,20 +862,24 @@ __device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk) {
         Xk[q * b + r] = cconj(h);
       }
     }
-    for (int e = threadIdx.x; e < bb; e += blockDim.x) Mm[e] = cmk(e / b == e % b ? 1.0 : 0.0, 0.0);
     __syncthreads();
     for (int e = threadIdx.x; e < b; e += blockDim.x) Xk[e * b + e].y = 0.0;
     __syncthreads();
+    floquet_start(Xk, Mm, b, wk);
     const bool conv = floquet_sweeps(Xk, Mm, b, kMaxSweeps, wk);
     if (!conv) atomicOr(s.status, kNoConvergeFloquet);
-    // Rayleigh quotients lam_r = v_r^H U v_r
+    // Rayleigh quotients lam_r = v_r^H (U V)_r, U V in Xk (K is done with)
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
+      int r;
+      const int kk = fdiv(e, 1.f / float(b), b, r);
+      double2 uv = cmk(0, 0);
+      for (int l = 0; l < b; ++l) uv = cfma(Ug(kk, l), Mm[l * b + r], uv);
+      Xk[e] = uv;
+    }
+    __syncthreads();
     for (int r = threadIdx.x; r < b; r += blockDim.x) {
       double2 acc = cmk(0, 0);
-      for (int kk = 0; kk < b; ++kk) {
-        double2 uv = cmk(0, 0);
-        for (int l = 0; l < b; ++l) uv = cfma(Ug(kk, l), Mm[l * b + r], uv);
-        acc = cfmaconj(Mm[kk * b + r], uv, acc);
-      }
+      for (int kk = 0; kk < b; ++kk) acc = cfmaconj(Mm[kk * b + r], Xk[kk * b + r], acc);
       lam[r] = acc;
     }
     __syncthreads();
@@ -1005,14 +1216,6 @@ __device__ __forceinline__ float4 cdf_mul(float4 x, float4 y) {
   CdfAcc a = {{0.f, 0.f}, {0.f, 0.f}};
   cdf_mac(a, x, y);
   return cdf_fin(a);
-}
-
-// q = e / d and r = e - q d without an integer division: (e + 1/2) / d in FP32 is at least
-// 1/(2 d) away from an integer and its rounding error is far smaller (e < 2^20, d <= 2^8)
-__device__ __forceinline__ int fdiv(int e, float invd, int d, int &r) {
-  const int q = __float2int_rz((float(e) + 0.5f) * invd);
-  r = e - q * d;
-  return q;
 }
 
 // The sweeps over the FP32 K (Kf) with V (double-float, Vd) accumulating the rotations.
