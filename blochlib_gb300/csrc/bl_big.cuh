@@ -15,7 +15,9 @@
 //   k_big_dyson_df  (c)         A_{i+1} = U_i A_i in double-float
 
 constexpr int kMaxBigBlock = 74;   // 5 real b x b matrices fit 227 KB of shared memory
-constexpr int kBigThreads = 256;   // k_big_floquet
+// k_big_floquet: a block from kFloqWide on has an SM's shared memory to itself and needs the warps
+constexpr int kBigThreads = 512, kFloqWide = 40;
+__host__ __device__ constexpr int floquet_threads(int b) { return b >= kFloqWide ? kBigThreads : 256; }
 constexpr int kBigPSMax = 63;      // 7 real b x b matrices (Paterson-Stockmeyer step) fit
 constexpr int kMaxInt = 128;       // interactions per system on the large-block path
 
@@ -632,30 +634,130 @@ __device__ bool floquet_sweeps(C *K, C *V, int b, int max_sweeps, const FloqWork
   return conv;
 }
 
-// Start of the FP64 sweeps: K = V^H K0 V nearly diagonal (Xk) and its V, orthonormal in FP64 (Mm),
-// from the eigenvectors of K0 (Xk on entry) in single precision.  The FP64 pipe issues 2 FMAs per
-// clock and SM against 128 in FP32, and all sweeps but the last two only bring the off-diagonal
-// down to where single precision leaves it: those run in FP32 (K and V in Mm's two halves), V is
-// widened and orthonormalised by the Cholesky factor of its Gram matrix (which departs from one by
-// ~1e-6: the reciprocals are short series), and K0 is transformed: 11 b^3 FMAs against 12 b^3 for
-// each sweep that it saves (~5).  Where single precision does not deliver (not finite, or far from
-// orthonormal), V = I and the FP64 sweeps do all of the work.
-// Blocks below kFloqStartMin stay with FP64 sweeps alone (blocks of 10, 320 crystallites: 0.66 ms
-// against 0.73; blocks of 20 to 35, 7 spins, 144 crystallites: 8.5 -> 3.0 ms).
-constexpr int kFloqSweeps32 = 12, kFloqStartMin = 16;
-__device__ void floquet_start(double2 *Xk, double2 *Mm, int b, const FloqWork &wk) {
+// x - f y, complex double-float
+__device__ __forceinline__ float4 cdf_fms(float4 x, float4 f, float4 y) {
+  CdfAcc a = {{x.x, x.z}, {x.y, x.w}};
+  cdf_mac(a, make_float4(-f.x, -f.y, -f.z, -f.w), y);
+  return cdf_fin(a);
+}
+__device__ __forceinline__ float4 cdf_mul(float4 x, float4 y) {
+  CdfAcc a = {{0.f, 0.f}, {0.f, 0.f}};
+  cdf_mac(a, x, y);
+  return cdf_fin(a);
+}
+
+// Element arithmetic of floquet_start: FP64, or double-float on the FP32 pipe (mixed form).  A
+// diagonal element of the work matrix holds K_ii in its real part and E_ii in its imaginary part.
+struct FloqF64 {
+  static constexpr int kStartMin = 16;  // smallest block that takes floquet_start
+  using E = double2;
+  using Acc = double2;
+  static __device__ __forceinline__ E of(float2 v) { return cmk(v.x, v.y); }
+  static __device__ __forceinline__ float2 narrow(E v) { return make_float2(float(v.x), float(v.y)); }
+  static __device__ __forceinline__ E conj(E v) { return cconj(v); }
+  static __device__ __forceinline__ Acc acc(E v) { return v; }
+  static __device__ __forceinline__ void mac(Acc &a, E x, E y) { a = cfma(x, y, a); }
+  static __device__ __forceinline__ void macj(Acc &a, E x, E y) { a = cfmaconj(x, y, a); }  // conj(x) y
+  static __device__ __forceinline__ E fin(const Acc &a) { return a; }
+  static __device__ __forceinline__ E im_of(E d) { return cmk(d.y, 0.0); }  // E_ii of a diagonal element
+  static __device__ __forceinline__ void set_im(E &d, E e) { d.y = e.x; }
+  static __device__ __forceinline__ E real(E d) { return cmk(d.x, 0.0); }
+  static __device__ __forceinline__ float dev_re(E v, float id) { return float(v.x - double(id)); }
+  static __device__ __forceinline__ float dev_im(E v) { return float(v.y); }
+  static __device__ __forceinline__ E neg_over(E g, E e) {  // -g / e for e = 1 + d, |d| <= 1e-4
+    const double d = e.x - 1.0;
+    return cscale(g, -fma(-d, fma(-d, fma(-d, fma(-d, 1.0, 1.0), 1.0), 1.0), 1.0));
+  }
+  static __device__ __forceinline__ E over_sqrt(E v, E e) {
+    const double d = e.x - 1.0;
+    return cscale(v, fma(-d, fma(-d, fma(-d, 0.3125, 0.375), 0.5), 1.0));
+  }
+};
+struct FloqDf {
+  static constexpr int kStartMin = 32;
+  using E = float4;
+  using Acc = CdfAcc;
+  static __device__ __forceinline__ E of(float2 v) { return make_float4(v.x, v.y, 0.f, 0.f); }
+  static __device__ __forceinline__ float2 narrow(E v) { return make_float2(v.x + v.z, v.y + v.w); }
+  static __device__ __forceinline__ E conj(E v) { return make_float4(v.x, -v.y, v.z, -v.w); }
+  static __device__ __forceinline__ Acc acc(E v) { return {{v.x, v.z}, {v.y, v.w}}; }
+  static __device__ __forceinline__ void mac(Acc &a, E x, E y) { cdf_mac(a, x, y); }
+  static __device__ __forceinline__ void macj(Acc &a, E x, E y) { cdf_mac(a, conj(x), y); }
+  static __device__ __forceinline__ E fin(const Acc &a) { return cdf_fin(a); }
+  static __device__ __forceinline__ E im_of(E d) { return make_float4(d.y, 0.f, d.w, 0.f); }
+  static __device__ __forceinline__ void set_im(E &d, E e) { d.y = e.x, d.w = e.z; }
+  static __device__ __forceinline__ E real(E d) { return make_float4(d.x, 0.f, d.z, 0.f); }
+  static __device__ __forceinline__ float dev_re(E v, float id) { return (v.x - id) + v.z; }
+  static __device__ __forceinline__ float dev_im(E v) { return v.y + v.w; }
+  static __device__ __forceinline__ E neg_over(E g, E e) {  // -(g - g d (1 - d)), g of the size of d
+    const float d = dev_re(e, 1.f), f = d * (1.f - d);
+    const float2 re = dfv_add(make_float2(-g.x, -g.z), make_float2(g.x * f, 0.f)),
+                 im = dfv_add(make_float2(-g.y, -g.w), make_float2(g.y * f, 0.f));
+    return make_float4(re.x, im.x, re.y, im.y);
+  }
+  static __device__ __forceinline__ E over_sqrt(E v, E e) {
+    const float2 d = dfv_add(make_float2(e.x, e.z), make_float2(-1.f, 0.f));
+    const float q = d.x * d.x * (0.375f - 0.3125f * d.x);
+    const float2 f = dfv_add(make_float2(1.f, 0.f), dfv_add(make_float2(-0.5f * d.x, -0.5f * d.y), make_float2(q, 0.f)));
+    const float2 re = dfv_mul(f, make_float2(v.x, v.z)), im = dfv_mul(f, make_float2(v.y, v.w));
+    return make_float4(re.x, im.x, re.y, im.y);
+  }
+};
+
+// Start of the final sweeps: K = V^H K0 V nearly diagonal (Xk) and its V, orthonormal (Mm), from
+// the eigenvectors of K0 (Xk on entry) in single precision.  FP64 issues 2 FMAs per clock and SM
+// against 128 in FP32, and a double-float product takes about 30 FP32 operations; all sweeps but
+// the last ones only bring the off-diagonal down to where single precision leaves it.  Those run
+// in FP32 (K and V in Mm's two halves), V is widened and orthonormalised by the Cholesky factor of
+// its Gram matrix (which departs from one by ~1e-6: the reciprocals are short series), and K0 is
+// transformed: 11 b^3 multiply-adds against 12 b^3 (FP64; V alone in double-float: 6 b^3) for each
+// of the ~5 sweeps that it saves.  Where single precision does not deliver (not finite, or far
+// from orthonormal), V = I and the final sweeps do all of the work.
+// Blocks below kStartMin stay with the final sweeps alone (FP64, blocks of 10, 320 crystallites:
+// 0.66 ms against 0.73; blocks of 20 to 35, 7 spins, 144 crystallites: 8.5 -> 3.0 ms.  Double-float,
+// blocks of 20, 677 crystallites: 1.08 ms against 1.62; blocks of 28 to 70, 8 spins, 1154
+// crystallites: 74 -> 48 ms, with K's off-diagonal left at 1e-10 of its norm instead of 1e-7).
+constexpr int kFloqSweeps32 = 12;
+constexpr int kFloqPer = 4;  // elements per thread and group of the in-place products (b <= 4 blockDim.x)
+
+// X <- X V by groups of whole rows, in place
+template <class A>
+__device__ void mul_in_place(typename A::E *X, const typename A::E *V, int b) {
+  constexpr int kPer = kFloqPer;
+  const int nt = blockDim.x, tid = threadIdx.x, bb = b * b, group = min(b, kPer * nt / b);
+  const float invb = 1.f / float(b);
+  for (int r0 = 0; r0 < b; r0 += group) {
+    typename A::E out[kPer];
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      int j;
+      const int e = tid + t * nt, r = r0 + fdiv(e, invb, b, j);
+      if (e < group * b && r < b) {
+        auto a = A::acc(A::of(make_float2(0.f, 0.f)));
+        for (int l = 0; l < b; ++l) A::mac(a, X[r * b + l], V[l * b + j]);
+        out[t] = A::fin(a);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      const int e = tid + t * nt;
+      if (e < group * b && r0 * b + e < bb) X[r0 * b + e] = out[t];
+    }
+  }
+  __syncthreads();
+}
+
+template <class A>
+__device__ void floquet_start(typename A::E *Xk, typename A::E *Mm, int b, const FloqWork &wk) {
+  using E = typename A::E;
   const int bb = b * b, nt = blockDim.x, tid = threadIdx.x;
   const float invb = 1.f / float(b), invb1 = 1.f / float(b + 1);
-  constexpr int kPer = 4;  // elements per thread of a group in the products below
   float2 *K32 = reinterpret_cast<float2 *>(Mm), *V32 = K32 + bb;
-  if (b < kFloqStartMin || b > kPer * nt) {
-    for (int e = tid; e < bb; e += nt) Mm[e] = cmk(e % (b + 1) == 0 ? 1.0 : 0.0, 0.0);
-    __syncthreads();
-    return;
-  }
+  auto one = [&](int e) { return make_float2(e % (b + 1) == 0 ? 1.f : 0.f, 0.f); };
   for (int e = tid; e < bb; e += nt) {
-    K32[e] = make_float2(float(Xk[e].x), float(Xk[e].y));
-    V32[e] = make_float2(e % (b + 1) == 0 ? 1.f : 0.f, 0.f);
+    K32[e] = A::narrow(Xk[e]);
+    V32[e] = one(e);
   }
   __syncthreads();
   floquet_sweeps(K32, V32, b, kFloqSweeps32, wk);
@@ -668,7 +770,7 @@ __device__ void floquet_start(double2 *Xk, double2 *Mm, int b, const FloqWork &w
     if (e < bb) v = V32[e];
     bad = bad || !(fabsf(v.x) <= 2.f && fabsf(v.y) <= 2.f);
     __syncthreads();
-    if (e < bb) Mm[e] = cmk(v.x, v.y);
+    if (e < bb) Mm[e] = A::of(v);
   }
   bad = __syncthreads_or(bad);
   // Gram matrix E of V: E_ij (i < j) in Xk's lower triangle (element j, i), E_ii in the diagonal's
@@ -677,105 +779,86 @@ __device__ void floquet_start(double2 *Xk, double2 *Mm, int b, const FloqWork &w
   for (int e = tid; e < ntri && !bad; e += nt) {
     int j;
     const int i = tri_pair(e, b, invb1, j);
-    double2 g = cmk(0, 0);
-    for (int r = 0; r < b; ++r) g = cfmaconj(Mm[r * b + i], Mm[r * b + j], g);
-    if (i == j) Xk[i * b + i].y = g.x;
+    auto a = A::acc(A::of(make_float2(0.f, 0.f)));
+    for (int r = 0; r < b; ++r) A::macj(a, Mm[r * b + i], Mm[r * b + j]);
+    const E g = A::fin(a);
+    if (i == j) A::set_im(Xk[i * b + i], g);
     else Xk[j * b + i] = g;
-    const double d = i == j ? g.x - 1.0 : g.x;
-    bad = !(fabs(d) <= 1e-4 && fabs(g.y) <= 1e-4);
+    bad = !(fabsf(A::dev_re(g, i == j ? 1.f : 0.f)) <= 1e-4f && fabsf(A::dev_im(g)) <= 1e-4f);
   }
   bad = __syncthreads_or(bad);
   // V <- V R^-1 with E = R^H R, right-looking: step k takes column k's part out of the columns
   // above it, in V and in what is left of E; the columns' norms follow at the end
   for (int k = 0; k < b - 1 && !bad; ++k) {
-    const double d = Xk[k * b + k].y - 1.0;
-    const double inv = fma(-d, fma(-d, fma(-d, fma(-d, 1.0, 1.0), 1.0), 1.0), 1.0);  // 1 / E_kk
+    const E piv = A::im_of(Xk[k * b + k]);
     const int w = b - 1 - k, nv = b * w, ng = w * (w + 1) / 2;
     const float invw = 1.f / float(w), invw1 = 1.f / float(w + 1);
     for (int e = tid; e < nv + ng; e += nt) {
+      int j;
       if (e < nv) {
-        int j;
         const int r = fdiv(e, invw, w, j);
         j += k + 1;
-        const double2 f = cscale(Xk[j * b + k], -inv);
-        Mm[r * b + j] = cfma(Mm[r * b + k], f, Mm[r * b + j]);
+        auto a = A::acc(Mm[r * b + j]);
+        A::mac(a, Mm[r * b + k], A::neg_over(Xk[j * b + k], piv));
+        Mm[r * b + j] = A::fin(a);
       } else {
-        int j;
         const int i = k + 1 + tri_pair(e - nv, w, invw1, j);
         j += k + 1;
-        const double2 f = cscale(Xk[j * b + k], -inv);
-        if (i == j) Xk[i * b + i].y = fma(Xk[i * b + k].x, f.x, fma(Xk[i * b + k].y, f.y, Xk[i * b + i].y));
-        else Xk[j * b + i] = cfmaconj(Xk[i * b + k], f, Xk[j * b + i]);
+        auto a = A::acc(i == j ? A::im_of(Xk[i * b + i]) : Xk[j * b + i]);
+        A::macj(a, Xk[i * b + k], A::neg_over(Xk[j * b + k], piv));
+        if (i == j) A::set_im(Xk[i * b + i], A::fin(a));
+        else Xk[j * b + i] = A::fin(a);
       }
     }
     __syncthreads();
   }
   for (int e = tid; e < bb; e += nt) {
     int q;
-    const int r = fdiv(e, invb, b, q);
-    if (bad) {
-      Mm[e] = cmk(r == q ? 1.0 : 0.0, 0.0);
-    } else {
-      const double d = Xk[q * b + q].y - 1.0;  // E_qq^-1/2
-      Mm[e] = cscale(Mm[e], fma(-d, fma(-d, fma(-d, 0.3125, 0.375), 0.5), 1.0));
-    }
+    fdiv(e, invb, b, q);
+    Mm[e] = bad ? A::of(one(e)) : A::over_sqrt(Mm[e], A::im_of(Xk[q * b + q]));
   }
   __syncthreads();
   auto mirror = [&]() {
     for (int e = tid; e < ntri; e += nt) {
       int j;
       const int i = tri_pair(e, b, invb1, j);
-      if (i == j) Xk[i * b + i].y = 0.0;
-      else Xk[j * b + i] = cconj(Xk[i * b + j]);
+      if (i == j) Xk[i * b + i] = A::real(Xk[i * b + i]);
+      else Xk[j * b + i] = A::conj(Xk[i * b + j]);
     }
     __syncthreads();
   };
   mirror();
   if (bad) return;
-  // Xk <- K0 V by groups of rows, then V^H (K0 V) by groups of columns, each in place
+  // Xk <- K0 V by rows, then V^H (K0 V) by groups of columns, in place
+  mul_in_place<A>(Xk, Mm, b);
+  constexpr int kPer = kFloqPer;
   const int group = min(b, kPer * nt / b);
-  for (int r0 = 0; r0 < b; r0 += group) {
-    double2 acc[kPer];
-#pragma unroll
-    for (int t = 0; t < kPer; ++t) {
-      acc[t] = cmk(0, 0);
-      int j;
-      const int e = tid + t * nt, r = r0 + fdiv(e, invb, b, j);
-      if (e < group * b && r < b)
-        for (int l = 0; l < b; ++l) acc[t] = cfma(Xk[r * b + l], Mm[l * b + j], acc[t]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int t = 0; t < kPer; ++t) {
-      const int e = tid + t * nt;
-      if (e < group * b && r0 * b + e < bb) Xk[r0 * b + e] = acc[t];
-    }
-  }
-  __syncthreads();
   for (int j0 = 0; j0 < b; j0 += group) {
-    double2 acc[kPer];
+    E out[kPer];
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
-      acc[t] = cmk(0, 0);
       int i;
       const int e = tid + t * nt, j = j0 + fdiv(e, invb, b, i);
-      if (e < group * b && j < b && i <= j)
-        for (int l = 0; l < b; ++l) acc[t] = cfmaconj(Mm[l * b + i], Xk[l * b + j], acc[t]);
+      if (e < group * b && j < b && i <= j) {
+        auto a = A::acc(A::of(make_float2(0.f, 0.f)));
+        for (int l = 0; l < b; ++l) A::macj(a, Mm[l * b + i], Xk[l * b + j]);
+        out[t] = A::fin(a);
+      }
     }
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
       int i;
       const int e = tid + t * nt, j = j0 + fdiv(e, invb, b, i);
-      if (e < group * b && j < b && i <= j) Xk[i * b + j] = acc[t];
+      if (e < group * b && j < b && i <= j) Xk[i * b + j] = out[t];
     }
   }
   __syncthreads();
   mirror();
 }
 
-// DFA: A_n is double-float (mixed form).
-template <bool DFA>
+// DFA: A_n is double-float (mixed form); START: the sweeps begin with floquet_start.
+template <bool DFA, bool START>
 __device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk) {
   constexpr bool dfA = DFA;
   __shared__ int piv_s;
@@ -865,18 +948,18 @@ __device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk) {
     __syncthreads();
     for (int e = threadIdx.x; e < b; e += blockDim.x) Xk[e * b + e].y = 0.0;
     __syncthreads();
-    floquet_start(Xk, Mm, b, wk);
+    if constexpr (START) {
+      floquet_start<FloqF64>(Xk, Mm, b, wk);
+    } else {
+      for (int e = threadIdx.x; e < bb; e += blockDim.x) Mm[e] = cmk(e / b == e % b ? 1.0 : 0.0, 0.0);
+      __syncthreads();
+    }
     const bool conv = floquet_sweeps(Xk, Mm, b, kMaxSweeps, wk);
     if (!conv) atomicOr(s.status, kNoConvergeFloquet);
     // Rayleigh quotients lam_r = v_r^H (U V)_r, U V in Xk (K is done with)
-    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
-      int r;
-      const int kk = fdiv(e, 1.f / float(b), b, r);
-      double2 uv = cmk(0, 0);
-      for (int l = 0; l < b; ++l) uv = cfma(Ug(kk, l), Mm[l * b + r], uv);
-      Xk[e] = uv;
-    }
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) Xk[e] = Ug(e / b, e % b);
     __syncthreads();
+    mul_in_place<FloqF64>(Xk, Mm, b);
     for (int r = threadIdx.x; r < b; r += blockDim.x) {
       double2 acc = cmk(0, 0);
       for (int kk = 0; kk < b; ++kk) acc = cfmaconj(Mm[kk * b + r], Xk[kk * b + r], acc);
@@ -915,25 +998,24 @@ __device__ void floquet_cta(const DevSys &s, int k, int c, FloqWork wk) {
     s.L[at(bo + r, c, s.Cpad)] = cmk(log(hypot(lam[r].x, lam[r].y)), atan2(lam[r].y, lam[r].x));
 }
 
+template <bool START>
 __device__ void floquet_cta_df(const DevSys &s, int k, int c, FloqWork wk, bool a64 = false);
 
-// One CTA per crystallite: unitary eigen-decomposition of a large block of A_n.
-__global__ void __launch_bounds__(kBigThreads) k_big_floquet(DevSys s, int k) {
+// One CTA per crystallite: unitary eigen-decomposition of a large block of A_n.  DF: the mixed
+// form's double-float path (K in single precision after the two b x b arrays).  The variants are
+// kernels of their own: floquet_start's registers would cost the small blocks their occupancy.
+template <bool DF, bool DFA, bool START>
+__global__ void __launch_bounds__(START ? kBigThreads : 256) k_big_floquet(DevSys s, int k) {
   extern __shared__ double2 bsc[];
   __shared__ double2 rot[(kMaxBigBlock / 2 + 1) * 2];  // (c, 0), (s e^{i ph}) per pair
   __shared__ int rpair[(kMaxBigBlock / 2 + 1) * 2];
   __shared__ double2 fv[kMaxBigBlock];
   __shared__ double2 lam[kMaxBigBlock];
-  __shared__ double red[kBigThreads];
+  __shared__ double red[START ? kBigThreads : 256];
   const int b = s.bs[k];
-  if (s.floq32) {  // K in single precision after the two b x b arrays; the rest double-float
-    floquet_cta_df(s, k, blockIdx.x, FloqWork{bsc, bsc + b * b, rot, fv, lam, rpair, red,
-                                              reinterpret_cast<float2 *>(bsc + 2 * b * b)});
-  } else if (s.mixed) {
-    floquet_cta<true>(s, k, blockIdx.x, FloqWork{bsc, bsc + b * b, rot, fv, lam, rpair, red, nullptr});
-  } else {
-    floquet_cta<false>(s, k, blockIdx.x, FloqWork{bsc, bsc + b * b, rot, fv, lam, rpair, red, nullptr});
-  }
+  const FloqWork wk{bsc, bsc + b * b, rot, fv, lam, rpair, red, reinterpret_cast<float2 *>(bsc + 2 * b * b)};
+  if constexpr (DF) floquet_cta_df<START>(s, k, blockIdx.x, wk);
+  else floquet_cta<DFA, START>(s, k, blockIdx.x, wk);
 }
 
 // ------------------------------------------------------------------ mixed form, double-float
@@ -1206,18 +1288,6 @@ __global__ void __launch_bounds__(NT == 1 ? 1024 : 768) k_big_dyson_df(DevSys s,
 // (re.hi, im.hi, re.lo, im.lo) in the 16-byte slots of the FP64 work arrays; the results
 // (V, ln lambda) are stored in FP64 as by floquet_cta.
 
-// x - f y, complex double-float
-__device__ __forceinline__ float4 cdf_fms(float4 x, float4 f, float4 y) {
-  CdfAcc a = {{x.x, x.z}, {x.y, x.w}};
-  cdf_mac(a, make_float4(-f.x, -f.y, -f.z, -f.w), y);
-  return cdf_fin(a);
-}
-__device__ __forceinline__ float4 cdf_mul(float4 x, float4 y) {
-  CdfAcc a = {{0.f, 0.f}, {0.f, 0.f}};
-  cdf_mac(a, x, y);
-  return cdf_fin(a);
-}
-
 // The sweeps over the FP32 K (Kf) with V (double-float, Vd) accumulating the rotations.
 __device__ bool floquet_sweeps_df(float2 *Xk, float4 *Vd, int b, int max_sweeps, const FloqWork &wk) {
   float4 *rot = reinterpret_cast<float4 *>(wk.rot);  // per pair: (c.hi, 0, c.lo, 0), (s as complex df)
@@ -1354,6 +1424,7 @@ __device__ bool floquet_sweeps_df(float2 *Xk, float4 *Vd, int b, int max_sweeps,
 }
 
 // a64: A_n is FP64 (double2, the huge-block path's storage) instead of double-float
+template <bool START>
 __device__ void floquet_cta_df(const DevSys &s, int k, int c, FloqWork wk, bool a64) {
   __shared__ int piv_s;
   __shared__ double a_s;
@@ -1436,7 +1507,7 @@ __device__ void floquet_cta_df(const DevSys &s, int k, int c, FloqWork wk, bool 
       }
       __syncthreads();
     }
-    // X' = diag(M)^-1 X, then K = Hermitian part of i X' in FP32, V = I (double-float)
+    // X' = diag(M)^-1 X, then K = Hermitian part of i X'
     for (int r = threadIdx.x; r < b; r += blockDim.x) {
       const double2 d = df_load(M4[r * b + r]);
       fv[r] = df_store(cdiv(cmk(1, 0), d));
@@ -1446,26 +1517,33 @@ __device__ void floquet_cta_df(const DevSys &s, int k, int c, FloqWork wk, bool 
     __syncthreads();
     for (int e = threadIdx.x; e < bb; e += blockDim.x) {
       const int r = e / b, q = e % b;
+      if (r > q) continue;
       const float4 xrq = X4[r * b + q], xqr = X4[q * b + r];
-      // i X_rq = (-Im, Re); conj(i X_qr) = (-Im X_qr, -Re X_qr)
-      const float re = 0.5f * (-(xrq.y + xrq.w) - (xqr.y + xqr.w));
-      const float im = r == q ? 0.f : 0.5f * ((xrq.x + xrq.z) - (xqr.x + xqr.z));
-      Kf[e] = make_float2(re, im);
+      // i X_rq = (-Im, Re); conj(i X_qr) = (-Im X_qr, -Re X_qr); halves are exact
+      const float2 re = dfv_add(make_float2(-0.5f * xrq.y, -0.5f * xrq.w), make_float2(-0.5f * xqr.y, -0.5f * xqr.w));
+      float2 im = dfv_add(make_float2(0.5f * xrq.x, 0.5f * xrq.z), make_float2(-0.5f * xqr.x, -0.5f * xqr.z));
+      if (r == q) im = make_float2(0.f, 0.f);
+      X4[r * b + q] = make_float4(re.x, im.x, re.y, im.y);
+      X4[q * b + r] = make_float4(re.x, -im.x, re.y, -im.y);
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < bb; e += blockDim.x) M4[e] = make_float4(e / b == e % b ? 1.f : 0.f, 0.f, 0.f, 0.f);
+    if constexpr (START) {
+      floquet_start<FloqDf>(X4, M4, b, wk);
+    } else {
+      for (int e = threadIdx.x; e < bb; e += blockDim.x)
+        M4[e] = make_float4(e / b == e % b ? 1.f : 0.f, 0.f, 0.f, 0.f);
+      __syncthreads();
+    }
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) Kf[e] = FloqDf::narrow(X4[e]);
     __syncthreads();
     const int max_sweeps = kMaxSweeps;
     const bool conv = floquet_sweeps_df(Kf, M4, b, max_sweeps, wk);
     if (!conv) atomicOr(s.status, kNoConvergeFloquet);
-    // Rayleigh quotients: Y = A_n V (into X's array), lam_r = sum_k conj(V_kr) Y_kr
-    for (int e = threadIdx.x; e < bb; e += blockDim.x) {
-      const int kr = e / b, r = e % b;
-      CdfAcc a = {{0.f, 0.f}, {0.f, 0.f}};
-      for (int l = 0; l < b; ++l) cdf_mac(a, Ug(kr, l), M4[l * b + r]);
-      X4[e] = cdf_fin(a);
-    }
+    // Rayleigh quotients: Y = A_n V in X's array (A_n converted once: with a64 the conversions run
+    // at the FP64 rate), lam_r = sum_k conj(V_kr) Y_kr
+    for (int e = threadIdx.x; e < bb; e += blockDim.x) X4[e] = Ug(e / b, e % b);
     __syncthreads();
+    mul_in_place<FloqDf>(X4, M4, b);
     for (int r = threadIdx.x; r < b; r += blockDim.x) {
       CdfAcc a = {{0.f, 0.f}, {0.f, 0.f}};
       for (int kk = 0; kk < b; ++kk) {

@@ -2963,7 +2963,10 @@ static void ready_kernels(Context &ctx) {
         (const void *)k_tc_step, (const void *)k_tc_step_stk, (const void *)k_tc_dyson, (const void *)k_tc_dyson_stk,
         (const void *)k_big_seg_frame<false>, (const void *)k_big_seg_frame<true>,
         (const void *)k_big_eigframe<1, double2>, (const void *)k_big_eigframe<2, double2>,
-        (const void *)k_big_eigframe4, (const void *)k_big_floquet, (const void *)k_huge_floquet,
+        (const void *)k_big_eigframe4, (const void *)k_big_floquet<true, true, true>, (const void *)k_big_floquet<true, true, false>,
+        (const void *)k_big_floquet<false, true, true>, (const void *)k_big_floquet<false, true, false>,
+        (const void *)k_big_floquet<false, false, true>, (const void *)k_big_floquet<false, false, false>,
+        (const void *)k_huge_floquet,
         (const void *)k_big_qr4, (const void *)k_big_qr<1, float2>, (const void *)k_big_qr<1, double2>,
         (const void *)k_big_qr<2, double2>,
         (const void *)k_fave_fft<8, double2, true>, (const void *)k_fave_fft<8, double2, false>,
@@ -4113,7 +4116,18 @@ static void launch_stage(JobImpl &J, DevSys &s, int stage) {
         }
         break;
       case 2:  // the mixed form's single-precision K follows the two b x b double2 arrays
-        k_big_floquet<<<unsigned(s.C), kBigThreads, smat + (s.floq32 ? sizeof(float2) * size_t(b) * b : 0), st>>>(s, k);
+        if (s.floq32 && b >= FloqDf::kStartMin)
+          k_big_floquet<true, true, true><<<unsigned(s.C), floquet_threads(b), smat + sizeof(float2) * size_t(b) * b, st>>>(s, k);
+        else if (s.floq32)
+          k_big_floquet<true, true, false><<<unsigned(s.C), 256, smat + sizeof(float2) * size_t(b) * b, st>>>(s, k);
+        else if (s.mixed && b >= FloqF64::kStartMin)
+          k_big_floquet<false, true, true><<<unsigned(s.C), floquet_threads(b), smat, st>>>(s, k);
+        else if (s.mixed)
+          k_big_floquet<false, true, false><<<unsigned(s.C), 256, smat, st>>>(s, k);
+        else if (b >= FloqF64::kStartMin)
+          k_big_floquet<false, false, true><<<unsigned(s.C), floquet_threads(b), smat, st>>>(s, k);
+        else
+          k_big_floquet<false, false, false><<<unsigned(s.C), 256, smat, st>>>(s, k);
         break;
       case 3:
         if (b <= s.seg_max) {
@@ -4151,8 +4165,8 @@ static void launch_stage(JobImpl &J, DevSys &s, int stage) {
       case 2:
         if (J.xs_from <= kMaxBigBlock) {  // fits shared memory
           const int k = J.huge_blocks[kh], b = J.L.size[k];
-          k_big_floquet<<<unsigned(s.C), kBigThreads, sizeof(double2) * 2 * size_t(b) * b,
-                          aux_stream(J, J.big_blocks.size() + kh)>>>(s, k);
+          k_big_floquet<false, false, true><<<unsigned(s.C), floquet_threads(b), sizeof(double2) * 2 * size_t(b) * b,
+                                             aux_stream(J, J.big_blocks.size() + kh)>>>(s, k);
           ++J.launches;
         } else if (kh == 0) {
           huge_floquet_all(J, s);

@@ -325,10 +325,10 @@ __global__ void __launch_bounds__(kHugeFloqThreads) k_huge_floquet(DevSys s, Hug
   int *rpair = reinterpret_cast<int *>(red + (b > kHugeFloqThreads ? b : kHugeFloqThreads));
   double2 *Mm = ws + hf.ws[blockIdx.y] + size_t(blockIdx.x) * hf.mats * b * b;
   if (s.floq32)  // mixed form: FP32 sweeps, double-float Cayley solve, V and Rayleigh quotients
-    floquet_cta_df(s, k, c,
+    floquet_cta_df<true>(s, k, c,
                    FloqWork{Mm, Mm + size_t(b) * b, rot, fv, lam, rpair, red,
                             reinterpret_cast<float2 *>(Mm + 2 * size_t(b) * b)},
                    true);
   else
-    floquet_cta<false>(s, k, c, FloqWork{Mm, Mm + size_t(b) * b, rot, fv, lam, rpair, red, nullptr});
+    floquet_cta<false, true>(s, k, c, FloqWork{Mm, Mm + size_t(b) * b, rot, fv, lam, rpair, red, nullptr});
 }
