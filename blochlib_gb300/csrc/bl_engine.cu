@@ -2847,6 +2847,8 @@ struct JobImpl {
   DevBuf<double> phase;                    // per step: cos, sin of the rotor phase and of twice it
   DevBuf<double2> frames;                  // rf schedule: per chunk frame (permuted index)
   DevBuf<float2> Tk_df, Hc_df;             // mixed form: double-float operators and constant parts
+  DevBuf<int> hl_elem;                    // tensor-core blocks: the elements k_tc_hamil assembles
+  std::vector<int> hl_off, hl_n;
   DevBuf<int> tk_ptr, tk_term, tk_order;  // blocks above kMaxBlock: the operators' non-zeros by element
   DevBuf<float2> tk_val;
   DevBuf<double> tk_val64;
@@ -3528,6 +3530,22 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     }
     up.add(J.tk_ptr, ptr), up.add(J.tk_term, term), up.add(J.tk_val, val), up.add(J.tk_val64, val64);
     up.add(J.tk_order, order);
+    if (J.tc) {
+      std::vector<int> elem;
+      J.hl_off.assign(L.size.size(), 0), J.hl_n.assign(L.size.size(), 0);
+      for (size_t kb = 0; kb < L.size.size(); ++kb) {
+        const int b = L.size[kb], bp = L.poff[kb];
+        if (b < tc::kMinB || b > tc::kMaxB) continue;
+        J.hl_off[kb] = int(elem.size());
+        for (int x = 0; x < b * b; ++x) {
+          const int e = order[size_t(bp) + x];
+          if (e / b <= e % b && (ptr[size_t(bp) + e + 1] > ptr[size_t(bp) + e] || Hc[size_t(bp) + e] != 0.0))
+            elem.push_back(e);
+        }
+        J.hl_n[kb] = int(elem.size()) - J.hl_off[kb];
+      }
+      up.add(J.hl_elem, elem);
+    }
   }
   if (sched) {  // per chunk: the rf frame of each permuted index (1 where a chunk has none)
     bool any = false;
@@ -4087,11 +4105,17 @@ static void launch_stage(JobImpl &J, DevSys &s, int stage) {
     const bool nt1 = big_nt(b, b) == 1;
     switch (stage) {
       case 0:
+        if (J.tc && b >= tc::kMinB) {
+          k_tc_hamil<<<unsigned(s.Cpad / 32) * unsigned(s.n), 256, sizeof(float2) * 32 * size_t(s.nint), st>>>(
+              s, k, J.hl_elem.p + J.hl_off[k], J.hl_n[k]);
+          ++J.launches;
+        }
         if (J.tc && b >= tc::kMinB && tc::up16(b) <= 64)  // the two Horner chains stacked in one M = 128 tile
           k_tc_step_stk<<<unsigned(s.C) * unsigned(s.n), tc::kTcThreads, tc_step_stk_smem(b), st>>>(
-              s, k, J.usl.p + J.usl_off[k]);
+              s, k, J.hl_elem.p + J.hl_off[k], J.hl_n[k], J.usl.p + J.usl_off[k]);
         else if (J.tc && b >= tc::kMinB)
-          k_tc_step<<<unsigned(s.C) * unsigned(s.n), tc::kTcThreads, tc_step_smem(b), st>>>(s, k, J.usl.p + J.usl_off[k]);
+          k_tc_step<<<unsigned(s.C) * unsigned(s.n), tc::kTcThreads, tc_step_smem(b), st>>>(
+              s, k, J.hl_elem.p + J.hl_off[k], J.hl_n[k], J.usl.p + J.usl_off[k]);
         else if (s.mixed) k_big_step_df<<<unsigned(s.C) * unsigned(s.n), th_step, big_step_df_smem(b), st>>>(s, k);
         else k_big_step<<<unsigned(s.C) * unsigned(s.n), th_step, big_step_smem(b), st>>>(s, k);
         break;

@@ -224,28 +224,25 @@ __device__ __forceinline__ float2 normal(float2 v) {
 }
 
 // Issues the 10 slice pairs of one real product into the three accumulators at TMEM column
-// `col` (level 0, 1, 2+3 at col, col + R, col + 2R): A tile planes at a (plane stride pl
-// bytes), B tile planes at b, R = up16(b) output columns, R / 16 K steps.  `accumulate`
-// adds to what the accumulators hold instead of starting them.
+// `col` (level 0, 1, 2+3 at col, col + R, col + 2R): A tile planes at a (plane stride plA bytes), B
+// an R-row tile at b, R = up16(b) output columns, R / 16 K steps.  `accumulate` adds to what the
+// accumulators hold instead of starting them.  B's planes follow one another in whole row groups,
+// as the accumulators do in columns, so pairs of one A plane with consecutive B planes are one MMA
+// of N = 2R or 3R: seven MMAs a K step, each reading its A plane once (an MMA of N = 64 is bound by
+// the shared-memory reads, two thirds of them A's).
 __device__ __forceinline__ void issue_product(uint32_t tmem, uint32_t col, uint32_t a, uint32_t plA, uint32_t b,
-                                              uint32_t plB, int R, bool negA, bool accumulate) {
-  const uint32_t id = idesc_bf16(R, negA);
-  const int sp[10] = {0, 0, 1, 0, 1, 2, 0, 1, 2, 3}, tp[10] = {0, 1, 0, 2, 1, 0, 3, 2, 1, 0};
-  const int lev[10] = {0, 1, 1, 2, 2, 2, 2, 2, 2, 2};
+                                              int R, bool negA, bool accumulate) {
+  const uint32_t plB = uint32_t(R / 8 * sbo_bytes(R));
+  const int sp[7] = {0, 0, 1, 1, 2, 2, 3}, tp[7] = {0, 3, 0, 2, 0, 1, 0};
+  const int lev[7] = {0, 2, 1, 2, 2, 2, 2}, wide[7] = {3, 1, 2, 1, 1, 1, 1};
 #pragma unroll
-  for (int q = 0; q < 10; ++q) {
-    const uint32_t d = tmem + col + uint32_t(lev[q] * R);
-    const bool first = !accumulate && (q == 0 || q == 1 || q == 3);
+  for (int q = 0; q < 7; ++q) {
+    const uint32_t id = idesc_bf16(wide[q] * R, negA), d = tmem + col + uint32_t(lev[q] * R);
     const uint32_t a0 = a + uint32_t(sp[q]) * plA, b0 = b + uint32_t(tp[q]) * plB;
     for (int kk = 0; kk < R / 16; ++kk)
-      mma(d, sdesc(a0 + kk * 256, R), sdesc(b0 + kk * 256, R), id, (first && kk == 0) ? 0u : 1u);
+      mma(d, sdesc(a0 + kk * 256, R), sdesc(b0 + kk * 256, R), id, (!accumulate && q == 0 && kk == 0) ? 0u : 1u);
   }
 }
-__device__ __forceinline__ void issue_product(uint32_t tmem, uint32_t col, uint32_t a, uint32_t b, uint32_t pl,
-                                              int R, bool negA, bool accumulate) {
-  issue_product(tmem, col, a, pl, b, pl, R, negA, accumulate);
-}
-
 // -2^-8 / (k (k + 1)) (the units of slice4f) as double-float for the Horner steps (k = 1 .. 31), folded at compile time
 // into constant memory (k is the same in every thread), so that no epilogue divides in FP64
 #define BL_HC(k) dfv_const(-0x1p-8 / (double(k) * double((k) + 1)))
@@ -278,66 +275,76 @@ enum { kTcTimeout = 64 };  // status bit: a tensor-core wait ran out
 // K-major slice layout, four planes of 16 row groups each.
 __host__ __device__ constexpr size_t tc_stk_plane_bytes(int b) { return size_t(16) * tc::sbo_bytes(tc::up16(b)); }
 
-// The step's prologue (every thread): the term coefficients into fk, H_i (double-float) into
-// H, row sums of |H| into red, then the scale, squarings and Taylor degree into scl, nsq and
-// nterms.  The block's operator non-zeros (CSR rows bp .. bp + bb) are first copied into
-// `stage` (tiles that are free until X is sliced): coalesced, independent loads, after which
-// each entry's walk over its terms (36 on a diagonal of eight coupled spins) reads shared
-// memory instead of waiting on L2.
-__device__ __forceinline__ void tc_step_prologue(const DevSys &s, int k, int c, int i, float2 *fk, float *red,
-                                                 float2 *H, unsigned char *stage, size_t stage_bytes, float2 &scl,
-                                                 int &nsq, int &nterms) {
+// The Hamiltonians of one tensor-core block for every crystallite and step, as double-float values
+// of the elements that can be non-zero (elem: packed index r b + q, r <= q, by descending term
+// count): a lane per crystallite, a warp per element, so the walk over an element's terms is
+// uniform and the coefficients are read once per 32 crystallites.  (Assembled by the step kernel's
+// own CTA, one per SM, the lists' loads and the diagonal's 36 dependent sums took 16k of its 46k
+// clocks at b = 56.)  They wait in the block's part of U, which the tensor-core blocks do not use.
+__device__ __forceinline__ float2 *tc_hamil(const DevSys &s, int bp, int i) {
+  return reinterpret_cast<float2 *>(s.U + (size_t(i) * s.S2 + bp) * s.Cpad);
+}
+__global__ void __launch_bounds__(256) k_tc_hamil(DevSys s, int k, const int *__restrict__ elem, int nel) {
+  extern __shared__ float2 fkw[];  // nint x 32
+  const int groups = s.Cpad / 32, c0 = int(blockIdx.x % groups) * 32, i = blockIdx.x / groups;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int bp = s.bpoff[k];
+  const float2 *fk2 = reinterpret_cast<const float2 *>(s.fk);  // double-float pairs from k_coef
+  for (int x = warp; x < s.nint; x += 8) fkw[32 * x + lane] = fk2[at(i * s.nint + x, c0 + lane, s.Cpad)];
+  __syncthreads();
+  float2 *out = tc_hamil(s, bp, i);
+  for (int x = warp; x < nel; x += 8) {
+    const int e = elem[x];
+    float2 h = s.Hc_df[bp + e];
+    for (int j = s.tk_ptr[bp + e]; j < s.tk_ptr[bp + e + 1]; ++j)
+      h = dfv_add(h, dfv_mul(fkw[32 * s.tk_term[j] + lane], s.tk_val[j]));
+    out[at(x, c0 + lane, s.Cpad)] = h;
+  }
+}
+
+// The step's prologue (every thread): H_i (double-float, from k_tc_hamil's elements) into H, row
+// sums of |H| into red, then the scale, squarings and Taylor degree into scl, nsq and nterms.
+__device__ __forceinline__ void tc_step_prologue(const DevSys &s, int k, int c, int i, const int *elem, int nel,
+                                                 float *red, float2 *H, float2 &scl, int &nsq, int &nterms) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = s.bs[k], bp = s.bpoff[k], bb = b * b;
-  {  // term coefficients (double-float pairs from k_coef)
-    const float2 *fk2 = reinterpret_cast<const float2 *>(s.fk);
-    for (int kk = tid; kk < s.nint; kk += tc::kTcThreads) fk[kk] = fk2[at(i * s.nint + kk, c, s.Cpad)];
+  constexpr int kPer = (tc::kMaxB * (tc::kMaxB + 1) / 2 + tc::kTcThreads - 1) / tc::kTcThreads;
+  const float2 *Hl = tc_hamil(s, bp, i);
+  float2 v[kPer];
+  int el[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int x = tid + u * tc::kTcThreads;
+    if (x < nel) el[u] = __ldg(elem + x), v[u] = Hl[at(x, c, s.Cpad)];
   }
+  for (int e = tid; e < bb; e += tc::kTcThreads) H[e] = make_float2(0.f, 0.f);
   __syncthreads();
-  const float2 *Hcb = s.Hc_df + bp;
-  {
-    const int j0 = s.tk_ptr[bp], nz = s.tk_ptr[bp + bb] - j0;
-    const size_t need = size_t(2 * bb + 1 + nz) * sizeof(int) + size_t(nz) * sizeof(float2) + 16;
-    if (need <= stage_bytes) {
-      int *sp = reinterpret_cast<int *>(stage);
-      float2 *sv = reinterpret_cast<float2 *>(sp + ((2 * bb + 1 + nz + 3) & ~3));
-      int *so = sp + bb + 1, *st = so + bb;
-      // unrolled so that each thread's loads are in flight together (they do not depend on
-      // one another); Hc goes straight into H, so the walk below touches no global memory
-#pragma unroll 8
-      for (int x = tid; x <= bb; x += tc::kTcThreads) sp[x] = s.tk_ptr[bp + x] - j0;
-#pragma unroll 8
-      for (int x = tid; x < bb; x += tc::kTcThreads) so[x] = s.tk_order[bp + x];
-#pragma unroll 8
-      for (int x = tid; x < nz; x += tc::kTcThreads) st[x] = s.tk_term[j0 + x], sv[x] = s.tk_val[j0 + x];
-#pragma unroll 8
-      for (int e = tid; e < bb; e += tc::kTcThreads) H[e] = Hcb[e];
-      __syncthreads();
-      // elements by descending term count: the 32 lanes of a warp walk similar lengths (the
-      // diagonal, with a term for every interaction, together)
-      for (int x = tid; x < bb; x += tc::kTcThreads) {
-        const int e = so[x];
-        float2 h = H[e];
-        for (int j = sp[e]; j < sp[e + 1]; ++j) h = dfv_add(h, dfv_mul(fk[st[j]], sv[j]));
-        H[e] = h;
-      }
-    } else {
-      for (int e = tid; e < bb; e += tc::kTcThreads) {
-        float2 h = Hcb[e];
-        for (int j = s.tk_ptr[bp + e]; j < s.tk_ptr[bp + e + 1]; ++j)
-          h = dfv_add(h, dfv_mul(fk[s.tk_term[j]], s.tk_val[j]));
-        H[e] = h;
-      }
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    if (tid + u * tc::kTcThreads < nel) {
+      const int r = el[u] / b, q = el[u] - r * b;
+      H[r * b + q] = v[u], H[q * b + r] = v[u];
     }
   }
   __syncthreads();
   // row sums of |H| (a warp per row, lanes over the columns), then their maximum: the norm
-  for (int p = warp; p < b; p += tc::kTcThreads / 32) {
-    float rs = 0.f;
-    for (int q = lane; q < b; q += 32) rs += fabsf(H[p * b + q].x);
+  constexpr int kRows = (tc::kMaxB + 15) / 16;
+  float rs[kRows];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
-    if (lane == 0) red[p] = rs;
+  for (int u = 0; u < kRows; ++u) {
+    const int p = warp + u * (tc::kTcThreads / 32);
+    rs[u] = 0.f;
+    if (p < b)
+      for (int q = lane; q < b; q += 32) rs[u] += fabsf(H[p * b + q].x);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) rs[u] += __shfl_xor_sync(0xffffffffu, rs[u], o);
+#pragma unroll
+  for (int u = 0; u < kRows; ++u) {
+    const int p = warp + u * (tc::kTcThreads / 32);
+    if (p < b && lane == 0) red[p] = rs[u];
   }
   __syncthreads();
   if (warp == 0) {
@@ -376,12 +383,12 @@ __host__ __device__ constexpr size_t tc_step_smem(int b) {
   return 4 * tc::tile_bytes(b) + tc::overread_bytes(b) + 1024;
 }
 
-__global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, unsigned char *slab0) {
+__global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, const int *elem, int nel,
+                                                               unsigned char *slab0) {
   using tc::kTcThreads;
   extern __shared__ __align__(1024) unsigned char tsm[];
   __shared__ uint32_t tbase;
   __shared__ __align__(8) uint64_t mbar[2];
-  __shared__ float2 fk[kMaxInt];
   __shared__ float red[tc::kMaxB];
   __shared__ float2 scl;
   __shared__ int nsq, nterms, gfail[2];
@@ -400,10 +407,8 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
   }
   if (warp == 0) tc::tmem_alloc(&tbase, ncols);
   if (tid == 0) tc::mbar_init(&mbar[0]), tc::mbar_init(&mbar[1]);
-  // H (double-float) into the fourth tile as scratch, the other three as the staging area
-  float2 *H = reinterpret_cast<float2 *>(Bf[3]);
-  tc_step_prologue(s, k, c, i, fk, red, H, reinterpret_cast<unsigned char *>(Bf[0]), 3 * tc::tile_bytes(b), scl, nsq,
-                   nterms);
+  float2 *H = reinterpret_cast<float2 *>(Bf[3]);  // H (double-float) into the fourth tile as scratch
+  tc_step_prologue(s, k, c, i, elem, nel, red, H, scl, nsq, nterms);
   const int sq = nsq, K = nterms;
   const int mC = K / 2, mS = (K - 1) / 2;  // C to X^(2 mC), S to X^(2 mS + 1)
   {  // X slices into the first tile: one 8-column row chunk per thread and iteration, rows
@@ -495,7 +500,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
   const uint32_t aX = ba[0], aY = ba[1], aTC = ba[2], aTS = ba[3];
   // Y = X X, then the innermost Horner terms straight from Y (all 16 warps)
   if (tid == 0) {
-    tc::issue_product(tmem, set_col[0], aX, aX, pl, R, false, false);
+    tc::issue_product(tmem, set_col[0], aX, pl, aX, R, false, false);
     tc::commit(&mbar[0]);
   }
   if (!wait_all(0)) ok = false;
@@ -533,14 +538,14 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
     const uint32_t aT = grp == 0 ? aTC : aTS;
     int j = grp == 0 ? mC - 1 : mS - 1;
     while (j >= 1) {
-      if (tid == leader) tc::issue_product(tmem, set_col[set], aY, aT, pl, R, false, false), tc::commit(&mbar[set]);
+      if (tid == leader) tc::issue_product(tmem, set_col[set], aY, pl, aT, R, false, false), tc::commit(&mbar[set]);
       if (!wait_grp(set)) break;
       epilogue(set, hcoef(grp == 0 ? 2 * j - 1 : 2 * j), true, false, T, gpart, 2);
       --j;
       sync_grp();
     }
     if (grp == 1 && mS >= 1 && gfail[1] == 0) {
-      if (tid == leader) tc::issue_product(tmem, set_col[1], aX, aTS, pl, R, false, false), tc::commit(&mbar[1]);
+      if (tid == leader) tc::issue_product(tmem, set_col[1], aX, pl, aTS, R, false, false), tc::commit(&mbar[1]);
       if (wait_grp(1)) {
         epilogue(1, one, false, false, X, gpart, 2);
         sync_grp();
@@ -562,9 +567,9 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
     for (int u = 0; u < 4; ++u)
       if (Bf[u] != Ct && Bf[u] != St && nf < 2) fr[nf] = Bf[u], fa[nf] = ba[u], ++nf;
     if (tid == 0) {
-      tc::issue_product(tmem, set_col[0], aC, aC, pl, R, false, false);
+      tc::issue_product(tmem, set_col[0], aC, pl, aC, R, false, false);
       tc::commit(&mbar[0]);
-      tc::issue_product(tmem, set_col[1], aS, aS, pl, R, false, false);
+      tc::issue_product(tmem, set_col[1], aS, pl, aS, R, false, false);
       tc::commit(&mbar[1]);
     }
     const bool w0 = wait_all(0), w1 = wait_all(1);
@@ -574,7 +579,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
     }
     epilogue(0, one, false, true, fr[0], warp >> 2, 4);
     sync_all();
-    if (tid == 0) tc::issue_product(tmem, set_col[0], aC, aS, pl, R, false, false), tc::commit(&mbar[0]);
+    if (tid == 0) tc::issue_product(tmem, set_col[0], aC, pl, aS, R, false, false), tc::commit(&mbar[0]);
     if (!wait_all(0)) {
       ok = false;
       break;
@@ -609,7 +614,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
 // Y's rows in lanes m and R + m; the two Horner chains run as one, T = [T_C; T_S] stacked,
 // T <- [I + c_C Y T_C; I + c_S Y T_S] from the single product T Y (T_C, T_S and Y are
 // polynomials in Y and commute), the sine series carried to the same number of terms as the
-// cosine (one more than it needs); S = T_S X from the same stacked T.  Every TMEM lane
+// cosine (one more than it needs); S = T_S X from the same stacked T (X as B operand in Wt).  Every TMEM lane
 // quarter holds rows for each epilogue.  C and S end in R-row tiles, where the squarings
 // (as in k_tc_step) and the slab copy take them.  Shared memory: XS and T (stacked), two
 // R-row tiles (Y, then C; H's scratch, then S), the over-read margin of an R-row A tile.
@@ -617,12 +622,12 @@ __host__ __device__ constexpr size_t tc_step_stk_smem(int b) {
   return 8 * tc_stk_plane_bytes(b) + 2 * tc::tile_bytes(b) + tc::overread_bytes(b) + 1024;
 }
 
-__global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int k, unsigned char *slab0) {
+__global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int k, const int *elem, int nel,
+                                                                   unsigned char *slab0) {
   using tc::kTcThreads;
   extern __shared__ __align__(1024) unsigned char tsm[];
   __shared__ uint32_t tbase;
   __shared__ __align__(8) uint64_t mbar[2];
-  __shared__ float2 fk[kMaxInt];
   __shared__ float red[tc::kMaxB];
   __shared__ float2 scl;
   __shared__ int nsq, nterms;
@@ -641,12 +646,11 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
   const uint32_t aXS = tc::saddr(XS), aT = tc::saddr(T), aY = tc::saddr(Yt), aW = tc::saddr(Wt);
   if (warp == 0) tc::tmem_alloc(&tbase, ncols);
   if (tid == 0) tc::mbar_init(&mbar[0]), tc::mbar_init(&mbar[1]);
-  // H into Wt as scratch; XS, T and Yt as the staging area
-  float2 *H = reinterpret_cast<float2 *>(Wt);
-  tc_step_prologue(s, k, c, i, fk, red, H, base, 8 * plS + tc::tile_bytes(b), scl, nsq, nterms);
+  float2 *H = reinterpret_cast<float2 *>(Yt);  // H into Yt as scratch
+  tc_step_prologue(s, k, c, i, elem, nel, red, H, scl, nsq, nterms);
   const int sq = nsq, K = nterms;
   const int mC = K / 2;  // C to X^(2 mC), S to X^(2 mC + 1)
-  {  // X slices into both halves of XS: one 8-column row chunk per thread and iteration, rows
+  {  // X slices into both halves of XS and, as the products' B operand, Wt: one 8-column row chunk per thread and iteration, rows
      // fastest, H read down its columns (as in k_tc_step)
     const float2 sc = make_float2(scl.x * 256.f, scl.y * 256.f);
     const int nch = R * (R / 8);
@@ -663,6 +667,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
       const tc::Row8 x8 = tc::slice_row8(hi, lo);
       tc::put_row8(XS, peS, tc::tix(r, c0, R), x8);
       tc::put_row8(XS, peS, tc::tix(R + r, c0, R), x8);
+      tc::put_row8(Wt, pe, tc::tix(r, c0, R), x8);
     }
   }
   tc::fence_smem_async();
@@ -730,7 +735,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
   // Horner terms T_C = I + c Y (to T, or straight to Yt as C when no chain step follows) and
   // T_S = I + c' Y (to T's bottom half); c = 0 when the series stops at the identity
   if (tid == 0) {
-    tc::issue_product(tmem, 0, aXS, plS, aXS, plS, R, false, false);
+    tc::issue_product(tmem, 0, aXS, plS, aW, R, false, false);
     tc::commit(&mbar[0]);
   }
   if (!wait_all(0)) ok = false;
@@ -747,7 +752,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
   // T_C (= C) goes to Yt, free once its product has run
   for (int j = mC - 1; ok && j >= 1; --j) {
     if (tid == 0) {
-      tc::issue_product(tmem, 0, aT, plS, aY, pl, R, false, false);
+      tc::issue_product(tmem, 0, aT, plS, aY, R, false, false);
       tc::commit(&mbar[0]);
     }
     if (!wait_all(0)) {
@@ -762,7 +767,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
   // S = T_S X (the bottom half of T times X, X from XS's top half) into Wt
   if (ok) {
     if (tid == 0) {
-      tc::issue_product(tmem, 0, aT, plS, aXS, plS, R, false, false);
+      tc::issue_product(tmem, 0, aT, plS, aW, R, false, false);
       tc::commit(&mbar[0]);
     }
     if (!wait_all(0)) ok = false;
@@ -813,9 +818,9 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
     for (int u = 0; u < 4; ++u)
       if (Bf[u] != Ct && Bf[u] != St && nf < 2) fr[nf] = Bf[u], fa[nf] = ba[u], ++nf;
     if (tid == 0) {
-      tc::issue_product(tmem, set_col[0], aC, aC, pl, R, false, false);
+      tc::issue_product(tmem, set_col[0], aC, pl, aC, R, false, false);
       tc::commit(&mbar[0]);
-      tc::issue_product(tmem, set_col[1], aS, aS, pl, R, false, false);
+      tc::issue_product(tmem, set_col[1], aS, pl, aS, R, false, false);
       tc::commit(&mbar[1]);
     }
     const bool w0 = wait_all(0), w1 = wait_all(1);
@@ -825,7 +830,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step_stk(DevSys s, int
     }
     epi_sq(0, one, true, fr[0]);
     sync_all();
-    if (tid == 0) tc::issue_product(tmem, set_col[0], aC, aS, pl, R, false, false), tc::commit(&mbar[0]);
+    if (tid == 0) tc::issue_product(tmem, set_col[0], aC, pl, aS, R, false, false), tc::commit(&mbar[0]);
     if (!wait_all(0)) {
       ok = false;
       break;
@@ -916,10 +921,10 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_dyson(DevSys s, int k,
     }
     if (tid == 0) {
       tc::fence_after();
-      tc::issue_product(tmem, 0, aAr, aC, pl, R, false, false);                // re  = Ar^T C
-      tc::issue_product(tmem, 0, aAi, aS, pl, R, false, true);                 // re += Ai^T S
-      tc::issue_product(tmem, uint32_t(3 * R), aAi, aC, pl, R, false, false);  // im  = Ai^T C
-      tc::issue_product(tmem, uint32_t(3 * R), aAr, aS, pl, R, true, true);    // im -= Ar^T S
+      tc::issue_product(tmem, 0, aAr, pl, aC, R, false, false);                // re  = Ar^T C
+      tc::issue_product(tmem, 0, aAi, pl, aS, R, false, true);                 // re += Ai^T S
+      tc::issue_product(tmem, uint32_t(3 * R), aAi, pl, aC, R, false, false);  // im  = Ai^T C
+      tc::issue_product(tmem, uint32_t(3 * R), aAr, pl, aS, R, true, true);    // im -= Ar^T S
       tc::commit(&mbar[0]);
     }
     {
@@ -1053,8 +1058,8 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_dyson_stk(DevSys s, in
     }
     if (tid == 0) {
       tc::fence_after();
-      tc::issue_product(tmem, 0, aA1, plA, aC, plB, R, false, false);  // [Ar^T C; Ai^T C]
-      tc::issue_product(tmem, 0, aA2, plA, aS, plB, R, false, true);   // + [Ai^T S; -Ar^T S]
+      tc::issue_product(tmem, 0, aA1, plA, aC, R, false, false);  // [Ar^T C; Ai^T C]
+      tc::issue_product(tmem, 0, aA2, plA, aS, R, false, true);   // + [Ai^T S; -Ar^T S]
       tc::commit(&mbar[0]);
     }
     {
