@@ -66,10 +66,10 @@ __device__ __forceinline__ int tix(int r, int k, int R) {
 
 // Shared-memory matrix descriptor of a plane (start >> 4 in bits 0-13, leading byte offset
 // >> 4 in 16-29, stride byte offset >> 4 in 32-45, version 1 at bit 46, no swizzle).
-__device__ __forceinline__ uint64_t sdesc(uint32_t addr, int R) {
-  return uint64_t((addr & 0x3FFFF) >> 4) | (uint64_t(128 >> 4) << 16) | (uint64_t(sbo_bytes(R) >> 4) << 32) |
-         (1ull << 46);
-}
+// As its two words: the high one is the layout's, the low one moves with the address (in units of
+// 16 bytes).
+__device__ __forceinline__ uint32_t sdesc_lo(uint32_t addr) { return ((addr & 0x3FFFF) >> 4) | ((128u >> 4) << 16); }
+__host__ __device__ constexpr uint32_t sdesc_hi(int R) { return uint32_t(sbo_bytes(R) >> 4) | (1u << 14); }
 // Instruction descriptor, kind::f16: FP32 accumulator (bits 4-5 = 1), A and B BF16 (bits
 // 7-9, 10-12 = 1), optional negation of A (bit 13), both K-major, N >> 3 in bits 17-22,
 // M >> 4 in bits 24-28 (M = 128).
@@ -78,11 +78,12 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int N, bool negA) {
          (uint32_t(128 >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+// operand tiles of one layout (hi): a, b from sdesc_lo
+__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc, uint32_t acc) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc));
+      "{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %5, 0;\n mov.b64 da, {%1, %3};\n mov.b64 db, {%2, %3};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}" ::"r"(d),
+      "r"(a), "r"(b), "r"(hi), "r"(idesc), "r"(acc));
 }
 __device__ __forceinline__ void commit(uint64_t *mbar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(mbar))
@@ -230,19 +231,33 @@ __device__ __forceinline__ float2 normal(float2 v) {
 // as the accumulators do in columns, so pairs of one A plane with consecutive B planes are one MMA
 // of N = 2R or 3R: seven MMAs a K step, each reading its A plane once (an MMA of N = 64 is bound by
 // the shared-memory reads, two thirds of them A's).
-__device__ __forceinline__ void issue_product(uint32_t tmem, uint32_t col, uint32_t a, uint32_t plA, uint32_t b,
-                                              int R, bool negA, bool accumulate) {
-  const uint32_t plB = uint32_t(R / 8 * sbo_bytes(R));
-  const int sp[7] = {0, 0, 1, 1, 2, 2, 3}, tp[7] = {0, 3, 0, 2, 0, 1, 0};
-  const int lev[7] = {0, 2, 1, 2, 2, 2, 2}, wide[7] = {3, 1, 2, 1, 1, 1, 1};
+// The K steps are unrolled (KS = R / 16) and a descriptor costs one addition: with 64-bit
+// descriptors built per MMA, one thread took 144 clocks to issue each, more than the MMA runs.
+template <int KS>
+__device__ __noinline__ void issue_product_k(uint32_t tmem, uint32_t col, uint32_t a, uint32_t plA, uint32_t b,
+                                             bool negA, bool accumulate) {
+  constexpr int R = 16 * KS;
+  constexpr uint32_t plB = uint32_t(R / 8 * sbo_bytes(R)) / 16, hi = sdesc_hi(R);
+  constexpr int sp[7] = {0, 0, 1, 1, 2, 2, 3}, tp[7] = {0, 3, 0, 2, 0, 1, 0};
+  constexpr int lev[7] = {0, 2, 1, 2, 2, 2, 2}, wide[7] = {3, 1, 2, 1, 1, 1, 1};
+  const uint32_t alo = sdesc_lo(a), blo = sdesc_lo(b), pa = plA / 16, neg = idesc_bf16(0, negA);
 #pragma unroll
   for (int q = 0; q < 7; ++q) {
-    const uint32_t id = idesc_bf16(wide[q] * R, negA), d = tmem + col + uint32_t(lev[q] * R);
-    const uint32_t a0 = a + uint32_t(sp[q]) * plA, b0 = b + uint32_t(tp[q]) * plB;
-    for (int kk = 0; kk < R / 16; ++kk)
-      mma(d, sdesc(a0 + kk * 256, R), sdesc(b0 + kk * 256, R), id, (!accumulate && q == 0 && kk == 0) ? 0u : 1u);
+    const uint32_t a0 = alo + uint32_t(sp[q]) * pa, b0 = blo + uint32_t(tp[q]) * plB;
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk)
+      mma(tmem + col + uint32_t(lev[q] * R), a0 + 16u * kk, b0 + 16u * kk, hi, neg | idesc_bf16(wide[q] * R, false),
+          (q == 0 && kk == 0) ? uint32_t(accumulate) : 1u);
   }
 }
+__device__ __forceinline__ void issue_product(uint32_t tmem, uint32_t col, uint32_t a, uint32_t plA, uint32_t b,
+                                              int R, bool negA, bool accumulate) {
+  static_assert(kMinB > 32 && up16(kMaxB) <= 80, "K steps: 3 to 5");
+  if (R == 48) issue_product_k<3>(tmem, col, a, plA, b, negA, accumulate);
+  else if (R == 64) issue_product_k<4>(tmem, col, a, plA, b, negA, accumulate);
+  else issue_product_k<5>(tmem, col, a, plA, b, negA, accumulate);
+}
+
 // -2^-8 / (k (k + 1)) (the units of slice4f) as double-float for the Horner steps (k = 1 .. 31), folded at compile time
 // into constant memory (k is the same in every thread), so that no epilogue divides in FP64
 #define BL_HC(k) dfv_const(-0x1p-8 / (double(k) * double((k) + 1)))
@@ -395,7 +410,7 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c = blockIdx.x % s.C, i = blockIdx.x / s.C;
   if (tid < 2) gfail[tid] = 0;
-  const int b = s.bs[k], bp = s.bpoff[k], bb = b * b;
+  const int b = s.bs[k];
   const int R = tc::up16(b), pe = int(tc::plane_bytes(b) / 2);  // plane stride in BF16 units
   const int ncols = tc::pow2_cols(6 * R);
   unsigned char *base = tsm + ((1024 - (tc::saddr(tsm) & 1023)) & 1023);

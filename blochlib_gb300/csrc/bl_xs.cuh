@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(xs::kThreadsXs, 1)
   const int c = int(g % Cb), sl = int(g / Cb);
   const int tn = (n + kN - 1) / kN;
   const int r0 = int(blockIdx.x / tn) * TM, q0 = int(blockIdx.x % tn) * kN;
-  const int rows = min(TM, m - r0), cols = min(kN, n - q0), N16 = (cols + 15) / 16 * 16;
+  const int rows = min(TM, m - r0), cols = min(kN, n - q0);
   const int kc = CPLX ? kK / 2 : kK;  // source k per chunk
   const int nch = (k + kc - 1) / kc;
   unsigned char *base = xsm + ((1024 - (tc::saddr(xsm) & 1023)) & 1023);
@@ -216,7 +216,6 @@ __global__ void __launch_bounds__(xs::kThreadsXs, 1)
     if (bad) bad_s = 1;
     if (ok && !tc::wait_parity(&done, 0)) failed = 1;
   } else if (lane == 0) {
-    const uint32_t id = tc::idesc_bf16(N16, false);
     for (int ch = 0; ch < nch; ++ch) {
       const int buf = ch & 1;
       if (!tc::wait_parity(&full[buf], uint32_t((ch / 2) & 1))) {
@@ -224,19 +223,29 @@ __global__ void __launch_bounds__(xs::kThreadsXs, 1)
         break;
       }
       tc::fence_after();
-      const uint32_t a = tc::saddr(base + buf * buf_bytes<S>()), b = a + S * kPlaneA;
+      const uint32_t a = tc::sdesc_lo(tc::saddr(base + buf * buf_bytes<S>())), b = a + S * kPlaneA / 16;
       // the last chunk's K entries beyond k are zeros; a whole 16-entry half of them is skipped
       const int ks = (ch == nch - 1 && (k - ch * kc) * (CPLX ? 2 : 1) <= 16) ? 1 : 2;
-#pragma unroll 1
-      for (int lev = 0; lev <= kTop; ++lev) {
-        const uint32_t d = tmem + uint32_t(min(lev, kLev - 1) * kN);
-        for (int i = max(0, lev - (S - 1)); i <= min(lev, S - 1); ++i) {
-          const int j = lev - i;
-          const bool first = ch == 0 && lev < kLev && i == max(0, lev - (S - 1));
-          for (int kk = 0; kk < ks; ++kk)
-            tc::mma(d, tc::sdesc(a + i * kPlaneA + kk * 256, kK), tc::sdesc(b + j * kPlaneB + kk * 256, kK), id,
-                    first && kk == 0 ? 0u : 1u);
-        }
+      // A's digit i with B's digits j, j + 1, ..: the digit planes of B follow one another in whole
+      // row groups as the levels' accumulators do in columns, so up to four pairs are one MMA
+      // (N <= 256; columns beyond the tile's are not read).  Unrolled, a descriptor costs one
+      // addition: 16 MMAs a K step for 34 pairs (S = 7), 8 for 21 (S = 6).
+      auto pairs = [&](int i, int j, int w, int lev) {
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk)
+          if (kk < ks)
+            tc::mma(tmem + uint32_t(lev * kN), a + uint32_t(i * kPlaneA / 16 + kk * 16),
+                    b + uint32_t(j * kPlaneB / 16 + kk * 16), tc::sdesc_hi(kK), tc::idesc_bf16(w * kN, false),
+                    i == 0 && lev < kLev && kk == 0 && j == lev ? uint32_t(ch != 0) : 1u);
+      };
+#pragma unroll
+      for (int i = 0; i < S; ++i) {
+#pragma unroll
+        for (int j = 0; j < kLev - i; j += 4) pairs(i, j, min(4, kLev - i - j), i + j);
+      }
+      if (kTop >= kLev) {  // the last level shares an accumulator with the one before
+#pragma unroll
+        for (int i = kTop - (S - 1); i < S; ++i) pairs(i, kTop - i, 1, kLev - 1);
       }
       tc::commit(&empty[buf]);
     }
