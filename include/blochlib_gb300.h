@@ -73,7 +73,8 @@ typedef struct {
                       Jacobi sweeps (FIDs of at most 64 rotor periods) and a double-float or
                       FP64 Cayley transform, eigenvectors and eigenvalues; single-precision
                       eigenframe, Q/R, Fave and FID terms; powder sum in FP64.  Blocks above
-                      74 stay FP64. */
+                      74: step and Dyson products as exact digit slices on the tensor cores
+                      (six base-256 digits, FP64 storage). */
   int step_method; /* step exponential exp(-i 2pi tau H): 0 = eigen-decomposition (Jacobi),
                       1 = Taylor series with scaling and squaring; FP64, or in the mixed form
                       as above (blocks up to 8 with step_method 1, blocks 9-74 always) */
