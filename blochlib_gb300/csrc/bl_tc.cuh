@@ -38,11 +38,10 @@ namespace tc {
 
 constexpr int kTcThreads = 512;          // 16 warps: four per TMEM lane quarter
 constexpr int kMaxB = kMaxBigBlock;      // largest block on these kernels (up16 = 80)
-// smallest block on these kernels: below it the per-item costs (TMEM allocation, H assembly,
-// one synchronised epilogue per product) outweigh the products, and the double-float kernels
-// are faster (b = 28: the tensor-core step takes 3x the double-float step's time per item;
-// with the stacked kernels, moving c3's 35-blocks here took its 512-system batch from 57.0
-// to 54.2 FIDs/s)
+// smallest block on these kernels: smaller ones keep the double-float products (2^-48 each against
+// 2^-32 here).  From 33 on these kernels are the faster ones (16 requests of 2 to 7 spins through
+// the serving loop: 211 ms against 235), but 7- and 9-spin FIDs then differ from 64-bit propagation
+// by 4.9e-8 instead of 4.5e-8 on average; below 33 the M = 128 tile is mostly padding.
 constexpr int kMinB = 40;
 constexpr unsigned long long kWaitNs = 1000000000ull;  // an mbarrier wait gives up after 1 s
 
