@@ -1,19 +1,20 @@
 // Huge-block kernels (Hamiltonian blocks kMaxBigBlock < b <= kMaxHugeBlock, 9-12 like
 // spins 1/2), included by bl_engine.cu after bl_big.cuh.  A block no longer fits shared
-// memory, so each stage is a sequence of batched products of per-crystallite matrices:
-// 64 x 64 output tiles per CTA, 16-wide k panels staged in shared memory, 4 x 4 outputs
-// per thread.  Operands are addressed in place in the engine's [item][c] buffers (HMat
-// with element stride Cpad) or in a workspace of contiguous per-item matrices (element
-// stride 1).  With FP64 issue as the bound (one 64x64x16 complex panel is 262k FMA against
-// 32 KB of loads), the strided panel loads cost well under 1 B/clock per SM.
-//   step       k_huge_fk, k_huge_hbuild, k_huge_norm, k_huge_sym x 7, k_huge_low, squarings,
+// memory, so each stage is a sequence of batched products of per-crystallite matrices, by digit
+// slices on the tensor cores (k_xs_gemm in bl_xs.cuh) or, where its sums would not stay exact or
+// the operands are single precision, as 64 x 64 output tiles per CTA, 16-wide k panels staged in
+// shared memory, 4 x 4 outputs per thread.  Operands are addressed in place in the engine's
+// [item][c] buffers (HMat with element stride Cpad) or in a workspace of contiguous per-item
+// matrices (element stride 1).  With FP64 issue as the tiles' bound (one 64x64x16 complex panel is
+// 262k FMA against 32 KB of loads), the strided panel loads cost well under 1 B/clock per SM.
+//   step       k_huge_fk, k_huge_hbuild, k_huge_norm, products, k_huge_low, squarings,
 //              k_huge_store_u: the same symmetric Paterson-Stockmeyer exponential as
 //              k_big_step, over a chunk of (crystallite, step) items at a time
 //   Dyson      products per step of all segments at once (A_{i+1} = U_i A_i), then the chain over
 //              the segments' last products; k_huge_copy starts each
 //   Floquet    k_huge_floquet: floquet_cta with its two b x b matrices in global memory
-//   eigenframe k_huge_zgemm (A_{i+1} V_F) into the workspace, copied back in FP64
-//   Q/R        k_huge_mx (X = M_ab W_b from M's non-zeros) and k_huge_zgemm (W_a^H X)
+//   eigenframe products (A_{i+1} V_F) into the workspace, copied back in FP64
+//   Q/R        k_huge_mx (X = M_ab W_b from M's non-zeros), then W_a^H X
 // Items are numbered g = sl*C + c (crystallite c, step sl); a launch covers
 // g = j0 + blockIdx.y, and the workspace holds the launch's items by blockIdx.y.
 

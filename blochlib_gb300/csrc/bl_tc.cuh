@@ -628,10 +628,13 @@ __global__ void __launch_bounds__(tc::kTcThreads, 1) k_tc_step(DevSys s, int k, 
 // Y's rows in lanes m and R + m; the two Horner chains run as one, T = [T_C; T_S] stacked,
 // T <- [I + c_C Y T_C; I + c_S Y T_S] from the single product T Y (T_C, T_S and Y are
 // polynomials in Y and commute), the sine series carried to the same number of terms as the
-// cosine (one more than it needs); S = T_S X from the same stacked T (X as B operand in Wt).  Every TMEM lane
-// quarter holds rows for each epilogue.  C and S end in R-row tiles, where the squarings
-// (as in k_tc_step) and the slab copy take them.  Shared memory: XS and T (stacked), two
-// R-row tiles (Y, then C; H's scratch, then S), the over-read margin of an R-row A tile.
+// cosine (one more than it needs); S = T_S X from the same stacked T (X as B operand in Wt).
+// Every TMEM lane quarter holds rows for each epilogue.  C and S end in R-row tiles, where the
+// squarings (as in k_tc_step) and the slab copy take them.  Shared memory: XS and T (stacked), two
+// R-row tiles (H's scratch, Y, then C; X, then S), the over-read margin of an R-row A tile.
+// Bound by one CTA per SM taking its phases in turn: at b = 56 and degree 5 prologue 6k clocks, X
+// slices 2.6k, three products of 2.2 to 2.5k, their epilogues 2 to 4k each, the slab 2.4k (46k
+// clocks a step with H assembled here, a 62-operation epilogue and per-MMA descriptors: 27k now).
 __host__ __device__ constexpr size_t tc_step_stk_smem(int b) {
   return 8 * tc_stk_plane_bytes(b) + 2 * tc::tile_bytes(b) + tc::overread_bytes(b) + 1024;
 }
