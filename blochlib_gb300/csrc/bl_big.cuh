@@ -498,7 +498,7 @@ __device__ __forceinline__ C rot_mix(T c, C x, C s, C y) {
 
 // The parallel Jacobi sweeps of floquet_cta over the Hermitian K with V accumulating the rotations;
 // returns convergence.  The angles come from single precision; in FP64 each rotation is scaled to
-// c^2 + |s|^2 = 1, as in lanes_sweeps.  A round's pairs are disjoint, so K <- G^H K G splits into
+// c^2 + |s|^2 = 1 and elements at the diagonal's rounding are set to zero, as in lanes_sweeps.  A round's pairs are disjoint, so K <- G^H K G splits into
 // 2 x 2 blocks (pair t1's rows, pair t2's columns): only t1 <= t2 is computed and its conjugate
 // stored with it, 24 FP64 operations per element pair against 48 for columns then rows of the
 // whole of K, and one barrier less per round.
@@ -506,7 +506,7 @@ template <class C>
 __device__ bool floquet_sweeps(C *K, C *V, int b, int max_sweeps, const FloqWork &wk) {
   using T = decltype(C::x);
   constexpr bool kF64 = sizeof(T) == 8;
-  C *rot = reinterpret_cast<C *>(wk.rot);  // per pair: (c, 0), (s e^{i ph})
+  C *rot = reinterpret_cast<C *>(wk.rot);  // per pair: (c, 1 to set K_pq to zero), (s e^{i ph})
   auto rpair = [&](int t, int q) -> int & { return wk.rpair[2 * t + q]; };
   double *red = wk.red;
   const int bb = b * b;
@@ -562,9 +562,11 @@ __device__ bool floquet_sweeps(C *K, C *V, int b, int max_sweeps, const FloqWork
         C rc = mkc<C>(1, 0), rs = mkc<C>(0, 0);
         if (q < b) {
           const float hx = float(K[p * b + q].x), hy = float(K[p * b + q].y);
-          const float ab = hypotf(hx, hy);
-          if (ab != 0.f) {
-            const float theta = 0.5f * float(K[q * b + q].x - K[p * b + p].x) / ab;
+          const T kpp = K[p * b + p].x, kqq = K[q * b + q].x;
+          const float ab = hypotf(hx, hy), dmax = kF64 ? fmaxf(fabsf(float(kpp)), fabsf(float(kqq))) : 0.f;
+          if (kF64 && ab <= kSweepZero * dmax) rc.y = 1;
+          if (ab > kSweepRound * dmax) {
+            const float theta = 0.5f * float(kqq - kpp) / ab;
             float tt;
             if (fabsf(theta) > 1e18f) tt = 0.5f / theta;  // theta^2 stays finite
             else tt = copysignf(1.f, theta) / (fabsf(theta) + sqrtf(fmaf(theta, theta, 1.f)));
@@ -607,7 +609,10 @@ __device__ bool floquet_sweeps(C *K, C *V, int b, int max_sweeps, const FloqWork
             kqp = rot_mix(c1, kqp, j1, kpp), kqq = rot_mix(c1, kqq, j1, kpq);
             kpp = x, kpq = y;
           }
-          if (t1 == t2) kpp.y = 0, kqq.y = 0, kqp = cconj(kpq);  // the diagonal stays real
+          if (t1 == t2) {  // the diagonal stays real
+            if (rot[2 * t1].y != 0) kpq = zero;
+            kpp.y = 0, kqq.y = 0, kqp = cconj(kpq);
+          }
           K[p1 * b + p2] = kpp;
           if (t1 != t2) K[p2 * b + p1] = cconj(kpp);
           if (h2) K[p1 * b + q2] = kpq;

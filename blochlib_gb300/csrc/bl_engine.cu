@@ -1439,11 +1439,21 @@ __device__ __forceinline__ int lanes_cayley(const LaneGroup<B> &g, int r, const 
   return st;
 }
 
+// FP64 sweeps: a rotated element is set to zero when it was at most kSweepZero of the pair's larger
+// diagonal element (an angle from single precision leaves under 2^-21 of it), and neither rotated nor
+// kept at kSweepRound of it.
+constexpr float kSweepZero = 0x1p-32f, kSweepRound = 0x1p-52f;
 // Parallel (round-robin) complex Jacobi sweeps over K, at most `sweeps`; with VEC, V (FP64)
 // accumulates the rotations from the identity.  The rotation angles come from single precision
 // in both forms (an FP64 hypot, three divisions and two square roots per rotation were more than
 // half of the kernel's FP64 instructions): a rotation that misses its angle by 1e-7 of it leaves
-// 1e-7 of the element, which the next sweep removes, so the sweep count stays.  Each rotation is
+// 1e-7 of the element, which the next sweep removes.  Where that is below the rounding of the
+// diagonal (kSweepZero), the element is set to zero after its rotation, and one at the rounding
+// itself (kSweepRound) without a rotation: between equal eigenvalues (equivalent spins, spins
+// without couplings) the angle is of order one, and what such a rotation leaves is fresh rounding of
+// the diagonal, sweep after sweep.  Sweeps of matrices with two to b distinct eigenvalues, b = 2 to
+// 35, in this arithmetic on the host: 5.5 on average and at most 17 (with FP64 angles and every rotated
+// element set to zero 5.4 and at most 30); of generic ones 5.6 (5.1).  Each rotation is
 // scaled to c^2 + |s|^2 = 1 in FP64 (n^-1/2 = 1 - d/2 + 3 d^2/8 for n = 1 + d, d ~ 1e-7), so V
 // stays unitary to FP64 rounding; K takes the scaled rotation in FP64 and the single-precision
 // one otherwise.  T = double stops at off(K)^2 <= 1e-34 diag(K)^2 (or 1e-60: K = tan(phase / 2), so
@@ -1501,10 +1511,12 @@ __device__ __forceinline__ bool lanes_sweeps(const LaneGroup<B> &g, int r, typen
       const CT hpq = g.shfl(own_q, mp);
       const T kpp = g.shfl(own_d.x, mp), kqq = g.shfl(own_d.x, mq);
       float cf = 1.f, sx = 0.f, sy = 0.f;
+      bool zero = false;
       if (paired) {
         const float hx = float(hpq.x), hy = float(hpq.y);
-        const float ab = hypotf(hx, hy);
-        if (ab != 0.f) {
+        const float ab = hypotf(hx, hy), dmax = F32 ? 0.f : fmaxf(fabsf(float(kpp)), fabsf(float(kqq)));
+        zero = !F32 && ab <= kSweepZero * dmax;
+        if (ab > kSweepRound * dmax) {
           const float theta = 0.5f * float(kqq - kpp) / ab;
           float tt;
           if (fabsf(theta) > 1e18f) tt = 0.5f / theta;  // theta^2 stays finite
@@ -1560,6 +1572,7 @@ __device__ __forceinline__ bool lanes_sweeps(const LaneGroup<B> &g, int r, typen
           const CT u = isp ? kpk : kqk, v = isp ? kqk : kpk, sg = isp ? be : al;
           K[q2] = cadd(cscale(u, cs), cmul(sg, v));
           if (q2 == r) K[q2].y = T(0);
+          if (zero && q2 == (isp ? mq : mp)) K[q2] = cxm(T(0), T(0));
         }
       }
     }
