@@ -564,8 +564,8 @@ __device__ bool floquet_sweeps(C *K, C *V, int b, int max_sweeps, const FloqWork
           const float hx = float(K[p * b + q].x), hy = float(K[p * b + q].y);
           const T kpp = K[p * b + p].x, kqq = K[q * b + q].x;
           const float ab = hypotf(hx, hy), dmax = kF64 ? fmaxf(fabsf(float(kpp)), fabsf(float(kqq))) : 0.f;
-          if (kF64 && ab <= kSweepZero * dmax) rc.y = 1;
-          if (ab > kSweepRound * dmax) {
+          if (kF64 && ab <= fmaxf(kSweepZero * dmax, kSweepTiny)) rc.y = 1;
+          if (ab > fmaxf(kSweepRound * dmax, kSweepTiny)) {
             const float theta = 0.5f * float(kqq - kpp) / ab;
             float tt;
             if (fabsf(theta) > 1e18f) tt = 0.5f / theta;  // theta^2 stays finite
@@ -1349,7 +1349,7 @@ __device__ bool floquet_sweeps_df(float2 *Xk, float4 *Vd, int b, int max_sweeps,
         if (q < b) {
           const float2 hpq = Xk[p * b + q];
           const float ab = hypotf(hpq.x, hpq.y);
-          if (ab != 0.f) {
+          if (ab > kSweepTiny) {  // (a denormal element's phase has too few bits to be a rotation's)
             const float phx = hpq.x / ab, phy = hpq.y / ab;
             const float theta = 0.5f * (Xk[q * b + q].x - Xk[p * b + p].x) / ab;
             float tt;

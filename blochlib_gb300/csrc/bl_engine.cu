@@ -1441,8 +1441,10 @@ __device__ __forceinline__ int lanes_cayley(const LaneGroup<B> &g, int r, const 
 
 // FP64 sweeps: a rotated element is set to zero when it was at most kSweepZero of the pair's larger
 // diagonal element (an angle from single precision leaves under 2^-21 of it), and neither rotated nor
-// kept at kSweepRound of it.
-constexpr float kSweepZero = 0x1p-32f, kSweepRound = 0x1p-52f;
+// kept at kSweepRound of it.  Either form: no rotation for an element of at most kSweepTiny (off(K)^2
+// is below 1e-60 then; 1 / |K_pq| overflows from 2^-128 down, and equal diagonal elements make that
+// factor count).
+constexpr float kSweepZero = 0x1p-32f, kSweepRound = 0x1p-52f, kSweepTiny = 1e-30f;
 // Parallel (round-robin) complex Jacobi sweeps over K, at most `sweeps`; with VEC, V (FP64)
 // accumulates the rotations from the identity.  The rotation angles come from single precision
 // in both forms (an FP64 hypot, three divisions and two square roots per rotation were more than
@@ -1515,8 +1517,8 @@ __device__ __forceinline__ bool lanes_sweeps(const LaneGroup<B> &g, int r, typen
       if (paired) {
         const float hx = float(hpq.x), hy = float(hpq.y);
         const float ab = hypotf(hx, hy), dmax = F32 ? 0.f : fmaxf(fabsf(float(kpp)), fabsf(float(kqq)));
-        zero = !F32 && ab <= kSweepZero * dmax;
-        if (ab > kSweepRound * dmax) {
+        zero = !F32 && ab <= fmaxf(kSweepZero * dmax, kSweepTiny);
+        if (ab > fmaxf(kSweepRound * dmax, kSweepTiny)) {
           const float theta = 0.5f * float(kqq - kpp) / ab;
           float tt;
           if (fabsf(theta) > 1e18f) tt = 0.5f / theta;  // theta^2 stays finite

@@ -42,3 +42,19 @@ def test_equal_eigenphases_match_oracle(name, form):
                      rng.uniform(0, 2 * np.pi, count), rng.uniform(0.1, 1, count)], axis=1)
     ref, _ = oracle_fid(job, rows)
     assert rel(gpu_fid(job, rows, precision=int(mixed)), ref) <= (1e-6 if mixed else 1e-10)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("coupling", [1e-34, 1e-37, 1e-40])
+@pytest.mark.parametrize("nspin", [4, 6])
+def test_couplings_below_the_single_precision_range(nspin, coupling, precision):
+    """A pair with a coupling near and below the smallest normal FP32 number, equal shifts, beside a
+    strongly coupled pair: the element's reciprocal overflows in FP32."""
+    lines = [f"numspin {nspin}"] + [f"T 1H {k}" for k in range(nspin)]
+    lines += ["D 5000 0 1 30 50 0", f"D {coupling!r} 2 3 70 20 0"] + [f"D 900 1 {k} 10 80 0" for k in range(4, nspin)]
+    n, wr = 24, 1.0e4
+    job = "".join(f"spin: {l}\n" for l in lines) + (
+        f"npts: 40\nsw: {n * wr!r}\nwr: {wr!r}\nrotb: 54.7356\nrho: Ix 0\ndet: Fp\n")
+    rows = np.array([[0.3, 1.1, 0.2, 1.0], [2.0, 0.4, 1.5, 0.5], [4.1, 2.2, 5.0, 0.7]])
+    ref, _ = oracle_fid(job, rows)
+    assert rel(gpu_fid(job, rows, precision=precision), ref) <= (1e-6 if precision else 1e-10)
