@@ -207,6 +207,7 @@ struct DevSys {
   const int *srp, *seo;      // per D pair (a,b): the rho pair (b,a) and first element, or -1
   const double2 *tw;         // exp(-2 pi i k / M), k < M
   double tau, wr, sin_rotb, cos_rotb, scale;
+  double wref, wscale;  // mixed form's FID terms: largest |weight|; wref scale / fftq, applied in FP64
   // per block
   const int *bs, *boff, *bpoff;
   // per interaction: crystal tensor (xx xy xz yy yz zz), scale, packed operator
@@ -2324,7 +2325,8 @@ __global__ void __launch_bounds__(128) k_fave_fft(DevSys s) {
     const C wo = cmul(twb[q], mkc<C>(0.5 * d.y, -0.5 * d.x));
     return p < Mh ? cadd(ev, wo) : csub(ev, wo);
   };
-  const double invM = 1.0 / double(M);
+  // 1/M; in single precision its power of two only (exact), 1/q follows with the weights (wscale)
+  const double invM = 1.0 / double(kF ? M / q5 : M);
   C *Gb = Bufs<C>::G(s);
   if (half && twist) {  // n == M: frequencies q and q + M/2 share E_q and w^q O_q
     for (int idx = threadIdx.x; idx < Mh * CG; idx += blockDim.x) {
@@ -2514,7 +2516,7 @@ __global__ void __launch_bounds__(kThreads) k_p2p_elems(DevSys s) {
 // Per element it stages z_e^j and G_p(e) of its 32 crystallites in shared memory by
 // asynchronous copies (coalesced: crystallites are fastest in HBM; double-buffered, so the
 // next element's copies are in flight while this one is summed), and each thread updates its
-// tile with w_c scale z, accumulating one element in FP32 and folding it into double-float
+// tile with (w_c / wref) z, accumulating one element in FP32 and folding it into double-float
 // (hi + lo) sums.  ft_sub groups of 64 threads each take a part of the
 // range and add up their double-float sums in order (one or two 64-thread CTAs an SM before where
 // there are few elements or crystallites: 4 spins, 3722 crystallites 0.315 -> 0.274 ms; 9 spins, 32
@@ -2547,7 +2549,7 @@ __global__ void __launch_bounds__(kFtThreads * 4) k_fid_tiled(DevSys s) {
   const int c0 = g * 32;
   if (threadIdx.x < 32) {
     const int c = c0 + tid;
-    ws[tid] = c < s.C ? float(s.w[c] * s.scale) : 0.f;
+    ws[tid] = c < s.C ? float(s.w[c] / s.wref) : 0.f;
   }
   __syncthreads();
   auto sub_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(sub + 1), "n"(kFtThreads) : "memory"); };
@@ -2647,8 +2649,8 @@ __global__ void __launch_bounds__(kFtThreads * 4) k_fid_tiled(DevSys s) {
       const int j = j0 + 4 * jt + a, p = p0 + 4 * pt + b;
       const long k = long(j) * s.gper + p;
       if (j < s.J && p < s.gper && k < s.npts)
-        s.partial[row * s.npts + k] = make_double2(double(hi[a][b].x) + double(lo[a][b].x),
-                                                   double(hi[a][b].y) + double(lo[a][b].y));
+        s.partial[row * s.npts + k] = make_double2((double(hi[a][b].x) + double(lo[a][b].x)) * s.wscale,
+                                                   (double(hi[a][b].y) + double(lo[a][b].y)) * s.wscale);
     }
 }
 
@@ -3744,6 +3746,12 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     s.scale = 1.0 / dd;
     s.gper = J.pb;
   }
+  // A factor that every term shares (1/M, the scale, equal weights) is no single-precision number in
+  // general, and its rounding, up to 2^-24, would shift the whole FID: 6e-8 at 48 steps.
+  s.wref = 0.0;
+  for (int c = 0; c < J.C; ++c) s.wref = std::max(s.wref, std::fabs(pw.weight[c]));
+  if (!(s.wref > 0.0 && std::isfinite(s.wref))) s.wref = 1.0;
+  s.wscale = s.wref * s.scale / double(s.fftq);
   s.bs = J.bs.p, s.boff = J.boff.p, s.bpoff = J.bpoff.p;
   s.pas = J.pas.p, s.iscale = J.iscale.p, s.Tk = J.Tk.p, s.Hc = J.Hc.p;
   s.fk = use_fk ? J.fkc.p : nullptr;
