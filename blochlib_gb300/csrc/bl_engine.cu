@@ -1369,13 +1369,9 @@ __device__ __forceinline__ int lanes_cayley(const LaneGroup<B> &g, int r, const 
 #pragma unroll
   for (int q = 0; q < B; ++q) {
     const double id = (q == r) ? 1.0 : 0.0;
-    if constexpr (sizeof(T) == sizeof(float)) {
-      const float2 w = cmul(cvt<float2>(ea), cvt<float2>(U[q]));
-      M[q] = cxm(T(id) + w.x, w.y), X[q] = cxm(T(id) - w.x, -w.y);
-    } else {
-      const double2 w = cmul(ea, U[q]);
-      M[q] = cxm(T(id + w.x), T(w.y)), X[q] = cxm(T(id - w.x), T(-w.y));
-    }
+    // I + W and I - W rounded once: W rounded on its own would add 2^-24 where they are small
+    const double2 w = soft ? todbl(cmul(cvt<float2>(ea), cvt<float2>(U[q]))) : cmul(ea, U[q]);
+    M[q] = cxm(T(id + w.x), T(w.y)), X[q] = cxm(T(id - w.x), T(-w.y));
   }
 #pragma unroll
   for (int kc = 0; kc < B; ++kc) {
@@ -1456,8 +1452,9 @@ constexpr float kSweepZero = 0x1p-32f, kSweepRound = 0x1p-52f, kSweepTiny = 1e-3
 // without couplings) the angle is of order one, and what such a rotation leaves is fresh rounding of
 // the diagonal, sweep after sweep.  Sweeps of matrices with two to b distinct eigenvalues, b = 2 to
 // 35, in this arithmetic on the host: 5.5 on average and at most 17 (with FP64 angles and every rotated
-// element set to zero 5.4 and at most 30); of generic ones 5.6 (5.1).  Each rotation is
-// scaled to c^2 + |s|^2 = 1 in FP64 (n^-1/2 = 1 - d/2 + 3 d^2/8 for n = 1 + d, d ~ 1e-7), so V
+// element set to zero 5.4 and at most 30); of generic ones 5.6 (5.1).  In single precision the angle
+// has all of K's bits and every rotated element is set to zero: turning what its rounding leaves once
+// more would put that into V.  Each rotation is scaled to c^2 + |s|^2 = 1 in FP64 (n^-1/2 = 1 - d/2 + 3 d^2/8 for n = 1 + d, d ~ 1e-7), so V
 // stays unitary to FP64 rounding; K takes the scaled rotation in FP64 and the single-precision
 // one otherwise.  T = double stops at off(K)^2 <= 1e-34 diag(K)^2 (or 1e-60: K = tan(phase / 2), so
 // what is left is far below any phase); T = float one sweep after 1e-10 diag(K)^2 (quadratic
@@ -1527,6 +1524,7 @@ __device__ __forceinline__ bool lanes_sweeps(const LaneGroup<B> &g, int r, typen
           cf = rsqrtf(fmaf(tt, tt, 1.f));
           const float ts = tt * cf / ab;
           sx = hx * ts, sy = hy * ts;
+          zero = zero || F32;
         }
       }
       double cd = cf;
