@@ -3882,24 +3882,27 @@ static void huge_mm(JobImpl &J, const DevSys &s, cudaStream_t st, bool conjA, HM
                     int eb) {
   const unsigned tx = unsigned(((m + 63) / 64) * ((n + xs::kN - 1) / xs::kN));
   const XsReal none{};
-  if (s.mixed) {
-    k_xs_gemm<true, 6, false, double2><<<dim3(tx, unsigned(items)), xs::kThreadsXs, xs::smem<6>(), st>>>(
-        A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
-  } else if (2 * k <= 512) {
-    if (conjA)
-      k_xs_gemm<true, 7, true, double2><<<dim3(tx, unsigned(items)), xs::kThreadsXs, xs::smem<7>(), st>>>(
+  for (; items > 0; j0 += kHugeMaxItems, items -= kHugeMaxItems) {  // grid y is limited
+    const unsigned gy = unsigned(std::min(items, kHugeMaxItems));
+    if (s.mixed) {
+      k_xs_gemm<true, 6, false, double2><<<dim3(tx, gy), xs::kThreadsXs, xs::smem<6>(), st>>>(
           A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
-    else
-      k_xs_gemm<true, 7, false, double2><<<dim3(tx, unsigned(items)), xs::kThreadsXs, xs::smem<7>(), st>>>(
-          A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
-  } else if (conjA) {
-    k_huge_zgemm<double2, true, double2, double2, double2>
-        <<<dim3(tiles(m, n), unsigned(items)), kHThreads, 0, st>>>(A, B, O, m, n, k, Cb, j0, 1.0);
-  } else {
-    k_huge_zgemm<double2, false, double2, double2, double2>
-        <<<dim3(tiles(m, n), unsigned(items)), kHThreads, 0, st>>>(A, B, O, m, n, k, Cb, j0, 1.0);
+    } else if (2 * k <= 512) {
+      if (conjA)
+        k_xs_gemm<true, 7, true, double2><<<dim3(tx, gy), xs::kThreadsXs, xs::smem<7>(), st>>>(
+            A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
+      else
+        k_xs_gemm<true, 7, false, double2><<<dim3(tx, gy), xs::kThreadsXs, xs::smem<7>(), st>>>(
+            A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
+    } else if (conjA) {
+      k_huge_zgemm<double2, true, double2, double2, double2>
+          <<<dim3(tiles(m, n), gy), kHThreads, 0, st>>>(A, B, O, m, n, k, Cb, j0, 1.0);
+    } else {
+      k_huge_zgemm<double2, false, double2, double2, double2>
+          <<<dim3(tiles(m, n), gy), kHThreads, 0, st>>>(A, B, O, m, n, k, Cb, j0, 1.0);
+    }
+    ++J.launches;
   }
-  ++J.launches;
 }
 
 // U_i of huge block k for every (crystallite, step): symmetric Paterson-Stockmeyer.
@@ -3971,19 +3974,24 @@ static void huge_dyson(JobImpl &J, DevSys &s, size_t kh, cudaStream_t st) {
   const unsigned ge = unsigned((long(b) * b + 255) / 256);
   const int len = s.nseg > 1 ? kSegLen : n;
   const size_t step = size_t(s.S2) * s.Cpad;
-  k_huge_copy<<<dim3(ge, unsigned(s.C), unsigned(s.nseg)), 256, 0, st>>>(s, s.U, s.A, 0, 0, len, bp, b);
-  ++J.launches;
+  auto copy = [&](const double2 *src, double2 *dst, int src0, int dst0, int stride, int segs) {
+    const long items = long(segs) * s.C;
+    for (long g0 = 0; g0 < items; g0 += kHugeMaxItems) {
+      k_huge_copy<<<dim3(ge, unsigned(std::min<long>(kHugeMaxItems, items - g0))), 256, 0, st>>>(s, src, dst, src0, dst0,
+                                                                                              stride, bp, b, g0);
+      ++J.launches;
+    }
+  };
+  copy(s.U, s.A, 0, 0, len, s.nseg);
   for (int t = 1; t < len; ++t) {
     const int segs = (n - t + len - 1) / len;  // segments that have a step t
     const auto U = item_mat<const double2>(s.U + t * step, bp, long(len) * s.S2, b, s.Cpad);
     const auto Ain = item_mat<const double2>(s.A + (t - 1) * step, bp, long(len) * s.S2, b, s.Cpad);
     const auto Aout = item_mat<double2>(s.A + t * step, bp, long(len) * s.S2, b, s.Cpad);
-    for (int g0 = 0; g0 < segs * s.C; g0 += kHugeMaxItems)
-      huge_mm(J, s, st, false, U, Ain, Aout, b, b, b, s.C, g0, std::min(kHugeMaxItems, segs * s.C - g0), 0, 0);
+    huge_mm(J, s, st, false, U, Ain, Aout, b, b, b, s.C, 0, segs * s.C, 0, 0);
   }
   if (s.nseg <= 1) return;
-  k_huge_copy<<<dim3(ge, unsigned(s.C), 1), 256, 0, st>>>(s, s.A, s.U, std::min(len, n) - 1, 0, 0, bp, b);
-  ++J.launches;
+  copy(s.A, s.U, std::min(len, n) - 1, 0, 0, 1);
   for (int t = 1; t < s.nseg; ++t) {
     const auto P = item_mat<const double2>(s.A + (std::min((t + 1) * len, n) - 1) * step, bp, 0, b, s.Cpad);
     const auto Ein = item_mat<const double2>(s.U + (t - 1) * step, bp, 0, b, s.Cpad);
@@ -4036,9 +4044,7 @@ static void huge_eigframe(JobImpl &J, DevSys &s, size_t kh) {
     const auto E = item_mat<const double2>(s.U, bp, s.S2, b, s.Cpad);  // E_{sl+1}
     const auto V = item_mat<const double2>(s.VF, bp, 0, b, s.Cpad);
     const auto O = item_mat<double2>(Vseg + step, bp, s.S2, b, s.Cpad);
-    const int items = s.C * (s.nseg - 1);
-    for (int g0 = 0; g0 < items; g0 += kHugeMaxItems)
-      huge_mm(J, s, st, false, E, V, O, b, b, b, s.C, g0, std::min(kHugeMaxItems, items - g0), 0, 0);
+    huge_mm(J, s, st, false, E, V, O, b, b, b, s.C, 0, s.C * (s.nseg - 1), 0, 0);
   }
   const int len = s.nseg > 1 ? kSegLen : J.n;
   for (int seg = 0; seg < s.nseg; ++seg) {

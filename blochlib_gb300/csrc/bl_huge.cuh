@@ -260,12 +260,14 @@ __global__ void k_huge_store_u(DevSys s, const double *ws, int bp, int bo, int b
   s.U[(size_t(i) * s.S2 + bp + e) * s.Cpad + c] = u;
 }
 
-// dst = src for block (bp, b), crystallite blockIdx.y, segment blockIdx.z: step slots src0 + z
-// stride of one [item][c] buffer to dst0 + z stride of another.
-__global__ void k_huge_copy(DevSys s, const double2 *src, double2 *dst, int src0, int dst0, int stride, int bp, int b) {
+// dst = src for block (bp, b) of item g = g0 + blockIdx.y (crystallite g % C, segment z = g / C): step
+// slot src0 + z stride of one [item][c] buffer to dst0 + z stride of another.
+__global__ void k_huge_copy(DevSys s, const double2 *src, double2 *dst, int src0, int dst0, int stride, int bp, int b,
+                            long g0) {
   const long bb = long(b) * b, e = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y, z = blockIdx.z;
   if (e >= bb) return;
+  const long g = g0 + blockIdx.y;
+  const int c = int(g % s.C), z = int(g / s.C);
   const size_t x = (size_t(bp) + e) * s.Cpad + c, step = size_t(s.S2) * s.Cpad;
   dst[size_t(dst0 + z * stride) * step + x] = src[size_t(src0 + z * stride) * step + x];
 }
