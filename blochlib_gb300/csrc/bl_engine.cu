@@ -3126,6 +3126,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
   const int nhc = sched ? J.pb : 1;
   std::vector<double> pas, isc, Hc(size_t(L.S2) * nhc, 0.0);
   std::vector<TermEntry> Tnz;  // non-zeros of the packed operators, term by term
+  size_t nnz = 0;              // their number (counted also where only the plan is wanted)
   auto pack = [&](const std::vector<double> &M, double *dst) {
     for (int k = 0; k < nb; ++k)
       for (int r = 0; r < L.size[k]; ++r)
@@ -3153,6 +3154,7 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     pas.insert(pas.end(), {I.pas[0][0], I.pas[0][1], I.pas[0][2], I.pas[1][1], I.pas[1][2], I.pas[2][2]});
     isc.push_back(scale);
     ikind.push_back(kind);
+    nnz += kind == 0 ? sys.h_nonzeros()[kk].size() : size_t(N);
     if (!g_sizing) {
       if (kind == 0) {
         for (const auto &e : sys.h_nonzeros()[kk]) entry(e.r, e.c, e.v);
@@ -3322,6 +3324,20 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     const size_t tk = size_t(J.nint) * L.S2, hc = size_t(L.S2) * (sched ? J.pb : 1);
     plan.tables = (tk + hc) * sizeof(double) * ((p.precision == 1 && !J.is_static) ? 2 : 1) +
                   (Dblk.size() + Rhoblk.size()) * sizeof(double2) + size_t(N) * J.pb * sizeof(double2) + 64 * 256;
+    // the tables in index form: FID elements, pairs, M_ab by row, operators by term and by element.  Up
+    // to 9 spins they fit the allowance of fixed_bytes; what goes beyond it is counted here (11 spins:
+    // 24 MB)
+    auto nonzeros = [](const std::vector<double2> &v) {
+      return size_t(std::count_if(v.begin(), v.end(), [](double2 z) { return z.x != 0.0 || z.y != 0.0; }));
+    };
+    size_t rows = 0;
+    for (int pr = 0; pr < J.npq + J.npr; ++pr) rows += size_t(L.size[pr < J.npq ? qa[pr] : ra[pr - J.npq]]) + 1;
+    const size_t index = size_t(J.ne) * 5 * sizeof(int) + size_t(J.npq + J.npr) * 6 * sizeof(int) + rows * sizeof(int) +
+                         (nonzeros(Dblk) + nonzeros(Rhoblk)) * (sizeof(int) + sizeof(double2) + sizeof(float2)) +
+                         nnz * (sizeof(TermEntry) + sizeof(int) + sizeof(double) + sizeof(float2)) +
+                         size_t(L.S2) * 3 * sizeof(int) + size_t(J.n) * 4 * sizeof(double) + 4096 * sizeof(double2);
+    constexpr size_t kAllowance = size_t(7) << 20;  // of fixed_bytes' 8 MiB
+    if (index > kAllowance) plan.tables += index - kAllowance;
   }
   if (g_sizing) {
     *g_sizing = plan;
@@ -3351,6 +3367,10 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     size_t fr = 0, tot = 0;
     CUDA_OK(cudaMemGetInfo(&fr, &tot));
     budget = size_t(0.6 * double(fr));
+  }
+  if (g_arena && g_arena->aux_streams) {  // a region holds the tables too
+    const size_t tables = plan.tables + 40 * 256;
+    budget = budget > tables ? budget - tables : 0;
   }
   budget = budget > huge_fixed ? budget - huge_fixed : 0;
   long cb = long(budget / std::max<size_t>(per_c, 1));
