@@ -3896,7 +3896,8 @@ static unsigned tiles(int m, int n) { return unsigned(((m + kHT - 1) / kHT) * ((
 
 // Products O = op(A) B of `items` items from j0 on: exact digit slices on the tensor cores
 // (bl_xs.cuh) where their sums stay exact (K' = 2k <= 512 digits; the mixed form, which needs
-// 2^-44, always), else FP64 tiles.  |A| <= 2^ea, |B| <= 2^eb.
+// 2^-44, always) and the result's exponents stay within FP64 (the slices' joining has no denormals),
+// else FP64 tiles.  |A| <= 2^ea, |B| <= 2^eb.
 static void huge_mm(JobImpl &J, const DevSys &s, cudaStream_t st, bool conjA, HMat<const double2> A,
                     HMat<const double2> B, HMat<double2> O, int m, int n, int k, int Cb, long j0, int items, int ea,
                     int eb) {
@@ -3907,7 +3908,7 @@ static void huge_mm(JobImpl &J, const DevSys &s, cudaStream_t st, bool conjA, HM
     if (s.mixed) {
       k_xs_gemm<true, 6, false, double2><<<dim3(tx, gy), xs::kThreadsXs, xs::smem<6>(), st>>>(
           A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
-    } else if (2 * k <= 512) {
+    } else if (2 * k <= 512 && std::abs(ea + eb) <= 900) {
       if (conjA)
         k_xs_gemm<true, 7, true, double2><<<dim3(tx, gy), xs::kThreadsXs, xs::smem<7>(), st>>>(
             A, B, O, m, n, k, Cb, j0, ea, eb, none, s.status);
