@@ -4,12 +4,18 @@
 //
 // An operand (|x| <= 2^e, e given per operand) becomes a fixed-point integer x 2^(8S-1-e),
 // written as S balanced base-256 digits q_j (exact in BF16), and the product takes the digit
-// pairs with i + j <= top level into one FP32 accumulator per level in tensor memory.  A
-// level's sums are integers below 2^24 (rows and columns of norm ~1, K' <= 512 digits long),
-// so the tensor core's FP32 accumulation is exact; the epilogue joins the levels in 64-bit
-// integers and rounds once to FP64, without touching the FP64 pipe.
-//   S = 7 (FP64 form): levels 0..7, the last two in one accumulator: 34 pairs, operand rounding
-//     2^-56 and dropped levels below 2^-60 for |O| ~ 1: at or below a 252-term FP64 dot product;
+// pairs with i + j <= top level into one FP32 accumulator per level in tensor memory; the epilogue
+// joins the levels in 64-bit integers and rounds once to FP64, without touching the FP64 pipe.
+// A level's sums are integers, accumulated exactly below 2^24.  Norms (rows and columns of length
+// ~1) bound the leading digit only; the others reach 128, so exactness is certain where (l - 1) K'
+// <= 992 at level l: every level up to K' = 165 digits, levels 0 to 4 at 252 (blocks of 126).
+// Digits beyond the first are close to uniform and of either sign: on propagators of 9 and 10 spins
+// (K' = 252 and 504) the largest sum was 0.05 and 0.08 of 2^24, which the dispatch's limit of K' <=
+// 512 rests on.  With all entries of both operands equal, K' = 504, it reaches 1.5 from level 4 on; a
+// sum in [2^24, 2^25) is rounded to 2 units, of 2^-46 at level 4.
+//   S = 7 (FP64 form): levels 0..7, the last two in one accumulator (rounded at 2^-24 of its sum,
+//     2^-68): 34 pairs, operand rounding 2^-56 and dropped levels below 2^-60 for |O| ~ 1.  9 spins,
+//     one crystallite, n = 24: 1.0e-15 from 80-bit propagation, 1.4e-15 with FP64 step products;
 //   S = 6 (mixed form): levels 0..5, 21 pairs, dropped levels ~2^-44, the size of the compensated
 //     double-float sums they take the place of.
 // Why: GB300 issues 2 FP64 FMAs per clock and SM (a 126 x 126 complex product: 3.9 M clocks on
