@@ -718,7 +718,7 @@ struct FloqDf {
 // transformed: 11 b^3 multiply-adds against 12 b^3 (FP64; V alone in double-float: 6 b^3) for each
 // of the ~5 sweeps that it saves.  Where single precision does not deliver (not finite, or far
 // from orthonormal), V = I and the final sweeps do all of the work.
-// Blocks below kStartMin stay with the final sweeps alone (FP64, blocks of 10, 320 crystallites:
+// Blocks below kStartMin stay with the final sweeps alone (sizes measured: FP64, blocks of 10, 320 crystallites:
 // 0.66 ms against 0.73; blocks of 20 to 35, 7 spins, 144 crystallites: 8.5 -> 3.0 ms.  Double-float,
 // blocks of 20, 677 crystallites: 1.08 ms against 1.62; blocks of 28 to 70, 8 spins, 1154
 // crystallites: 74 -> 48 ms, with K's off-diagonal left at 1e-10 of its norm instead of 1e-7).
@@ -1728,7 +1728,7 @@ __global__ void __launch_bounds__(384) k_big_eigframe4(DevSys s, int k) {
 // k_big_qr in single precision for row blocks from kQr4Min on: W_a, a column chunk of W_b and of X =
 // M_ab W_b in shared memory, loaded by asynchronous copies, a warp per row.  Smaller row blocks
 // stay with the 2 x 2 tiles: 20 x 20 has 25 tiles of 4 x 4, one warp (6 spins: 2.01 ms by 2 x 2, 2.65
-// by 4 x 4).
+// by 4 x 4; 56 and 70 are faster by 4 x 4, sizes between 20 and 56 were not measured on their own).
 constexpr int kQr4Min = 40;
 __host__ __device__ constexpr size_t big_qr4_smem(int ba, int bb, int w) {
   return sizeof(float2) * (size_t(ba) * up4(ba) + size_t(bb) * w + size_t(ba) * up4(w));

@@ -2520,9 +2520,9 @@ __global__ void __launch_bounds__(kThreads) k_p2p_elems(DevSys s) {
 // there are few elements or crystallites: 4 spins, 3722 crystallites 0.315 -> 0.274 ms; 9 spins, 32
 // crystallites 11.5 -> 4.1 ms; 8 spins, 1154 crystallites 26.6 -> 22.7 ms).  The CTA writes its tile to partial row (warp * ft_r + range); k_reduce
 // sums the rows of the populated warps in a fixed order.  Each output's summation order
-// (crystallites 0..31 per element, elements in order within a range) depends on neither
-// the tile shape nor the batch, so a crystallite's contribution does not depend on its
-// neighbours.
+// (crystallites 0..31 per element, elements in order within a sub-range, sub-ranges in order) follows
+// from the element count and the tile shape (ft_sub does), that is from the job's points and steps,
+// and not from the batch, so a crystallite's contribution does not depend on its neighbours.
 constexpr int kFtThreads = 64, kFtR = 16, kFtJmax = 32;
 // Dynamic shared memory of k_fid_tiled: two buffers of 32 crystallites x (4 jt + 4 pt).
 // Groups per CTA: as many as leave their buffers within 200 KB.
@@ -3613,8 +3613,8 @@ Job::Job(Context &ctx, const SpinSystem &sys, const Powder &pw, const CMatrix &r
     up.add(J.angles, ang), up.add(J.t0_all, t0), up.add(J.w_all, w);
   }
   // FFT length of the Fave correlation: n itself when it is a power of two (twisted circular
-  // correlation; FP64 form only, its twist factors are FP64 work), else the power of two >= 2n
-  // (zero-padded linear correlation, the single-precision transforms of the mixed form)
+  // correlation; FP64 form only, its twist factors are FP64 work), else the cheapest of 2^a, 3 2^a and
+  // 5 2^a from 2n on (zero-padded linear correlation; fave_length)
   DevSys &s = J.base;
   if (!J.p2p) {
     s.fave_twist = (!J.mixed && J.n >= 8 && (J.n & (J.n - 1)) == 0) ? 1 : 0;
@@ -3895,7 +3895,7 @@ static HMat<T> ws_mat(T *p, long j0, long mat, int C, int ld) {
 static unsigned tiles(int m, int n) { return unsigned(((m + kHT - 1) / kHT) * ((n + kHT - 1) / kHT)); }
 
 // Products O = op(A) B of `items` items from j0 on: exact digit slices on the tensor cores
-// (bl_xs.cuh) where their sums stay exact (K' = 2k <= 512 digits; the mixed form, which needs
+// (bl_xs.cuh) up to K' = 2k = 512 digits (its comment on exactness; the mixed form, which needs
 // 2^-44, always) and the result's exponents stay within FP64 (the slices' joining has no denormals),
 // else FP64 tiles.  |A| <= 2^ea, |B| <= 2^eb.
 static void huge_mm(JobImpl &J, const DevSys &s, cudaStream_t st, bool conjA, HMat<const double2> A,
@@ -4628,8 +4628,9 @@ std::string Job::describe() const {
 // kNoAllocScratch bytes; larger jobs are processed in crystallite batches that fit it, and
 // a job whose smallest batch does not fit is rejected with BL_ERR_NOMEM.  Every GPU that
 // loads this library holds the array until the process exits.  All calls share it and it
-// keeps the previous call's contents: each call zeroes what must start at zero (the status
-// word and the warp partials), and calls that overlap on the GPU race on it.
+// keeps the previous call's contents: each call zeroes what must start at zero (the status word,
+// the counters, scattered operator tables) and writes every warp partial that it sums, and calls
+// that overlap on the GPU race on it.
 namespace {
 constexpr size_t kNoAllocScratch = size_t(64) << 20;
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch];
